@@ -1135,6 +1135,7 @@ void AmgHierarchy::buildDevice(const FinestDevice& in, const SolverOptions& opt,
   // host may queue or prepare other work while it runs
   CUDA_OK(cudaStreamSynchronize(st));
   prepareChebyshev();
+  buildTail();
   tunePlans();
   lap("launch plans");
   // coarsest direct solve: dense inverse built on the GPU (no pivoting when

@@ -89,6 +89,8 @@ void AmgHierarchy::release() {
   keep_spares(c2f_, spareC2f_);
   coarseInv_ = nullptr;
   coarseInvF_ = nullptr;
+  tailStart_ = -1;
+  tailPrograms_.clear();
 }
 
 RefLevel AmgHierarchy::spareLevel(int l) { return take_spare(spareRef_, (size_t)l); }
@@ -295,6 +297,7 @@ void AmgHierarchy::build(std::vector<RefLevel>& levels, int finestLocalSize, con
     lap(gjUnpivoted ? "coarsest inverse (unpivoted)" : "coarsest inverse");
   }
   prepareChebyshev();
+  buildTail();
   tunePlans();
   lap("launch plans");
   if (trace) {
@@ -390,7 +393,9 @@ void AmgHierarchy::tunePlans() {
     std::sort(t.begin(), t.end());
     return t[2];
   };
-  for (int l = 0; l < L; l++) {
+  // (levels of the cluster kernel launch nothing of their own)
+  const int Lp = tailStart_ >= 0 ? tailStart_ : L;
+  for (int l = 0; l < Lp; l++) {
     DevLevel& d = lv_[l];
     d.plan = dev::RowPlan();
     if (d.ellWidth) {
@@ -464,7 +469,7 @@ void AmgHierarchy::tunePlans() {
   // residual + restriction of each level above the coarsest: the fused
   // kernel (gathers of scattered fine rows) or the coalesced residual pass
   // followed by the gather of r, whichever is faster (same result bits)
-  for (int l = 0; l + 1 < L; l++) {
+  for (int l = 0; l + 1 < L && l < Lp; l++) {
     DevLevel& d = lv_[l];
     d.splitRestrict = false;
     if (!opt_.autotune || d.n < kTuneMinRows) continue;
@@ -705,6 +710,7 @@ void AmgHierarchy::sweeps(int nSweeps, int l, cudaStream_t st, const T* xc, cons
 template <class T>
 void AmgHierarchy::cycle(CycleType t, int l, cudaStream_t st, bool xZero) {
   const int L = (int)lv_.size();
+  if (l == tailStart_ && runTail<T>(t, xZero, st)) return;
   DevLevel& d = lv_[l];
   const bool coarsest = (l == L - 1);
   if (coarsest && coarseInv_) {
@@ -744,6 +750,224 @@ void AmgHierarchy::cycle(CycleType t, int l, cudaStream_t st, bool xZero) {
     dev::prolong<T>(d.n, d.ci, vec_x<T>(c), vec_x<T>(d), st, rhsOnly);
   }
   sweeps<T>(opt_.postSweeps(l), l, st);
+}
+
+// ---- the coarse levels as one cluster kernel ----------------------------------
+// Which levels: those whose rows the cluster's threads hold in registers,
+// one row a thread (16 CTAs x 512) or, at up to kTailTwo entries a row, two.
+// A pass there takes 0.12-0.27 us on levels of at most 512 rows (one CTA)
+// and 0.5-1.2 us on larger ones, against 2.0-2.6 us as a launch; streaming
+// more rows through the same 16 SMs took 1.5-4 us per pass, more than the
+// launch on all SMs. kTailSmem bounds the vectors (24 KB a level at most).
+namespace {
+constexpr size_t kTailSmem = 160 * 1024;
+}  // namespace
+
+void AmgHierarchy::buildTail() {
+  tailStart_ = -1;
+  tailPrograms_.clear();
+  const int L = (int)lv_.size();
+  const bool f32 = opt_.precision == kMixed;
+  // (a forced launch plan asks for launches)
+  if (L == 0 || opt_.coarseSolver == kCoarseDirect || opt_.finestOnly() || opt_.planTpr || opt_.planEllRows ||
+      (opt_.smootherType == kGaussSeidel && opt_.ordering == kSequential))
+    return;
+  // from the coarsest level up, as many as the shared memory holds
+  const size_t vb = f32 ? sizeof(float) : sizeof(double);
+  const int lc = dev::cycle_tail_cluster(f32, kTailSmem);
+  if (lc < 0) return;
+  struct Shape {
+    int slices, lc, width;
+    unsigned x, vec;  // shared-memory offset of x; bytes of a vector (b and r follow)
+  };
+  std::vector<Shape> shape(L);
+  size_t used = 0;
+  int first = L;
+  for (int l = L - 1; l >= 0 && L - l <= dev::kTailMaxLevels; l--) {
+    const DevLevel& d = lv_[l];
+    Shape& q = shape[l];
+    q.slices = d.ellWidth ? (d.n + 31) / 32 : d.nSlices;
+    q.width = std::max(1, d.ellWidth ? d.ellWidth : d.maxWidth);
+    const int warps = dev::kTailWarps * (q.width <= dev::kTailTwo ? dev::kTailRowsMax : 1);
+    if (chebyshevLevel(l) || q.slices > warps << lc || d.nColors > dev::kTailMaxColors) break;
+    q.lc = q.slices <= dev::kTailWarps ? 0 : lc;
+    q.vec = (unsigned)(((q.slices + (1 << q.lc) - 1) >> q.lc) * 32 * vb);
+    q.x = (unsigned)used;
+    if (used + 3 * (size_t)q.vec > kTailSmem) break;
+    used += 3 * (size_t)q.vec;
+    first = l;
+  }
+  if (first == L) return;
+  // first rows of a level's colours, on the device
+  auto colourRows = [&](int l) -> const int* {
+    const DevLevel& d = lv_[l];
+    if (d.nColors <= 1) return nullptr;
+    return arena_.upload(d.ellWidth ? d.colorSliceStart : packed(l).colorStart);
+  };
+  // a level's slices by their relative place within their colour, then
+  // their inverse order
+  auto sliceOrder = [&](int l) {
+    const DevLevel& d = lv_[l];
+    const int S = shape[l].slices;
+    std::vector<std::pair<double, int>> key(S);
+    int c = 0;
+    for (int s = 0; s < S; s++) {
+      const int at = d.ellWidth ? 32 * s : s;  // colorSliceStart holds rows on ELL-32 levels
+      while (c + 1 < d.nColors && at >= d.colorSliceStart[c + 1]) c++;
+      const int c0 = d.nColors > 1 ? d.colorSliceStart[c] : 0;
+      const int c1 = d.nColors > 1 ? d.colorSliceStart[c + 1] : (d.ellWidth ? d.n : S);
+      key[s] = {(at - c0 + 0.5) / std::max(1, c1 - c0), s};
+    }
+    std::sort(key.begin(), key.end());
+    std::vector<int> o(2 * (size_t)S);
+    for (int h = 0; h < S; h++) {
+      o[h] = key[h].second;
+      o[S + key[h].second] = h;
+    }
+    return o;
+  };
+  auto fill = [&](auto& args) {
+    using T = std::remove_const_t<decltype(args.w)>;
+    args.lc = lc;
+    args.w = (T)opt_.jacobiWeight;
+    dev::TailPackArgs<T> pack = {};
+    pack.levels = L - first;
+    for (int l = first; l < L; l++) {
+      DevLevel& d = lv_[l];
+      const Shape& s = shape[l];
+      auto& q = args.lv[l - first];
+      auto& p = pack.lv[l - first];
+      const size_t slots = (size_t)s.slices * 32, entries = slots * s.width;
+      p.a = view<T>(d);
+      p.rowSlice = d.rowSlice;
+      p.colorRow = colourRows(l);
+      p.order = arena_.upload(sliceOrder(l));
+      p.home = p.order + s.slices;
+      p.slot = (int*)arena_.alloc(sizeof(int) * slots);
+      p.idx = (int*)arena_.alloc(sizeof(int) * entries);
+      p.val = (T*)arena_.alloc(sizeof(T) * entries);
+      p.diag = (T*)arena_.alloc(sizeof(T) * slots);
+      p.rdiag = (T*)arena_.alloc(sizeof(T) * slots);
+      if (l + 1 < L) {
+        p.ci = d.ci;
+        p.ciOut = (int*)arena_.alloc(sizeof(int) * slots);
+        p.c2fRow = d.c2fRow;
+        p.c2fCol = d.c2fCol;
+        p.nCoarse = lv_[l + 1].n;
+        p.c2fOut = (int*)arena_.alloc(sizeof(int) * (size_t)d.n);
+      }
+      q.n = d.n;
+      q.slices = s.slices;
+      q.lc = s.lc;
+      q.per = (s.slices + (1 << s.lc) - 1) >> s.lc;
+      q.width = s.width;
+      q.colors = d.nColors;
+      q.slot = p.slot;
+      q.idx = p.idx;
+      q.val = p.val;
+      q.diag = p.diag;
+      q.rdiag = p.rdiag;
+      q.ci = p.ciOut;
+      q.c2fRow = d.c2fRow;
+      q.c2fIdx = p.c2fOut;
+      q.x = s.x;
+      q.b = s.x + s.vec;
+      q.r = s.x + 2 * s.vec;
+    }
+    dev::cycle_tail_pack<T>(args, pack, nullptr);
+    CUDA_OK(cudaGetLastError());
+  };
+  if (f32)
+    fill(tail32_);
+  else
+    fill(tail64_);
+  // the steps of one visit of level l, as cycle() orders its launches
+  std::vector<dev::TailStep> steps;
+  auto solo = [&](int l) { return shape[l].lc == 0; };
+  auto add = [&](int op, int l, bool one, int n = 0, int flags = 0) {
+    if (!steps.empty()) {
+      const bool both = one && ((steps.back().op >> 8) & dev::kTailSolo);
+      flags |= both ? dev::kTailBarCta : dev::kTailBarCluster;
+    }
+    if (one) flags |= dev::kTailSolo;
+    steps.push_back({op | flags << 8, l - first, n, 0});
+  };
+  auto smoothStep = [&](int nSweeps, int l, int flags) {
+    if (nSweeps <= 0 && !flags) return;
+    const int op = dampedLevel(l, lv_[l].n)                ? dev::kTailDamped
+                   : opt_.smootherType != kGaussSeidel ? dev::kTailJacobi
+                                                       : dev::kTailGs;
+    add(op, l, solo(l), std::max(0, nSweeps), flags | (opt_.gsReverse ? 0 : dev::kTailForward));
+  };
+  constexpr size_t kMaxSteps = 1 << 16;
+  // zeroed: the step that led here has set x = 0
+  std::function<void(CycleType, int, bool, bool)> visit = [&](CycleType t, int l, bool xZero, bool zeroed) {
+    if (steps.size() > kMaxSteps) return;
+    const bool coarsest = l == L - 1;
+    const bool rhsOnly = xZero && opt_.nPreSweeps == 0 && !coarsest;
+    const int zero = xZero && !rhsOnly && !zeroed ? dev::kTailZero : 0;
+    smoothStep(opt_.nPreSweeps, l, zero | (!coarsest && !rhsOnly ? dev::kTailResidual : 0));
+    if (!coarsest) {
+      add(rhsOnly ? dev::kTailRestrictRhs : dev::kTailRestrict, l, solo(l + 1));
+      visit(t, l + 1, true, true);
+      if (t == kWCycle)
+        visit(kWCycle, l + 1, false, false);
+      else if (t == kFCycle)
+        visit(kVCycle, l + 1, false, false);
+      add(rhsOnly ? dev::kTailAssign : dev::kTailProlong, l, solo(l));
+    }
+    smoothStep(opt_.postSweeps(l), l, 0);
+  };
+  std::vector<TailProgram> programs;
+  std::vector<size_t> start;
+  std::vector<dev::TailStep> all;
+  auto program = [&](CycleType t, bool xZero) {
+    steps.clear();
+    add(dev::kTailLoad, first, solo(first), 0, xZero ? dev::kTailZero : 0);
+    visit(t, first, xZero, xZero);
+    add(dev::kTailStore, first, solo(first));
+    programs.push_back({t, xZero, nullptr, (int)steps.size()});
+    start.push_back(all.size());
+    all.insert(all.end(), steps.begin(), steps.end());
+    return steps.size() <= kMaxSteps;
+  };
+  bool ok = program(opt_.cycleType, true) && program(opt_.cycleType, false);
+  if (opt_.cycleType == kFCycle) ok = ok && program(kVCycle, true) && program(kVCycle, false);
+  if (!ok) return;  // a W cycle of very many levels: launches of their own
+  const dev::TailStep* d = arena_.upload(all);
+  CUDA_OK(cudaStreamSynchronize(nullptr));
+  for (size_t k = 0; k < programs.size(); k++) programs[k].steps = d + start[k];
+  tailPrograms_ = std::move(programs);
+  tailSmem_ = used;
+  if (getenv("FVM_TRACE"))
+    fprintf(stderr, "[fvm setup] cluster kernel: levels %d (%d rows) to %d, %d CTAs\n", first, lv_[first].n, L - 1,
+            1 << lc);
+  tailStart_ = first;
+}
+
+template <class T>
+bool AmgHierarchy::runTail(CycleType t, bool xZero, cudaStream_t st) {
+  if constexpr (std::is_same<T, float>::value) {
+    if (opt_.precision != kMixed) return false;
+  } else {
+    if (opt_.precision == kMixed) return false;
+  }
+  for (const TailProgram& p : tailPrograms_) {
+    if (p.type != t || p.xZero != xZero) continue;
+    auto go = [&](auto args) {
+      args.steps = p.steps;
+      args.nSteps = p.n;
+      args.bIn = vec_b<T>(lv_[tailStart_]);
+      args.xIo = vec_x<T>(lv_[tailStart_]);
+      dev::cycle_tail<T>(args, tailSmem_, st);
+    };
+    if constexpr (std::is_same<T, float>::value)
+      go(tail32_);
+    else
+      go(tail64_);
+    return true;
+  }
+  return false;
 }
 
 bool AmgHierarchy::fusedProlong(int l) const {
@@ -856,6 +1080,10 @@ int AmgHierarchy::kernelsPerCycle() const {
   const int L = (int)lv_.size();
   for (int l = 0; l < L; l++) {
     const DevLevel& d = lv_[l];
+    if (l == tailStart_) {
+      k += 1;
+      break;
+    }
     if (l == L - 1 && coarseInv_) {
       k += 1;
       continue;

@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "amg_setup.hpp"
+#include "cycle_tail.cuh"
 #include "kernels.cuh"
 #include "learned.hpp"
 
@@ -334,6 +335,23 @@ class AmgHierarchy {
   double chebBound_ = 0.0;
   void prepareChebyshev();
   bool chebyshevLevel(int l) const { return l == 0 && !chebC1_.empty(); }
+  // Levels tailStart_ .. L-1 of a cycle run as one cluster kernel (-1: none
+  // do). Its steps are listed once per build for every way a cycle enters
+  // level tailStart_ (cycle type, zero guess).
+  int tailStart_ = -1;
+  size_t tailSmem_ = 0;
+  struct TailProgram {
+    CycleType type;
+    bool xZero;
+    const dev::TailStep* steps;
+    int n;
+  };
+  std::vector<TailProgram> tailPrograms_;
+  dev::TailArgs<double> tail64_ = {};
+  dev::TailArgs<float> tail32_ = {};
+  void buildTail();
+  template <class T>
+  bool runTail(CycleType t, bool xZero, cudaStream_t st);
   // one smoother pass of level l with a given plan (what the tuner times)
   void smootherPass(int l, dev::RowPlan plan, cudaStream_t st);
   // level l's residual restricted to level l + 1, fused or split
