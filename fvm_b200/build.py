@@ -31,9 +31,9 @@ NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "--expt-relaxed-constexpr",
               "-Xcompiler", "-fPIC,-ffp-contract=off"] + ARCH
 
 HOST_SOURCES = ["mesh.cpp", "amg_setup.cpp", "capi.cpp", "fluent.cpp"]
-CUDA_SOURCES = ["kernels.cu", "solver.cu", "thermal.cu", "cycle_tail.cu", "residual_noalloc.cu", "learned.cu", "amg_device.cu"]
+CUDA_SOURCES = ["kernels.cu", "solver.cu", "thermal.cu", "cycle_tail.cu", "coarse_inverse.cu", "residual_noalloc.cu", "learned.cu", "amg_device.cu"]
 # device code free to contract a * b + c into one rounding
-FMA_SOURCES = {"learned.cu", "amg_device.cu"}
+FMA_SOURCES = {"learned.cu", "amg_device.cu", "coarse_inverse.cu"}
 
 
 def _nvcc() -> str:

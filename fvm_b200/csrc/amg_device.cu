@@ -6,6 +6,7 @@
 // thread (or one warp) that reads its inputs in a fixed order; the only
 // atomics place fine rows into coarse-row lists, which are then sorted.
 #include "amg_device.cuh"
+#include "coarse_inverse.cuh"
 
 #include <algorithm>
 #include <chrono>
@@ -482,20 +483,6 @@ __global__ void k_compose(int n, int* ci, const int* __restrict__ ci2) {
   if (i < n) ci[i] = ci2[ci[i]];
 }
 
-__global__ void k_dominance(LevelRows a, int* flag) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= a.n) return;
-  int base, w;
-  row_range(a, i, base, w);
-  double s = 0.0;
-  for (int k = 0; k < w; k++) {
-    const int j = a.cols[base + 32 * k];
-    if (j != i) s += fabs(a.vals[base + 32 * k]);
-  }
-  const double d = a.diag[i];
-  if (!(d != 0.0 && s <= fabs(d) * (1.0 + 1e-8))) atomicOr(flag, 1);
-}
-
 // ---- level-0 pattern of a mesh on the device -------------------------------
 // Self-column entries per self row of cellCells.
 __global__ void k_ip_count(int n, const int* __restrict__ ccRow, const int* __restrict__ ccCol, int* cnt) {
@@ -715,10 +702,6 @@ void slice_meta_fill(int n, const int* sliceOff, int4* meta, int* sliceRow, int*
 
 void compose_index(int n, int* ci, const int* ci2, cudaStream_t st) {
   if (n > 0) k_compose<<<cdiv(n, kT), kT, 0, st>>>(n, ci, ci2);
-}
-
-void dominance_check(const LevelRows& a, int* flag, cudaStream_t st) {
-  k_dominance<<<cdiv(a.n, kT), kT, 0, st>>>(a, flag);
 }
 
 }  // namespace dev
@@ -1178,37 +1161,47 @@ void AmgHierarchy::buildDevice(const FinestDevice& in, const SolverOptions& opt,
       coarseInv_ = arena_.upload(inv);
     } else {
       FVM_REQUIRE(c.ellWidth == 0, kUnsupported, "coarsest level in ELL-32 layout");
-      const dev::LevelRows a{c.n, c.cols, c.vals, c.diag, c.meta, c.rowSlice, c.ellWidth};
+      auto alloc = [&](size_t bytes) { return arena_.alloc(size_class(bytes)); };
       CUDA_OK(cudaMemsetAsync(flags + 2, 0, sizeof(int), st));
-      dev::dominance_check(a, flags + 2, st);
+      dev::dominant_symmetric_check(c.view64(), c.rowSlice, flags + 2, st);
       CUDA_OK(cudaMemcpyAsync(hflags, flags + 2, sizeof(int), cudaMemcpyDeviceToHost, st));
       CUDA_OK(cudaStreamSynchronize(st));
-      const bool dominant = hflags[0] == 0;
-      void* gjScratch = arena_.alloc(size_class(dev::gauss_jordan_scratch_bytes(c.n)));
-      coarseInv_ = (double*)arena_.alloc(size_class(sizeof(double) * nn));
-      if (dominant) {
-        dev::dense_from_sell(c.view64(), c.nSlices, coarseInv_, st);
-        // a symmetric level (a diffusion operator's Galerkin level) takes
-        // the symmetric sweep: half the products
-        CUDA_OK(cudaMemsetAsync(flags + 2, 0, sizeof(int), st));
-        dev::dense_symmetry_check(c.n, coarseInv_, flags + 2, st);
-        CUDA_OK(cudaMemcpyAsync(hflags, flags + 2, sizeof(int), cudaMemcpyDeviceToHost, st));
-        CUDA_OK(cudaStreamSynchronize(st));
-        if (hflags[0] == 0)
-          dev::gauss_jordan_inverse_symmetric(c.n, coarseInv_, gjScratch, st);
+      if (hflags[0] == 0) {
+        // a diffusion operator's Galerkin level
+        int* status = (int*)alloc(sizeof(int));
+        CUDA_OK(cudaMemsetAsync(status, 0, sizeof(int), st));
+        if (mixed)
+          coarseInvF_ = (float*)alloc(sizeof(float) * nn);
         else
-          dev::gauss_jordan_inverse_dominant(c.n, coarseInv_, gjScratch, st);
+          coarseInv_ = (double*)alloc(sizeof(double) * nn);
+        // the rows' points, averaged down from the cell centroids
+        float* points = nullptr;
+        for (int l = 0; in.xyz && l + 1 < L; l++) {
+          float* fine = points;
+          points = (float*)alloc(sizeof(float) * 3 * (size_t)lv_[l + 1].n);
+          dev::coarse_points(lv_[l + 1].n, lv_[l].c2fRow, lv_[l].c2fCol, l == 0 ? finest_->iperm : nullptr,
+                             l == 0 ? in.xyz : nullptr, lv_[l].n, fine, points, st);
+        }
+        dev::inverse_symmetric(c.view64(), c.rowSlice, points, coarseInv_, coarseInvF_, status, alloc, st);
+        CUDA_OK(cudaMemcpyAsync(pendingStatus(), status, sizeof(int), cudaMemcpyDeviceToHost, st));
       } else {
-        double* dA = (double*)arena_.alloc(size_class(sizeof(double) * nn));
-        dev::dense_from_sell(c.view64(), c.nSlices, dA, st);
-        dev::gauss_jordan_inverse(c.n, dA, coarseInv_, gjScratch, st);
+        void* gjScratch = alloc(dev::gauss_jordan_scratch_bytes(c.n));
+        coarseInv_ = (double*)alloc(sizeof(double) * nn);
+        if ((hflags[0] & 1) == 0) {
+          dev::dense_from_sell(c.view64(), c.nSlices, coarseInv_, st);
+          dev::gauss_jordan_inverse_dominant(c.n, coarseInv_, gjScratch, st);
+        } else {
+          double* dA = (double*)alloc(sizeof(double) * nn);
+          dev::dense_from_sell(c.view64(), c.nSlices, dA, st);
+          dev::gauss_jordan_inverse(c.n, dA, coarseInv_, gjScratch, st);
+        }
+        CUDA_OK(cudaMemcpyAsync(pendingStatus(), dev::gauss_jordan_status(c.n, gjScratch), sizeof(int),
+                                cudaMemcpyDeviceToHost, st));
       }
       // the status is read by finishBuild
-      CUDA_OK(cudaMemcpyAsync(pendingStatus(), dev::gauss_jordan_status(c.n, gjScratch), sizeof(int),
-                              cudaMemcpyDeviceToHost, st));
       inversePending_ = true;
     }
-    if (mixed) {
+    if (mixed && !coarseInvF_) {
       coarseInvF_ = (float*)arena_.alloc(size_class(sizeof(float) * nn));
       dev::cast_d2f(nn, coarseInv_, coarseInvF_, st);
     }

@@ -82,9 +82,5 @@ void slice_meta_fill(int n, const int* sliceOff, int4* meta, int* sliceRow, int*
 // ci[i] = ci2[ci[i]]: two aggregations composed
 void compose_index(int n, int* ci, const int* ci2, cudaStream_t st);
 
-// *flag = 1 unless every row is diagonally dominant (|a_ii| >= sum |a_ij|
-// up to a relative slack of 1e-8); *flag must be 0 on entry
-void dominance_check(const LevelRows& a, int* flag, cudaStream_t st);
-
 }  // namespace dev
 }  // namespace fvm

@@ -1,6 +1,8 @@
 // GPU AMG hierarchy and the linear solvers built on it.
 #include "solver.hpp"
 
+#include "coarse_inverse.cuh"
+
 #include <math_constants.h>
 
 #include <algorithm>
@@ -186,7 +188,7 @@ void AmgHierarchy::build(std::vector<RefLevel>& levels, int finestLocalSize, con
   // its own, overlapping the packing and uploads of the other levels.
   const bool direct = opt.coarseSolver == kCoarseDirect && !opt.finestOnly();
   cudaStream_t gjStream = nullptr;
-  void* gjScratch = nullptr;
+  const int* gjStatus = nullptr;
   int coarseN = 0;
   bool gjUnpivoted = false;
   auto startCoarseInverse = [&](int l) {
@@ -229,16 +231,26 @@ void AmgHierarchy::build(std::vector<RefLevel>& levels, int finestLocalSize, con
           }
         symmetric = found;
       }
-    gjScratch = arena_.alloc(dev::gauss_jordan_scratch_bytes(c.n));
-    coarseInv_ = (double*)arena_.alloc(sizeof(double) * nn);
     CUDA_OK(cudaStreamCreateWithFlags(&gjStream, cudaStreamNonBlocking));
     gjUnpivoted = dominant;
+    if (symmetric) {
+      gjStatus = (int*)arena_.alloc(sizeof(int));
+      CUDA_OK(cudaMemsetAsync(const_cast<int*>(gjStatus), 0, sizeof(int), gjStream));
+      if (mixed)
+        coarseInvF_ = (float*)arena_.alloc(sizeof(float) * nn);
+      else
+        coarseInv_ = (double*)arena_.alloc(sizeof(double) * nn);
+      dev::inverse_symmetric(lv_[l].view64(), lv_[l].rowSlice, nullptr, coarseInv_, coarseInvF_,
+                             const_cast<int*>(gjStatus),
+                             [&](size_t bytes) { return arena_.alloc(bytes); }, gjStream);
+      return;
+    }
+    void* gjScratch = arena_.alloc(dev::gauss_jordan_scratch_bytes(c.n));
+    gjStatus = dev::gauss_jordan_status(c.n, gjScratch);
+    coarseInv_ = (double*)arena_.alloc(sizeof(double) * nn);
     if (dominant) {
       dev::dense_from_sell(lv_[l].view64(), lv_[l].nSlices, coarseInv_, gjStream);
-      if (symmetric)
-        dev::gauss_jordan_inverse_symmetric(c.n, coarseInv_, gjScratch, gjStream);
-      else
-        dev::gauss_jordan_inverse_dominant(c.n, coarseInv_, gjScratch, gjStream);
+      dev::gauss_jordan_inverse_dominant(c.n, coarseInv_, gjScratch, gjStream);
       return;
     }
     double* dA = (double*)arena_.alloc(sizeof(double) * nn);
@@ -280,15 +292,14 @@ void AmgHierarchy::build(std::vector<RefLevel>& levels, int finestLocalSize, con
   if (direct) {
     if (gjStream) {
       int singular = 0;
-      const cudaError_t e1 = cudaMemcpyAsync(&singular, dev::gauss_jordan_status(coarseN, gjScratch), sizeof(int),
-                                             cudaMemcpyDeviceToHost, gjStream);
+      const cudaError_t e1 = cudaMemcpyAsync(&singular, gjStatus, sizeof(int), cudaMemcpyDeviceToHost, gjStream);
       const cudaError_t e2 = cudaStreamSynchronize(gjStream);
       cudaStreamDestroy(gjStream);
       CUDA_OK(e1);
       CUDA_OK(e2);
       FVM_REQUIRE(singular == 0, kBadArgument, "singular coarsest-level matrix");
     }
-    if (mixed) {
+    if (mixed && !coarseInvF_) {
       const size_t nn = (size_t)coarseN * coarseN;
       coarseInvF_ = (float*)arena_.alloc(sizeof(float) * nn);
       dev::cast_d2f(nn, coarseInv_, coarseInvF_, 0);
@@ -713,7 +724,7 @@ void AmgHierarchy::cycle(CycleType t, int l, cudaStream_t st, bool xZero) {
   if (l == tailStart_ && runTail<T>(t, xZero, st)) return;
   DevLevel& d = lv_[l];
   const bool coarsest = (l == L - 1);
-  if (coarsest && coarseInv_) {
+  if (coarsest && hasCoarseInverse()) {
     if constexpr (std::is_same<T, float>::value) {
       if (coarseInvF_) {
         dev::dense_solve_f32(d.n, coarseInvF_, d.bF, d.xF, st);
@@ -1039,7 +1050,7 @@ double AmgHierarchy::cycleBytes() const {
   for (int l = 0; l < L; l++) {
     const DevLevel& d = lv_[l];
     const double pass = d.n * (4.0 * vb) + d.entries * (4.0 + vb);
-    if (l == L - 1 && coarseInv_) {
+    if (l == L - 1 && hasCoarseInverse()) {
       total += (double)d.n * d.n * (opt_.precision == kMixed && coarseInvF_ ? 4.0 : 8.0) + 2.0 * vb * d.n;
       continue;
     }
@@ -1084,7 +1095,7 @@ int AmgHierarchy::kernelsPerCycle() const {
       k += 1;
       break;
     }
-    if (l == L - 1 && coarseInv_) {
+    if (l == L - 1 && hasCoarseInverse()) {
       k += 1;
       continue;
     }
@@ -1129,7 +1140,7 @@ void AmgHierarchy::profileLevels(int reps, void* flush, size_t flushBytes, cudaS
     o[0] = d.n;
     o[1] = (double)d.entries;
     const double pass = d.n * 4.0 * vb + d.entries * (4.0 + vb);
-    if (l == L - 1 && coarseInv_) {
+    if (l == L - 1 && hasCoarseInverse()) {
       o[2] = timed([&] {
         if (f32 && coarseInvF_)
           dev::dense_solve_f32(d.n, coarseInvF_, d.bF, d.xF, st);

@@ -187,6 +187,9 @@ struct FinestDevice {
   // ascending (cfRow, cfCol) and faceCells (2 per face). conn is then the
   // self-column part of cellCells and entrySrc the face behind each entry.
   const int *ccRow = nullptr, *ccCol = nullptr, *cfRow = nullptr, *cfCol = nullptr, *faceCells = nullptr;
+  // cell centroids (3 per row of the pattern, reference order) on the device,
+  // or null: they only shape the elimination order of the coarsest inverse
+  const double* xyz = nullptr;
 };
 
 // Cached level-0 structure of device-built hierarchies (pattern only).
@@ -308,7 +311,8 @@ class AmgHierarchy {
   int* pendingStatus();
   std::vector<DevLevel> lv_;
   double* coarseInv_ = nullptr;  // dense inverse of the coarsest level
-  float* coarseInvF_ = nullptr;  // its FP32 copy for the FP32 cycle
+  float* coarseInvF_ = nullptr;  // in FP32 for the FP32 cycle (which may hold it alone)
+  bool hasCoarseInverse() const { return coarseInv_ || coarseInvF_; }
   DeviceArena arena_;
   // level l (of n rows) smooths with damped Jacobi (coarseJacobiRows)
   bool dampedLevel(int l, int n) const;

@@ -962,6 +962,7 @@ void ThermalModel::ensureMatrix() {
     in.cfRow = dCfRow_;
     in.cfCol = dCfCol_;
     in.faceCells = dFaceCells_;
+    in.xyz = dCentroid_;
     CUDA_OK(cudaStreamSynchronize(stream_));
     hier_.buildDevice(in, opt_.linear, true);
     lap("hierarchy on the device");
