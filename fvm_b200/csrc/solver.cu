@@ -1296,36 +1296,67 @@ __global__ void k_add_vec(int n, const double* __restrict__ a, const double* __r
   if (i < n) y[i] = a[i] + b[i];
 }
 
-// Device-side loop control of the CG graph. Status: 0 running, 1
-// converged, 2 non-finite residual, 3 iteration limit.
-__global__ void k_cg_loop_init(double* scal, int* loopInt, double* history, double absTol, int maxIt,
-                               cudaGraphConditionalHandle h) {
+// Device-side loop control of a solve's graph. Status: 0 running, 1
+// converged, 2 non-finite residual, 3 iteration limit. testFirst: the
+// initial norm may already meet the absolute tolerance.
+__global__ void k_loop_init(double* scal, int* loopInt, double* history, double absTol, int maxIt, int testFirst,
+                            cudaGraphConditionalHandle h) {
   const double r0 = scal[kNorm];
   history[0] = r0;
   loopInt[0] = 0;
-  const bool finite = isfinite(r0);
-  const bool done = !finite || r0 < absTol || maxIt <= 0;
-  loopInt[1] = !finite ? 2 : (r0 < absTol ? 1 : (maxIt <= 0 ? 3 : 0));
-  scal[kRho] = CUDART_INF;  // first beta = 0
-  cudaGraphSetConditional(h, done ? 0u : 1u);
+  const bool finite = isfinite(r0), met = testFirst && r0 < absTol;
+  loopInt[1] = !finite ? 2 : (met ? 1 : (maxIt <= 0 ? 3 : 0));
+  // the Krylov solvers' first pass: beta = 0 (rho / inf), alpha / omega = 0
+  scal[kRho] = CUDART_INF;
+  scal[kAlpha] = 0.0;
+  scal[kOmega] = 1.0;
+  cudaGraphSetConditional(h, loopInt[1] == 0 ? 1u : 0u);
 }
 
-__global__ void k_cg_loop_check(const double* scal, int* loopInt, double* history, double relTol, double absTol,
-                                int maxIt, cudaGraphConditionalHandle h) {
-  const double rn = scal[kNorm];
+// The norm of an iteration's residual from its np partial sums (summed as
+// sum_partials sums them) and the test on it. Half: the test BiCGStab makes
+// half way, on the absolute tolerance alone; the second half runs unless the
+// solve ended (condition hHalf).
+template <bool Half>
+__global__ void __launch_bounds__(1024) k_loop_check(int np, const double* __restrict__ p, double* scal, int* loopInt,
+                                                     double* history, double relTol, double absTol, int maxIt,
+                                                     cudaGraphConditionalHandle h, cudaGraphConditionalHandle hHalf) {
+  __shared__ double sh[32];
+  double v = 0.0;
+  const int bd = blockDim.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  int k = threadIdx.x;
+  for (; k + 3 * bd < np; k += 4 * bd) {
+    const double a0 = p[k], a1 = p[k + bd], a2 = p[k + 2 * bd], a3 = p[k + 3 * bd];
+    v += a0;
+    v += a1;
+    v += a2;
+    v += a3;
+  }
+  for (; k < np; k += bd) v += p[k];
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  if (lane == 0) sh[w] = v;
+  __syncthreads();
+  if (w) return;
+  v = sh[lane];
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  if (lane) return;
+  const double rn = v;
+  scal[kNorm] = rn;
   const int i = loopInt[0] + 1;
-  loopInt[0] = i;
-  history[i] = rn;
-  const double r0 = history[0];
   int status = 0;
   if (!isfinite(rn))
     status = 2;
-  else if (rn < absTol || rn / r0 < relTol)
+  else if (rn < absTol || (!Half && rn / history[0] < relTol))
     status = 1;
-  else if (i >= maxIt)
+  else if (!Half && i >= maxIt)
     status = 3;
   loopInt[1] = status;
-  cudaGraphSetConditional(h, status == 0 ? 1u : 0u);
+  if (!Half || status) {
+    loopInt[0] = i;
+    history[i] = rn;
+  }
+  if (!Half || status) cudaGraphSetConditional(h, status == 0 ? 1u : 0u);
+  if (Half) cudaGraphSetConditional(hHalf, status == 0 ? 1u : 0u);
 }
 }  // namespace
 
@@ -1436,6 +1467,7 @@ SolveReport LinearSolve::solveAMG(cudaStream_t st) {
   const SolverOptions& o = h_.options();
   DevLevel& d = h_.level(0);
   SolveReport rep;
+  if (deviceSolvable() && solveDeviceLoop(st, rep)) return rep;
   CUDA_OK(cudaMemsetAsync(d.x, 0, sizeof(double) * (size_t)n_, st));
   if (learned_) CUDA_OK(cudaMemsetAsync(scal_ + kLsAccepted, 0, 3 * sizeof(double), st));
   dev::residual<double>(d.view64(), d.nSlices, d.x, d.b, d.r, d.partials, st);
@@ -1639,9 +1671,7 @@ SolveReport LinearSolve::solveCG(cudaStream_t st) {
   SolveReport rep;
   // the whole solve on the device when nothing needs the host between
   // iterations (no learned step, no printing)
-  if (o.preconditioner == kPrecAMG && o.useGraphs && o.verbosity <= 0 && !(learned_ && learnedActive_) &&
-      !graphsFailed_ && solveCGLoop(st, flexible, rep))
-    return rep;
+  if (deviceSolvable() && solveDeviceLoop(st, rep)) return rep;
   if (getenv("FVM_TRACE"))
     fprintf(stderr, "[fvm solve] CG on the host loop (learned step %s, graphs %s, loop graph %s)\n",
             learned_ && learnedActive_ ? "active" : "inactive", graphsFailed_ ? "failed" : "ok",
@@ -1806,121 +1836,236 @@ bool graph_leaves(cudaGraph_t g, std::vector<cudaGraphNode_t>& leaves) {
   return true;
 }
 
-bool LinearSolve::addCGLoop(cudaGraph_t g, cudaStream_t st, bool flexible, bool hostCopies) {
+bool graph_capture(cudaGraph_t g, cudaStream_t st, const std::function<void()>& fn) {
+  std::vector<cudaGraphNode_t> leaves;
+  if (!graph_leaves(g, leaves)) return false;
+  if (cudaStreamBeginCaptureToGraph(st, g, leaves.empty() ? nullptr : leaves.data(), nullptr, leaves.size(),
+                                    cudaStreamCaptureModeThreadLocal) != cudaSuccess)
+    return false;
+  bool ok = true;
+  try {
+    fn();
+  } catch (const Error&) {
+    ok = false;
+  }
+  cudaGraph_t out = nullptr;
+  return cudaStreamEndCapture(st, &out) == cudaSuccess && ok;
+}
+
+bool graph_conditional(cudaGraph_t g, cudaGraphConditionalHandle h, cudaGraphConditionalNodeType type,
+                       cudaGraph_t* body) {
+  std::vector<cudaGraphNode_t> leaves;
+  if (!graph_leaves(g, leaves) || leaves.empty()) return false;
+  cudaGraphNodeParams cp = {};
+  cp.type = cudaGraphNodeTypeConditional;
+  cp.conditional.handle = h;
+  cp.conditional.type = type;
+  cp.conditional.size = 1;
+  cudaGraphNode_t node = nullptr;
+  if (cudaGraphAddNode(&node, g, leaves.data(), leaves.size(), &cp) != cudaSuccess) return false;
+  *body = cp.conditional.phGraph_out[0];
+  return true;
+}
+
+// A solver's loop in g: prologue, while node, epilogue. The norm of the
+// initial residual is left in scal_[kNorm] by `prologue`; `iteration` is
+// captured into the while node's body and leaves np partial sums of the
+// residual's norm in partials; with `half` (BiCGStab) it is the second half,
+// under a condition that the first half's norm sets.
+bool LinearSolve::addLoop(cudaGraph_t g, cudaStream_t st, int maxIt, bool testFirst,
+                          const std::function<void()>& prologue, const std::function<void()>& half,
+                          const std::function<void()>& iteration, int np, const double* partials,
+                          const std::function<void()>& epilogue) {
   const SolverOptions& o = h_.options();
-  DevLevel& d = h_.level(0);
-  const bool mixedCycle = o.precision == kMixed;
-  // The FP32 cycle works on level 0's FP32 vectors only, so the iterate and
-  // the right-hand side can be level 0's own FP64 x and b: no copy in, no
-  // restore. The FP64 cycle overwrites them, so it keeps copies.
-  double* X = mixedCycle ? d.x : work_;
-  double* R = work_ + (size_t)n_;
-  double* Z = work_ + 2 * (size_t)n_;
-  double* P = work_ + 3 * (size_t)n_;
-  double* Q = work_ + 4 * (size_t)n_;
-  double* B = mixedCycle ? d.b : work_ + 5 * (size_t)n_;
   if (!loopInt_) loopInt_ = (int*)h_.scratch(4 * sizeof(int));
   if (!history_ || historyCap_ < o.nMaxIterations + 2) {
     history_ = (double*)h_.scratch(sizeof(double) * (size_t)(o.nMaxIterations + 2));
     historyCap_ = o.nMaxIterations + 2;
   }
-  const cudaStreamCaptureMode mode = cudaStreamCaptureModeThreadLocal;
-  cudaGraphConditionalHandle h = 0;
-  // the loop goes after whatever g already holds
-  std::vector<cudaGraphNode_t> before;
-  bool ok = graph_leaves(g, before) &&
-            cudaGraphConditionalHandleCreate(&h, g, 0, cudaGraphCondAssignDefault) == cudaSuccess;
-  // prologue: x = 0, p = 0, z = 0, r = b, |r| (host copies of b kept in B)
-  ok = ok && cudaStreamBeginCaptureToGraph(st, g, before.empty() ? nullptr : before.data(), nullptr, before.size(),
-                                           mode) == cudaSuccess;
-  if (ok) {
-    try {
-      CUDA_OK(cudaMemsetAsync(X, 0, sizeof(double) * (size_t)n_, st));
-      CUDA_OK(cudaMemsetAsync(P, 0, sizeof(double) * (size_t)n_, st));
-      CUDA_OK(cudaMemsetAsync(Z, 0, sizeof(double) * (size_t)n_, st));
-      if (B != d.b) dev::copy_d(n_, d.b, B, st);
-      // r = b at x = 0, with its norm and the FP32 cycle's right-hand side
-      dev::cg_start(n_, B, R, mixedCycle ? d.bF : nullptr, partials_, st);
-      dev::sum_partials(dev::vec_blocks(n_), partials_, scal_ + kNorm, st);
-      k_cg_loop_init<<<1, 1, 0, st>>>(scal_, loopInt_, history_, o.absoluteTolerance, o.nMaxIterations, h);
-    } catch (const Error&) {
-      ok = false;
-    }
-    cudaGraph_t gg = nullptr;
-    ok = cudaStreamEndCapture(st, &gg) == cudaSuccess && ok;
+  cudaGraphConditionalHandle h = 0, hHalf = 0;
+  cudaGraph_t body = nullptr, second = nullptr;
+  bool ok = cudaGraphConditionalHandleCreate(&h, g, 0, cudaGraphCondAssignDefault) == cudaSuccess;
+  ok = ok && graph_capture(g, st, [&] {
+    prologue();
+    k_loop_init<<<1, 1, 0, st>>>(scal_, loopInt_, history_, o.absoluteTolerance, maxIt, testFirst ? 1 : 0, h);
+    CUDA_OK(cudaGetLastError());
+  });
+  ok = ok && graph_conditional(g, h, cudaGraphCondTypeWhile, &body);
+  if (half) {
+    ok = ok && cudaGraphConditionalHandleCreate(&hHalf, body, 0, cudaGraphCondAssignDefault) == cudaSuccess;
+    ok = ok && graph_capture(body, st, [&] {
+      half();
+      k_loop_check<true><<<1, 1024, 0, st>>>(np, partials, scal_, loopInt_, history_, o.relativeTolerance,
+                                             o.absoluteTolerance, maxIt, h, hHalf);
+      CUDA_OK(cudaGetLastError());
+    });
+    ok = ok && graph_conditional(body, hHalf, cudaGraphCondTypeIf, &second);
   }
-  // the while node after the prologue's last node
-  cudaGraphNode_t cnode = nullptr;
-  cudaGraph_t body = nullptr;
+  ok = ok && graph_capture(half ? second : body, st, [&] {
+    iteration();
+    k_loop_check<false><<<1, 1024, 0, st>>>(np, partials, scal_, loopInt_, history_, o.relativeTolerance,
+                                            o.absoluteTolerance, maxIt, h, hHalf);
+    CUDA_OK(cudaGetLastError());
+  });
   if (ok) {
-    std::vector<cudaGraphNode_t> leaves;
-    ok = graph_leaves(g, leaves);
-    cudaGraphNodeParams cp = {};
-    cp.type = cudaGraphNodeTypeConditional;
-    cp.conditional.handle = h;
-    cp.conditional.type = cudaGraphCondTypeWhile;
-    cp.conditional.size = 1;
-    ok = ok && !leaves.empty() && cudaGraphAddNode(&cnode, g, leaves.data(), leaves.size(), &cp) == cudaSuccess;
-    if (ok) body = cp.conditional.phGraph_out[0];
+    size_t nb = 0, ns = 0;
+    cudaGraphGetNodes(body, nullptr, &nb);
+    if (half) cudaGraphGetNodes(second, nullptr, &ns);
+    loopBodyNodes_ = (long long)nb + (long long)ns - (half ? 1 : 0);
   }
-  // body: one fused iteration and the convergence check
-  ok = ok && cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0, mode) == cudaSuccess;
-  if (ok) {
-    try {
-      // the FP32 cycle runs on level 0's bF, which the prologue and each
-      // update write (r in FP32)
-      if (mixedCycle)
-        h_.runCycle<float>(st, true);
-      else
-        h_.applyCycle(R, st);
-      if (mixedCycle)
-        dev::cg_take_z<float>(n_, d.xF, R, Z, partials2_, st);
-      else
-        dev::cg_take_z<double>(n_, d.x, R, Z, partials2_, st);
-      dev::cg_beta(dev::vec_blocks(n_), partials2_, scal_ + kRho, scal_ + kRhoPrev, scal_ + kBeta, flexible, st);
-      // p = p * beta + z is formed by the SpMV where it reads p and written
-      // by the update: no pass of its own
-      dev::spmv_dot_pby(d.view64(), d.nSlices, Z, P, scal_ + kBeta, Q, partials2_, st);
-      dev::cg_alpha(dev::spmv_dot_blocks(d.view64(), d.nSlices), partials2_, scal_ + kRho, scal_ + kAlpha, st);
-      dev::cg_update_pby(n_, scal_ + kAlpha, Z, scal_ + kBeta, P, Q, X, R, partials_, st,
-                         mixedCycle ? d.bF : nullptr);
-      dev::sum_partials(dev::vec_blocks(n_), partials_, scal_ + kNorm, st);
-      k_cg_loop_check<<<1, 1, 0, st>>>(scal_, loopInt_, history_, o.relativeTolerance, o.absoluteTolerance,
-                                       o.nMaxIterations, h);
-    } catch (const Error&) {
-      ok = false;
-    }
-    cudaGraph_t bb = nullptr;
-    ok = cudaStreamEndCapture(st, &bb) == cudaSuccess && ok;
-    size_t nb = 0;
-    if (ok) cudaGraphGetNodes(body, nullptr, &nb);
-    loopBodyNodes_ = (long long)nb;
-  }
-  // epilogue: the system restored; with hostCopies the true residual's norm
-  // and the results to the pinned host scalars (inside an outer loop nothing
-  // reads that norm)
-  ok = ok && cudaStreamBeginCaptureToGraph(st, g, &cnode, nullptr, 1, mode) == cudaSuccess;
-  if (ok) {
-    try {
-      if (hostCopies) {
-        dev::residual<double>(d.view64(), d.nSlices, X, B, R, nullptr, st);
-        norm_into(R, scal_ + kNorm, st);
-      }
-      if (X != d.x) dev::copy_d(n_, X, d.x, st);
-      if (B != d.b) dev::copy_d(n_, B, d.b, st);
-      if (hostCopies) {
-        CUDA_OK(cudaMemcpyAsync(hostScal_, scal_ + kNorm, sizeof(double), cudaMemcpyDeviceToHost, st));
-        CUDA_OK(cudaMemcpyAsync(hostScal_ + 1, history_, sizeof(double), cudaMemcpyDeviceToHost, st));
-        CUDA_OK(cudaMemcpyAsync(hostScal_ + 2, loopInt_, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
-      }
-    } catch (const Error&) {
-      ok = false;
-    }
-    cudaGraph_t ee = nullptr;
-    ok = cudaStreamEndCapture(st, &ee) == cudaSuccess && ok;
-  }
+  ok = ok && graph_capture(g, st, epilogue);
   if (!ok) cudaGetLastError();
   return ok;
+}
+
+bool LinearSolve::addDeviceLoop(cudaGraph_t g, cudaStream_t st, bool hostCopies) {
+  const SolverOptions& o = h_.options();
+  DevLevel& d = h_.level(0);
+  const bool mixedCycle = o.precision == kMixed;
+  // the results to the pinned host scalars
+  auto copies = [&] {
+    if (!hostCopies) return;
+    CUDA_OK(cudaMemcpyAsync(hostScal_, scal_ + kNorm, sizeof(double), cudaMemcpyDeviceToHost, st));
+    CUDA_OK(cudaMemcpyAsync(hostScal_ + 1, history_, sizeof(double), cudaMemcpyDeviceToHost, st));
+    CUDA_OK(cudaMemcpyAsync(hostScal_ + 2, loopInt_, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
+  };
+  const size_t nb = sizeof(double) * (size_t)n_;
+  if (o.solver == kSolverAMG) {
+    // solveAMG's iterations: cycles (mixed: FP32 refinement steps) and the
+    // residual, all on level 0's own vectors
+    return addLoop(
+        g, st, o.nMaxIterations - 1, true,
+        [&] {
+          CUDA_OK(cudaMemsetAsync(d.x, 0, nb, st));
+          dev::residual<double>(d.view64(), d.nSlices, d.x, d.b, d.r, d.partials, st);
+          dev::sum_partials(d.nPartials, d.partials, scal_ + kNorm, st);
+        },
+        nullptr,
+        [&] {
+          if (mixedCycle) {
+            dev::convert_d2f(n_, d.r, d.bF, st);
+            h_.runCycle<float>(st, true);
+            dev::add_f2d(n_, d.xF, d.x, st);
+          } else {
+            h_.runCycle<double>(st);
+          }
+          dev::residual<double>(d.view64(), d.nSlices, d.x, d.b, d.r, d.partials, st);
+        },
+        d.nPartials, d.partials, copies);
+  }
+  // The FP32 cycle works on level 0's FP32 vectors only, so under CG the
+  // iterate and the right-hand side can be level 0's own FP64 x and b: no
+  // copy in, no restore. The FP64 cycle overwrites them, so it keeps copies.
+  const bool own = mixedCycle && o.solver == kSolverCG;
+  double* X = own ? d.x : work_;
+  double* R = work_ + (size_t)n_;
+  const int vb = dev::vec_blocks(n_);
+  if (o.solver == kSolverCG) {
+    double* Z = work_ + 2 * (size_t)n_;
+    double* P = work_ + 3 * (size_t)n_;
+    double* Q = work_ + 4 * (size_t)n_;
+    double* B = own ? d.b : work_ + 5 * (size_t)n_;
+    return addLoop(
+        g, st, o.nMaxIterations, true,
+        [&] {
+          // x = 0, p = 0, z = 0, r = b, |r| (b kept in B)
+          CUDA_OK(cudaMemsetAsync(X, 0, nb, st));
+          CUDA_OK(cudaMemsetAsync(P, 0, nb, st));
+          CUDA_OK(cudaMemsetAsync(Z, 0, nb, st));
+          if (B != d.b) dev::copy_d(n_, d.b, B, st);
+          // r = b at x = 0, with its norm and the FP32 cycle's right-hand side
+          dev::cg_start(n_, B, R, mixedCycle ? d.bF : nullptr, partials_, st);
+          dev::sum_partials(vb, partials_, scal_ + kNorm, st);
+        },
+        nullptr,
+        [&] {
+          // the FP32 cycle runs on level 0's bF, which the prologue and each
+          // update write (r in FP32)
+          if (mixedCycle)
+            h_.runCycle<float>(st, true);
+          else
+            h_.applyCycle(R, st);
+          if (mixedCycle)
+            dev::cg_take_z<float>(n_, d.xF, R, Z, partials2_, st);
+          else
+            dev::cg_take_z<double>(n_, d.x, R, Z, partials2_, st);
+          dev::cg_beta(vb, partials2_, scal_ + kRho, scal_ + kRhoPrev, scal_ + kBeta, cgFlexible(), st);
+          // p = p * beta + z is formed by the SpMV where it reads p and written
+          // by the update: no pass of its own
+          dev::spmv_dot_pby(d.view64(), d.nSlices, Z, P, scal_ + kBeta, Q, partials2_, st);
+          dev::cg_alpha(dev::spmv_dot_blocks(d.view64(), d.nSlices), partials2_, scal_ + kRho, scal_ + kAlpha, st);
+          dev::cg_update_pby(n_, scal_ + kAlpha, Z, scal_ + kBeta, P, Q, X, R, partials_, st,
+                             mixedCycle ? d.bF : nullptr);
+        },
+        vb, partials_,
+        [&] {
+          // the system restored; with hostCopies the true residual's norm
+          // (inside an outer loop nothing reads it)
+          if (hostCopies) {
+            dev::residual<double>(d.view64(), d.nSlices, X, B, R, nullptr, st);
+            norm_into(R, scal_ + kNorm, st);
+          }
+          if (X != d.x) dev::copy_d(n_, X, d.x, st);
+          if (B != d.b) dev::copy_d(n_, B, d.b, st);
+          copies();
+        });
+  }
+  // BiCGStab (BCGStab.cpp:27-170)
+  double* RT = work_ + 2 * (size_t)n_;
+  double* P = work_ + 3 * (size_t)n_;
+  double* PH = work_ + 4 * (size_t)n_;
+  double* V = work_ + 5 * (size_t)n_;
+  double* Tt = work_ + 6 * (size_t)n_;
+  double* B = work_ + 7 * (size_t)n_;
+  return addLoop(
+      g, st, o.nMaxIterations, false,
+      [&] {
+        CUDA_OK(cudaMemsetAsync(X, 0, nb, st));
+        CUDA_OK(cudaMemsetAsync(P, 0, nb, st));
+        CUDA_OK(cudaMemsetAsync(V, 0, nb, st));
+        dev::copy_d(n_, d.b, B, st);
+        dev::residual<double>(d.view64(), d.nSlices, X, B, R, nullptr, st);
+        dev::copy_d(n_, R, RT, st);
+        norm_into(R, scal_ + kNorm, st);
+      },
+      [&] { bcgFirst(R, RT, V, P, PH, X, st); }, [&] { bcgSecond(R, Tt, PH, X, st); }, vb, partials_,
+      [&] {
+        if (hostCopies) {
+          dev::residual<double>(d.view64(), d.nSlices, X, B, R, nullptr, st);
+          norm_into(R, scal_ + kNorm, st);
+        }
+        dev::copy_d(n_, X, d.x, st);
+        dev::copy_d(n_, B, d.b, st);
+        copies();
+      });
+}
+
+// The two halves of a BiCGStab iteration; each ends with the partial sums of
+// the residual's norm.
+void LinearSolve::bcgFirst(double* R, double* RT, double* V, double* P, double* PH, double* X, cudaStream_t st) {
+  const DevLevel& d = h_.level(0);
+  dev::copy_d(1, scal_ + kRho, scal_ + kRhoPrev, st);
+  dot_into(R, RT, scal_ + kRho, st);
+  dev::scalar_ratio_product(scal_ + kRho, scal_ + kRhoPrev, scal_ + kAlpha, scal_ + kOmega, scal_ + kBeta, st);
+  dev::bicg_p_update(n_, R, V, scal_ + kOmega, scal_ + kBeta, P, st);
+  h_.apply(P, PH, st);
+  dev::spmv(d.view64(), d.nSlices, PH, V, st);
+  dot_into(RT, V, scal_ + kRtv, st);
+  dev::scalar_div(scal_ + kRho, scal_ + kRtv, scal_ + kAlpha, st);
+  dev::axpy_dev(n_, scal_ + kAlpha, -1.0, PH, X, st);
+  dev::axpy_dev(n_, scal_ + kAlpha, -1.0, V, R, st);
+  dev::l1_partials(n_, R, partials_, st);
+}
+void LinearSolve::bcgSecond(double* R, double* Tt, double* SH, double* X, cudaStream_t st) {
+  const DevLevel& d = h_.level(0);
+  h_.apply(R, SH, st);
+  dev::spmv(d.view64(), d.nSlices, SH, Tt, st);
+  dot_into(Tt, R, scal_ + kTdotr, st);
+  dot_into(Tt, Tt, scal_ + kTdott, st);
+  dev::scalar_div(scal_ + kTdotr, scal_ + kTdott, scal_ + kOmega, st);
+  dev::axpy_dev(n_, scal_ + kOmega, -1.0, SH, X, st);
+  dev::axpy_dev(n_, scal_ + kOmega, -1.0, Tt, R, st);
+  dev::l1_partials(n_, R, partials_, st);
 }
 
 // The FP32 cycle, unequal sweeps, W cycles, one-directional or Chebyshev
@@ -1935,30 +2080,29 @@ bool LinearSolve::cgFlexible() const {
 
 bool LinearSolve::deviceSolvable() const {
   const SolverOptions& o = h_.options();
-  return o.solver == kSolverCG && o.preconditioner == kPrecAMG && o.useGraphs && o.verbosity <= 0 &&
-         !(learned_ && learnedActive_) && !graphsFailed_ && !loopFailed_;
+  return o.solver != kSolverJacobi && (o.preconditioner == kPrecAMG || o.solver == kSolverBCGStab) && o.useGraphs &&
+         o.verbosity <= 0 && !(learned_ && learnedActive_) && !graphsFailed_ && !loopFailed_;
 }
 
 LinearSolve::LoopKey LinearSolve::loopKey() const {
   const SolverOptions& o = h_.options();
-  return LoopKey{cgFlexible(), o.nMaxIterations, o.relativeTolerance, o.absoluteTolerance};
+  return LoopKey{cgFlexible(), (int)o.solver, o.nMaxIterations, o.relativeTolerance, o.absoluteTolerance};
 }
 
 void LinearSolve::prebuild(cudaStream_t st) {
   if (!deviceSolvable() || gLoop_) return;
-  if (!buildCGLoop(st, cgFlexible())) loopFailed_ = true;
+  if (!buildDeviceLoop(st)) loopFailed_ = true;
 }
 
 bool LinearSolve::appendDeviceSolve(cudaGraph_t g, cudaStream_t st) {
-  return deviceSolvable() && addCGLoop(g, st, cgFlexible(), false);
+  return outerSolvable() && addDeviceLoop(g, st, false);
 }
 
-bool LinearSolve::buildCGLoop(cudaStream_t st, bool flexible) {
-  const SolverOptions& o = h_.options();
+bool LinearSolve::buildDeviceLoop(cudaStream_t st) {
   if (gLoop_) cudaGraphExecDestroy(gLoop_);
   gLoop_ = nullptr;
   cudaGraph_t g = nullptr;
-  bool ok = cudaGraphCreate(&g, 0) == cudaSuccess && addCGLoop(g, st, flexible, true);
+  bool ok = cudaGraphCreate(&g, 0) == cudaSuccess && addDeviceLoop(g, st, true);
   if (ok) {
     size_t nn = 0;
     cudaGraphGetNodes(g, nullptr, &nn);
@@ -1972,22 +2116,15 @@ bool LinearSolve::buildCGLoop(cudaStream_t st, bool flexible) {
     cudaGetLastError();
     return false;
   }
-  loopFlexible_ = flexible;
-  loopMaxIt_ = o.nMaxIterations;
-  loopRel_ = o.relativeTolerance;
-  loopAbs_ = o.absoluteTolerance;
+  loopBuilt_ = loopKey();
   return true;
 }
 
-bool LinearSolve::solveCGLoop(cudaStream_t st, bool flexible, SolveReport& rep) {
-  const SolverOptions& o = h_.options();
+bool LinearSolve::solveDeviceLoop(cudaStream_t st, SolveReport& rep) {
   if (loopFailed_) return false;
-  if (!gLoop_ || loopFlexible_ != flexible || loopMaxIt_ != o.nMaxIterations || loopRel_ != o.relativeTolerance ||
-      loopAbs_ != o.absoluteTolerance) {
-    if (!buildCGLoop(st, flexible)) {
-      loopFailed_ = true;
-      return false;
-    }
+  if ((!gLoop_ || !(loopBuilt_ == loopKey())) && !buildDeviceLoop(st)) {
+    loopFailed_ = true;
+    return false;
   }
   CUDA_OK(cudaGraphLaunch(gLoop_, st));
   CUDA_OK(cudaStreamSynchronize(st));
@@ -2026,6 +2163,7 @@ SolveReport LinearSolve::solveBCGStab(cudaStream_t st) {
   double* Tt = work_ + 6 * (size_t)n_;
   double* B = work_ + 7 * (size_t)n_;
   SolveReport rep;
+  if (deviceSolvable() && solveDeviceLoop(st, rep)) return rep;
   CUDA_OK(cudaMemsetAsync(X, 0, sizeof(double) * (size_t)n_, st));
   CUDA_OK(cudaMemsetAsync(P, 0, sizeof(double) * (size_t)n_, st));
   CUDA_OK(cudaMemsetAsync(V, 0, sizeof(double) * (size_t)n_, st));
@@ -2048,18 +2186,8 @@ SolveReport LinearSolve::solveBCGStab(cudaStream_t st) {
   if (!std::isfinite(r0)) throw Error(kNaN, "initial residual is not finite");
   for (int i = 0; i < o.nMaxIterations; i++) {
     run(g1_, st, [&] {
-      dev::copy_d(1, scal_ + kRho, scal_ + kRhoPrev, st);
-      dot_into(R, RT, scal_ + kRho, st);
-      dev::scalar_ratio_product(scal_ + kRho, scal_ + kRhoPrev, scal_ + kAlpha, scal_ + kOmega,
-                                scal_ + kBeta, st);
-      dev::bicg_p_update(n_, R, V, scal_ + kOmega, scal_ + kBeta, P, st);
-      h_.apply(P, PH, st);
-      dev::spmv(d.view64(), d.nSlices, PH, V, st);
-      dot_into(RT, V, scal_ + kRtv, st);
-      dev::scalar_div(scal_ + kRho, scal_ + kRtv, scal_ + kAlpha, st);
-      dev::axpy_dev(n_, scal_ + kAlpha, -1.0, PH, X, st);
-      dev::axpy_dev(n_, scal_ + kAlpha, -1.0, V, R, st);
-      norm_into(R, scal_ + kNorm, st);
+      bcgFirst(R, RT, V, P, PH, X, st);
+      dev::sum_partials(dev::vec_blocks(n_), partials_, scal_ + kNorm, st);
       CUDA_OK(cudaMemcpyAsync(hostScal_, scal_ + kNorm, sizeof(double), cudaMemcpyDeviceToHost, st));
     });
     CUDA_OK(cudaStreamSynchronize(st));
@@ -2073,15 +2201,8 @@ SolveReport LinearSolve::solveBCGStab(cudaStream_t st) {
       break;
     }
     run(g2_, st, [&] {
-      double* SH = PH;
-      h_.apply(R, SH, st);
-      dev::spmv(d.view64(), d.nSlices, SH, Tt, st);
-      dot_into(Tt, R, scal_ + kTdotr, st);
-      dot_into(Tt, Tt, scal_ + kTdott, st);
-      dev::scalar_div(scal_ + kTdotr, scal_ + kTdott, scal_ + kOmega, st);
-      dev::axpy_dev(n_, scal_ + kOmega, -1.0, SH, X, st);
-      dev::axpy_dev(n_, scal_ + kOmega, -1.0, Tt, R, st);
-      norm_into(R, scal_ + kNorm, st);
+      bcgSecond(R, Tt, PH, X, st);
+      dev::sum_partials(dev::vec_blocks(n_), partials_, scal_ + kNorm, st);
       CUDA_OK(cudaMemcpyAsync(hostScal_, scal_ + kNorm, sizeof(double), cudaMemcpyDeviceToHost, st));
     });
     CUDA_OK(cudaStreamSynchronize(st));

@@ -364,6 +364,11 @@ class AmgHierarchy {
 
 // nodes of g that no node depends on
 bool graph_leaves(cudaGraph_t g, std::vector<cudaGraphNode_t>& leaves);
+// fn's launches on st go into g after its current leaves
+bool graph_capture(cudaGraph_t g, cudaStream_t st, const std::function<void()>& fn);
+// a conditional node after g's leaves; its body graph in *body
+bool graph_conditional(cudaGraph_t g, cudaGraphConditionalHandle h, cudaGraphConditionalNodeType type,
+                       cudaGraph_t* body);
 
 // Linear solve of the finest system held by the hierarchy: level 0's b is
 // the right-hand side, level 0's x the delta (zeroed on entry).
@@ -381,28 +386,33 @@ class LinearSolve {
   int solveRecording(cudaStream_t st, double relTol, int maxIter, int record, const std::vector<double*>& rs,
                      const std::vector<double*>& xs, SolveReport& rep);
 
-  // The whole solve can run inside a graph with no host step: CG under the
-  // AMG cycle, graphs on, no printing, no active learned step.
+  // The whole solve can run inside a graph with no host step: AMG, CG under
+  // the AMG cycle or BiCGStab, graphs on, no printing, no active learned
+  // step.
   bool deviceSolvable() const;
+  // ... and inside the outer loop's graph: CG only, as the thermal model's
+  // report and its tests state it (an AMG or BiCGStab solve is one graph of
+  // its own per outer iteration)
+  bool outerSolvable() const { return h_.options().solver == kSolverCG && deviceSolvable(); }
   // Appends that solve to g after its current leaves (no host copies):
   // afterwards deviceLoopState() holds {iterations, status} (status 1
   // converged, 2 non-finite, 3 iteration limit) and deviceInitialNorm()
   // the L1 norm of the right-hand side. False when a graph call failed (g
   // is then unusable).
   bool appendDeviceSolve(cudaGraph_t g, cudaStream_t st);
-  // builds the graph of solveCG's device loop now (when it will be used)
+  // builds the graph of the solve's device loop now (when it will be used)
   // rather than in the first solve
   void prebuild(cudaStream_t st);
   const int* deviceLoopState() const { return loopInt_; }
   const double* deviceInitialNorm() const { return history_; }
   long long loopBodyNodes() const { return loopBodyNodes_; }
-  // the CG settings a graph from appendDeviceSolve bakes in
+  // the settings a graph from appendDeviceSolve bakes in
   struct LoopKey {
-    bool flexible;
-    int maxIt;
-    double rel, abs;
+    bool flexible = false;
+    int solver = -1, maxIt = -1;
+    double rel = 0.0, abs = 0.0;
     bool operator==(const LoopKey& o) const {
-      return flexible == o.flexible && maxIt == o.maxIt && rel == o.rel && abs == o.abs;
+      return flexible == o.flexible && solver == o.solver && maxIt == o.maxIt && rel == o.rel && abs == o.abs;
     }
   };
   LoopKey loopKey() const;
@@ -411,22 +421,25 @@ class LinearSolve {
   bool cgFlexible() const;
   SolveReport solveAMG(cudaStream_t st);
   SolveReport solveCG(cudaStream_t st);
-  // CG with the fused iteration, every iteration of one solve inside one
-  // CUDA graph (a conditional while node whose condition a device kernel
-  // sets from the residual norm): one host synchronisation per solve.
-  // Returns false (and is not used again) when the graph cannot be built.
-  bool solveCGLoop(cudaStream_t st, bool flexible, SolveReport& rep);
-  bool buildCGLoop(cudaStream_t st, bool flexible);
-  // appends the CG loop (prologue, while node, epilogue) to g after its
-  // current leaves; hostCopies: the epilogue also copies the final norm,
-  // the initial norm and the loop state to the pinned host scalars
-  bool addCGLoop(cudaGraph_t g, cudaStream_t st, bool flexible, bool hostCopies);
+  // Every iteration of one solve inside one CUDA graph (a conditional while
+  // node whose condition a device kernel sets from the residual norm): one
+  // host synchronisation per solve. Returns false (and is not used again)
+  // when the graph cannot be built.
+  bool solveDeviceLoop(cudaStream_t st, SolveReport& rep);
+  bool buildDeviceLoop(cudaStream_t st);
+  // appends the solve's loop (prologue, while node, epilogue) to g after its
+  // current leaves; hostCopies: the epilogue also copies the final norm, the
+  // initial norm and the loop state to the pinned host scalars
+  bool addDeviceLoop(cudaGraph_t g, cudaStream_t st, bool hostCopies);
+  bool addLoop(cudaGraph_t g, cudaStream_t st, int maxIt, bool testFirst, const std::function<void()>& prologue,
+               const std::function<void()>& half, const std::function<void()>& iteration, int np,
+               const double* partials, const std::function<void()>& epilogue);
+  void bcgFirst(double* R, double* RT, double* V, double* P, double* PH, double* X, cudaStream_t st);
+  void bcgSecond(double* R, double* Tt, double* SH, double* X, cudaStream_t st);
   int historyCap_ = 0;
   cudaGraphExec_t gLoop_ = nullptr;
   bool loopFailed_ = false;
-  bool loopFlexible_ = false;
-  int loopMaxIt_ = -1;
-  double loopRel_ = 0.0, loopAbs_ = 0.0;
+  LoopKey loopBuilt_;
   int* loopInt_ = nullptr;       // device: iterations, status
   long long loopBodyNodes_ = 0, loopOtherNodes_ = 0;  // kernels and copies per iteration / per solve
   double* history_ = nullptr;    // device: norms of iterations 0..nMaxIterations

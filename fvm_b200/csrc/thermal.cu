@@ -491,45 +491,13 @@ bool ThermalModel::buildAdvanceGraph(int historyCap) {
   double* hist = (double*)((char*)dOuter_ + kOuterHead);
   const dev::BoundaryData bd = boundaryData();
   const int nCells = mesh_->nCells;
-  const cudaStreamCaptureMode mode = cudaStreamCaptureModeThreadLocal;
-  // fn's launches on stream_ go into gr after its current leaves
-  auto capture = [&](cudaGraph_t gr, const std::function<void()>& fn) {
-    std::vector<cudaGraphNode_t> leaves;
-    if (!graph_leaves(gr, leaves)) return false;
-    if (cudaStreamBeginCaptureToGraph(stream_, gr, leaves.empty() ? nullptr : leaves.data(), nullptr, leaves.size(),
-                                      mode) != cudaSuccess)
-      return false;
-    bool ok = true;
-    try {
-      fn();
-    } catch (const Error&) {
-      ok = false;
-    }
-    cudaGraph_t out = nullptr;
-    return cudaStreamEndCapture(stream_, &out) == cudaSuccess && ok;
-  };
-  // a conditional node after gr's leaves; its body graph in *bodyOut
-  auto conditional = [&](cudaGraph_t gr, cudaGraphConditionalHandle h, cudaGraphConditionalNodeType type,
-                         cudaGraph_t* bodyOut) {
-    std::vector<cudaGraphNode_t> leaves;
-    if (!graph_leaves(gr, leaves) || leaves.empty()) return false;
-    cudaGraphNodeParams cp = {};
-    cp.type = cudaGraphNodeTypeConditional;
-    cp.conditional.handle = h;
-    cp.conditional.type = type;
-    cp.conditional.size = 1;
-    cudaGraphNode_t node = nullptr;
-    if (cudaGraphAddNode(&node, gr, leaves.data(), leaves.size(), &cp) != cudaSuccess) return false;
-    *bodyOut = cp.conditional.phGraph_out[0];
-    return true;
-  };
   cudaGraph_t g = nullptr, body = nullptr, upd = nullptr;
   cudaGraphConditionalHandle hOuter = 0, hUpdate = 0;
   bool ok = cudaGraphCreate(&g, 0) == cudaSuccess &&
             cudaGraphConditionalHandleCreate(&hOuter, g, 0, cudaGraphCondAssignDefault) == cudaSuccess;
   const int aaM = opt_.linear.outerAcceleration;
   if (aaM > 0) ensureAcceleration(aaM);
-  ok = ok && capture(g, [&] {
+  ok = ok && graph_capture(g, stream_, [&] {
     k_outer_init<<<1, 1, 0, stream_>>>(state, hOuter);
     CUDA_OK(cudaGetLastError());
     if (aaM > 0) accelerationStart(stream_);
@@ -539,17 +507,17 @@ bool ThermalModel::buildAdvanceGraph(int historyCap) {
     cudaGraphGetNodes(g, nullptr, &np);
     advPrologueNodes_ = (long long)np;
   }
-  ok = ok && conditional(g, hOuter, cudaGraphCondTypeWhile, &body);
+  ok = ok && graph_conditional(g, hOuter, cudaGraphCondTypeWhile, &body);
   ok = ok && cudaGraphConditionalHandleCreate(&hUpdate, body, 0, cudaGraphCondAssignDefault) == cudaSuccess;
-  ok = ok && capture(body, [&] { linearize(); });
+  ok = ok && graph_capture(body, stream_, [&] { linearize(); });
   ok = ok && solver_->appendDeviceSolve(body, stream_);
-  ok = ok && capture(body, [&] {
+  ok = ok && graph_capture(body, stream_, [&] {
     k_outer_check<<<1, 1, 0, stream_>>>(state, hist, solver_->deviceInitialNorm(), solver_->deviceLoopState(),
                                         hOuter, hUpdate);
     CUDA_OK(cudaGetLastError());
   });
-  ok = ok && conditional(body, hUpdate, cudaGraphCondTypeIf, &upd);
-  ok = ok && capture(upd, [&] {
+  ok = ok && graph_conditional(body, hUpdate, cudaGraphCondTypeIf, &upd);
+  ok = ok && graph_capture(upd, stream_, [&] {
     dev::update_solution(nCells, dPerm_, hier_.level(0).x, bd, dFaceCells_, dCoeff_, dT_, stream_);
     // skipped on the device once the loop has ended (converged or out of
     // iterations), as the host loop skips it
@@ -584,7 +552,7 @@ bool ThermalModel::buildAdvanceGraph(int historyCap) {
 
 bool ThermalModel::outerGraphUsable() const {
   return !advanceFailed_ && opt_.linear.outerOnDevice && !matrixDependsOnT_ && !dSegNorm_ &&
-         opt_.linear.verbosity <= 0 && solver_ && solver_->deviceSolvable();
+         opt_.linear.verbosity <= 0 && solver_ && solver_->outerSolvable();
 }
 
 bool ThermalModel::advanceOnDevice(int niter, AdvanceReport& rep) {
