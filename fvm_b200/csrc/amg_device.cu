@@ -1171,7 +1171,7 @@ void AmgHierarchy::buildDevice(const FinestDevice& in, const SolverOptions& opt,
         int* status = (int*)alloc(sizeof(int));
         CUDA_OK(cudaMemsetAsync(status, 0, sizeof(int), st));
         if (mixed)
-          coarseInvF_ = (float*)alloc(sizeof(float) * nn);
+          coarseInvF_ = (float*)alloc(sizeof(float) * (size_t)c.n * dev::inverse_f32_stride(c.n));
         else
           coarseInv_ = (double*)alloc(sizeof(double) * nn);
         // the rows' points, averaged down from the cell centroids
@@ -1202,8 +1202,8 @@ void AmgHierarchy::buildDevice(const FinestDevice& in, const SolverOptions& opt,
       inversePending_ = true;
     }
     if (mixed && !coarseInvF_) {
-      coarseInvF_ = (float*)arena_.alloc(size_class(sizeof(float) * nn));
-      dev::cast_d2f(nn, coarseInv_, coarseInvF_, st);
+      coarseInvF_ = (float*)arena_.alloc(size_class(sizeof(float) * (size_t)c.n * dev::inverse_f32_stride(c.n)));
+      dev::inverse_to_f32(c.n, coarseInv_, coarseInvF_, st);
     }
     if (trace) {
       finishBuild();

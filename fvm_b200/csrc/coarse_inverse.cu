@@ -840,11 +840,12 @@ __global__ void __launch_bounds__(256, 3) k_inv_update(int NB, int np, const int
 
 // out = the negated, unpermuted matrix: a CTA takes W consecutive rows of
 // the padded order, mirrors them from the stored triangle into shared
-// memory and writes each to its own row, columns gathered there
+// memory and writes each to its own row (ld apart, zero past column n),
+// columns gathered there
 template <class T, int W>
 __global__ void __launch_bounds__(512) k_inv_finish(int n, int NB, const int* __restrict__ pos,
                                                     const int* __restrict__ rowAt, const double* __restrict__ A,
-                                                    const unsigned char* __restrict__ nz, T* __restrict__ out) {
+                                                    const unsigned char* __restrict__ nz, T* __restrict__ out, int ld) {
   extern __shared__ __align__(16) unsigned char raw[];
   T* strip = reinterpret_cast<T*>(raw);  // [W][NB * 32]
   const int N = NB * kBlk, p0 = blockIdx.x * W, I = p0 / kBlk, r0 = p0 % kBlk;
@@ -864,7 +865,8 @@ __global__ void __launch_bounds__(512) k_inv_finish(int n, int NB, const int* __
   for (int r = 0; r < W; r++) {
     const int i = rowAt[p0 + r];
     if (i < 0) continue;
-    for (int j = threadIdx.x; j < n; j += 512) out[(size_t)i * n + j] = strip[(size_t)r * N + pos[j]];
+    for (int j = threadIdx.x; j < ld; j += 512)
+      out[(size_t)i * ld + j] = j < n ? strip[(size_t)r * N + pos[j]] : T(0);
   }
 }
 __global__ void k_inv_rows(int n, const int* __restrict__ pos, int* rowAt) {
@@ -953,12 +955,13 @@ void inverse_symmetric(const SellView<double>& a, const int* rowSlice, const flo
     const size_t smem = sizeof(double) * 4 * (size_t)N;
     ok(cudaFuncSetAttribute(k_inv_finish<double, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
        "cudaFuncSetAttribute");
-    k_inv_finish<double, 4><<<N / 4, 512, smem, st>>>(n, NB, pos, rowAt, A, nz, out64);
+    k_inv_finish<double, 4><<<N / 4, 512, smem, st>>>(n, NB, pos, rowAt, A, nz, out64, n);
   } else {
     const size_t smem = sizeof(float) * 8 * (size_t)N;
     ok(cudaFuncSetAttribute(k_inv_finish<float, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
        "cudaFuncSetAttribute");
-    k_inv_finish<float, 8><<<N / 8, 512, smem, st>>>(n, NB, pos, rowAt, A, nz, outF);
+    k_inv_finish<float, 8><<<N / 8, 512, smem, st>>>(n, NB, pos, rowAt, A, nz, outF,
+                                                             inverse_f32_stride(n));
   }
   ok(cudaGetLastError(), "coarsest inverse");
 }

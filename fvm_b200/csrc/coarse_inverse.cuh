@@ -23,7 +23,7 @@ void coarse_points(int nc, const int* c2fRow, const int* c2fCol, const int* fine
                    const float* finePoints, float* points, cudaStream_t st);
 
 // The inverse, n x n row-major in a's row numbering, to out64 or (out64
-// null) in FP32 to outF. alloc gives device memory that lives until the
+// null) in FP32 to outF with rows inverse_f32_stride(n) apart. alloc gives device memory that lives until the
 // stream has finished; *status (device, 0 on entry) becomes 1 when a pivot
 // is exactly zero. points (may be null): the rows' points, which only shape
 // the order of elimination. The order of elimination is read back to the host (one

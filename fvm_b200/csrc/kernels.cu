@@ -51,22 +51,26 @@ __device__ __forceinline__ double block_sum(double v) {
 // (the same value, without the prolongation's launch and x round trip)
 template <class T>
 struct XDirect {
-  const T* __restrict__ x;
+  const T* x;
   __device__ __forceinline__ T operator()(int j) const { return x[j]; }
 };
 // CG's new search direction read where it is needed: p_j = p_old_j * beta +
 // z_j, rounded as k_xpby_dev rounds it (contraction off in this file)
+template <class S>
 struct XPby {
-  const double* __restrict__ z;
-  const double* __restrict__ p;
+  const S* z;
+  const double* p;
   double beta;
-  __device__ __forceinline__ double operator()(int j) const { return p[j] * beta + z[j]; }
+  __device__ __forceinline__ double operator()(int j) const { return p[j] * beta + (double)z[j]; }
 };
 template <class T>
 struct XProlonged {
-  const T* __restrict__ xc;
+  const T* xc;
   const int* __restrict__ ci;
-  __device__ __forceinline__ T operator()(int j) const { return xc[ci[j]]; }
+  __device__ __forceinline__ T operator()(int j) const {
+    const int c = ci[j];
+    return c >= 0 ? xc[c] : T(0);
+  }
 };
 
 // Up to K entries of a row: every column and value load is issued, then
@@ -112,8 +116,7 @@ __device__ __forceinline__ T row_sum_g(const SellView<T>& a, const int4 m, int l
   return sum;
 }
 template <class T>
-__device__ __forceinline__ T row_sum(const SellView<T>& a, const int4 m, int lane, const T* __restrict__ x,
-                                     T sum) {
+__device__ __forceinline__ T row_sum(const SellView<T>& a, const int4 m, int lane, const T* x, T sum) {
   return row_sum_g(a, m, lane, XDirect<T>{x}, sum);
 }
 
@@ -121,13 +124,24 @@ __device__ __forceinline__ T row_sum(const SellView<T>& a, const int4 m, int lan
 // Programmatic dependent launch: every hot-path kernel lets the next
 // kernel in the stream be scheduled as soon as all of its own blocks are
 // running (launch_dependents), and waits for its predecessor's completion
-// and memory before touching any data (griddepcontrol.wait). The launch
-// latency of the next kernel then overlaps this one. Kernels launched
-// without the attribute see both instructions as no-ops.
-#define FVM_PDL()                                                  \
-  do {                                                             \
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); \
-    asm volatile("griddepcontrol.wait;" ::: "memory");             \
+// and memory before touching any data an earlier kernel writes
+// (griddepcontrol.wait). The launch latency of the next kernel then overlaps
+// this one. Kernels launched without the attribute see both instructions as
+// no-ops.
+//
+// What no kernel of a solve writes -- a level's columns, values, diagonal,
+// slice metadata and transfer maps, complete before the solve's first launch
+// (the setup ends with a synchronisation) -- is loaded between the two
+// instructions, so a pass whose predecessor is still running has its row in
+// registers when the wait ends and only gathers then. (The vectors such a
+// kernel reads after the wait are not declared __restrict__: as read-only
+// parameters the compiler would be free to load them ahead of it.)
+#define FVM_PDL_TRIGGER() asm volatile("griddepcontrol.launch_dependents;" ::: "memory")
+#define FVM_PDL_WAIT() asm volatile("griddepcontrol.wait;" ::: "memory")
+#define FVM_PDL()      \
+  do {                 \
+    FVM_PDL_TRIGGER(); \
+    FVM_PDL_WAIT();    \
   } while (0)
 
 // A slice's {first row, rows, offset, width}: loaded (SELL-32) or computed
@@ -154,28 +168,6 @@ __global__ void k_zero(int n, T* x) {
 
 // ---------------------------------------------------------------------------
 template <class T>
-__global__ void __launch_bounds__(kBlock, 8) k_gs_color(SellView<T> a, int s0, int s1, T* x, const T* __restrict__ b) {
-  FVM_PDL();
-  const int lane = threadIdx.x & 31;
-  if (a.ellWidth) {
-    // rows [s0, s1) of the aligned 32-row groups
-    const int s = (s0 >> 5) + blockIdx.x * kSlicesPerBlock + (threadIdx.x >> 5);
-    const int i = (s << 5) + lane;
-    if (i < s0 || i >= s1) return;
-    const T sum = row_sum(a, slice_meta(a, s), lane, x, b[i]);
-    x[i] = -sum / a.diag[i];
-    return;
-  }
-  const int s = s0 + blockIdx.x * kSlicesPerBlock + (threadIdx.x >> 5);
-  if (s >= s1) return;
-  const int4 m = slice_meta(a, s);
-  if (lane >= m.y) return;
-  const int i = m.x + lane;
-  const T sum = row_sum(a, m, lane, x, b[i]);
-  x[i] = -sum / a.diag[i];
-}
-
-template <class T>
 __global__ void k_gs_sequential(SellView<T> a, T* x, const T* __restrict__ b, int reverse) {
   FVM_PDL();
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
@@ -188,7 +180,7 @@ __global__ void k_gs_sequential(SellView<T> a, T* x, const T* __restrict__ b, in
 }
 
 template <class T>
-__global__ void __launch_bounds__(kBlock, 8) k_jacobi(SellView<T> a, int nSlices, const T* __restrict__ xold, T* xnew,
+__global__ void __launch_bounds__(kBlock, 4) k_jacobi(SellView<T> a, int nSlices, const T* __restrict__ xold, T* xnew,
                          const T* __restrict__ b) {
   FVM_PDL();
   const int lane = threadIdx.x & 31;
@@ -201,28 +193,130 @@ __global__ void __launch_bounds__(kBlock, 8) k_jacobi(SellView<T> a, int nSlices
   }
 }
 
-// damped Jacobi: xnew = xold + w (xJacobi - xold); Pro: xold is the
-// prolongation xc[ci] a pass would otherwise have assigned first
-template <class T, bool Pro>
-__global__ void __launch_bounds__(kBlock, 8) k_jacobi_damped(SellView<T> a, int nSlices, const T* __restrict__ xold,
-                                                             T* xnew, const T* __restrict__ b, T w,
-                                                             const T* __restrict__ xc, const int* __restrict__ ci) {
-  FVM_PDL();
-  const int lane = threadIdx.x & 31;
-  for (int s = blockIdx.x * kSlicesPerBlock + (threadIdx.x >> 5); s < nSlices; s += gridDim.x * kSlicesPerBlock) {
-    const int4 m = slice_meta(a, s);
-    if (lane >= m.y) continue;
-    const int i = m.x + lane;
-    T sum, xo;
-    if constexpr (Pro) {
-      sum = row_sum_g(a, m, lane, XProlonged<T>{xc, ci}, b[i]);
-      xo = xc[ci[i]];
-    } else {
-      sum = row_sum(a, m, lane, xold, b[i]);
-      xo = xold[i];
+// Up to K entries of a row held ahead of the wait, and their sum after it
+// (stored order, four gathers in flight at a time)
+template <class T, int K>
+struct RowHead {
+  int c[K];
+  T v[K];
+  __device__ __forceinline__ void load(const SellView<T>& a, int e0, int cnt) {
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      c[k] = 0;
+      v[k] = T(0);
+      if (k < cnt) {
+        c[k] = a.cols[e0 + (k << 5)];
+        v[k] = a.vals[e0 + (k << 5)];
+      }
     }
-    xnew[i] = xo + w * (-sum / a.diag[i] - xo);
   }
+  // columns as the rows of the next level they are prolonged from
+  __device__ __forceinline__ void prolonged(const int* __restrict__ ci, int cnt) {
+#pragma unroll
+    for (int k = 0; k < K; k++)
+      if (k < cnt) c[k] = ci[c[k]];
+  }
+  template <class X>
+  __device__ __forceinline__ T sum(int cnt, const X& xg, T s) const {
+#pragma unroll
+    for (int k0 = 0; k0 < K; k0 += 4) {
+      T xv[4];
+#pragma unroll
+      for (int k = k0; k < k0 + 4 && k < K; k++)
+        if (k < cnt) xv[k - k0] = xg(c[k]);
+#pragma unroll
+      for (int k = k0; k < k0 + 4 && k < K; k++)
+        if (k < cnt) s = s + v[k] * xv[k - k0];
+    }
+    return s;
+  }
+};
+// x as a prolongation would have assigned it, read by coarse row (-1: none)
+template <class T>
+struct XCoarse {
+  const T* xc;
+  __device__ __forceinline__ T operator()(int c) const { return c >= 0 ? xc[c] : T(0); }
+};
+
+// One colour of a SELL-32 level: one warp per slice, its first eight entries
+// ahead of the wait
+template <class T>
+__global__ void __launch_bounds__(kBlock) k_gs_color(SellView<T> a, int s0, int s1, T* x, const T* b) {
+  FVM_PDL_TRIGGER();
+  constexpr int K = 8;
+  const int lane = threadIdx.x & 31;
+  int4 m = make_int4(0, 0, 0, 0);
+  bool live;
+  if (a.ellWidth) {
+    // rows [s0, s1) of the aligned 32-row groups
+    const int s = (s0 >> 5) + blockIdx.x * kSlicesPerBlock + (threadIdx.x >> 5);
+    const int i = (s << 5) + lane;
+    live = i >= s0 && i < s1;
+    if (live) m = slice_meta(a, s);
+  } else {
+    const int s = s0 + blockIdx.x * kSlicesPerBlock + (threadIdx.x >> 5);
+    if (s < s1) m = slice_meta(a, s);
+    live = lane < m.y;
+  }
+  const int i = m.x + lane;
+  RowHead<T, K> h;
+  int cnt = 0;
+  T d = T(1);
+  if (live) {
+    cnt = min(m.w, K);
+    h.load(a, m.z + lane, cnt);
+    d = a.diag[i];
+  }
+  FVM_PDL_WAIT();
+  if (!live) return;
+  T sum = h.sum(cnt, XDirect<T>{x}, b[i]);
+  if (m.w > K) sum = row_sum(a, make_int4(m.x, m.y, m.z + (K << 5), m.w - K), lane, x, sum);
+  x[i] = -sum / d;
+}
+
+// damped Jacobi: xnew = xold + w (xJacobi - xold); Pro: xold is the
+// prolongation xc[ci] a pass would otherwise have assigned first. One warp
+// per slice, its first entries (FP32 twelve, FP64 eight) ahead of the wait.
+template <class T, bool Pro>
+__global__ void __launch_bounds__(kBlock) k_jacobi_damped(SellView<T> a, int nSlices, const T* xold,
+                                                          T* xnew, const T* b, T w,
+                                                          const T* xc, const int* __restrict__ ci) {
+  FVM_PDL_TRIGGER();
+  constexpr int K = sizeof(T) == 4 ? 12 : 8;
+  const int lane = threadIdx.x & 31;
+  const int s = blockIdx.x * kSlicesPerBlock + (threadIdx.x >> 5);
+  int4 m = make_int4(0, 0, 0, 0);
+  if (s < nSlices) m = slice_meta(a, s);
+  const bool live = lane < m.y;
+  const int i = m.x + lane;
+  RowHead<T, K> h;
+  int cnt = 0, own = i;
+  T d = T(1);
+  if (live) {
+    cnt = min(m.w, K);
+    h.load(a, m.z + lane, cnt);
+    d = a.diag[i];
+    if constexpr (Pro) {
+      own = ci[i];
+      h.prolonged(ci, cnt);
+    }
+  }
+  FVM_PDL_WAIT();
+  if (!live) return;
+  T sum = b[i], xo;
+  const int4 rest = make_int4(m.x, m.y, m.z + (K << 5), m.w - K);
+  if constexpr (Pro) {
+    const XCoarse<T> xg{xc};
+    xo = xg(own);
+    sum = h.sum(cnt, xg, sum);
+    if (m.w > K) sum = row_sum_g(a, rest, lane, XProlonged<T>{xc, ci}, sum);
+  } else {
+    const XDirect<T> xg{xold};
+    xo = xg(own);
+    sum = h.sum(cnt, xg, sum);
+    if (m.w > K) sum = row_sum_g(a, rest, lane, xg, sum);
+  }
+  xnew[i] = xo + w * (-sum / d - xo);
 }
 
 // One step of a Chebyshev polynomial smoother on D^-1 A: with the row's
@@ -230,7 +324,7 @@ __global__ void __launch_bounds__(kBlock, 8) k_jacobi_damped(SellView<T> a, int 
 // written, not read) and xnew = x + dv. dv is indexed by row only, so it
 // is updated in place; x and xnew are distinct.
 template <class T, bool First>
-__global__ void __launch_bounds__(kBlock, 8) k_cheb(SellView<T> a, int nSlices, const T* __restrict__ x, T* xnew,
+__global__ void __launch_bounds__(kBlock, 4) k_cheb(SellView<T> a, int nSlices, const T* __restrict__ x, T* xnew,
                                                     T* dv, const T* __restrict__ b, T c1, T c2) {
   FVM_PDL();
   const int lane = threadIdx.x & 31;
@@ -265,7 +359,7 @@ __global__ void __launch_bounds__(kBlock) k_gershgorin(SellView<double> a, int n
 }
 
 template <class T>
-__global__ void __launch_bounds__(kBlock, 8) k_residual(SellView<T> a, int nSlices, const T* __restrict__ x,
+__global__ void __launch_bounds__(kBlock, 4) k_residual(SellView<T> a, int nSlices, const T* __restrict__ x,
                            const T* __restrict__ b, T* r, double* partials) {
   FVM_PDL();
   const int lane = threadIdx.x & 31;
@@ -302,7 +396,7 @@ __global__ void k_csr_residual(int n, const int* __restrict__ row, const int* __
   if (threadIdx.x == 0) partials[blockIdx.x] = t;
 }
 
-__global__ void __launch_bounds__(kBlock, 8) k_spmv(SellView<double> a, int nSlices, const double* __restrict__ x, double* y) {
+__global__ void __launch_bounds__(kBlock, 4) k_spmv(SellView<double> a, int nSlices, const double* __restrict__ x, double* y) {
   FVM_PDL();
   const int lane = threadIdx.x & 31;
   for (int s = blockIdx.x * kSlicesPerBlock + (threadIdx.x >> 5); s < nSlices; s += gridDim.x * kSlicesPerBlock) {
@@ -337,82 +431,103 @@ __device__ __forceinline__ T ell_row(const SellView<T>& a, int i, const T* __res
   return ell_row_g<T, W>(a, i, XDirect<T>{x}, sum);
 }
 
+// blocks of 256 threads an SM must hold: what a row of W entries kept in
+// registers leaves room for
+template <class T, int W>
+constexpr int ell_blocks() {
+  return sizeof(T) == 4 ? (W <= 6 ? 8 : 6) : (W <= 4 ? 7 : 5);
+}
+
+// rows [r0, r1) of one colour. The pass is bounded by the latency of its two
+// dependent rounds of loads, not by bytes; the first round, the matrix, is
+// done while the previous colour still runs.
+template <class T, int W>
+__global__ void __launch_bounds__(kBlock, ell_blocks<T, W>()) k_gs_color_ell(SellView<T> a, int r0, int r1, T* x,
+                                                                            const T* b) {
+  FVM_PDL_TRIGGER();
+  const int i = (((r0 >> 5) + blockIdx.x * kSlicesPerBlock) << 5) + threadIdx.x;
+  const bool live = i >= r0 && i < r1;
+  RowHead<T, W> h;
+  T d = T(1);
+  if (live) {
+    h.load(a, (i >> 5) * (32 * W) + (i & 31), W);
+    d = a.diag[i];
+  }
+  FVM_PDL_WAIT();
+  if (!live) return;
+  x[i] = -h.sum(W, XDirect<T>{x}, b[i]) / d;
+}
+
 // The first forward Gauss-Seidel sweep after a prolongation that would
-// assign x = xc[ci]: rows of earlier colours (below r0 in the colour-major
-// order) already hold their new values, rows of later colours still the
-// prolonged ones, read from xc
+// assign x = xc[ci] (bitwise the values of prolongation + pass): rows of
+// earlier colours (below r0 in the colour-major order) already hold their
+// new values, rows of later colours are still the prolonged ones, read from
+// xc. Which of the two a column is, and its coarse row (c < 0: -2 - ci, -1
+// for none), is known ahead of the wait.
 template <class T>
 struct XSweepProlonged {
   const T* x;
-  const T* __restrict__ xc;
-  const int* __restrict__ ci;
-  int r0;
-  __device__ __forceinline__ T operator()(int j) const { return j < r0 ? x[j] : xc[ci[j]]; }
+  const T* xc;
+  __device__ __forceinline__ T operator()(int c) const { return c >= 0 ? x[c] : c == -1 ? T(0) : xc[-2 - c]; }
 };
-
-// rows [r0, r1) of one colour
 template <class T, int W>
-__global__ void __launch_bounds__(kBlock, 8) k_gs_color_ell(SellView<T> a, int r0, int r1, T* x,
-                                                            const T* __restrict__ b) {
-  FVM_PDL();
+__global__ void __launch_bounds__(kBlock, ell_blocks<T, W>()) k_gs_color_ell_pro(SellView<T> a, int r0, int r1, T* x,
+                                                                                const T* b,
+                                                                                const T* xc,
+                                                                                const int* __restrict__ ci) {
+  FVM_PDL_TRIGGER();
   const int i = (((r0 >> 5) + blockIdx.x * kSlicesPerBlock) << 5) + threadIdx.x;
-  if (i < r0 || i >= r1) return;
-  const T sum = ell_row<T, W>(a, i, x, b[i]);
-  x[i] = -sum / a.diag[i];
+  const bool live = i >= r0 && i < r1;
+  RowHead<T, W> h;
+  T d = T(1);
+  if (live) {
+    h.load(a, (i >> 5) * (32 * W) + (i & 31), W);
+    d = a.diag[i];
+#pragma unroll
+    for (int k = 0; k < W; k++)
+      if (h.c[k] >= r0) h.c[k] = -2 - ci[h.c[k]];
+  }
+  FVM_PDL_WAIT();
+  if (!live) return;
+  x[i] = -h.sum(W, XSweepProlonged<T>{x, xc}, b[i]) / d;
 }
 
-// the same colour pass in the first forward sweep after a fused
-// prolongation (XSweepProlonged): bitwise the values of prolongation + pass
-template <class T, int W>
-__global__ void __launch_bounds__(kBlock, 8) k_gs_color_ell_pro(SellView<T> a, int r0, int r1, T* x,
-                                                                const T* __restrict__ b, const T* __restrict__ xc,
-                                                                const int* __restrict__ ci) {
-  FVM_PDL();
-  const int i = (((r0 >> 5) + blockIdx.x * kSlicesPerBlock) << 5) + threadIdx.x;
-  if (i < r0 || i >= r1) return;
-  const T sum = ell_row_g<T, W>(a, i, XSweepProlonged<T>{x, xc, ci, r0}, b[i]);
-  x[i] = -sum / a.diag[i];
-}
-
-// The same pass with two rows per thread (32-row groups g and g + 8 of a
-// block's 16): both rows' column, value, b and diagonal loads are issued
-// first, then both rows' x gathers, then the two sums, so a thread keeps
-// twice the loads in flight and a colour of a few hundred thousand rows
-// fits in one wave. Each row sums b then its products in stored order, as
-// ell_row does, and rows of one colour never read each other, so the
-// result is bitwise that of k_gs_color_ell.
+// The same colour pass with two rows per thread (32-row groups g and g + 8
+// of a block's 16): half the blocks, so a colour of a few hundred thousand
+// rows fits in one wave and the next colour's blocks find room beside it.
+// Rows of one colour never read each other, so the result is bitwise that
+// of k_gs_color_ell.
 template <class T, int W>
 __global__ void __launch_bounds__(kBlock) k_gs_color_ell2(SellView<T> a, int r0, int r1, T* x,
-                                                          const T* __restrict__ b) {
-  FVM_PDL();
+                                                          const T* b) {
+  FVM_PDL_TRIGGER();
   const int g0 = (r0 >> 5) + blockIdx.x * (2 * kSlicesPerBlock) + (threadIdx.x >> 5);
-  const int i0 = (g0 << 5) + (threadIdx.x & 31);
-  const int i1 = i0 + (kSlicesPerBlock << 5);
-  const bool v0 = i0 >= r0 && i0 < r1, v1 = i1 >= r0 && i1 < r1;
-  const int o0 = (i0 >> 5) * (32 * W) + (i0 & 31), o1 = (i1 >> 5) * (32 * W) + (i1 & 31);
-  int c0[W], c1[W];
-  T a0[W], a1[W], x0[W], x1[W];
+  int i[2];
+  bool live[2];
+  RowHead<T, W> h[2];
+  T d[2], sum[2];
 #pragma unroll
-  for (int k = 0; k < W; k++) {
-    c0[k] = v0 ? a.cols[o0 + (k << 5)] : 0;
-    a0[k] = v0 ? a.vals[o0 + (k << 5)] : T(0);
-    c1[k] = v1 ? a.cols[o1 + (k << 5)] : 0;
-    a1[k] = v1 ? a.vals[o1 + (k << 5)] : T(0);
+  for (int q = 0; q < 2; q++) {
+    i[q] = ((g0 + q * kSlicesPerBlock) << 5) + (threadIdx.x & 31);
+    live[q] = i[q] >= r0 && i[q] < r1;
+    d[q] = T(1);
+    h[q].load(a, (i[q] >> 5) * (32 * W) + (i[q] & 31), live[q] ? W : 0);
+    if (live[q]) d[q] = a.diag[i[q]];
   }
-  T s0 = v0 ? b[i0] : T(0), s1 = v1 ? b[i1] : T(0);
-  const T d0 = v0 ? a.diag[i0] : T(1), d1 = v1 ? a.diag[i1] : T(1);
+  FVM_PDL_WAIT();
+  T xv[2][W];
 #pragma unroll
-  for (int k = 0; k < W; k++) {
-    x0[k] = v0 ? x[c0[k]] : T(0);
-    x1[k] = v1 ? x[c1[k]] : T(0);
+  for (int q = 0; q < 2; q++) {
+    sum[q] = live[q] ? b[i[q]] : T(0);
+#pragma unroll
+    for (int k = 0; k < W; k++) xv[q][k] = live[q] ? x[h[q].c[k]] : T(0);
   }
 #pragma unroll
-  for (int k = 0; k < W; k++) {
-    s0 = s0 + a0[k] * x0[k];
-    s1 = s1 + a1[k] * x1[k];
+  for (int q = 0; q < 2; q++) {
+#pragma unroll
+    for (int k = 0; k < W; k++) sum[q] = sum[q] + h[q].v[k] * xv[q][k];
+    if (live[q]) x[i[q]] = -sum[q] / d[q];
   }
-  if (v0) x[i0] = -s0 / d0;
-  if (v1) x[i1] = -s1 / d1;
 }
 
 template <class T, int W>
@@ -452,13 +567,21 @@ __global__ void __launch_bounds__(kBlock, 8) k_cheb_ell(SellView<T> a, const T* 
 
 // residual with one L1 partial per block (256 rows)
 template <class T, int W>
-__global__ void __launch_bounds__(kBlock, 8) k_residual_ell(SellView<T> a, const T* __restrict__ x,
-                                                            const T* __restrict__ b, T* r, double* partials) {
-  FVM_PDL();
+__global__ void __launch_bounds__(kBlock, ell_blocks<T, W>()) k_residual_ell(SellView<T> a, const T* x,
+                                                                            const T* b, T* r,
+                                                                            double* partials) {
+  FVM_PDL_TRIGGER();
   const int i = blockIdx.x * kBlock + threadIdx.x;
+  RowHead<T, W> h;
+  T d = T(0);
+  if (i < a.n) {
+    h.load(a, (i >> 5) * (32 * W) + (i & 31), W);
+    d = a.diag[i];
+  }
+  FVM_PDL_WAIT();
   double l1 = 0.0;
   if (i < a.n) {
-    const T ri = ell_row<T, W>(a, i, x, b[i] + a.diag[i] * x[i]);
+    const T ri = h.sum(W, XDirect<T>{x}, b[i] + d * x[i]);
     r[i] = ri;
     l1 = fabs((double)ri);
   }
@@ -517,31 +640,42 @@ __global__ void __launch_bounds__(kBlock, 8) k_spmv_dot_ell(SellView<double> a, 
 
 // q = A p with p = p_old * beta + z formed on the fly (p itself is written
 // by k_cg_update_pby, after every row has read its neighbours' p_old), one
-// partial of p.q per block
-template <int W>
-__global__ void __launch_bounds__(kBlock, 8) k_spmv_dot_pby_ell(SellView<double> a, const double* __restrict__ z,
-                                                                const double* __restrict__ p, const double* beta,
+// partial of p.q per block. z is the cycle's own result (FP32 for the FP32
+// cycle: the conversion is exact). p_old and the matrix, which the kernels
+// just before do not write, are loaded ahead of the wait.
+template <class S, int W>
+__global__ void __launch_bounds__(kBlock, W <= 6 ? 6 : 5) k_spmv_dot_pby_ell(SellView<double> a, const S* z,
+                                                                const double* p, const double* beta,
                                                                 double* y, double* partials) {
-  FVM_PDL();
+  FVM_PDL_TRIGGER();
   const int i = blockIdx.x * kBlock + threadIdx.x;
-  const XPby pg{z, p, beta[0]};
-  double d = 0.0;
+  RowHead<double, W> h;
+  double pv = 0.0, d = 0.0;
   if (i < a.n) {
-    const double xi = pg(i);
-    const double yi = ell_row_g<double, W>(a, i, pg, a.diag[i] * xi);
-    y[i] = yi;
-    d = xi * yi;
+    h.load(a, (i >> 5) * (32 * W) + (i & 31), W);
+    d = a.diag[i];
+    pv = p[i];
   }
-  d = block_sum(d);
-  if (threadIdx.x == 0) partials[blockIdx.x] = d;
+  FVM_PDL_WAIT();
+  const XPby<S> pg{z, p, beta[0]};
+  double dot = 0.0;
+  if (i < a.n) {
+    const double xi = pv * pg.beta + (double)z[i];
+    const double yi = h.sum(W, pg, d * xi);
+    y[i] = yi;
+    dot = xi * yi;
+  }
+  dot = block_sum(dot);
+  if (threadIdx.x == 0) partials[blockIdx.x] = dot;
 }
 
-__global__ void __launch_bounds__(kBlock, 8) k_spmv_dot_pby(SellView<double> a, int nSlices,
-                                                            const double* __restrict__ z, const double* __restrict__ p,
-                                                            const double* beta, double* y, double* partials) {
+template <class S>
+__global__ void __launch_bounds__(kBlock, 4) k_spmv_dot_pby(SellView<double> a, int nSlices, const S* __restrict__ z,
+                                                            const double* __restrict__ p, const double* beta,
+                                                            double* y, double* partials) {
   FVM_PDL();
   const int lane = threadIdx.x & 31;
-  const XPby pg{z, p, beta[0]};
+  const XPby<S> pg{z, p, beta[0]};
   double d = 0.0;
   for (int s = blockIdx.x * kSlicesPerBlock + (threadIdx.x >> 5); s < nSlices; s += gridDim.x * kSlicesPerBlock) {
     const int4 m = slice_meta(a, s);
@@ -557,7 +691,7 @@ __global__ void __launch_bounds__(kBlock, 8) k_spmv_dot_pby(SellView<double> a, 
 }
 
 // the same over a SELL-32 level (grid-stride over slices)
-__global__ void __launch_bounds__(kBlock, 8) k_spmv_dot(SellView<double> a, int nSlices, const double* __restrict__ x,
+__global__ void __launch_bounds__(kBlock, 4) k_spmv_dot(SellView<double> a, int nSlices, const double* __restrict__ x,
                                                         double* y, double* partials) {
   FVM_PDL();
   const int lane = threadIdx.x & 31;
@@ -575,25 +709,15 @@ __global__ void __launch_bounds__(kBlock, 8) k_spmv_dot(SellView<double> a, int 
   if (threadIdx.x == 0) partials[blockIdx.x] = d;
 }
 
-// z <- src (as FP64), with block partials of r.z_old and r.z_new
+// block partials of (r, z), z the cycle's result, beside those of (r, z_old)
+// that the update left (pairs: z_old, z)
 template <class S>
-__global__ void k_cg_take_z(int n, const S* __restrict__ src, const double* __restrict__ r, double* z,
-                            double* partials) {
+__global__ void k_cg_dot_z(int n, const S* __restrict__ z, const double* __restrict__ r, double* partials) {
   FVM_PDL();
-  double a = 0.0, b = 0.0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const double ri = r[i];
-    const double zo = z[i];
-    const double zn = (double)src[i];
-    z[i] = zn;
-    a += ri * zo;
-    b += ri * zn;
-  }
-  block_sum2(a, b);
-  if (threadIdx.x == 0) {
-    partials[2 * blockIdx.x] = a;
-    partials[2 * blockIdx.x + 1] = b;
-  }
+  double b = 0.0;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) b += r[i] * (double)z[i];
+  b = block_sum(b);
+  if (threadIdx.x == 0) partials[2 * blockIdx.x + 1] = b;
 }
 
 // rho_prev <- rho, rho <- (r, z_new), beta (flexible: (rho - (r, z_old)) / rho_prev)
@@ -617,49 +741,72 @@ __global__ void k_cg_beta(int np, const double* __restrict__ p, double* rho, dou
 // alpha = rho / sum of the partials (p.Ap)
 __global__ void k_cg_alpha(int np, const double* __restrict__ p, const double* rho, double* alpha) {
   FVM_PDL();
+  // four loads in flight per thread, added in order
   double s = 0.0;
-  for (int i = threadIdx.x; i < np; i += blockDim.x) s += p[i];
+  const int bd = blockDim.x;
+  int i = threadIdx.x;
+  for (; i + 3 * bd < np; i += 4 * bd) {
+    const double a0 = p[i], a1 = p[i + bd], a2 = p[i + 2 * bd], a3 = p[i + 3 * bd];
+    s += a0;
+    s += a1;
+    s += a2;
+    s += a3;
+  }
+  for (; i < np; i += bd) s += p[i];
   s = block_sum(s);
   if (threadIdx.x == 0) alpha[0] = rho[0] / s;
 }
 
-// x += -alpha p; r += -alpha q; block partials of |r|
+// x += -alpha p; r += -alpha q; block partials of |r| and, for the next
+// flexible beta, of (r, z) with the new r and this iteration's z (pairs,
+// first entry)
+template <class S>
 __global__ void k_cg_update(int n, const double* alpha, const double* __restrict__ p, const double* __restrict__ q,
-                            double* x, double* r, double* partials, float* rF) {
+                            double* x, double* r, const S* __restrict__ z, double* partials, double* zPartials,
+                            float* rF) {
   FVM_PDL();
   const double am = -1.0 * alpha[0];
-  double l1 = 0.0;
+  double l1 = 0.0, rz = 0.0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     x[i] = x[i] + am * p[i];
     const double ri = r[i] + am * q[i];
     r[i] = ri;
     if (rF) rF[i] = (float)ri;
     l1 += fabs(ri);
+    rz += ri * (double)z[i];
   }
-  l1 = block_sum(l1);
-  if (threadIdx.x == 0) partials[blockIdx.x] = l1;
+  block_sum2(l1, rz);
+  if (threadIdx.x == 0) {
+    partials[blockIdx.x] = l1;
+    zPartials[2 * blockIdx.x] = rz;
+  }
 }
 
-// p = p_old * beta + z (written here), x += -alpha p; r += -alpha q; block
-// partials of |r|
-__global__ void k_cg_update_pby(int n, const double* alpha, const double* __restrict__ z, const double* beta,
-                                double* p, const double* __restrict__ q, double* x, double* r, double* partials,
-                                float* rF) {
+// the same with p = p_old * beta + z, written here
+template <class S>
+__global__ void k_cg_update_pby(int n, const double* alpha, const S* __restrict__ z, const double* beta, double* p,
+                                const double* __restrict__ q, double* x, double* r, double* partials,
+                                double* zPartials, float* rF) {
   FVM_PDL();
   const double am = -1.0 * alpha[0];
   const double b = beta[0];
-  double l1 = 0.0;
+  double l1 = 0.0, rz = 0.0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const double pi = p[i] * b + z[i];
+    const double zi = (double)z[i];
+    const double pi = p[i] * b + zi;
     p[i] = pi;
     x[i] = x[i] + am * pi;
     const double ri = r[i] + am * q[i];
     r[i] = ri;
     if (rF) rF[i] = (float)ri;
     l1 += fabs(ri);
+    rz += ri * zi;
   }
-  l1 = block_sum(l1);
-  if (threadIdx.x == 0) partials[blockIdx.x] = l1;
+  block_sum2(l1, rz);
+  if (threadIdx.x == 0) {
+    partials[blockIdx.x] = l1;
+    zPartials[2 * blockIdx.x] = rz;
+  }
 }
 
 // ---- SELL-32 smoothers with several threads per row (autotuned plans) ---------
@@ -670,31 +817,51 @@ __global__ void k_cg_update_pby(int n, const double* alpha, const double* __rest
 // exactly as row_sum's does.
 // Lanes of rows past the slice's last row (live = false) take part in the
 // shuffles but load nothing: their slots of the slice hold no entries.
-template <class T, int TPR, class X>
-__device__ __forceinline__ T row_sum_tpr(const SellView<T>& a, const int4 m, int l, bool live, const X& xg,
-                                         T sum) {
-  constexpr int C = 4;
-  const int lane = threadIdx.x & 31, sub = lane & (TPR - 1), g0 = lane & ~(TPR - 1);
-  const int o = m.z + l, w = m.w;
-  for (int k0 = 0; k0 < w; k0 += TPR * C) {
-    int c[C];
-    T v[C], p[C];
+constexpr int kTprChunk = 4;
+// a thread's entries of the chunk that starts at k0
+template <class T, int TPR>
+struct TprChunk {
+  int c[kTprChunk];
+  T v[kTprChunk];
+  __device__ __forceinline__ void load(const SellView<T>& a, const int4 m, int l, bool live, int k0) {
+    const int sub = threadIdx.x & (TPR - 1), o = m.z + l;
 #pragma unroll
-    for (int q = 0; q < C; q++) {
+    for (int q = 0; q < kTprChunk; q++) {
       const int k = k0 + q * TPR + sub;
-      const bool ok = live && k < w;
+      const bool ok = live && k < m.w;
       c[q] = ok ? a.cols[o + (k << 5)] : 0;
       v[q] = ok ? a.vals[o + (k << 5)] : T(0);
     }
+  }
+  __device__ __forceinline__ void prolonged(const int* __restrict__ ci) {
 #pragma unroll
-    for (int q = 0; q < C; q++) p[q] = v[q] * xg(c[q]);
+    for (int q = 0; q < kTprChunk; q++) c[q] = ci[c[q]];
+  }
+  template <class X>
+  __device__ __forceinline__ T sum(const int4 m, int k0, const X& xg, T s) const {
+    const int lane = threadIdx.x & 31, g0 = lane & ~(TPR - 1);
+    T p[kTprChunk];
 #pragma unroll
-    for (int q = 0; q < C; q++)
+    for (int q = 0; q < kTprChunk; q++) p[q] = v[q] * xg(c[q]);
+#pragma unroll
+    for (int q = 0; q < kTprChunk; q++)
 #pragma unroll
       for (int s2 = 0; s2 < TPR; s2++) {
         const T pv = __shfl_sync(0xffffffffu, p[q], g0 + s2);
-        if (k0 + q * TPR + s2 < w) sum = sum + pv;
+        if (k0 + q * TPR + s2 < m.w) s = s + pv;
       }
+    return s;
+  }
+};
+// the entries after the first chunk
+template <class T, int TPR, bool Pro, class X>
+__device__ __forceinline__ T tpr_rest(const SellView<T>& a, const int4 m, int l, bool live, const X& xg,
+                                      const int* __restrict__ ci, T sum) {
+  for (int k0 = TPR * kTprChunk; k0 < m.w; k0 += TPR * kTprChunk) {
+    TprChunk<T, TPR> h;
+    h.load(a, m, l, live, k0);
+    if constexpr (Pro) h.prolonged(ci);
+    sum = h.sum(m, k0, xg, sum);
   }
   return sum;
 }
@@ -708,8 +875,8 @@ __device__ __forceinline__ void tpr_row(int gw, int& sliceOffset, int& l) {
 
 template <class T, int TPR, int BLOCK>
 __global__ void __launch_bounds__(BLOCK) k_gs_color_tpr(SellView<T> a, int s0, int s1, T* x,
-                                                        const T* __restrict__ b) {
-  FVM_PDL();
+                                                        const T* b) {
+  FVM_PDL_TRIGGER();
   int so, l;
   tpr_row<TPR>(blockIdx.x * (BLOCK / 32) + (threadIdx.x >> 5), so, l);
   const int s = s0 + so;
@@ -717,32 +884,51 @@ __global__ void __launch_bounds__(BLOCK) k_gs_color_tpr(SellView<T> a, int s0, i
   const int4 m = a.meta[s];
   const bool live = l < m.y;
   const int i = m.x + (live ? l : 0);
-  const T sum = row_sum_tpr<T, TPR>(a, m, l, live, XDirect<T>{x}, live ? b[i] : T(0));
-  if (live && (threadIdx.x & (TPR - 1)) == 0) x[i] = -sum / a.diag[i];
+  TprChunk<T, TPR> h;
+  h.load(a, m, l, live, 0);
+  const T d = a.diag[i];
+  FVM_PDL_WAIT();
+  const XDirect<T> xg{x};
+  T sum = h.sum(m, 0, xg, live ? b[i] : T(0));
+  sum = tpr_rest<T, TPR, false>(a, m, l, live, xg, nullptr, sum);
+  if (live && (threadIdx.x & (TPR - 1)) == 0) x[i] = -sum / d;
 }
 
 // Pro: the pass right after a prolongation that would assign x = xc[ci]
 // reads those values from xc directly (xold unused)
 template <class T, int TPR, int BLOCK, bool Pro>
-__global__ void __launch_bounds__(BLOCK) k_jacobi_damped_tpr(SellView<T> a, int nSlices, const T* __restrict__ xold,
-                                                             T* xnew, const T* __restrict__ b, T w,
-                                                             const T* __restrict__ xc, const int* __restrict__ ci) {
-  FVM_PDL();
+__global__ void __launch_bounds__(BLOCK) k_jacobi_damped_tpr(SellView<T> a, int nSlices, const T* xold,
+                                                             T* xnew, const T* b, T w,
+                                                             const T* xc, const int* __restrict__ ci) {
+  FVM_PDL_TRIGGER();
   int s, l;
   tpr_row<TPR>(blockIdx.x * (BLOCK / 32) + (threadIdx.x >> 5), s, l);
   if (s >= nSlices) return;  // whole warp
   const int4 m = a.meta[s];
   const bool live = l < m.y;
   const int i = m.x + (live ? l : 0);
-  T sum;
-  if constexpr (Pro)
-    sum = row_sum_tpr<T, TPR>(a, m, l, live, XProlonged<T>{xc, ci}, live ? b[i] : T(0));
-  else
-    sum = row_sum_tpr<T, TPR>(a, m, l, live, XDirect<T>{xold}, live ? b[i] : T(0));
-  if (live && (threadIdx.x & (TPR - 1)) == 0) {
-    const T xo = Pro ? xc[ci[i]] : xold[i];
-    xnew[i] = xo + w * (-sum / a.diag[i] - xo);
+  TprChunk<T, TPR> h;
+  h.load(a, m, l, live, 0);
+  const T d = a.diag[i];
+  int own = i;
+  if constexpr (Pro) {
+    h.prolonged(ci);
+    own = ci[i];
   }
+  FVM_PDL_WAIT();
+  T sum = live ? b[i] : T(0), xo;
+  if constexpr (Pro) {
+    const XCoarse<T> xg{xc};
+    xo = xg(own);
+    sum = h.sum(m, 0, xg, sum);
+    sum = tpr_rest<T, TPR, true>(a, m, l, live, xg, ci, sum);
+  } else {
+    const XDirect<T> xg{xold};
+    xo = xg(own);
+    sum = h.sum(m, 0, xg, sum);
+    sum = tpr_rest<T, TPR, false>(a, m, l, live, xg, nullptr, sum);
+  }
+  if (live && (threadIdx.x & (TPR - 1)) == 0) xnew[i] = xo + w * (-sum / d - xo);
 }
 
 // Calls LAUNCH(TPR, BLOCK) for a supported plan; false otherwise.
@@ -777,14 +963,31 @@ __global__ void __launch_bounds__(BLOCK) k_jacobi_damped_tpr(SellView<T> a, int 
     }                                 \
   }()
 
+// one thread per coarse row; its first six fine rows ahead of the wait
 template <class T>
-__global__ void k_restrict(int nc, const int* __restrict__ c2fRow, const int* __restrict__ c2fCol,
-                           const T* __restrict__ r, T* bc, T* xc) {
-  FVM_PDL();
+__global__ void __launch_bounds__(kBlock) k_restrict(int nc, const int* __restrict__ c2fRow,
+                                                     const int* __restrict__ c2fCol, const T* r, T* bc,
+                                                     T* xc) {
+  FVM_PDL_TRIGGER();
+  constexpr int K = 6;
   const int I = blockIdx.x * blockDim.x + threadIdx.x;
+  int e0 = 0, e1 = 0, c[K];
+  if (I < nc) {
+    e0 = c2fRow[I];
+    e1 = c2fRow[I + 1];
+  }
+#pragma unroll
+  for (int k = 0; k < K; k++) c[k] = e0 + k < e1 ? c2fCol[e0 + k] : -1;
+  FVM_PDL_WAIT();
   if (I >= nc) return;
+  T v[K];
+#pragma unroll
+  for (int k = 0; k < K; k++) v[k] = c[k] >= 0 ? r[c[k]] : T(0);
   T s = T(0);
-  for (int k = c2fRow[I]; k < c2fRow[I + 1]; k++) s = s + r[c2fCol[k]];
+#pragma unroll
+  for (int k = 0; k < K; k++)
+    if (c[k] >= 0) s = s + v[k];
+  for (int k = e0 + K; k < e1; k++) s = s + r[c2fCol[k]];
   bc[I] = s;
   if (xc) xc[I] = T(0);
 }
@@ -811,11 +1014,12 @@ __global__ void __launch_bounds__(kBlock, 4) k_residual_restrict(SellView<T> a, 
 }
 
 template <class T>
-__global__ void k_prolong(int n, const int* __restrict__ ci, const T* __restrict__ xc, T* x, int assign) {
-  FVM_PDL();
+__global__ void k_prolong(int n, const int* __restrict__ ci, const T* xc, T* x, int assign) {
+  FVM_PDL_TRIGGER();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int c = i < n ? ci[i] : -1;
+  FVM_PDL_WAIT();
   if (i >= n) return;
-  const int c = ci[i];
   if (assign)
     x[i] = c >= 0 ? xc[c] : T(0);
   else if (c >= 0)
@@ -835,16 +1039,64 @@ __global__ void k_dense_solve(int n, const double* __restrict__ ainv, const T* _
   if (lane == 0) x[row] = (T)(-s);
 }
 
-__global__ void k_dense_solve_f32(int n, const float* __restrict__ ainv, const float* __restrict__ b,
-                                  float* x) {
-  FVM_PDL();
-  const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (row >= n) return;
-  float s = 0.0f;
-  for (int j = lane; j < n; j += 32) s += ainv[(size_t)row * n + j] * b[j];
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-  if (lane == 0) x[row] = -s;
+// x = -inv b with the FP32 inverse (row stride ld, a multiple of four,
+// columns past n zero). A CTA of four warps takes R rows; a thread holds K
+// float4 of each, loaded ahead of the wait: the inverse, the largest read of
+// a cycle's coarse levels (18 MB at 2151 rows), arrives in registers while
+// the restrictions above still run, and after the wait only b is read.
+// Measured against one warp per row reading the row after the wait: 2151
+// rows 10.5 -> 4 us in a cycle.
+template <int R, int K>
+__global__ void __launch_bounds__(128) k_dense_solve_f32(int n, int ld, const float* __restrict__ ainv,
+                                                         const float* b, float* x) {
+  FVM_PDL_TRIGGER();
+  __shared__ float part[4][R];
+  const int row0 = blockIdx.x * R, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  float4 v[R][K];
+#pragma unroll
+  for (int r = 0; r < R; r++)
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      const int c = 4 * (threadIdx.x + 128 * k);
+      v[r][k] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (c < ld && row0 + r < n) v[r][k] = *reinterpret_cast<const float4*>(ainv + (size_t)(row0 + r) * ld + c);
+    }
+  FVM_PDL_WAIT();
+  float s[R];
+#pragma unroll
+  for (int r = 0; r < R; r++) s[r] = 0.0f;
+#pragma unroll
+  for (int k = 0; k < K; k++) {
+    const int c = 4 * (threadIdx.x + 128 * k);
+    float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (c + 3 < n) {
+      q = *reinterpret_cast<const float4*>(b + c);
+    } else {
+      if (c < n) q.x = b[c];
+      if (c + 1 < n) q.y = b[c + 1];
+      if (c + 2 < n) q.z = b[c + 2];
+    }
+#pragma unroll
+    for (int r = 0; r < R; r++) s[r] += (v[r][k].x * q.x + v[r][k].y * q.y) + (v[r][k].z * q.z + v[r][k].w * q.w);
+  }
+#pragma unroll
+  for (int r = 0; r < R; r++) {
+    for (int o = 16; o > 0; o >>= 1) s[r] += __shfl_down_sync(0xffffffffu, s[r], o);
+    if (lane == 0) part[w][r] = s[r];
+  }
+  __syncthreads();
+  if (threadIdx.x < R && row0 + (int)threadIdx.x < n) {
+    const int r = threadIdx.x;
+    x[row0 + r] = -((part[0][r] + part[1][r]) + (part[2][r] + part[3][r]));
+  }
+}
+
+// the FP32 copy of an n x n FP64 inverse, row stride ld, padding zero
+__global__ void k_inverse_f32(int n, int ld, const double* __restrict__ a, float* b) {
+  const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= (size_t)n * ld) return;
+  const int i = (int)(e / ld), j = (int)(e % ld);
+  b[e] = j < n ? (float)a[(size_t)i * n + j] : 0.0f;
 }
 
 // Blocked in-place Gauss-Jordan inversion with partial (row) pivoting.
@@ -1012,20 +1264,25 @@ __global__ void k_l1_partials(int n, const double* __restrict__ a, double* parti
   if (threadIdx.x == 0) partials[blockIdx.x] = s;
 }
 // The start of a CG solve from x = 0: r = b + A x is b itself. r, its FP32
-// copy (the FP32 cycle's right-hand side; null: none) and the |r|_1
-// partials in k_l1_partials' layout, in one pass over b.
+// copy (the FP32 cycle's right-hand side; null: none), x = p = 0 and the
+// |r|_1 partials in k_l1_partials' layout, in one pass over b.
 __global__ void k_cg_start(int n, const double* __restrict__ b, double* __restrict__ r, float* __restrict__ rF,
-                           double* partials) {
+                           double* __restrict__ x, double* __restrict__ p, double* partials, double* zPartials) {
   FVM_PDL();
   double s = 0.0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const double v = b[i];
     r[i] = v;
     if (rF) rF[i] = (float)v;
+    x[i] = 0.0;
+    p[i] = 0.0;
     s += fabs(v);
   }
   s = block_sum(s);
-  if (threadIdx.x == 0) partials[blockIdx.x] = s;
+  if (threadIdx.x == 0) {
+    partials[blockIdx.x] = s;
+    zPartials[2 * blockIdx.x] = 0.0;  // (r, z_old) of the first beta
+  }
 }
 __global__ void k_dot_partials(int n, const double* __restrict__ a, const double* __restrict__ b,
                                double* partials) {
@@ -1414,9 +1671,9 @@ void jacobi_damped(const SellView<T>& a, int nSlices, const T* xold, T* xnew, co
 #undef FVM_P
   }
   if (pro)
-    pdl_launch(k_jacobi_damped<T, true>, reduce_blocks(nSlices), kBlock, st, a, nSlices, xold, xnew, b, w, xc, ci);
+    pdl_launch(k_jacobi_damped<T, true>, ceil_div(nSlices, kSlicesPerBlock), kBlock, st, a, nSlices, xold, xnew, b, w, xc, ci);
   else
-    pdl_launch(k_jacobi_damped<T, false>, reduce_blocks(nSlices), kBlock, st, a, nSlices, xold, xnew, b, w, xc, ci);
+    pdl_launch(k_jacobi_damped<T, false>, ceil_div(nSlices, kSlicesPerBlock), kBlock, st, a, nSlices, xold, xnew, b, w, xc, ci);
 }
 template <class T>
 void chebyshev_step(const SellView<T>& a, int nSlices, const T* x, T* xnew, T* dv, const T* b, T c1, T c2,
@@ -1481,23 +1738,23 @@ void spmv_dot(const SellView<double>& a, int nSlices, const double* x, double* y
 #undef FVM_L
   pdl_launch(k_spmv_dot, reduce_blocks(nSlices), kBlock, st, a, nSlices, x, y, partials);
 }
-void spmv_dot_pby(const SellView<double>& a, int nSlices, const double* z, const double* p, const double* beta,
-                  double* y, double* partials, cudaStream_t st) {
-#define FVM_L(W) pdl_launch(k_spmv_dot_pby_ell<W>, ceil_div(a.n, kBlock), kBlock, st, a, z, p, beta, y, partials)
+template <class S>
+void spmv_dot_pby(const SellView<double>& a, int nSlices, const S* z, const double* p, const double* beta, double* y,
+                  double* partials, cudaStream_t st) {
+#define FVM_L(W) pdl_launch(k_spmv_dot_pby_ell<S, W>, ceil_div(a.n, kBlock), kBlock, st, a, z, p, beta, y, partials)
   if (a.ellWidth && FVM_ELL_SWITCH(a.ellWidth, FVM_L)) return;
 #undef FVM_L
-  pdl_launch(k_spmv_dot_pby, reduce_blocks(nSlices), kBlock, st, a, nSlices, z, p, beta, y, partials);
-}
-void cg_update_pby(int n, const double* alpha, const double* z, const double* beta, double* p, const double* q,
-                   double* x, double* r, double* partials, cudaStream_t st, float* rF) {
-  pdl_launch(k_cg_update_pby, vec_blocks(n), kBlock, st, n, alpha, z, beta, p, q, x, r, partials, rF);
+  pdl_launch(k_spmv_dot_pby<S>, reduce_blocks(nSlices), kBlock, st, a, nSlices, z, p, beta, y, partials);
 }
 template <class S>
-void cg_take_z(int n, const S* src, const double* r, double* z, double* partials, cudaStream_t st) {
-  pdl_launch(k_cg_take_z<S>, vec_blocks(n), kBlock, st, n, src, r, z, partials);
+void cg_update_pby(int n, const double* alpha, const S* z, const double* beta, double* p, const double* q, double* x,
+                   double* r, double* partials, double* zPartials, cudaStream_t st, float* rF) {
+  pdl_launch(k_cg_update_pby<S>, vec_blocks(n), kBlock, st, n, alpha, z, beta, p, q, x, r, partials, zPartials, rF);
 }
-template void cg_take_z<float>(int, const float*, const double*, double*, double*, cudaStream_t);
-template void cg_take_z<double>(int, const double*, const double*, double*, double*, cudaStream_t);
+template <class S>
+void cg_dot_z(int n, const S* z, const double* r, double* partials, cudaStream_t st) {
+  pdl_launch(k_cg_dot_z<S>, vec_blocks(n), kBlock, st, n, z, r, partials);
+}
 void cg_beta(int np, const double* partials, double* rho, double* rhoPrev, double* beta, bool flexible,
              cudaStream_t st) {
   pdl_launch(k_cg_beta, 1, 1024, st, np, partials, rho, rhoPrev, beta, flexible ? 1 : 0);
@@ -1505,10 +1762,22 @@ void cg_beta(int np, const double* partials, double* rho, double* rhoPrev, doubl
 void cg_alpha(int np, const double* partials, const double* rho, double* alpha, cudaStream_t st) {
   pdl_launch(k_cg_alpha, 1, 1024, st, np, partials, rho, alpha);
 }
-void cg_update(int n, const double* alpha, const double* p, const double* q, double* x, double* r, double* partials,
-               cudaStream_t st, float* rF) {
-  pdl_launch(k_cg_update, vec_blocks(n), kBlock, st, n, alpha, p, q, x, r, partials, rF);
+template <class S>
+void cg_update(int n, const double* alpha, const double* p, const double* q, double* x, double* r, const S* z,
+               double* partials, double* zPartials, cudaStream_t st, float* rF) {
+  pdl_launch(k_cg_update<S>, vec_blocks(n), kBlock, st, n, alpha, p, q, x, r, z, partials, zPartials, rF);
 }
+template void cg_update<double>(int, const double*, const double*, const double*, double*, double*, const double*,
+                                double*, double*, cudaStream_t, float*);
+#define FVM_CG_STEP(S)                                                                                               \
+  template void spmv_dot_pby<S>(const SellView<double>&, int, const S*, const double*, const double*, double*,       \
+                                double*, cudaStream_t);                                                              \
+  template void cg_update_pby<S>(int, const double*, const S*, const double*, double*, const double*, double*,       \
+                                 double*, double*, double*, cudaStream_t, float*);                                   \
+  template void cg_dot_z<S>(int, const S*, const double*, double*, cudaStream_t);
+FVM_CG_STEP(float)
+FVM_CG_STEP(double)
+#undef FVM_CG_STEP
 template <class T>
 void restrict_sum(int nc, const int* c2fRow, const int* c2fCol, const T* r, T* bc, cudaStream_t st) {
   pdl_launch(k_restrict<T>, ceil_div(nc, kBlock), kBlock, st, nc, c2fRow, c2fCol, r, bc, (T*)nullptr);
@@ -1539,8 +1808,28 @@ template <class T>
 void dense_solve(int n, const double* ainv, const T* b, T* x, cudaStream_t st) {
   pdl_launch(k_dense_solve<T>, ceil_div(n, kBlock / 32), kBlock, st, n, ainv, b, x);
 }
+int inverse_f32_stride(int n) { return (n + 3) / 4 * 4; }
+void inverse_to_f32(int n, const double* a, float* b, cudaStream_t st) {
+  const int ld = inverse_f32_stride(n);
+  k_inverse_f32<<<ceil_div((long long)n * ld, kBlock), kBlock, 0, st>>>(n, ld, a, b);
+}
 void dense_solve_f32(int n, const float* ainv, const float* b, float* x, cudaStream_t st) {
-  pdl_launch(k_dense_solve_f32, ceil_div(n, kBlock / 32), kBlock, st, n, ainv, b, x);
+  const int ld = inverse_f32_stride(n);
+  // K float4 per thread and row (n <= 4096: at most 8), as many rows as 64
+  // registers hold
+#define FVM_D(K, R) \
+  case K: pdl_launch(k_dense_solve_f32<R, K>, ceil_div(n, R), 128, st, n, ld, ainv, b, x); break
+  switch (ceil_div(ld, 512)) {
+    FVM_D(1, 4);
+    FVM_D(2, 4);
+    FVM_D(3, 4);
+    FVM_D(4, 4);
+    FVM_D(5, 3);
+    FVM_D(6, 2);
+    FVM_D(7, 2);
+    default: pdl_launch(k_dense_solve_f32<2, 8>, ceil_div(n, 2), 128, st, n, ld, ainv, b, x);
+  }
+#undef FVM_D
 }
 namespace {
 constexpr int kGjMaxPanel = 8;
@@ -1941,8 +2230,9 @@ int vec_blocks(int n) {
 void l1_partials(int n, const double* a, double* partials, cudaStream_t st) {
   pdl_launch(k_l1_partials, vec_blocks(n), kBlock, st, n, a, partials);
 }
-void cg_start(int n, const double* b, double* r, float* rF, double* partials, cudaStream_t st) {
-  pdl_launch(k_cg_start, vec_blocks(n), kBlock, st, n, b, r, rF, partials);
+void cg_start(int n, const double* b, double* r, float* rF, double* x, double* p, double* partials, double* zPartials,
+              cudaStream_t st) {
+  pdl_launch(k_cg_start, vec_blocks(n), kBlock, st, n, b, r, rF, x, p, partials, zPartials);
 }
 void dot_partials(int n, const double* a, const double* b, double* partials, cudaStream_t st) {
   pdl_launch(k_dot_partials, vec_blocks(n), kBlock, st, n, a, b, partials);

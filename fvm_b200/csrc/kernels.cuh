@@ -88,15 +88,19 @@ int reduce_blocks(int nSlices);  // grid of the SELL-32 whole-level row kernels
 int spmv_dot_blocks(const SellView<double>& a, int nSlices);
 void spmv_dot(const SellView<double>& a, int nSlices, const double* x, double* y, double* partials, cudaStream_t st);
 // the same with p = p_old * beta + z formed on the fly (spmv_dot_blocks
-// partials); cg_update_pby then writes that p and updates x and r
-void spmv_dot_pby(const SellView<double>& a, int nSlices, const double* z, const double* p, const double* beta,
-                  double* y, double* partials, cudaStream_t st);
-void cg_update_pby(int n, const double* alpha, const double* z, const double* beta, double* p, const double* q,
-                   double* x, double* r, double* partials, cudaStream_t st, float* rF = nullptr);
-// z <- src (converted to FP64) with per-block partials of r.z_old and
-// r.z_new (interleaved, vec_blocks(n) pairs)
+// partials), z the cycle's result in its own precision; cg_update_pby then
+// writes that p and updates x and r
 template <class S>
-void cg_take_z(int n, const S* src, const double* r, double* z, double* partials, cudaStream_t st);
+void spmv_dot_pby(const SellView<double>& a, int nSlices, const S* z, const double* p, const double* beta, double* y,
+                  double* partials, cudaStream_t st);
+template <class S>
+void cg_update_pby(int n, const double* alpha, const S* z, const double* beta, double* p, const double* q, double* x,
+                   double* r, double* partials, double* zPartials, cudaStream_t st, float* rF = nullptr);
+// per-block partials of (r, z) into the second entries of the pairs
+// (r, z_old), (r, z) (vec_blocks(n) of them); the first entries are those
+// cg_update(_pby) left in zPartials, with the new r and its iteration's z
+template <class S>
+void cg_dot_z(int n, const S* z, const double* r, double* partials, cudaStream_t st);
 // from those pairs: *rhoPrev <- *rho, *rho <- (r, z_new), *beta <- *rho /
 // *rhoPrev, or with flexible (Polak-Ribiere) (*rho - (r, z_old)) / *rhoPrev
 void cg_beta(int np, const double* partials, double* rho, double* rhoPrev, double* beta, bool flexible,
@@ -106,8 +110,9 @@ void cg_alpha(int np, const double* partials, const double* rho, double* alpha, 
 // x += -alpha p, r += -alpha q, and per-block L1 partials of the new r
 // (vec_blocks(n) of them); rF (optional) gets the new r in FP32, the
 // right-hand side of the next FP32 cycle
-void cg_update(int n, const double* alpha, const double* p, const double* q, double* x, double* r, double* partials,
-               cudaStream_t st, float* rF = nullptr);
+template <class S>
+void cg_update(int n, const double* alpha, const double* p, const double* q, double* x, double* r, const S* z,
+               double* partials, double* zPartials, cudaStream_t st, float* rF = nullptr);
 // number of L1 partials residual() writes for a level (one per block)
 int residual_partials(int nSlices, int n, int ellWidth);
 
@@ -148,7 +153,10 @@ void prolong(int n, const int* ci, const T* xc, T* x, cudaStream_t st, bool assi
 // x = -Ainv b with a dense FP64 inverse (n x n, row-major)
 template <class T>
 void dense_solve(int n, const double* ainv, const T* b, T* x, cudaStream_t st);
-// same with an FP32 copy of the inverse (half the bytes; FP32 V-cycle)
+// same with an FP32 copy of the inverse (half the bytes; FP32 V-cycle), whose
+// rows are inverse_f32_stride(n) apart, zero past column n; n <= 4096
+int inverse_f32_stride(int n);
+void inverse_to_f32(int n, const double* a, float* b, cudaStream_t st);
 void dense_solve_f32(int n, const float* ainv, const float* b, float* x, cudaStream_t st);
 // Inverse of the dense n x n matrix `a` (row-major, FP64, device;
 // overwritten) by blocked in-place Gauss-Jordan elimination with partial
@@ -180,7 +188,8 @@ void dot_partials(int n, const double* a, const double* b, double* partials, cud
 void sum_partials(int np, const double* partials, double* out, cudaStream_t st);
 // r = b (the residual at x = 0), rF = (float) b when rF is not null, and the
 // |b|_1 partials of l1_partials (vec_blocks(n) of them)
-void cg_start(int n, const double* b, double* r, float* rF, double* partials, cudaStream_t st);
+void cg_start(int n, const double* b, double* r, float* rF, double* x, double* p, double* partials, double* zPartials,
+              cudaStream_t st);
 // scalar recurrences for the Krylov solvers, all on the device:
 // out = num / den (out, num, den are device scalars)
 void scalar_div(const double* num, const double* den, double* out, cudaStream_t st);

@@ -237,7 +237,7 @@ void AmgHierarchy::build(std::vector<RefLevel>& levels, int finestLocalSize, con
       gjStatus = (int*)arena_.alloc(sizeof(int));
       CUDA_OK(cudaMemsetAsync(const_cast<int*>(gjStatus), 0, sizeof(int), gjStream));
       if (mixed)
-        coarseInvF_ = (float*)arena_.alloc(sizeof(float) * nn);
+        coarseInvF_ = (float*)arena_.alloc(sizeof(float) * (size_t)c.n * dev::inverse_f32_stride(c.n));
       else
         coarseInv_ = (double*)arena_.alloc(sizeof(double) * nn);
       dev::inverse_symmetric(lv_[l].view64(), lv_[l].rowSlice, nullptr, coarseInv_, coarseInvF_,
@@ -300,9 +300,8 @@ void AmgHierarchy::build(std::vector<RefLevel>& levels, int finestLocalSize, con
       FVM_REQUIRE(singular == 0, kBadArgument, "singular coarsest-level matrix");
     }
     if (mixed && !coarseInvF_) {
-      const size_t nn = (size_t)coarseN * coarseN;
-      coarseInvF_ = (float*)arena_.alloc(sizeof(float) * nn);
-      dev::cast_d2f(nn, coarseInv_, coarseInvF_, 0);
+      coarseInvF_ = (float*)arena_.alloc(sizeof(float) * (size_t)coarseN * dev::inverse_f32_stride(coarseN));
+      dev::inverse_to_f32(coarseN, coarseInv_, coarseInvF_, 0);
     }
     CUDA_OK(cudaDeviceSynchronize());
     lap(gjUnpivoted ? "coarsest inverse (unpivoted)" : "coarsest inverse");
@@ -1676,12 +1675,10 @@ SolveReport LinearSolve::solveCG(cudaStream_t st) {
     fprintf(stderr, "[fvm solve] CG on the host loop (learned step %s, graphs %s, loop graph %s)\n",
             learned_ && learnedActive_ ? "active" : "inactive", graphsFailed_ ? "failed" : "ok",
             loopFailed_ ? "failed" : "ok");
-  CUDA_OK(cudaMemsetAsync(X, 0, sizeof(double) * (size_t)n_, st));
-  CUDA_OK(cudaMemsetAsync(P, 0, sizeof(double) * (size_t)n_, st));
-  CUDA_OK(cudaMemsetAsync(Z, 0, sizeof(double) * (size_t)n_, st));  // z_0 enters the first flexible beta
+  CUDA_OK(cudaMemsetAsync(Z, 0, sizeof(double) * (size_t)n_, st));  // (Jacobi: z_0 enters the first flexible beta)
   dev::copy_d(n_, d.b, B, st);
   // r = b at x = 0, with its norm (the FP32 copy below, when the cycle takes it)
-  dev::cg_start(n_, B, R, nullptr, partials_, st);
+  dev::cg_start(n_, B, R, nullptr, X, P, partials_, partials2_, st);
   dev::sum_partials(dev::vec_blocks(n_), partials_, scal_ + kNorm, st);
   {
     const double inf = std::numeric_limits<double>::infinity();
@@ -1734,12 +1731,12 @@ SolveReport LinearSolve::solveCG(cudaStream_t st) {
         nn::step_trial(n_, R1, Q2, scal_ + kLsAlpha, RT, partials_, st);
         dev::sum_partials(dev::vec_blocks(n_), partials_, scal_ + kLsTrial, st);
         k_combine<<<gb, 256, 0, st>>>(n_, D1, scal_ + kLsAlpha, DN, D1);
-        dev::cg_take_z<double>(n_, D1, R, Z, partials2_, st);
+        dev::cg_dot_z<double>(n_, D1, R, partials2_, st);
         dev::cg_beta(dev::vec_blocks(n_), partials2_, scal_ + kRho, scal_ + kRhoPrev, scal_ + kBeta, flexible, st);
-        dev::xpby_dev(n_, Z, scal_ + kBeta, P, st);
+        dev::xpby_dev(n_, D1, scal_ + kBeta, P, st);
         dev::spmv_dot(d.view64(), d.nSlices, P, Q, partials2_, st);
         dev::cg_alpha(dev::spmv_dot_blocks(d.view64(), d.nSlices), partials2_, scal_ + kRho, scal_ + kAlpha, st);
-        dev::cg_update(n_, scal_ + kAlpha, P, Q, X, R, partials_, st, rF);
+        dev::cg_update<double>(n_, scal_ + kAlpha, P, Q, X, R, D1, partials_, partials2_, st, rF);
         dev::sum_partials(dev::vec_blocks(n_), partials_, scal_ + kNorm, st);
         CUDA_OK(cudaMemcpyAsync(hostScal_, scal_ + kNorm, sizeof(double), cudaMemcpyDeviceToHost, st));
         CUDA_OK(cudaMemcpyAsync(hostScal_ + 1, scal_ + kLsBefore, sizeof(double), cudaMemcpyDeviceToHost, st));
@@ -1753,13 +1750,9 @@ SolveReport LinearSolve::solveCG(cudaStream_t st) {
         else
           h_.applyCycle(R, st);
         if (mixedCycle)
-          dev::cg_take_z<float>(n_, d.xF, R, Z, partials2_, st);
+          cgStep<float>(d.xF, R, P, Q, X, flexible, rF, st);
         else
-          dev::cg_take_z<double>(n_, d.x, R, Z, partials2_, st);
-        dev::cg_beta(dev::vec_blocks(n_), partials2_, scal_ + kRho, scal_ + kRhoPrev, scal_ + kBeta, flexible, st);
-        dev::spmv_dot_pby(d.view64(), d.nSlices, Z, P, scal_ + kBeta, Q, partials2_, st);
-        dev::cg_alpha(dev::spmv_dot_blocks(d.view64(), d.nSlices), partials2_, scal_ + kRho, scal_ + kAlpha, st);
-        dev::cg_update_pby(n_, scal_ + kAlpha, Z, scal_ + kBeta, P, Q, X, R, partials_, st, rF);
+          cgStep<double>(d.x, R, P, Q, X, flexible, rF, st);
         dev::sum_partials(dev::vec_blocks(n_), partials_, scal_ + kNorm, st);
         CUDA_OK(cudaMemcpyAsync(hostScal_, scal_ + kNorm, sizeof(double), cudaMemcpyDeviceToHost, st));
       });
@@ -1961,20 +1954,16 @@ bool LinearSolve::addDeviceLoop(cudaGraph_t g, cudaStream_t st, bool hostCopies)
   double* R = work_ + (size_t)n_;
   const int vb = dev::vec_blocks(n_);
   if (o.solver == kSolverCG) {
-    double* Z = work_ + 2 * (size_t)n_;
     double* P = work_ + 3 * (size_t)n_;
     double* Q = work_ + 4 * (size_t)n_;
     double* B = own ? d.b : work_ + 5 * (size_t)n_;
     return addLoop(
         g, st, o.nMaxIterations, true,
         [&] {
-          // x = 0, p = 0, z = 0, r = b, |r| (b kept in B)
-          CUDA_OK(cudaMemsetAsync(X, 0, nb, st));
-          CUDA_OK(cudaMemsetAsync(P, 0, nb, st));
-          CUDA_OK(cudaMemsetAsync(Z, 0, nb, st));
+          // x = 0, p = 0, r = b at x = 0 with its norm and the FP32 cycle's
+          // right-hand side (b kept in B)
           if (B != d.b) dev::copy_d(n_, d.b, B, st);
-          // r = b at x = 0, with its norm and the FP32 cycle's right-hand side
-          dev::cg_start(n_, B, R, mixedCycle ? d.bF : nullptr, partials_, st);
+          dev::cg_start(n_, B, R, mixedCycle ? d.bF : nullptr, X, P, partials_, partials2_, st);
           dev::sum_partials(vb, partials_, scal_ + kNorm, st);
         },
         nullptr,
@@ -1986,16 +1975,9 @@ bool LinearSolve::addDeviceLoop(cudaGraph_t g, cudaStream_t st, bool hostCopies)
           else
             h_.applyCycle(R, st);
           if (mixedCycle)
-            dev::cg_take_z<float>(n_, d.xF, R, Z, partials2_, st);
+            cgStep<float>(d.xF, R, P, Q, X, cgFlexible(), d.bF, st);
           else
-            dev::cg_take_z<double>(n_, d.x, R, Z, partials2_, st);
-          dev::cg_beta(vb, partials2_, scal_ + kRho, scal_ + kRhoPrev, scal_ + kBeta, cgFlexible(), st);
-          // p = p * beta + z is formed by the SpMV where it reads p and written
-          // by the update: no pass of its own
-          dev::spmv_dot_pby(d.view64(), d.nSlices, Z, P, scal_ + kBeta, Q, partials2_, st);
-          dev::cg_alpha(dev::spmv_dot_blocks(d.view64(), d.nSlices), partials2_, scal_ + kRho, scal_ + kAlpha, st);
-          dev::cg_update_pby(n_, scal_ + kAlpha, Z, scal_ + kBeta, P, Q, X, R, partials_, st,
-                             mixedCycle ? d.bF : nullptr);
+            cgStep<double>(d.x, R, P, Q, X, cgFlexible(), nullptr, st);
         },
         vb, partials_,
         [&] {
@@ -2038,6 +2020,21 @@ bool LinearSolve::addDeviceLoop(cudaGraph_t g, cudaStream_t st, bool hostCopies)
         dev::copy_d(n_, B, d.b, st);
         copies();
       });
+}
+
+// A CG iteration after its cycle, z the cycle's result where the cycle left
+// it: (r, z), beta, q = A p, alpha, the updates. p = p * beta + z is formed
+// by the SpMV where it reads p and written by the update; (r_new, z) for the
+// next flexible beta is summed there too, so z is never copied.
+template <class S>
+void LinearSolve::cgStep(const S* z, double* R, double* P, double* Q, double* X, bool flexible, float* rF,
+                         cudaStream_t st) {
+  const DevLevel& d = h_.level(0);
+  dev::cg_dot_z<S>(n_, z, R, partials2_, st);
+  dev::cg_beta(dev::vec_blocks(n_), partials2_, scal_ + kRho, scal_ + kRhoPrev, scal_ + kBeta, flexible, st);
+  dev::spmv_dot_pby<S>(d.view64(), d.nSlices, z, P, scal_ + kBeta, Q, partials2_, st);
+  dev::cg_alpha(dev::spmv_dot_blocks(d.view64(), d.nSlices), partials2_, scal_ + kRho, scal_ + kAlpha, st);
+  dev::cg_update_pby<S>(n_, scal_ + kAlpha, z, scal_ + kBeta, P, Q, X, R, partials_, partials2_, st, rF);
 }
 
 // The two halves of a BiCGStab iteration; each ends with the partial sums of

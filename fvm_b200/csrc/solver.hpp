@@ -434,6 +434,8 @@ class LinearSolve {
   bool addLoop(cudaGraph_t g, cudaStream_t st, int maxIt, bool testFirst, const std::function<void()>& prologue,
                const std::function<void()>& half, const std::function<void()>& iteration, int np,
                const double* partials, const std::function<void()>& epilogue);
+  template <class S>
+  void cgStep(const S* z, double* R, double* P, double* Q, double* X, bool flexible, float* rF, cudaStream_t st);
   void bcgFirst(double* R, double* RT, double* V, double* P, double* PH, double* X, cudaStream_t st);
   void bcgSecond(double* R, double* Tt, double* SH, double* X, cudaStream_t st);
   int historyCap_ = 0;
