@@ -9,6 +9,7 @@
 // channel, so a neighbour's activations are one coalesced 128-byte load.
 // The graph is the finest level's SELL-32 matrix (neighbours j of row i:
 // its stored columns, padding entries carry a zero coupling).
+#include <algorithm>
 #include <cmath>
 #include <stdexcept>
 
@@ -34,6 +35,33 @@ int node_blocks(int n) {
   return b < 148 * 16 ? (b < 1 ? 1 : b) : 148 * 16;
 }
 
+// Every kernel of a pass lets the next one start (its launch, TMEM and
+// shared-memory set-up) and waits for all before it ahead of its first read
+// of anything a pass writes. Pointers to what a pass writes carry no
+// __restrict__ here: such loads may be moved above the wait.
+#define NN_PDL_TRIGGER() asm volatile("griddepcontrol.launch_dependents;" ::: "memory")
+#define NN_PDL_WAIT() asm volatile("griddepcontrol.wait;" ::: "memory")
+#define NN_PDL()      \
+  do {                \
+    NN_PDL_TRIGGER(); \
+    NN_PDL_WAIT();    \
+  } while (0)
+
+template <typename... KArgs, typename... Args>
+void launch(void (*kernel)(KArgs...), int grid, int block, size_t smem, cudaStream_t st, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
 __device__ __forceinline__ float relu(float x) { return x > 0.f ? x : 0.f; }
 
 __device__ __forceinline__ double block_sum(double v) {
@@ -49,39 +77,37 @@ __device__ __forceinline__ double block_sum(double v) {
   return s;
 }
 
-// sum_i |r_i| / |a_ii| per block (input scale)
-__global__ void k_scale_partials(int n, const double* __restrict__ r, const double* __restrict__ diag,
-                                 double* partials) {
-  double s = 0.0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    s += fabs(r[i]) / fabs(diag[i]);
-  s = block_sum(s);
-  if (threadIdx.x == 0) partials[blockIdx.x] = s;
-}
-
 // sum_i e_i^2 per block
 __global__ void k_sq_partials(int n, const double* __restrict__ e, double* partials) {
+  NN_PDL();
   double s = 0.0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) s += e[i] * e[i];
   s = block_sum(s);
   if (threadIdx.x == 0) partials[blockIdx.x] = s;
 }
 
-// u_i = r_i / (|a_ii| s), s = sum / n; s stored as scal[0] = sum / n
-__global__ void k_input(int n, const double* __restrict__ r, const double* __restrict__ diag,
-                        const double* __restrict__ sum, float* u, double* scale) {
+// u_i = r_i / (|a_ii| s), s = sum / n (stored as scale[0]), and the encoder's
+// h0_i = relu(we u_i + be): a warp takes 8 nodes, lane q < 8 forms u of node q
+__global__ void __launch_bounds__(kBlock) k_encode(int n, const double* r, const double* __restrict__ diag,
+                                                   const double* sum, const float* P, float* u, double* scale,
+                                                   float* H0) {
+  NN_PDL();
+  const int lane = threadIdx.x & 31;
+  const int i0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 8;
   const double s = sum[0] / (double)n;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i == 0) scale[0] = s;
-  if (i >= n) return;
-  u[i] = s > 0.0 ? (float)(r[i] / (fabs(diag[i]) * s)) : 0.f;
-}
-
-__global__ void k_encode(int n, const float* __restrict__ u, const float* __restrict__ P, float* H0) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (long long)n * 32) return;
-  const int i = (int)(t >> 5), c = (int)(t & 31);
-  H0[t] = relu(__fmaf_rn(P[kEncW + c], u[i], P[kEncB + c]));
+  if (i0 == 0 && lane == 0) scale[0] = s;
+  if (i0 >= n) return;
+  const float w = P[kEncW + lane], b = P[kEncB + lane];
+  float ui = 0.f;
+  if (lane < 8 && i0 + lane < n) {
+    ui = s > 0.0 ? (float)(r[i0 + lane] / (fabs(diag[i0 + lane]) * s)) : 0.f;
+    u[i0 + lane] = ui;
+  }
+#pragma unroll
+  for (int q = 0; q < 8; q++) {
+    const float uq = __shfl_sync(kFull, ui, q);
+    if (i0 + q < n) H0[(size_t)(i0 + q) * 32 + lane] = relu(__fmaf_rn(w, uq, b));
+  }
 }
 
 struct GraphArgs {
@@ -94,18 +120,30 @@ struct GraphArgs {
   const float* wb;  // per stored entry (i, j): |a_ij| / |a_jj| (its transpose's weight)
 };
 
-// The message weights of every stored entry, computed once per pass (the
-// same FP64 quotient rounded to FP32 that the layers used to form inline).
-__global__ void k_edge_weights(int nSlices, const int4* __restrict__ meta, const int* __restrict__ cols,
-                               const double* __restrict__ vals, const double* __restrict__ diag, float* wf,
-                               float* wb) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int s = t >> 5, lane = t & 31;
-  if (s >= nSlices) return;
-  const int4 m = meta[s];
+// The start of a pass, two independent parts in one launch: blocks below
+// scaleBlocks sum |r_i| / |a_ii| (input scale, one partial each); the others
+// compute the message weights of every stored entry (the same FP64 quotient
+// rounded to FP32 that the layers used to form inline), warp w of them
+// taking every fourth entry of the rows of slice w / 4.
+__global__ void __launch_bounds__(kBlock) k_pass_start(int n, const double* r, int scaleBlocks, double* partials,
+                                                       int nSlices, const int4* __restrict__ meta,
+                                                       const int* __restrict__ cols, const double* vals,
+                                                       const double* diag, float* wf, float* wb) {
+  NN_PDL();
+  if (blockIdx.x < scaleBlocks) {
+    double s = 0.0;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += scaleBlocks * blockDim.x)
+      s += fabs(r[i]) / fabs(diag[i]);
+    s = block_sum(s);
+    if (threadIdx.x == 0) partials[blockIdx.x] = s;
+    return;
+  }
+  const int w = ((blockIdx.x - scaleBlocks) * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (w >= 4 * nSlices) return;
+  const int4 m = meta[w >> 2];
   if (lane >= m.y) return;
   const double di = fabs(diag[m.x + lane]);
-  for (int k = 0; k < m.w; k++) {
+  for (int k = w & 3; k < m.w; k += 4) {
     const int e = m.z + (k << 5) + lane;
     const double a = fabs(vals[e]);
     wf[e] = (float)(a / di);
@@ -115,8 +153,8 @@ __global__ void k_edge_weights(int nSlices, const int4* __restrict__ meta, const
 
 // sum_k w[e_k] X[j_k][lane] over the entries e_k = base + 32 k (k < width)
 // of one row, in stored order, with the loads of four entries in flight
-__device__ __forceinline__ float gather_row(const int* __restrict__ cols, const float* __restrict__ w, int base,
-                                            int width, const float* __restrict__ X, int lane, float acc) {
+__device__ __forceinline__ float gather_row(const int* __restrict__ cols, const float* w, int base, int width,
+                                            const float* X, int lane, float acc) {
   int k = 0;
   for (; k + 4 <= width; k += 4) {
     int j[4];
@@ -138,11 +176,85 @@ __device__ __forceinline__ float gather_row(const int* __restrict__ cols, const 
   return acc;
 }
 
+// What a lane holds of the entries of 8 rows i0 + q stride (q = lane % 8;
+// rows from n on: none): where its row's entries lie, and the column of the
+// row's entry lane / 8 (-1 past its width). None of it changes in a pass, so
+// the kernels below fetch it ahead of their wait for the previous one.
+struct Rows8 {
+  int base, width, j;
+};
+__device__ __forceinline__ Rows8 rows8(const GraphArgs& g, int i0, int stride, int n, int lane) {
+  const int i = i0 + (lane & 7) * stride, k = lane >> 3;
+  Rows8 p = {0, 0, -1};
+  if (i < n) {
+    const int4 m = g.meta[g.rowSlice[i]];
+    p.base = m.z + (i - m.x);
+    p.width = m.w;
+    if (k < p.width) p.j = g.cols[p.base + (k << 5)];
+  }
+  return p;
+}
+// acc[q] += sum_k w[e_k] X[j_k][lane] over the entries of row q, each row's
+// sum in stored order. One row at a time a warp waited for four dependent L2
+// loads per row (slice, metadata, column, activations: 1600 cycles each when
+// other SMs have just written the line). Here gather8_issue starts the copies
+// of the first four neighbours of all 8 rows into the warp's 4 KB of shared
+// memory (16 bytes a lane, no registers held), the caller loads what else it
+// needs, and gather8_sum waits once. (24.6k nodes: the forward layer 24.6 ->
+// 8.4 us.)
+constexpr int kStage = 8 * 4 * 32;  // floats of a warp's staging
+__device__ __forceinline__ void gather8_issue(const float* X, Rows8 p, float* stage, int lane) {
+#pragma unroll
+  for (int q = 0; q < 8; q++) {
+    const int j = __shfl_sync(kFull, p.j, q + (lane & 24));
+    if (j >= 0) {
+      const uint32_t to = umma::smem_addr(stage + q * 128 + lane * 4);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to), "l"(X + (size_t)j * 32 + (lane & 7) * 4)
+                   : "memory");
+    }
+  }
+}
+__device__ __forceinline__ void gather8_sum(const GraphArgs& g, const float* wts, const float* X, Rows8 p, float* stage,
+                                            int lane, float (&acc)[8]) {
+  const int most = __reduce_max_sync(kFull, p.width);
+  for (int k0 = 0; k0 < most; k0 += 4) {
+    const int e = p.base + ((k0 + (lane >> 3)) << 5);
+    if (k0) {
+      p.j = k0 + (lane >> 3) < p.width ? g.cols[e] : -1;
+      gather8_issue(X, p, stage, lane);
+    }
+    const float w = p.j >= 0 ? wts[e] : 0.f;
+    const unsigned live = __ballot_sync(kFull, p.j >= 0);
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < 8; q++)
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const float wk = __shfl_sync(kFull, w, q + 8 * k);
+        if (live >> (q + 8 * k) & 1u) acc[q] = __fmaf_rn(wk, stage[q * 128 + k * 32 + lane], acc[q]);
+      }
+    __syncwarp();
+  }
+}
+
+// v[t] <- v[(t + g) % 8]
+__device__ __forceinline__ void rotate8(float (&v)[8], int g) {
+#pragma unroll
+  for (int b = 1; b < 8; b <<= 1) {
+    float s[8];
+#pragma unroll
+    for (int t = 0; t < 8; t++) s[t] = (g & b) ? v[(t + b) & 7] : v[t];
+#pragma unroll
+    for (int t = 0; t < 8; t++) v[t] = s[t];
+  }
+}
+
 // h_out = relu(Ws h + Wm m + b), m_i = sum_j w_ij h_j
-__global__ void __launch_bounds__(kBlock) k_layer(int n, GraphArgs g, const float* __restrict__ P,
-                                                  const float* __restrict__ Hin, float* __restrict__ Hout,
-                                                  float* __restrict__ Mout) {
+__global__ void __launch_bounds__(kBlock) k_layer(int n, GraphArgs g, const float* P, const float* Hin, float* Hout,
+                                                  float* Mout) {
   __shared__ float sWsT[32 * 32], sWmT[32 * 32], sb[32];
+  NN_PDL();
   for (int t = threadIdx.x; t < 1024; t += blockDim.x) {
     const int c = t >> 5, k = t & 31;
     sWsT[k * 32 + c] = P[t];
@@ -178,34 +290,65 @@ __global__ void __launch_bounds__(kBlock) k_layer(int n, GraphArgs g, const floa
 // MMA reads its operands as TF32 (10-bit mantissa); sums are FP32.
 
 constexpr int kTcRows = 128;
-constexpr int kTcThreads = 256;
+static_assert(kLayer0 % 4 == 0 && kLayerSize % 4 == 0, "layers read their weights as float4");
+constexpr int kTcThreads = 512;  // 16 warps, 8 rows of the tile each
+constexpr int kTcBlocks = 2;     // resident CTAs per SM
 constexpr uint32_t kTcWaitLimit = 1u << 22;  // tries of the completion wait before the kernel gives up
 
 __device__ __forceinline__ int kmajor(int r, int k, int K) {
   return (r >> 3) * (K << 3) + ((k >> 2) << 5) + ((r & 7) << 2) + (k & 3);
 }
 
-// The same layer as k_layer: the message gather on the CUDA cores (warp per
-// node, FP32, same order), then [h_i, m_i] (128 x 64) times [Ws Wm]^T (64 x
+// Stores rows rb .. rb + 7 (rb a multiple of 8; v[q] = row rb + q, column
+// lane) into columns col0 .. col0 + 31 of a K-wide operand. A row at a time
+// the 8 column groups of a row share 4 banks (8-way conflict): each group
+// writes its own row of the 8 instead.
+__device__ __forceinline__ void store_rows8(float* s, int rb, int col0, int K, int lane, float (&v)[8]) {
+  const int g = lane >> 2;
+  rotate8(v, g);
+  float* at = s + (rb >> 3) * (K << 3) + (((col0 >> 2) + g) << 5) + (lane & 3);
+#pragma unroll
+  for (int t = 0; t < 8; t++) at[((t + g) & 7) << 2] = v[t];
+}
+// The same rows transposed: element (f0 + lane, rb + q) of a kTcRows-wide
+// operand, four rows a 16-byte store.
+__device__ __forceinline__ void store_cols8(float* s, int f0, int rb, int lane, const float (&v)[8]) {
+  float* at = s + ((f0 + lane) >> 3) * (kTcRows << 3) + ((rb >> 2) << 5) + ((lane & 7) << 2);
+  *reinterpret_cast<float4*>(at) = make_float4(v[0], v[1], v[2], v[3]);
+  *reinterpret_cast<float4*>(at + 32) = make_float4(v[4], v[5], v[6], v[7]);
+}
+
+constexpr int kFwdSmem = (kTcRows * 64 + 32 * 64 + kTcThreads / 32 * kStage) * (int)sizeof(float);
+
+// The same layer as k_layer: the message gather on the CUDA cores (8
+// nodes a warp, FP32, same order), then [h_i, m_i] (128 x 64) times [Ws Wm]^T (64 x
 // 32) as 8 MMAs of K = 8 into TMEM, bias + ReLU in the epilogue. status
 // gets 1 if a completion wait runs out (outputs of that tile not written).
-__global__ void __launch_bounds__(kTcThreads, 4) k_layer_tc(int n, GraphArgs g, const float* __restrict__ P,
-                                                            const float* __restrict__ Hin, float* __restrict__ Hout,
-                                                            float* __restrict__ Mout, int* status) {
-  __shared__ __align__(128) float sA[kTcRows * 64];
-  __shared__ __align__(128) float sB[32 * 64];
+__global__ void __launch_bounds__(kTcThreads, kTcBlocks) k_layer_tc(int n, GraphArgs g, const float* P,
+                                                                    const float* Hin, float* Hout, float* Mout,
+                                                                    int* status) {
+  extern __shared__ __align__(1024) float smem[];
+  float* sA = smem;               // 128 x 64
+  float* sB = sA + kTcRows * 64;  // 32 x 64
   __shared__ float sBias[32];
   __shared__ __align__(8) uint64_t bar;
   __shared__ uint32_t sTmem;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  // B = [Ws Wm]: row = output channel, K = the 64 inputs (h then m)
-  for (int t = threadIdx.x; t < 2048; t += blockDim.x) {
-    const int o = t >> 6, k = t & 63;
-    sB[kmajor(o, k, 64)] = k < 32 ? P[o * 32 + k] : P[1024 + o * 32 + (k - 32)];
-  }
-  if (threadIdx.x < 32) sBias[threadIdx.x] = P[2048 + threadIdx.x];
+  float* stage = sB + 32 * 64 + warp * kStage;
+  NN_PDL_TRIGGER();
   if (warp == 0) umma::tmem_alloc(&sTmem, 32);
   if (threadIdx.x == 32) umma::mbar_init(&bar, 1);
+  Rows8 rows = rows8(g, blockIdx.x * kTcRows + 8 * warp, 1, n, lane);
+  NN_PDL_WAIT();
+  gather8_issue(Hin, rows, stage, lane);
+  // B = [Ws Wm]: row = output channel, K = the 64 inputs (h then m); a thread
+  // takes 4 inputs of a channel (every CTA reads these 8 KB at once: whole
+  // lines, a sector per lane cost 3 us). P is 16-byte aligned (run_forward).
+  {
+    const int t = threadIdx.x, o = (t >> 3) & 31, k = ((t & 7) << 2) + ((t >> 8) << 5);
+    *reinterpret_cast<float4*>(sB + kmajor(o, k, 64)) = reinterpret_cast<const float4*>(P)[t];
+  }
+  if (threadIdx.x < 32) sBias[threadIdx.x] = P[2048 + threadIdx.x];
   umma::fence_smem_for_mma();
   umma::fence_before_sync();
   __syncthreads();
@@ -218,18 +361,23 @@ __global__ void __launch_bounds__(kTcThreads, 4) k_layer_tc(int n, GraphArgs g, 
   bool pending = false;
   for (int tile = blockIdx.x; tile < nTiles; tile += gridDim.x) {
     const int row0 = tile * kTcRows;
-    for (int r = warp; r < kTcRows; r += kTcThreads / 32) {
-      const int i = row0 + r;
-      float h = 0.f, msg = 0.f;
-      if (i < n) {
-        const int4 m = g.meta[g.rowSlice[i]];
-        h = Hin[(size_t)i * 32 + lane];
-        msg = gather_row(g.cols, g.wf, m.z + (i - m.x), m.w, Hin, lane, 0.f);
-        if (Mout) Mout[(size_t)i * 32 + lane] = msg;
-      }
-      sA[kmajor(r, lane, 64)] = h;
-      sA[kmajor(r, 32 + lane, 64)] = msg;
+    const int rb = 8 * warp;  // the warp's rows of the tile
+    float h[8], m[8];
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+      h[q] = row0 + rb + q < n ? Hin[(size_t)(row0 + rb + q) * 32 + lane] : 0.f;
+      m[q] = 0.f;
     }
+    gather8_sum(g, g.wf, Hin, rows, stage, lane, m);
+    if (Mout) {
+#pragma unroll
+      for (int q = 0; q < 8; q++)
+        if (row0 + rb + q < n) Mout[(size_t)(row0 + rb + q) * 32 + lane] = m[q];
+    }
+    store_rows8(sA, rb, 0, 64, lane, h);
+    store_rows8(sA, rb, 32, 64, lane, m);
+    rows = rows8(g, row0 + (int)gridDim.x * kTcRows + rb, 1, n, lane);  // the next tile's
+    gather8_issue(Hin, rows, stage, lane);
     umma::fence_smem_for_mma();
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -249,23 +397,30 @@ __global__ void __launch_bounds__(kTcThreads, 4) k_layer_tc(int n, GraphArgs g, 
     pending = false;
     parity ^= 1u;
     umma::fence_after_sync();
-    // warp w reads TMEM lanes 32 (w % 4) .. +31 (its rows), columns 16 (w / 4) .. +15
-    const int q = warp & 3, half = warp >> 2;
-    float z[16];
-    umma::ld16(umma::tmem_at(tmem, 32 * q, 16 * half), z);
-    const int i = row0 + 32 * q + lane;
-    if (i < n) {
-      float4* out = reinterpret_cast<float4*>(Hout + (size_t)i * 32 + 16 * half);
+    // warp w reads TMEM lanes 32 (w % 4) .. +31 (its rows), columns 8 (w / 4) .. +7
+    const int q = warp & 3, part = warp >> 2;
+    float z[8];
+    umma::ld8(umma::tmem_at(tmem, 32 * q, 8 * part), z);
+    const int i = 32 * q + lane;
+    // through shared memory (the MMAs are done with A), 16-byte pieces rotated
+    // by row, to whole lines: a lane's own row is 32 separate lines a store
 #pragma unroll
-      for (int c = 0; c < 4; c++) {
-        const float* b = sBias + 16 * half + 4 * c;
-        out[c] = make_float4(relu(z[4 * c] + b[0]), relu(z[4 * c + 1] + b[1]), relu(z[4 * c + 2] + b[2]),
-                             relu(z[4 * c + 3] + b[3]));
-      }
+    for (int c = 0; c < 2; c++) {
+      const float* b = sBias + 8 * part + 4 * c;
+      reinterpret_cast<float4*>(sA)[i * 8 + ((2 * part + c) ^ (i & 7))] =
+          make_float4(relu(z[4 * c] + b[0]), relu(z[4 * c + 1] + b[1]), relu(z[4 * c + 2] + b[2]),
+                      relu(z[4 * c + 3] + b[3]));
     }
     umma::fence_before_sync();
     __syncthreads();
+    for (int t = threadIdx.x; t < kTcRows * 8; t += kTcThreads) {
+      const int r = t >> 3;
+      if (row0 + r < n)
+        reinterpret_cast<float4*>(Hout)[(size_t)row0 * 8 + t] = reinterpret_cast<float4*>(sA)[r * 8 + ((t & 7) ^ (r & 7))];
+    }
+    __syncthreads();
   }
+  asm volatile("cp.async.wait_all;" ::: "memory");
   // after a wait that ran out, give the MMAs in flight one more bounded wait
   // before their accumulator is released
   if (pending) __syncthreads_and(umma::mbar_wait(&bar, parity, kTcWaitLimit));
@@ -297,15 +452,22 @@ __device__ __forceinline__ float warp_sum(float v) {
   return __shfl_sync(kFull, v, 0);
 }
 
-__global__ void __launch_bounds__(kBlock) k_decode(int n, const float* __restrict__ P, const float* __restrict__ H3,
-                                                   const double* __restrict__ scale, double* out) {
+__global__ void __launch_bounds__(kBlock) k_decode(int n, const float* P, const float* H3, const double* scale,
+                                                   double* out) {
+  NN_PDL();
   const int lane = threadIdx.x & 31;
   const int nw = (gridDim.x * blockDim.x) >> 5;
   const float wd = P[kDecW + lane], bd = P[kDecB];
   const double s = scale[0];
-  for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += nw) {
-    const float y = warp_sum(wd * H3[(size_t)i * 32 + lane]) + bd;
-    if (lane == 0) out[i] = s * (double)y;
+  // four nodes a warp: one node's chain of five shuffles left it waiting
+  for (int i = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 4; i < n; i += nw * 4) {
+    float y[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) y[q] = i + q < n ? H3[(size_t)(i + q) * 32 + lane] : 0.f;
+#pragma unroll
+    for (int q = 0; q < 4; q++) y[q] = warp_sum(wd * y[q]) + bd;
+    if (lane < 4 && i + lane < n)
+      out[i + lane] = s * (double)(lane == 0 ? y[0] : lane == 1 ? y[1] : lane == 2 ? y[2] : y[3]);
   }
 }
 
@@ -322,11 +484,11 @@ __device__ void block_grad_store(const float* sv, int nv, float* gp, int off) {
   }
 }
 
-__global__ void __launch_bounds__(kBlock) k_decode_bwd(int n, const float* __restrict__ P,
-                                                       const float* __restrict__ H3, const double* __restrict__ scale,
-                                                       const double* __restrict__ e, const double* __restrict__ e2,
-                                                       float* __restrict__ dH3, float* gp, double* lossPartials) {
+__global__ void __launch_bounds__(kBlock) k_decode_bwd(int n, const float* P, const float* H3, const double* scale,
+                                                       const double* __restrict__ e, const double* e2, float* dH3,
+                                                       float* gp, double* lossPartials) {
   __shared__ float sv[kWarps * 33];
+  NN_PDL();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int nw = (gridDim.x * blockDim.x) >> 5;
   const float wd = P[kDecW + lane], bd = P[kDecB];
@@ -353,24 +515,35 @@ __global__ void __launch_bounds__(kBlock) k_decode_bwd(int n, const float* __res
 
 // Decoder backward from a given gradient of the loss with respect to the
 // FP64 output d = s y: gd[i] * gdScale[0] (dL/dy = s dL/dd).
-__global__ void __launch_bounds__(kBlock) k_decode_bwd_grad(int n, const float* __restrict__ P,
-                                                            const float* __restrict__ H3,
-                                                            const double* __restrict__ scale,
-                                                            const double* __restrict__ gd,
-                                                            const double* __restrict__ gdScale,
-                                                            float* __restrict__ dH3, float* gp) {
+__global__ void __launch_bounds__(kBlock) k_decode_bwd_grad(int n, const float* P, const float* H3,
+                                                            const double* scale, const double* gd,
+                                                            const double* gdScale, float* dH3, float* gp) {
   __shared__ float sv[kWarps * 33];
+  NN_PDL();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int nw = (gridDim.x * blockDim.x) >> 5;
   const float wd = P[kDecW + lane];
   const double s = scale[0] * gdScale[0];
   float gwd = 0.f, gbd = 0.f;
-  for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += nw) {
-    const float h = H3[(size_t)i * 32 + lane];
-    const float gy = (float)(s * gd[i]);
-    dH3[(size_t)i * 32 + lane] = gy * wd;
-    gwd = __fmaf_rn(gy, h, gwd);
-    gbd += gy;
+  for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += 4 * nw) {
+    // four nodes' loads in flight, summed in node order
+    float h[4];
+    double gi[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const int j = i + q * nw;
+      h[q] = j < n ? H3[(size_t)j * 32 + lane] : 0.f;
+      gi[q] = j < n ? gd[j] : 0.0;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const int j = i + q * nw;
+      if (j >= n) break;
+      const float gy = (float)(s * gi[q]);
+      dH3[(size_t)j * 32 + lane] = gy * wd;
+      gwd = __fmaf_rn(gy, h[q], gwd);
+      gbd += gy;
+    }
   }
   sv[w * 33 + lane] = gwd;
   if (lane == 0) sv[w * 33 + 32] = gbd;
@@ -378,7 +551,8 @@ __global__ void __launch_bounds__(kBlock) k_decode_bwd_grad(int n, const float* 
 }
 
 // t = r + q in place of q, with block partials of t.t and r.r
-__global__ void k_residual_loss(int n, const double* __restrict__ r, double* q, double* partials) {
+__global__ void k_residual_loss(int n, const double* r, double* q, double* partials) {
+  NN_PDL();
   double a = 0.0, b = 0.0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const double ri = r[i];
@@ -396,7 +570,8 @@ __global__ void k_residual_loss(int n, const double* __restrict__ r, double* q, 
 }
 
 // loss = sum t.t / sum r.r; gscale = 2 / sum r.r
-__global__ void k_residual_loss_finish(int np, const double* __restrict__ partials, double* loss, double* gscale) {
+__global__ void k_residual_loss_finish(int np, const double* partials, double* loss, double* gscale) {
+  NN_PDL();
   double a = 0.0, b = 0.0;
   for (int k = threadIdx.x; k < np; k += blockDim.x) {
     a += partials[2 * k];
@@ -412,13 +587,12 @@ __global__ void k_residual_loss_finish(int np, const double* __restrict__ partia
 }
 
 // dz = dHout * [Hout > 0]; dS = Ws^T dz; dM = Wm^T dz; gradients of Ws, Wm, b
-__global__ void __launch_bounds__(kBlock) k_layer_bwd_a(int n, const float* __restrict__ P,
-                                                        const float* __restrict__ Hin, const float* __restrict__ Hout,
-                                                        const float* __restrict__ Min, const float* __restrict__ dHout,
-                                                        float* __restrict__ dS, float* __restrict__ dM, float* gp,
-                                                        int off) {
+__global__ void __launch_bounds__(kBlock) k_layer_bwd_a(int n, const float* P, const float* Hin, const float* Hout,
+                                                        const float* Min, const float* dHout, float* dS, float* dM,
+                                                        float* gp, int off) {
   extern __shared__ float sv[];  // kWarps * kLayerSize (per-warp gradient sums)
   __shared__ float sWs[1024], sWm[1024];
+  NN_PDL();
   for (int t = threadIdx.x; t < 1024; t += blockDim.x) {
     sWs[t] = P[t];
     sWm[t] = P[1024 + t];
@@ -460,8 +634,10 @@ __global__ void __launch_bounds__(kBlock) k_layer_bwd_a(int n, const float* __re
 }
 
 // dHin_i = dS_i + sum_j w_ji dM_j (w_ji = |a_ji| / |a_jj|; symmetric couplings)
-__global__ void __launch_bounds__(kBlock) k_layer_bwd_b(int n, GraphArgs g, const float* __restrict__ dS,
-                                                        const float* __restrict__ dM, float* __restrict__ dHin) {
+// (the FP32 layers; the tensor-core ones form it where they read it)
+__global__ void __launch_bounds__(kBlock) k_layer_bwd_b(int n, GraphArgs g, const float* dS, const float* dM,
+                                                        float* dHin) {
+  NN_PDL();
   const int lane = threadIdx.x & 31;
   const int nw = (gridDim.x * blockDim.x) >> 5;
   for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += nw) {
@@ -482,31 +658,44 @@ __global__ void __launch_bounds__(kBlock) k_layer_bwd_b(int n, GraphArgs g, cons
 // (32 channels x 128 nodes), W^T (64 inputs x 32 channels).
 constexpr int kBwdSmem = (128 * kTcRows + kTcRows * 32 + 32 * kTcRows + 64 * 32) * (int)sizeof(float);
 
-__global__ void __launch_bounds__(kTcThreads, 2) k_layer_bwd_tc(int n, const float* __restrict__ P,
-                                                                const float* __restrict__ Hin,
-                                                                const float* __restrict__ Hout,
-                                                                const float* __restrict__ Min,
-                                                                const float* __restrict__ dHout,
-                                                                float* __restrict__ dS, float* __restrict__ dM,
-                                                                float* gp, int off, int* status) {
+// The incoming gradient is dHout as given (dMout null), or the previous
+// layer's input gradient, formed here row by row (dHout = its dS plus the
+// gather of its dM = dMout) instead of by a pass of its own between the two:
+// the layer with that pass took 22.9 + 6.5 us at 24.6k nodes, now 10.3.
+__global__ void __launch_bounds__(kTcThreads, 2) k_layer_bwd_tc(int n, GraphArgs g, const float* P, const float* Hin,
+                                                                const float* Hout, const float* Min,
+                                                                const float* dHout, const float* dMout, float* dS,
+                                                                float* dM, float* gp, int off, int* status) {
   extern __shared__ __align__(1024) float smem[];
-  float* sXT = smem;                // 128 x 128
-  float* sZ = sXT + 128 * kTcRows;  // 128 x 32
-  float* sZT = sZ + kTcRows * 32;   // 32 x 128
-  float* sW = sZT + 32 * kTcRows;   // 64 x 32
+  float* sZ = smem;                  // 128 x 32
+  float* sZT = sZ + kTcRows * 32;    // 32 x 128
+  float* sXT = sZT + 32 * kTcRows;   // 128 x 128
+  float* sW = sXT + 128 * kTcRows;   // 64 x 32
+  // before a tile's operands are written the space of Z, ZT and the first 64
+  // features of XT is the warps' gather staging; after its MMAs, that of the
+  // 64 features holds its outputs on their way to global memory
   __shared__ __align__(8) uint64_t bar;
   __shared__ uint32_t sTmem;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int t = threadIdx.x; t < 2048; t += blockDim.x) {
-    const int f = t >> 5, c = t & 31;  // W^T[f][c] = Ws[c][f] or Wm[c][f - 32]
-    sW[kmajor(f, c, 32)] = f < 32 ? P[c * 32 + f] : P[1024 + c * 32 + (f - 32)];
-  }
-  for (int t = threadIdx.x; t < 64 * kTcRows; t += blockDim.x) {
-    const int f = 64 + (t >> 7), r = t & 127;
-    sXT[kmajor(f, r, kTcRows)] = f == 64 ? 1.f : 0.f;
-  }
+  float* stage = smem + warp * kStage;
+  static_assert(kTcThreads / 32 * kStage == 2 * kTcRows * 32 + 64 * kTcRows, "staging overlays Z, ZT and 64 features");
+  NN_PDL_TRIGGER();
   if (warp == 0) umma::tmem_alloc(&sTmem, 128);
   if (threadIdx.x == 32) umma::mbar_init(&bar, 1);
+  // features 64 .. 127 of XT: the constant 1, then zeros
+  for (int t = threadIdx.x; t < 64 * kTcRows / 4; t += blockDim.x) {
+    const float one = t < 256 && (t & 7) == 0 ? 1.f : 0.f;
+    reinterpret_cast<float4*>(sXT + 64 * kTcRows)[t] = make_float4(one, one, one, one);
+  }
+  Rows8 rows = {0, 0, -1};
+  if (dMout) rows = rows8(g, blockIdx.x * kTcRows + 8 * warp, 1, n, lane);
+  NN_PDL_WAIT();
+  if (dMout) gather8_issue(dMout, rows, stage, lane);
+  {
+    const int f = threadIdx.x & 63, c = (threadIdx.x >> 6) << 2;  // W^T[f][c] = Ws[c][f] or Wm[c][f - 32]
+    const float* w = f < 32 ? P + c * 32 + f : P + 1024 + c * 32 + (f - 32);
+    *reinterpret_cast<float4*>(sW + kmajor(f, c, 32)) = make_float4(w[0], w[32], w[64], w[96]);
+  }
   umma::fence_smem_for_mma();
   umma::fence_before_sync();
   __syncthreads();
@@ -521,20 +710,30 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_layer_bwd_tc(int n, const flo
   bool pending = false, any = false, failed = false;
   for (int tile = blockIdx.x; tile < nTiles; tile += gridDim.x) {
     const int row0 = tile * kTcRows;
-    for (int r = warp; r < kTcRows; r += kTcThreads / 32) {
-      const int i = row0 + r;
-      float dz = 0.f, h = 0.f, m = 0.f;
-      if (i < n) {
-        const size_t o = (size_t)i * 32 + lane;
-        dz = Hout[o] > 0.f ? dHout[o] : 0.f;
-        h = Hin[o];
-        m = Min[o];
-      }
-      sZ[kmajor(r, lane, 32)] = dz;
-      sZT[kmajor(lane, r, kTcRows)] = dz;
-      sXT[kmajor(lane, r, kTcRows)] = h;
-      sXT[kmajor(32 + lane, r, kTcRows)] = m;
+    const int rw = 8 * warp;  // the warp's rows of the tile
+    float dz[8], h[8], m[8];
+#pragma unroll
+    for (int q = 0; q < 8; q++) dz[q] = row0 + rw + q < n ? dHout[(size_t)(row0 + rw + q) * 32 + lane] : 0.f;
+    float ho[8];
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+      const size_t o = (size_t)(row0 + rw + q) * 32 + lane;
+      const bool live = row0 + rw + q < n;
+      ho[q] = live ? Hout[o] : 0.f;
+      h[q] = live ? Hin[o] : 0.f;
+      m[q] = live ? Min[o] : 0.f;
     }
+    if (dMout) {
+      gather8_sum(g, g.wb, dMout, rows, stage, lane, dz);
+      rows = rows8(g, row0 + (int)gridDim.x * kTcRows + rw, 1, n, lane);  // the next tile's
+      __syncthreads();
+    }
+#pragma unroll
+    for (int q = 0; q < 8; q++) dz[q] = ho[q] > 0.f ? dz[q] : 0.f;
+    store_cols8(sZT, 0, rw, lane, dz);
+    store_cols8(sXT, 0, rw, lane, h);
+    store_cols8(sXT, 32, rw, lane, m);
+    store_rows8(sZ, rw, 0, 32, lane, dz);
     umma::fence_smem_for_mma();
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -559,45 +758,50 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_layer_bwd_tc(int n, const flo
     pending = false;
     parity ^= 1u;
     umma::fence_after_sync();
-    // warp w: rows 32 (w % 4) .., columns 32 (w / 4) ..: dS for w < 4, dM for w >= 4
-    const int q = warp & 3, half = warp >> 2;
+    // warp w: rows 32 (w % 4) .., columns 16 (w / 4) ..: dS for w < 8, dM for w >= 8
+    const int q = warp & 3, part = warp >> 2;
     float v[16];
-    const int i = row0 + 32 * q + lane;
-    float* dst = (half ? dM : dS) + (size_t)i * 32;
+    const int i = 32 * q + lane;
+    umma::ld16(umma::tmem_at(tmem, 32 * q, 16 * part), v);
+    // to whole lines through shared memory, 16-byte pieces rotated by row
+    float4* out = reinterpret_cast<float4*>(sXT);  // 128 rows x (dS, dM)
 #pragma unroll
-    for (int p = 0; p < 2; p++) {
-      umma::ld16(umma::tmem_at(tmem, 32 * q, 32 * half + 16 * p), v);
-      if (i < n) {
-        float4* o4 = reinterpret_cast<float4*>(dst + 16 * p);
-#pragma unroll
-        for (int c = 0; c < 4; c++) o4[c] = make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
-      }
-    }
+    for (int c = 0; c < 4; c++)
+      out[i * 16 + ((4 * part + c) ^ (i & 7))] = make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
     umma::fence_before_sync();
     __syncthreads();
+    umma::fence_after_sync();
+    for (int t = threadIdx.x; t < kTcRows * 8; t += kTcThreads) {
+      const int r = t >> 3, c = (t & 7) ^ (r & 7);
+      if (row0 + r < n) {
+        reinterpret_cast<float4*>(dS)[(size_t)row0 * 8 + t] = out[r * 16 + c];
+        reinterpret_cast<float4*>(dM)[(size_t)row0 * 8 + t] = out[r * 16 + 8 + c];
+      }
+    }
+    __syncthreads();
+    if (dMout) gather8_issue(dMout, rows, stage, lane);
   }
+  asm volatile("cp.async.wait_all;" ::: "memory");
   if (pending) __syncthreads_and(umma::mbar_wait(&bar, parity, kTcWaitLimit));
   umma::fence_after_sync();
-  // gradient partials of this CTA: warps 0..3 hold features 32 w + lane
+  // gradient partials of this CTA: warp w holds features 32 (w % 4) + lane,
+  // channels 8 (w / 4) .. +7
   float* gb = gp + (size_t)blockIdx.x * kParams + off;
-  if (warp < 4) {
-    const int f = 32 * warp + lane;
-    float v[16];
+  if ((warp & 3) < 3) {
+    const int f = 32 * (warp & 3) + lane, ch0 = 8 * (warp >> 2);
+    float v[8];
+    if (any && !failed) {
+      umma::ld8(umma::tmem_at(tmem, 32 * (warp & 3), 64 + ch0), v);
+    } else {
 #pragma unroll
-    for (int p = 0; p < 2; p++) {
-      if (any && !failed) {
-        umma::ld16(umma::tmem_at(tmem, 32 * warp, 64 + 16 * p), v);
-      } else {
+      for (int c = 0; c < 8; c++) v[c] = 0.f;
+    }
 #pragma unroll
-        for (int c = 0; c < 16; c++) v[c] = 0.f;
-      }
-#pragma unroll
-      for (int c = 0; c < 16; c++) {
-        const int ch = 16 * p + c;
-        if (f < 32) gb[ch * 32 + f] = v[c];
-        else if (f < 64) gb[1024 + ch * 32 + (f - 32)] = v[c];
-        else if (f == 64) gb[2048 + ch] = v[c];
-      }
+    for (int c = 0; c < 8; c++) {
+      const int ch = ch0 + c;
+      if (f < 32) gb[ch * 32 + f] = v[c];
+      else if (f < 64) gb[1024 + ch * 32 + (f - 32)] = v[c];
+      else if (f == 64) gb[2048 + ch] = v[c];
     }
   }
   if (failed && threadIdx.x == 0) atomicOr(status, 1);
@@ -607,32 +811,76 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_layer_bwd_tc(int n, const flo
   if (warp == 0) umma::tmem_free(tmem, 128);
 }
 
-__global__ void __launch_bounds__(kBlock) k_encode_bwd(int n, const float* __restrict__ u, const float* __restrict__ H0,
-                                                       const float* __restrict__ dH0, float* gp) {
+// dH0 as given (dM null), or formed from the first layer's dS (= dH0) and
+// dM as in k_layer_bwd_tc; 8 nodes of a warp at a time, summed in node order
+__global__ void __launch_bounds__(kBlock) k_encode_bwd(int n, GraphArgs g, const float* u, const float* H0,
+                                                       const float* dH0, const float* dM, float* gp) {
   __shared__ float sv[kWarps * 64];
+  __shared__ __align__(16) float sStage[kWarps * kStage];
+  NN_PDL();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int nw = (gridDim.x * blockDim.x) >> 5;
   float gw = 0.f, gb = 0.f;
-  for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += nw) {
-    const size_t o = (size_t)i * 32 + lane;
-    const float dz = H0[o] > 0.f ? dH0[o] : 0.f;
-    gw = __fmaf_rn(dz, u[i], gw);
-    gb += dz;
+  float* stage = sStage + w * kStage;
+  for (int i0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i0 < n; i0 += 8 * nw) {
+    float dh[8], h0[8], uq[8];
+    Rows8 rows = {0, 0, -1};
+    if (dM) {
+      rows = rows8(g, i0, nw, n, lane);
+      gather8_issue(dM, rows, stage, lane);
+    }
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+      const int i = i0 + q * nw;
+      dh[q] = i < n ? dH0[(size_t)i * 32 + lane] : 0.f;
+      h0[q] = i < n ? H0[(size_t)i * 32 + lane] : 0.f;
+      uq[q] = i < n ? u[i] : 0.f;
+    }
+    if (dM) gather8_sum(g, g.wb, dM, rows, stage, lane, dh);
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+      if (i0 + q * nw >= n) break;
+      const float dz = h0[q] > 0.f ? dh[q] : 0.f;
+      gw = __fmaf_rn(dz, uq[q], gw);
+      gb += dz;
+    }
   }
   sv[w * 64 + lane] = gw;
   sv[w * 64 + 32 + lane] = gb;
   block_grad_store(sv, 64, gp, kEncW);
 }
 
-__global__ void k_grad_reduce(int nBlocks, const float* __restrict__ gp, float* grad) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= kParams) return;
+// grad = sum over the blocks' partials, in block order (the layers' parameters
+// have layerBlocks of them, the others kGradBlocks). A block takes 32
+// parameters: its warps bring all their partials to shared memory at once and
+// one warp adds them up. (One thread a parameter with four loads in flight
+// took 9.4 us, now 6.7.)
+__global__ void __launch_bounds__(kBlock) k_grad_reduce(int layerBlocks, const float* gp, float* grad) {
+  __shared__ float part[kGradBlocks][32];
+  NN_PDL();
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int p = blockIdx.x * 32 + lane;
+  const bool layer = blockIdx.x * 32 >= kLayer0 && blockIdx.x * 32 + 32 <= kDecW;
+  const int nb = layer ? layerBlocks : kGradBlocks;
+  if (p < kParams) {
+#pragma unroll
+    for (int k = 0; k < kGradBlocks / kWarps; k++) {
+      const int b = w + k * kWarps;
+      if (b < nb) part[b][lane] = gp[(size_t)b * kParams + p];
+    }
+  }
+  __syncthreads();
+  if (w || p >= kParams) return;
   float s = 0.f;
-  for (int b = 0; b < nBlocks; b++) s += gp[(size_t)b * kParams + p];
+#pragma unroll 8
+  for (int b = 0; b < nb; b++) s += part[b][lane];
   grad[p] = s;
 }
+static_assert(kGradBlocks % kWarps == 0 && kLayer0 % 32 == 0 && kDecW % 32 == 0,
+              "the reduction's blocks hold parameters of one kind");
 
-__global__ void k_adam(float* P, const float* __restrict__ g, float* m, float* v, float lr, float c1, float c2) {
+__global__ void k_adam(float* P, const float* g, float* m, float* v, float lr, float c1, float c2) {
+  NN_PDL();
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= kParams) return;
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
@@ -654,32 +902,75 @@ void check(cudaError_t e, const char* what) {
 
 constexpr int kReduceBlocks = 592;
 
-// persistent grid of the forward tensor-core layer: up to 4 CTAs per SM
+// persistent grid of the forward tensor-core layer
 int tc_blocks(int n) {
   const int t = ceil_div(n, kTcRows);
-  return t < 148 * 4 ? (t < 1 ? 1 : t) : 148 * 4;
+  return t < 148 * kTcBlocks ? (t < 1 ? 1 : t) : 148 * kTcBlocks;
 }
 
 void run_forward(const Graph& g, const float* P, const double* r, Workspace& w, double* scal, bool keepMessages,
                  cudaStream_t st) {
   const int n = w.n;
-  k_scale_partials<<<kReduceBlocks, kBlock, 0, st>>>(n, r, g.a.diag, w.partials);
-  dev::sum_partials(kReduceBlocks, w.partials, scal + 1, st);
-  k_input<<<ceil_div(n, kBlock), kBlock, 0, st>>>(n, r, g.a.diag, scal + 1, w.u, scal);
-  k_encode<<<ceil_div((long long)n * 32, kBlock), kBlock, 0, st>>>(n, w.u, P, w.H[0]);
   FVM_REQUIRE(g.entries > 0 && g.entries <= w.wcap, kBadArgument,
               "learned correction: workspace not prepared for this graph's entries");
-  k_edge_weights<<<ceil_div((long long)g.nSlices * 32, kBlock), kBlock, 0, st>>>(g.nSlices, g.a.meta, g.a.cols,
-                                                                               g.a.vals, g.a.diag, w.wf, w.wb);
+  launch(k_pass_start, kReduceBlocks + ceil_div(4LL * g.nSlices, kWarps), kBlock, 0, st, n, r, kReduceBlocks,
+         w.partials, g.nSlices, g.a.meta, g.a.cols, g.a.vals, g.a.diag, w.wf, w.wb);
+  dev::sum_partials(kReduceBlocks, w.partials, scal + 1, st);
+  launch(k_encode, ceil_div(n, 8 * kWarps), kBlock, 0, st, n, r, g.a.diag, scal + 1, P, w.u, scal, w.H[0]);
+  FVM_REQUIRE(((uintptr_t)P & 15) == 0, kBadArgument, "learned correction: parameters not 16-byte aligned");
   const GraphArgs ga = args(g, w);
+  if (w.tensorCores)
+    check(cudaFuncSetAttribute(k_layer_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, kFwdSmem),
+          "k_layer_tc shared memory");
   for (int l = 0; l < kLayers; l++) {
     const float* Pl = P + kLayer0 + l * kLayerSize;
     float* Ml = keepMessages ? w.M[l] : nullptr;
     if (w.tensorCores)
-      k_layer_tc<<<tc_blocks(n), kTcThreads, 0, st>>>(n, ga, Pl, w.H[l], w.H[l + 1], Ml, w.status);
+      launch(k_layer_tc, tc_blocks(n), kTcThreads, kFwdSmem, st, n, ga, Pl, w.H[l], w.H[l + 1], Ml, w.status);
     else
-      k_layer<<<node_blocks(n), kBlock, 0, st>>>(n, ga, Pl, w.H[l], w.H[l + 1], Ml);
+      launch(k_layer, node_blocks(n), kBlock, 0, st, n, ga, Pl, w.H[l], w.H[l + 1], Ml);
   }
+}
+
+// From the decoder's gradient in w.dA: the layers' backward passes, the
+// encoder's, and the reduction of every block's gradient partials.
+void run_backward(const Graph& g, const float* P, float* grad, Workspace& w, cudaStream_t st) {
+  const int n = w.n;
+  const GraphArgs ga = args(g, w);
+  // a CTA without a tile has no gradient to add
+  const int layerBlocks = w.tensorCores ? std::min(kGradBlocks, ceil_div(n, kTcRows)) : kGradBlocks;
+  const float *dH = w.dA, *dM = nullptr;  // incoming gradient (and the message part still to gather)
+  if (w.tensorCores) {
+    check(cudaFuncSetAttribute(k_layer_bwd_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, kBwdSmem),
+          "k_layer_bwd_tc shared memory");
+    for (int l = kLayers - 1; l >= 0; l--) {
+      const int off = kLayer0 + l * kLayerSize;
+      // a layer reads the last one's dS, dM for every neighbour while it
+      // writes its own: two pairs in turn, the second of buffers that are
+      // free after the last layer (the decoder's gradient, its messages)
+      const bool odd = (kLayers - 1 - l) & 1;
+      float* outS = odd ? w.dA : w.dS;
+      float* outM = odd ? w.M[kLayers - 1] : w.dB;
+      launch(k_layer_bwd_tc, layerBlocks, kTcThreads, kBwdSmem, st, n, ga, P + off, w.H[l], w.H[l + 1], w.M[l], dH, dM,
+             outS, outM, w.gradPartials, off, w.status);
+      check(cudaGetLastError(), "layer backward launch");
+      dH = outS;
+      dM = outM;
+    }
+  } else {
+    const size_t smem = sizeof(float) * kWarps * kLayerSize;
+    check(cudaFuncSetAttribute(k_layer_bwd_a, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+          "k_layer_bwd_a shared memory");
+    for (int l = kLayers - 1; l >= 0; l--) {
+      const int off = kLayer0 + l * kLayerSize;
+      launch(k_layer_bwd_a, kGradBlocks, kBlock, smem, st, n, P + off, w.H[l], w.H[l + 1], w.M[l], w.dA, w.dS, w.dB,
+             w.gradPartials, off);
+      check(cudaGetLastError(), "layer backward launch");
+      launch(k_layer_bwd_b, node_blocks(n), kBlock, 0, st, n, ga, w.dS, w.dB, w.dA);
+    }
+  }
+  launch(k_encode_bwd, kGradBlocks, kBlock, 0, st, n, ga, w.u, w.H[0], dH, dM, w.gradPartials);
+  launch(k_grad_reduce, ceil_div(kParams, 32), kBlock, 0, st, layerBlocks, w.gradPartials, grad);
 }
 
 }  // namespace
@@ -753,37 +1044,19 @@ void Workspace::checkStatus() {
 void forward(const Graph& g, const float* params, const double* r, double* out, Workspace& w, double* scal,
              cudaStream_t st) {
   run_forward(g, params, r, w, scal, false, st);
-  k_decode<<<node_blocks(w.n), kBlock, 0, st>>>(w.n, params, w.H[kLayers], scal, out);
+  launch(k_decode, node_blocks(ceil_div(w.n, 4)), kBlock, 0, st, w.n, params, w.H[kLayers], scal, out);
 }
 
 void forward_backward(const Graph& g, const float* P, const double* r, const double* e, float* grad, double* loss,
                       Workspace& w, double* scal, cudaStream_t st) {
   const int n = w.n;
   run_forward(g, P, r, w, scal, true, st);
-  k_sq_partials<<<kReduceBlocks, kBlock, 0, st>>>(n, e, w.partials);
+  launch(k_sq_partials, kReduceBlocks, kBlock, 0, st, n, e, w.partials);
   dev::sum_partials(kReduceBlocks, w.partials, scal + 2, st);
-  k_decode_bwd<<<kGradBlocks, kBlock, 0, st>>>(n, P, w.H[kLayers], scal, e, scal + 2, w.dA, w.gradPartials,
-                                               w.partials);
+  launch(k_decode_bwd, kGradBlocks, kBlock, 0, st, n, P, w.H[kLayers], scal, e, scal + 2, w.dA, w.gradPartials,
+         w.partials);
   dev::sum_partials(kGradBlocks, w.partials, loss, st);
-  const GraphArgs ga = args(g, w);
-  const size_t smem = sizeof(float) * kWarps * kLayerSize;
-  check(cudaFuncSetAttribute(k_layer_bwd_a, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-        "k_layer_bwd_a shared memory");
-  check(cudaFuncSetAttribute(k_layer_bwd_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, kBwdSmem),
-        "k_layer_bwd_tc shared memory");
-  for (int l = kLayers - 1; l >= 0; l--) {
-    const int off = kLayer0 + l * kLayerSize;
-    if (w.tensorCores)
-      k_layer_bwd_tc<<<kGradBlocks, kTcThreads, kBwdSmem, st>>>(n, P + off, w.H[l], w.H[l + 1], w.M[l], w.dA, w.dS,
-                                                                 w.dB, w.gradPartials, off, w.status);
-    else
-      k_layer_bwd_a<<<kGradBlocks, kBlock, smem, st>>>(n, P + off, w.H[l], w.H[l + 1], w.M[l], w.dA, w.dS, w.dB,
-                                                       w.gradPartials, off);
-    check(cudaGetLastError(), "layer backward launch");
-    k_layer_bwd_b<<<node_blocks(n), kBlock, 0, st>>>(n, ga, w.dS, w.dB, w.dA);
-  }
-  k_encode_bwd<<<kGradBlocks, kBlock, 0, st>>>(n, w.u, w.H[0], w.dA, w.gradPartials);
-  k_grad_reduce<<<ceil_div(kParams, kBlock), kBlock, 0, st>>>(kGradBlocks, w.gradPartials, grad);
+  run_backward(g, P, grad, w, st);
 }
 
 void forward_backward_residual(const Graph& g, const float* P, const double* r, float* grad, double* loss,
@@ -792,31 +1065,14 @@ void forward_backward_residual(const Graph& g, const float* P, const double* r, 
   double* d = w.dv;
   double* t = w.dv + n;
   run_forward(g, P, r, w, scal, true, st);
-  k_decode<<<node_blocks(n), kBlock, 0, st>>>(n, P, w.H[kLayers], scal, d);
+  launch(k_decode, node_blocks(ceil_div(n, 4)), kBlock, 0, st, n, P, w.H[kLayers], scal, d);
   dev::spmv(g.a, g.nSlices, d, t, st);  // t = A d
-  k_residual_loss<<<kReduceBlocks, kBlock, 0, st>>>(n, r, t, w.partials);  // t = r + A d
-  k_residual_loss_finish<<<1, kBlock, 0, st>>>(kReduceBlocks, w.partials, loss, scal + 3);
+  launch(k_residual_loss, kReduceBlocks, kBlock, 0, st, n, r, t, w.partials);  // t = r + A d
+  launch(k_residual_loss_finish, 1, kBlock, 0, st, kReduceBlocks, w.partials, loss, scal + 3);
   dev::spmv(g.a, g.nSlices, t, d, st);  // d = A (r + A d): dL/dd / (2 / |r|^2)
-  k_decode_bwd_grad<<<kGradBlocks, kBlock, 0, st>>>(n, P, w.H[kLayers], scal, d, scal + 3, w.dA, w.gradPartials);
-  const GraphArgs ga = args(g, w);
-  const size_t smem = sizeof(float) * kWarps * kLayerSize;
-  check(cudaFuncSetAttribute(k_layer_bwd_a, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-        "k_layer_bwd_a shared memory");
-  check(cudaFuncSetAttribute(k_layer_bwd_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, kBwdSmem),
-        "k_layer_bwd_tc shared memory");
-  for (int l = kLayers - 1; l >= 0; l--) {
-    const int off = kLayer0 + l * kLayerSize;
-    if (w.tensorCores)
-      k_layer_bwd_tc<<<kGradBlocks, kTcThreads, kBwdSmem, st>>>(n, P + off, w.H[l], w.H[l + 1], w.M[l], w.dA, w.dS,
-                                                                 w.dB, w.gradPartials, off, w.status);
-    else
-      k_layer_bwd_a<<<kGradBlocks, kBlock, smem, st>>>(n, P + off, w.H[l], w.H[l + 1], w.M[l], w.dA, w.dS, w.dB,
-                                                       w.gradPartials, off);
-    check(cudaGetLastError(), "layer backward launch");
-    k_layer_bwd_b<<<node_blocks(n), kBlock, 0, st>>>(n, ga, w.dS, w.dB, w.dA);
-  }
-  k_encode_bwd<<<kGradBlocks, kBlock, 0, st>>>(n, w.u, w.H[0], w.dA, w.gradPartials);
-  k_grad_reduce<<<ceil_div(kParams, kBlock), kBlock, 0, st>>>(kGradBlocks, w.gradPartials, grad);
+  launch(k_decode_bwd_grad, kGradBlocks, kBlock, 0, st, n, P, w.H[kLayers], scal, d, scal + 3, w.dA,
+         w.gradPartials);
+  run_backward(g, P, grad, w, st);
 }
 
 int tc_wait_probe(unsigned limit) {
@@ -837,7 +1093,7 @@ int tc_wait_probe(unsigned limit) {
 void adam_step(float* params, const float* grad, float* m, float* v, float lr, int t, cudaStream_t st) {
   const float c1 = 1.f - std::pow(0.9f, (float)t);
   const float c2 = 1.f - std::pow(0.999f, (float)t);
-  k_adam<<<ceil_div(kParams, kBlock), kBlock, 0, st>>>(params, grad, m, v, lr, c1, c2);
+  launch(k_adam, ceil_div(kParams, kBlock), kBlock, 0, st, params, grad, m, v, lr, c1, c2);
 }
 
 std::vector<float> initial_parameters(uint64_t seed) {

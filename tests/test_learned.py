@@ -190,6 +190,58 @@ def test_tensor_core_layers_on_many_tiles():
     assert rel_l2(res[True][1], res[False][1]) <= 2e-2
 
 
+def _irregular(n, most, seed):
+    """Symmetric M-matrix whose rows hold between 0 and about 2 `most` entries."""
+    rng = np.random.default_rng(seed)
+    pairs = set()
+    for i in range(n):
+        for j in rng.integers(0, n, rng.integers(0, most + 1)):
+            if i != j:
+                pairs.add((min(i, int(j)), max(i, int(j))))
+    pairs = sorted(pairs)
+    rows = [[] for _ in range(n)]
+    for a, b in pairs:
+        c = rng.uniform(0.1, 2.0)
+        rows[a].append((b, c))
+        rows[b].append((a, c))
+    row = np.zeros(n + 1, np.int32)
+    row[1:] = np.cumsum([len(r) for r in rows])
+    col = np.array([j for r in rows for j, _ in r], np.int32)
+    off = np.array([c for r in rows for _, c in r])
+    diag = -np.array([sum(c for _, c in r) for r in rows]) - rng.uniform(0.1, 0.5, n)
+    return row, col, diag, off
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,most", [(9, 2), (127, 3), (128, 6), (129, 4), (1100, 9)])
+def test_tensor_core_layers_on_irregular_rows(n, most):
+    """The layers gather four entries of eight rows at a time: rows with none,
+    with more than four and of unequal lengths, on one tile, at its edges and
+    on several. Forward against the FP64 restatement; gradient against it too:
+    TF32 moves a pre-activation by about 2^-11 of its terms, so about 2 * 2^-11
+    * 0.4 = 4e-4 of the units of a layer change side of the ReLU and over three
+    layers a gradient block moves by about sqrt(3 * 4e-4) = 3.5e-2 of its norm
+    (one unit of a graph of n nodes by sqrt(1 / 16 n)); a missed entry by a
+    share of its row's sum, above 1e-1."""
+    from fvm_b200.learned import LearnedCorrection
+
+    row, col, diag, off = _irregular(n, most, seed=20 + n)
+    rng = np.random.default_rng(21)
+    lc = LearnedCorrection(seed=0)
+    P = rng.normal(0, 0.25, mo.N_PARAMS).astype(np.float32)
+    lc.setParams(P)
+    r = rng.normal(size=n)
+    e = rng.normal(size=n)
+    P64 = P.astype(np.float64)
+    assert rel_l2(lc.forward_csr(row, col, diag, off, r), mo.forward(P64, row, col, diag, off, r)) <= _TOL[True][0]
+    g, loss = lc.gradient_csr(row, col, diag, off, r, e)
+    lref, gref = mo.loss_and_gradient(P64, row, col, diag, off, r, e)
+    assert abs(loss - lref) <= _TOL[True][1] * lref
+    tol = 6e-2 + (1.0 / (16 * n)) ** 0.5
+    for a, b in _BLOCKS:
+        assert rel_l2(g[a:b], gref[a:b]) <= tol, a
+
+
 def _plain(nPre=1, nPost=1):
     from fvm_b200 import fvmbaseExt
 
