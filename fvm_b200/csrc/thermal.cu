@@ -46,6 +46,8 @@ ThermalModel::~ThermalModel() {
   if (hPinned_) cudaFreeHost(hPinned_);
   if (dSegOff_) cudaFree(dSegOff_);
   if (dSegNorm_) cudaFree(dSegNorm_);
+  if (dSegChunk_) cudaFree(dSegChunk_);
+  if (dSegPart_) cudaFree(dSegPart_);
 }
 
 void ThermalModel::freeDevice() {
@@ -92,11 +94,17 @@ void ThermalModel::init() {
   initialized_ = true;
 }
 
+namespace {
+constexpr int kSegChunk = 2048;  // cells of a segment a CUDA block takes in its norm
+}
+
 void ThermalModel::setSegments(const std::vector<int>& offsets) {
   if (dSegOff_) cudaFree(dSegOff_);
   if (dSegNorm_) cudaFree(dSegNorm_);
-  dSegOff_ = nullptr;
-  dSegNorm_ = nullptr;
+  if (dSegChunk_) cudaFree(dSegChunk_);
+  if (dSegPart_) cudaFree(dSegPart_);
+  dSegOff_ = dSegChunk_ = nullptr;
+  dSegNorm_ = dSegPart_ = nullptr;
   segOff_.clear();
   if (!offsets.empty()) {
     FVM_REQUIRE(offsets.size() >= 2 && offsets.front() == 0 && offsets.back() == mesh_->nCells, kBadArgument,
@@ -106,6 +114,13 @@ void ThermalModel::setSegments(const std::vector<int>& offsets) {
     segOff_ = offsets;
     CUDA_OK(cudaMalloc(&dSegOff_, sizeof(int) * segOff_.size()));
     CUDA_OK(cudaMemcpy(dSegOff_, segOff_.data(), sizeof(int) * segOff_.size(), cudaMemcpyHostToDevice));
+    std::vector<int> chunk(1, 0);
+    for (size_t s = 0; s + 1 < segOff_.size(); s++)
+      chunk.push_back(chunk.back() + (segOff_[s + 1] - segOff_[s] + kSegChunk - 1) / kSegChunk);
+    segChunks_ = chunk.back();
+    CUDA_OK(cudaMalloc(&dSegChunk_, sizeof(int) * chunk.size()));
+    CUDA_OK(cudaMemcpy(dSegChunk_, chunk.data(), sizeof(int) * chunk.size(), cudaMemcpyHostToDevice));
+    CUDA_OK(cudaMalloc(&dSegPart_, sizeof(double) * (size_t)segChunks_));
     CUDA_OK(cudaMalloc(&dSegNorm_, sizeof(double) * (segOff_.size() - 1)));
   }
   segFirst_.assign(numSegments(), -1.0);
@@ -121,21 +136,49 @@ void ThermalModel::segmentStatus(std::vector<double>& first, std::vector<double>
 }
 
 namespace {
-// L1 norm of b over each block of cells (reference order; b is in the
-// solver's permuted order), one CUDA block per segment, fixed summation order
-__global__ void k_segment_l1(const int* __restrict__ off, const int* __restrict__ perm, const double* __restrict__ b,
-                             double* out) {
-  __shared__ double red[256];
-  const int s = blockIdx.x;
-  double acc = 0.0;
-  for (int i = off[s] + threadIdx.x; i < off[s + 1]; i += blockDim.x) acc += fabs(b[perm[i]]);
-  red[threadIdx.x] = acc;
-  __syncthreads();
-  for (int o = blockDim.x >> 1; o > 0; o >>= 1) {
-    if ((int)threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
-    __syncthreads();
+// L1 norm of b over each segment of cells (reference order; b is in the
+// solver's permuted order): a CUDA block per chunk of at most kSegChunk cells
+// (chunk[s] .. chunk[s + 1] are segment s's), then a warp per segment over its
+// chunks' sums. The order depends on the segment's own length alone. With a
+// block per segment 24 meshes kept 24 of 148 SMs busy: 129 us at 686k cells,
+// now 4.1 (and 1.6 for the sums).
+__global__ void __launch_bounds__(256) k_segment_l1(int nSeg, const int* __restrict__ off,
+                                                    const int* __restrict__ chunk, const int* __restrict__ perm,
+                                                    const double* __restrict__ b, double* partial) {
+  __shared__ double red[8];
+  int lo = 0, hi = nSeg;  // chunk[lo] <= blockIdx.x < chunk[hi]
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (chunk[mid] <= (int)blockIdx.x) lo = mid;
+    else hi = mid;
   }
-  if (threadIdx.x == 0) out[s] = red[0];
+  const int first = off[lo] + ((int)blockIdx.x - chunk[lo]) * kSegChunk;
+  const int last = min(first + kSegChunk, off[lo + 1]);
+  int at[kSegChunk / 256];
+#pragma unroll
+  for (int k = 0; k < kSegChunk / 256; k++) {
+    const int i = first + k * 256 + (int)threadIdx.x;
+    at[k] = i < last ? perm[i] : -1;
+  }
+  double acc = 0.0;
+#pragma unroll
+  for (int k = 0; k < kSegChunk / 256; k++) acc += at[k] >= 0 ? fabs(b[at[k]]) : 0.0;
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; w++) acc += red[w];
+    partial[blockIdx.x] = acc;
+  }
+}
+__global__ void k_segment_sum(int nSeg, const int* __restrict__ chunk, const double* __restrict__ partial,
+                              double* out) {
+  const int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (s >= nSeg) return;
+  double acc = 0.0;
+  for (int c = chunk[s] + lane; c < chunk[s + 1]; c += 32) acc += partial[c];
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+  if (lane == 0) out[s] = acc;
 }
 
 // Outer-loop state of advance() on the device; the outer norms follow it at
@@ -1068,8 +1111,10 @@ void ThermalModel::advance(int niter, AdvanceReport& rep) {
     }
     rep.launches += 4;
     if (dSegNorm_) {
-      k_segment_l1<<<numSegments(), 256, 0, stream_>>>(dSegOff_, dPerm_, hier_.level(0).b, dSegNorm_);
-      rep.launches += 1;
+      const int ns = numSegments();
+      k_segment_l1<<<segChunks_, 256, 0, stream_>>>(ns, dSegOff_, dSegChunk_, dPerm_, hier_.level(0).b, dSegPart_);
+      k_segment_sum<<<(ns + 7) / 8, 256, 0, stream_>>>(ns, dSegChunk_, dSegPart_, dSegNorm_);
+      rep.launches += 2;
     }
     SolveReport sr;
     {

@@ -252,6 +252,9 @@ class ThermalModel {
   std::vector<int> segOff_;
   int* dSegOff_ = nullptr;
   double* dSegNorm_ = nullptr;
+  int* dSegChunk_ = nullptr;  // per segment the first of its chunks (one block's share of the norm)
+  double* dSegPart_ = nullptr;
+  int segChunks_ = 0;
   std::vector<double> segFirst_, segLast_;
   std::vector<int> segConvergedAt_;
   bool segmentsConverged();

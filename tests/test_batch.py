@@ -122,3 +122,35 @@ def test_parallel_block_aggregation_equals_sequential():
     assert s1 == s2
     for a, b in zip(c1, c2):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.gpu
+def test_segment_norms_at_chunk_edges():
+    """Each mesh's norm is summed in chunks of 2048 cells: meshes of fewer
+    cells, one chunk exactly, one cell less and more, and several chunks in
+    one batch. The first norm of every mesh equals the initial residual norm
+    of the mesh solved alone: the same n <= 10403 terms in another order, so
+    to n 2^-53 = 1.2e-12 at most."""
+    from fvm_b200 import fvmbaseExt
+
+    ms = []
+    for i, (nx, ny) in enumerate([(3, 3), (23, 89), (8, 256), (683, 3), (101, 103)]):
+        m = meshgen.quad_mesh(nx, jitter=0.2, seed=i, ny=ny)
+        rng = np.random.default_rng(40 + i)
+        ms.append((m, np.exp(rng.normal(size=m["nCells"])), rng.uniform(size=m["nCells"])))
+    assert [m["nCells"] for m, _, _ in ms] == [9, 2047, 2048, 2049, 10403]
+    bc = {1: ("T", 300.0), 2: ("T", 400.0)}
+
+    def solve(part):
+        amg = fvmbaseExt.AMG()
+        amg.relativeTolerance = 0.1
+        amg.nMaxIterations = 50
+        bt = batch.BatchedThermal([m for m, _, _ in part], bc, amg, relative_tolerance=1e-6)
+        _, rep = bt.solve([k for _, k, _ in part], [s for _, _, s in part])
+        return bt.status()[0], rep
+
+    first, _ = solve(ms)
+    for i, one in enumerate(ms):
+        alone, rep = solve([one])
+        assert abs(first[i] - rep.initialNorm) <= 2e-12 * rep.initialNorm
+        assert first[i] == alone[0]
