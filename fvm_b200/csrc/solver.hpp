@@ -138,10 +138,11 @@ struct DevLevel {
   size_t entries = 0;
 };
 
-// Device allocations of one owner. release() keeps the blocks for reuse by
-// later alloc() calls of the same size (a rebuilt AMG hierarchy on the same
-// mesh asks for the same sizes), so rebuilding does not pay cudaFree /
-// cudaMalloc again; the destructor frees everything.
+// Device allocations of one owner: small arrays from a few chunks, large ones
+// as blocks of their own (256-byte aligned all). release() keeps chunks and
+// blocks for later alloc() calls (blocks for the same size: a rebuilt AMG
+// hierarchy on the same mesh asks for the same sizes), so rebuilding does not
+// pay cudaFree / cudaMalloc again; the destructor frees everything.
 class DeviceArena {
  public:
   ~DeviceArena();
@@ -163,6 +164,12 @@ class DeviceArena {
   void copy_h2d(void* d, const void* h, size_t n);
   std::vector<std::pair<void*, size_t>> ptrs_;
   std::multimap<size_t, void*> free_;
+  struct Chunk {
+    void* p = nullptr;
+    size_t size = 0, used = 0;
+  };
+  std::vector<Chunk> chunks_;  // of the small arrays
+  size_t chunk_ = 0;           // the one being filled
   size_t bytes_ = 0;
   std::mutex mu_;  // levels are uploaded from several setup threads
 };
