@@ -15,6 +15,7 @@
 #include <cstdlib>
 
 #include "common.hpp"
+#include "pdl.cuh"
 #include "solver.hpp"
 
 namespace fvm {
@@ -67,13 +68,19 @@ __device__ __forceinline__ int block_exclusive_scan(int v, int& total) {
   return off + x - v;
 }
 
-__global__ void k_scan_tiles(const int* __restrict__ in, int* out, int n, int* tileSum) {
+// Exclusive scan in two kernels: each tile's own scan with its total, then
+// every tile adds the totals of those before it (a block sums them itself:
+// 1500 tiles are 6 loads a thread, less than a launch of their own). In is
+// what is scanned: In(i), and done(i) once it has been read.
+template <class In>
+__global__ void __launch_bounds__(kT) k_scan_tiles(In in, int* out, int n, int* tileSum) {
+  FVM_PDL();
   const int base = blockIdx.x * kScanTile + threadIdx.x * 4;
   int v[4];
   int s = 0;
 #pragma unroll
   for (int q = 0; q < 4; q++) {
-    v[q] = base + q < n ? in[base + q] : 0;
+    v[q] = base + q < n ? in(base + q) : 0;
     s += v[q];
   }
   int total;
@@ -86,29 +93,41 @@ __global__ void k_scan_tiles(const int* __restrict__ in, int* out, int n, int* t
   if (threadIdx.x == 0) tileSum[blockIdx.x] = total;
 }
 
-// one block: exclusive scan of the tile sums in place, total at [nTiles]
-__global__ void k_scan_tile_sums(int* tileSum, int nTiles) {
-  const int per = (nTiles + kT - 1) / kT;
-  const int b = threadIdx.x * per;
+// host (pinned) gets the total and, with extra, extra[0] and extra[1]
+__global__ void __launch_bounds__(kT) k_scan_add(int* out, int n, const int* tileSum, int* host, const int* extra) {
+  FVM_PDL();
+  __shared__ int part[kT / 32];
+  const int tile = blockIdx.x;
   int s = 0;
-  for (int q = 0; q < per; q++)
-    if (b + q < nTiles) s += tileSum[b + q];
-  int total;
-  int e = block_exclusive_scan(s, total);
-  for (int q = 0; q < per; q++)
-    if (b + q < nTiles) {
-      const int t = tileSum[b + q];
-      tileSum[b + q] = e;
-      e += t;
+  for (int t = threadIdx.x; t < tile; t += kT) s += tileSum[t];
+  s = __reduce_add_sync(kFull, s);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
+  __syncthreads();
+  int off = 0;
+#pragma unroll
+  for (int w = 0; w < kT / 32; w++) off += part[w];
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    const int i = tile * kScanTile + q * kT + threadIdx.x;
+    if (i < n) out[i] += off;
+  }
+  if (tile == (int)gridDim.x - 1 && threadIdx.x == 0) {
+    const int total = off + tileSum[tile];
+    out[n] = total;
+    if (host) {
+      host[0] = total;
+      if (extra) {
+        host[1] = extra[0];
+        host[2] = extra[1];
+      }
     }
-  if (threadIdx.x == 0) tileSum[nTiles] = total;
+  }
 }
 
-__global__ void k_scan_add(int* out, int n, const int* tileSum, int nTiles) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) out[i] += tileSum[i / kScanTile];
-  if (i == 0) out[n] = tileSum[nTiles];
-}
+struct ScanArray {
+  const int* in;
+  __device__ int operator()(int i) const { return in[i]; }
+};
 
 __global__ void k_fill_finest_vals(long long entries, const int* __restrict__ posSrc, const double* __restrict__ src,
                                    double* vals, float* valsF) {
@@ -140,7 +159,56 @@ __device__ __forceinline__ double strength(double v, double di, double dj) { ret
 // result with a quarter of the dependent round trips to memory.
 constexpr int kAggChunk = 4;
 
-__global__ void k_agg_init(LevelRows a, double* maxw, int* partner) {
+// the strongest candidate of row i among its entries whose neighbour is
+// unpaired (partner[j] == -1), paired (>= 0) or any, strength at least thr
+// (ties: smaller index); -1 when none
+enum Candidates { kUnpaired, kPaired, kAny };
+template <Candidates Which>
+__device__ __forceinline__ int agg_strongest(const LevelRows& a, int i, double thr, const int* partner) {
+  int base, w;
+  row_range(a, i, base, w);
+  const double di = fabs(a.diag[i]);
+  int bj = -1;
+  double bw = 0.0;
+  for (int k0 = 0; k0 < w; k0 += kAggChunk) {
+    int jj[kAggChunk];
+    double vv[kAggChunk], dj[kAggChunk];
+    bool use[kAggChunk];
+#pragma unroll
+    for (int u = 0; u < kAggChunk; u++) {
+      use[u] = false;
+      if (k0 + u < w) {
+        jj[u] = a.cols[base + 32 * (k0 + u)];
+        vv[u] = a.vals[base + 32 * (k0 + u)];
+        use[u] = !(jj[u] == i || vv[u] == 0.0);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kAggChunk; u++)
+      if (Which != kAny && use[u]) {
+        const int p = partner[jj[u]];
+        use[u] = Which == kPaired ? p >= 0 : p == -1;
+      }
+#pragma unroll
+    for (int u = 0; u < kAggChunk; u++)
+      if (use[u]) dj[u] = fabs(a.diag[jj[u]]);
+#pragma unroll
+    for (int u = 0; u < kAggChunk; u++) {
+      if (!use[u]) continue;
+      const double s = strength(vv[u], di, dj[u]);
+      if (!(s > 0.0) || s < thr) continue;
+      if (s > bw || (s == bw && jj[u] < bj)) {
+        bw = s;
+        bj = jj[u];
+      }
+    }
+  }
+  return bj;
+}
+
+// round one: every row's strongest entry, its strongest candidate, no partner
+__global__ void k_agg_first(LevelRows a, double beta, double* maxw, int* partner, int* best) {
+  FVM_PDL();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.n) return;
   int base, w;
@@ -169,68 +237,24 @@ __global__ void k_agg_init(LevelRows a, double* maxw, int* partner) {
   }
   maxw[i] = m;
   partner[i] = -1;
-}
-
-// the strongest candidate of row i among its entries whose neighbour j has
-// (paired ? partner[j] >= 0 : partner[j] == -1), strength at least thr
-// (ties: smaller index); -1 when none
-template <bool Paired>
-__device__ __forceinline__ int agg_strongest(const LevelRows& a, int i, double thr, const int* __restrict__ partner) {
-  int base, w;
-  row_range(a, i, base, w);
-  const double di = fabs(a.diag[i]);
-  int bj = -1;
-  double bw = 0.0;
-  for (int k0 = 0; k0 < w; k0 += kAggChunk) {
-    int jj[kAggChunk];
-    double vv[kAggChunk], dj[kAggChunk];
-    bool use[kAggChunk];
-#pragma unroll
-    for (int u = 0; u < kAggChunk; u++) {
-      use[u] = false;
-      if (k0 + u < w) {
-        jj[u] = a.cols[base + 32 * (k0 + u)];
-        vv[u] = a.vals[base + 32 * (k0 + u)];
-        use[u] = !(jj[u] == i || vv[u] == 0.0);
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < kAggChunk; u++)
-      if (use[u]) {
-        const int p = partner[jj[u]];
-        use[u] = Paired ? p >= 0 : p == -1;
-      }
-#pragma unroll
-    for (int u = 0; u < kAggChunk; u++)
-      if (use[u]) dj[u] = fabs(a.diag[jj[u]]);
-#pragma unroll
-    for (int u = 0; u < kAggChunk; u++) {
-      if (!use[u]) continue;
-      const double s = strength(vv[u], di, dj[u]);
-      if (!(s > 0.0) || s < thr) continue;
-      if (s > bw || (s == bw && jj[u] < bj)) {
-        bw = s;
-        bj = jj[u];
-      }
-    }
-  }
-  return bj;
+  best[i] = agg_strongest<kAny>(a, i, beta * m, partner);
 }
 
 // strongest unpaired candidate of every unpaired row (ties: smaller index)
-__global__ void k_agg_best(LevelRows a, const double* __restrict__ maxw, double beta, const int* __restrict__ partner,
-                           int* best) {
+__global__ void k_agg_best(LevelRows a, const double* maxw, double beta, const int* partner, int* best) {
+  FVM_PDL();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.n) return;
   if (partner[i] != -1) {
     best[i] = -1;
     return;
   }
-  best[i] = agg_strongest<false>(a, i, beta * maxw[i], partner);
+  best[i] = agg_strongest<kUnpaired>(a, i, beta * maxw[i], partner);
 }
 
 // handshake: i and j pair when each is the other's strongest candidate
-__global__ void k_agg_match(int n, const int* __restrict__ best, int* partner) {
+__global__ void k_agg_match(int n, const int* best, int* partner) {
+  FVM_PDL();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n || partner[i] != -1) return;
   const int j = best[i];
@@ -238,67 +262,80 @@ __global__ void k_agg_match(int n, const int* __restrict__ best, int* partner) {
 }
 
 // an unpaired row joins the pair of its strongest paired candidate
-__global__ void k_agg_join(LevelRows a, const double* __restrict__ maxw, double beta, const int* __restrict__ partner,
-                           int* join) {
+__global__ void k_agg_join(LevelRows a, const double* maxw, double beta, const int* partner, int* join) {
+  FVM_PDL();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.n) return;
   if (partner[i] != -1) {
     join[i] = -1;
     return;
   }
-  join[i] = agg_strongest<true>(a, i, beta * maxw[i], partner);
+  join[i] = agg_strongest<kPaired>(a, i, beta * maxw[i], partner);
 }
 
-__device__ __forceinline__ bool is_leader(int i, const int* partner, const int* join) {
+// the row whose coarse row i belongs to: the smaller of its pair, of the
+// pair it joins, or itself
+__device__ __forceinline__ int agg_leader(int i, const int* partner, const int* join) {
   const int p = partner[i];
-  return p >= 0 ? i < p : join[i] < 0;
+  if (p >= 0) return min(i, p);
+  const int j = join[i];
+  return j < 0 ? i : min(j, partner[j]);
 }
 
-__global__ void k_agg_flags(int n, const int* __restrict__ partner, const int* __restrict__ join,
-                            const int* __restrict__ order, int* flag) {
+// 1 for the leading rows, in the level's own order ...
+struct ScanLeaders {
+  const int *partner, *join;
+  __device__ int operator()(int i) const {
+    const int p = partner[i];
+    return (p >= 0 ? i < p : join[i] < 0) ? 1 : 0;
+  }
+};
+// ... or scattered into another
+__global__ void k_agg_flags(int n, const int* partner, const int* join, const int* order, int* flag) {
+  FVM_PDL();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) flag[order[i]] = ScanLeaders{partner, join}(i);
+}
+
+__global__ void k_agg_ci(int n, const int* partner, const int* join, const int* order, const int* pos, int* ci) {
+  FVM_PDL();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  flag[order ? order[i] : i] = is_leader(i, partner, join) ? 1 : 0;
-}
-
-__global__ void k_agg_ci_leaders(int n, const int* __restrict__ partner, const int* __restrict__ join,
-                                 const int* __restrict__ order, const int* __restrict__ pos, int* ci) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n || !is_leader(i, partner, join)) return;
-  ci[i] = pos[order ? order[i] : i];
-}
-
-__global__ void k_agg_ci_rest(int n, const int* __restrict__ partner, const int* __restrict__ join, int* ci) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n || is_leader(i, partner, join)) return;
-  const int p = partner[i];
-  if (p >= 0) {
-    ci[i] = ci[p];  // the pair's leader is its smaller row
-  } else {
-    const int j = join[i];
-    const int q = partner[j];
-    ci[i] = ci[j < q ? j : q];
-  }
+  const int l = agg_leader(i, partner, join);
+  ci[i] = pos[order ? order[l] : l];
 }
 
 // ---- coarse-to-fine lists ------------------------------------------------------
 
-__global__ void k_c2f_count(int n, const int* __restrict__ ci, int* cnt) {
+// cnt is zero on entry and again when the lists are done
+__global__ void k_c2f_count(int n, const int* ci, int* cnt) {
+  FVM_PDL();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) atomicAdd(&cnt[ci[i]], 1);
 }
+// the counts, cleared as they are read: next they are the lists' cursors
+struct ScanCounts {
+  int* cnt;
+  __device__ int operator()(int i) const {
+    const int c = cnt[i];
+    cnt[i] = 0;
+    return c;
+  }
+};
 
-__global__ void k_c2f_place(int n, const int* __restrict__ ci, const int* __restrict__ c2fRow, int* cursor,
-                            int* c2fCol) {
+__global__ void k_c2f_place(int n, const int* ci, const int* c2fRow, int* cursor, int* c2fCol) {
+  FVM_PDL();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int c = ci[i];
   c2fCol[c2fRow[c] + atomicAdd(&cursor[c], 1)] = i;
 }
 
-__global__ void k_c2f_sort(int nc, const int* __restrict__ c2fRow, int* c2fCol) {
+__global__ void k_c2f_sort(int nc, const int* c2fRow, int* cnt, int* c2fCol) {
+  FVM_PDL();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= nc) return;
+  cnt[c] = 0;
   const int b = c2fRow[c], e = c2fRow[c + 1];
   for (int q = b + 1; q < e; q++) {
     const int v = c2fCol[q];
@@ -315,34 +352,42 @@ __global__ void k_c2f_sort(int nc, const int* __restrict__ c2fRow, int* c2fCol) 
 
 constexpr int kGalWarps = 4;
 
+// One warp per coarse row. The entries of its fine rows (rows ascending,
+// entries in stored order) are taken 32 at a time, one a lane: lanes of one
+// coarse column find each other with a match, the lowest looks the column up
+// among those found before (U, in first-visit order; S their sums) and adds
+// the lanes' values in lane order, so every sum is in stored order. Scanning
+// all earlier entries of the row for each entry, and lane 0 summing the
+// diagonal over all of them, took 190 us a launch (70 for the counts) on the
+// levels of 1.5M tets; this takes GAL_US.
 template <bool kFill>
-__global__ void __launch_bounds__(32 * kGalWarps) k_galerkin(LevelRows a, int nc, const int* __restrict__ ci,
-                                                             const int* __restrict__ c2fRow,
-                                                             const int* __restrict__ c2fCol, int* count,
-                                                             int* overflow, const int* __restrict__ sliceOff,
-                                                             int* ccols, double* cvals, float* cvalsF,
-                                                             double* cdiag, float* cdiagF) {
-  __shared__ int sJ[kGalWarps][kGalerkinCap];
-  __shared__ double sV[kGalWarps][kGalerkinCap];
+__global__ void __launch_bounds__(32 * kGalWarps) k_galerkin(LevelRows a, int nc, const int* ci, const int* c2fRow,
+                                                             const int* c2fCol, int* count, int* overflow,
+                                                             const int* sliceOff, int* ccols, double* cvals,
+                                                             float* cvalsF, double* cdiag, float* cdiagF) {
+  __shared__ int sU[kGalWarps][kGalerkinCap];
+  __shared__ double sS[kFill ? kGalWarps : 1][kFill ? kGalerkinCap : 1];
   __shared__ int sOff[kGalWarps][32], sBase[kGalWarps][32], sRow[kGalWarps][32];
   __shared__ double sDiag[kGalWarps][32];
+  FVM_PDL();
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int I = blockIdx.x * kGalWarps + wid;
-  if (I >= nc) return;  // the whole warp leaves together
-  int* J = sJ[wid];
-  double* V = sV[wid];
+  if (I >= nc) {  // the whole warp leaves together
+    // lanes of the last slice past the last row: column 0, so that no index
+    // in the level is undefined (the fill covers whole slices)
+    if (kFill && I < ((nc + 31) & ~31)) {
+      const int s = I >> 5, cw = (sliceOff[s + 1] - sliceOff[s]) >> 5;
+      for (int slot = lane; slot < cw; slot += 32) ccols[sliceOff[s] + (I & 31) + 32 * (size_t)slot] = 0;
+    }
+    return;
+  }
+  int* U = sU[wid];
+  double* S = sS[kFill ? wid : 0];
   const int f0 = c2fRow[I], f1 = c2fRow[I + 1];
-  // the coarse diagonal (fill pass, lane 0): fine diagonals plus the entries
-  // inside the aggregate, fine rows ascending, entries in stored order,
-  // summed chunk by chunk from the values staged in shared memory
-  double dsum = 0.0;
-  // every entry of the aggregate's fine rows, fine rows ascending, entries
-  // in stored order; J = coarse column (-1: padding). Up to 32 fine rows at
-  // a time: each lane looks up one row's range, a warp scan places the rows,
-  // and the lanes then gather all their entries at once.
-  int L = 0;
-  bool over = false;
+  double dsum = 0.0;  // fine diagonals plus the entries inside the aggregate
+  int L = 0, nU = 0;
   for (int q0 = f0; q0 < f1; q0 += 32) {
+    // up to 32 fine rows: each lane looks one up, a warp scan places them
     const int nq = min(32, f1 - q0);
     int base = 0, w = 0, f = -1;
     if (lane < nq) {
@@ -357,128 +402,121 @@ __global__ void __launch_bounds__(32 * kGalWarps) k_galerkin(LevelRows a, int nc
     }
     const int tot = __shfl_sync(kFull, incl, 31);
     if (L + tot > kGalerkinCap) {
-      over = true;
-      break;
+      if (lane == 0) {
+        atomicExch(overflow, 1);
+        if (!kFill) count[I] = 0;
+      }
+      return;
     }
+    L += tot;
     sOff[wid][lane] = incl - w;
     sBase[wid][lane] = base;
     sRow[wid][lane] = f;
     __syncwarp();
-    for (int e = lane; e < tot; e += 32) {
-      // the last row q < nq whose range starts at or before e
-      int lo = 0, hi = nq - 1;
-      while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (sOff[wid][mid] <= e)
-          lo = mid;
-        else
-          hi = mid - 1;
+    int qd = 0;  // rows whose diagonal is in dsum
+    for (int e0 = 0; e0 < tot; e0 += 32) {
+      const int e = e0 + lane;
+      int J = -1;
+      double v = 0.0;
+      if (e < tot) {
+        // the last row q < nq whose range starts at or before e
+        int lo = 0, hi = nq - 1;
+        while (lo < hi) {
+          const int mid = (lo + hi + 1) >> 1;
+          if (sOff[wid][mid] <= e)
+            lo = mid;
+          else
+            hi = mid - 1;
+        }
+        const int idx = sBase[wid][lo] + 32 * (e - sOff[wid][lo]);
+        const int j = a.cols[idx];
+        v = a.vals[idx];
+        if (j != sRow[wid][lo] && v != 0.0) J = ci[j];  // else padding
       }
-      const int idx = sBase[wid][lo] + 32 * (e - sOff[wid][lo]);
-      const int j = a.cols[idx];
-      const double v = a.vals[idx];
-      J[L + e] = (j == sRow[wid][lo] || v == 0.0) ? -1 : ci[j];
-      V[L + e] = v;
+      if (kFill) {
+        unsigned in = __ballot_sync(kFull, J == I);
+        while (in) {
+          const int b = __ffs(in) - 1;
+          in &= in - 1;
+          while (qd < nq && sOff[wid][qd] <= e0 + b) dsum += sDiag[wid][qd++];
+          dsum += __shfl_sync(kFull, v, b);
+        }
+      }
+      const bool live = J >= 0 && J != I;
+      int slot = -1;
+      for (int k = 0; k < nU; k++)
+        if (U[k] == J) slot = k;
+      const unsigned same = __match_any_sync(kFull, live ? J : -2 - lane);
+      const bool leader = live && __ffs(same) - 1 == lane;
+      const unsigned found = __ballot_sync(kFull, leader && slot < 0);
+      const bool isNew = leader && slot < 0;
+      if (isNew) slot = nU + __popc(found & ((1u << lane) - 1u));
+      if (kFill) {
+        double s = leader && !isNew ? S[slot] : 0.0;
+        unsigned rest = leader ? same : 0u;
+        while (__any_sync(kFull, rest != 0u)) {
+          const double vb = __shfl_sync(kFull, v, rest ? __ffs(rest) - 1 : lane);
+          if (rest) s += vb;
+          rest &= rest - 1u;
+        }
+        if (leader) S[slot] = s;
+      }
+      __syncwarp();  // every lane has searched U
+      if (isNew) U[slot] = J;
+      nU += __popc(found);
+      __syncwarp();
     }
+    if (kFill)
+      while (qd < nq) dsum += sDiag[wid][qd++];
     __syncwarp();
-    if (kFill && lane == 0) {
-      int e = L;
-      for (int q = 0; q < nq; q++) {
-        dsum += sDiag[wid][q];
-        const int we = (q + 1 < nq ? sOff[wid][q + 1] : tot) - sOff[wid][q];
-        for (int k = 0; k < we; k++, e++)
-          if (J[e] == I) dsum += V[e];
-      }
-    }
-    __syncwarp();
-    L += tot;
-  }
-  __syncwarp();
-  if (over) {
-    if (lane == 0) {
-      atomicExch(overflow, 1);
-      if (!kFill) count[I] = 0;
-    }
-    return;
-  }
-  int cbase = 0, cw = 0;
-  if (kFill) {
-    const int s = I >> 5;
-    cbase = sliceOff[s] + (I & 31);
-    cw = (sliceOff[s + 1] - sliceOff[s]) >> 5;
-  }
-  // off-diagonal coarse columns in first-visit order; each first visit sums
-  // every later entry of its column in stored order
-  int nUnique = 0;
-  for (int e0 = 0; e0 < L; e0 += 32) {
-    const int e = e0 + lane;
-    bool first = false;
-    int Je = -1;
-    if (e < L) {
-      Je = J[e];
-      if (Je >= 0 && Je != I) {
-        first = true;
-        for (int e2 = 0; e2 < e; e2++)
-          if (J[e2] == Je) {
-            first = false;
-            break;
-          }
-      }
-    }
-    const unsigned m = __ballot_sync(kFull, first);
-    if (kFill && first) {
-      const int slot = nUnique + __popc(m & ((1u << lane) - 1u));
-      double s = 0.0;
-      for (int e2 = e; e2 < L; e2++)
-        if (J[e2] == Je) s += V[e2];
-      const size_t o = (size_t)cbase + 32 * (size_t)slot;
-      ccols[o] = Je;
-      cvals[o] = s;
-      if (cvalsF) cvalsF[o] = (float)s;
-    }
-    nUnique += __popc(m);
   }
   if constexpr (!kFill) {
-    if (lane == 0) count[I] = nUnique;
-    return;
+    if (lane == 0) count[I] = nU;
   } else {
-    for (int slot = nUnique + lane; slot < cw; slot += 32) {
+    const int s = I >> 5;
+    const int cbase = sliceOff[s] + (I & 31), cw = (sliceOff[s + 1] - sliceOff[s]) >> 5;
+    for (int slot = lane; slot < cw; slot += 32) {
       const size_t o = (size_t)cbase + 32 * (size_t)slot;
-      ccols[o] = I;
-      cvals[o] = 0.0;
-      if (cvalsF) cvalsF[o] = 0.f;
+      const bool used = slot < nU;  // else padding: own row, zero
+      const double v = used ? S[slot] : 0.0;
+      ccols[o] = used ? U[slot] : I;
+      cvals[o] = v;
+      if (cvalsF) cvalsF[o] = (float)v;
+    }
+    if (lane == 0) {
+      cdiag[I] = dsum;
+      if (cdiagF) cdiagF[I] = (float)dsum;
     }
   }
-  if (lane == 0) {
-    cdiag[I] = dsum;
-    if (cdiagF) cdiagF[I] = (float)dsum;
+}
+
+// a warp per slice; *maxWidth is zero on entry
+__global__ void k_slice_widths(int n, const int* count, int* width32, int* maxWidth) {
+  FVM_PDL();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if ((i & ~31) >= n) return;  // the whole warp leaves together
+  const int w = __reduce_max_sync(kFull, i < n ? count[i] : 0);
+  if ((i & 31) == 0) {
+    width32[i >> 5] = 32 * w;
+    atomicMax(maxWidth, w);
   }
 }
 
-__global__ void k_slice_widths(int n, const int* __restrict__ count, int* width32) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  const int ns = (n + 31) >> 5;
-  if (s >= ns) return;
-  int w = 0;
-  for (int r = s << 5; r < min(n, (s + 1) << 5); r++) w = max(w, count[r]);
-  width32[s] = 32 * w;
-}
-
-__global__ void k_slice_meta(int n, const int* __restrict__ sliceOff, int4* meta, int* sliceRow, int* sliceRows,
-                             int* rowSlice, int* maxWidth) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  const int ns = (n + 31) >> 5;
-  if (s >= ns) return;
-  const int r0 = s << 5, rows = min(32, n - r0);
-  const int w = (sliceOff[s + 1] - sliceOff[s]) >> 5;
-  meta[s] = make_int4(r0, rows, sliceOff[s], w);
-  sliceRow[s] = r0;
+__global__ void k_slice_meta(int n, const int* sliceOff, int4* meta, int* sliceRow, int* sliceRows, int* rowSlice) {
+  FVM_PDL();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int s = i >> 5;
+  rowSlice[i] = s;
+  if (i & 31) return;
+  const int rows = min(32, n - i), off = sliceOff[s];
+  meta[s] = make_int4(i, rows, off, (sliceOff[s + 1] - off) >> 5);
+  sliceRow[s] = i;
   sliceRows[s] = rows;
-  for (int r = 0; r < rows; r++) rowSlice[r0 + r] = s;
-  atomicMax(maxWidth, w);
 }
 
-__global__ void k_compose(int n, int* ci, const int* __restrict__ ci2) {
+__global__ void k_compose(int n, int* ci, const int* ci2) {
+  FVM_PDL();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) ci[i] = ci2[ci[i]];
 }
@@ -637,11 +675,18 @@ __global__ void k_ell_fill(int n, int rowsPadded, int W, const int* __restrict__
 
 int scan_scratch_ints(int n) { return cdiv(n, kScanTile) + 1; }
 
-void scan_exclusive(const int* in, int* out, int n, int* scratch, cudaStream_t st) {
+namespace {
+template <class In>
+void scan(const In& in, int* out, int n, int* scratch, cudaStream_t st, int* host = nullptr,
+          const int* extra = nullptr) {
   const int tiles = std::max(1, cdiv(n, kScanTile));
-  k_scan_tiles<<<tiles, kT, 0, st>>>(in, out, n, scratch);
-  k_scan_tile_sums<<<1, kT, 0, st>>>(scratch, tiles);
-  k_scan_add<<<std::max(1, cdiv(n, kT)), kT, 0, st>>>(out, n, scratch, tiles);
+  pdl_launch(k_scan_tiles<In>, tiles, kT, st, in, out, n, scratch);
+  pdl_launch(k_scan_add, tiles, kT, st, out, n, scratch, host, extra);
+}
+}  // namespace
+
+void scan_exclusive(const int* in, int* out, int n, int* scratch, cudaStream_t st, int* host, const int* extra) {
+  scan(ScanArray{in}, out, n, scratch, st, host, extra);
 }
 
 void fill_finest(long long entries, const int* posSrc, const double* src, double* vals, float* valsF, int n,
@@ -651,57 +696,55 @@ void fill_finest(long long entries, const int* posSrc, const double* src, double
 }
 
 void aggregate_pairs(const LevelRows& a, double beta, int rounds, const int* order, const AggWork& w, int* ci,
-                     cudaStream_t st) {
+                     int* nCoarse, cudaStream_t st) {
   const int n = a.n, g = cdiv(n, kT);
-  k_agg_init<<<g, kT, 0, st>>>(a, w.maxw, w.partner);
+  pdl_launch(k_agg_first, g, kT, st, a, beta, w.maxw, w.partner, w.best);
   for (int r = 0; r < rounds; r++) {
-    k_agg_best<<<g, kT, 0, st>>>(a, w.maxw, beta, w.partner, w.best);
-    k_agg_match<<<g, kT, 0, st>>>(n, w.best, w.partner);
+    if (r > 0) pdl_launch(k_agg_best, g, kT, st, a, w.maxw, beta, w.partner, w.best);
+    pdl_launch(k_agg_match, g, kT, st, n, w.best, w.partner);
   }
-  k_agg_join<<<g, kT, 0, st>>>(a, w.maxw, beta, w.partner, w.join);
-  k_agg_flags<<<g, kT, 0, st>>>(n, w.partner, w.join, order, w.flag);
-  scan_exclusive(w.flag, w.pos, n, w.scan, st);
-  k_agg_ci_leaders<<<g, kT, 0, st>>>(n, w.partner, w.join, order, w.pos, ci);
-  k_agg_ci_rest<<<g, kT, 0, st>>>(n, w.partner, w.join, ci);
+  pdl_launch(k_agg_join, g, kT, st, a, w.maxw, beta, w.partner, w.join);
+  if (order) {
+    pdl_launch(k_agg_flags, g, kT, st, n, w.partner, w.join, order, w.flag);
+    scan(ScanArray{w.flag}, w.pos, n, w.scan, st, nCoarse);
+  } else {
+    scan(ScanLeaders{w.partner, w.join}, w.pos, n, w.scan, st, nCoarse);
+  }
+  pdl_launch(k_agg_ci, g, kT, st, n, w.partner, w.join, order, w.pos, ci);
 }
 
 void coarse_to_fine(int n, int nc, const int* ci, int* cnt, int* c2fRow, int* c2fCol, int* scanScratch,
                     cudaStream_t st) {
-  cudaMemsetAsync(cnt, 0, sizeof(int) * (size_t)nc, st);
-  k_c2f_count<<<cdiv(n, kT), kT, 0, st>>>(n, ci, cnt);
-  scan_exclusive(cnt, c2fRow, nc, scanScratch, st);
-  cudaMemsetAsync(cnt, 0, sizeof(int) * (size_t)nc, st);
-  k_c2f_place<<<cdiv(n, kT), kT, 0, st>>>(n, ci, c2fRow, cnt, c2fCol);
-  k_c2f_sort<<<cdiv(nc, kT), kT, 0, st>>>(nc, c2fRow, c2fCol);
+  pdl_launch(k_c2f_count, cdiv(n, kT), kT, st, n, ci, cnt);
+  scan(ScanCounts{cnt}, c2fRow, nc, scanScratch, st);
+  pdl_launch(k_c2f_place, cdiv(n, kT), kT, st, n, ci, c2fRow, cnt, c2fCol);
+  pdl_launch(k_c2f_sort, cdiv(nc, kT), kT, st, nc, c2fRow, cnt, c2fCol);
 }
 
 void galerkin_count(const LevelRows& a, int nc, const int* ci, const int* c2fRow, const int* c2fCol, int* count,
                     int* overflow, cudaStream_t st) {
-  k_galerkin<false><<<cdiv(nc, kGalWarps), 32 * kGalWarps, 0, st>>>(a, nc, ci, c2fRow, c2fCol, count, overflow,
-                                                                      nullptr, nullptr, nullptr, nullptr, nullptr,
-                                                                      nullptr);
+  pdl_launch(k_galerkin<false>, cdiv(nc, kGalWarps), 32 * kGalWarps, st, a, nc, ci, c2fRow, c2fCol, count, overflow,
+             nullptr, nullptr, nullptr, nullptr, nullptr, nullptr);
 }
 
 void galerkin_fill(const LevelRows& a, int nc, const int* ci, const int* c2fRow, const int* c2fCol,
                    const int* sliceOff, int* cols, double* vals, float* valsF, double* diag, float* diagF,
-                   cudaStream_t st) {
-  k_galerkin<true><<<cdiv(nc, kGalWarps), 32 * kGalWarps, 0, st>>>(a, nc, ci, c2fRow, c2fCol, nullptr, nullptr,
-                                                                     sliceOff, cols, vals, valsF, diag, diagF);
+                   int* overflow, cudaStream_t st) {
+  pdl_launch(k_galerkin<true>, cdiv(cdiv(nc, 32) * 32, kGalWarps), 32 * kGalWarps, st, a, nc, ci, c2fRow, c2fCol,
+             nullptr, overflow, sliceOff, cols, vals, valsF, diag, diagF);
 }
 
-void slice_widths(int n, const int* count, int* width32, cudaStream_t st) {
-  const int ns = cdiv(n, 32);
-  k_slice_widths<<<cdiv(ns, kT), kT, 0, st>>>(n, count, width32);
+void slice_widths(int n, const int* count, int* width32, int* maxWidth, cudaStream_t st) {
+  pdl_launch(k_slice_widths, cdiv(n, kT), kT, st, n, count, width32, maxWidth);
 }
 
 void slice_meta_fill(int n, const int* sliceOff, int4* meta, int* sliceRow, int* sliceRows, int* rowSlice,
-                     int* maxWidth, cudaStream_t st) {
-  const int ns = cdiv(n, 32);
-  k_slice_meta<<<cdiv(ns, kT), kT, 0, st>>>(n, sliceOff, meta, sliceRow, sliceRows, rowSlice, maxWidth);
+                     cudaStream_t st) {
+  pdl_launch(k_slice_meta, cdiv(n, kT), kT, st, n, sliceOff, meta, sliceRow, sliceRows, rowSlice);
 }
 
 void compose_index(int n, int* ci, const int* ci2, cudaStream_t st) {
-  if (n > 0) k_compose<<<cdiv(n, kT), kT, 0, st>>>(n, ci, ci2);
+  if (n > 0) pdl_launch(k_compose, cdiv(n, kT), kT, st, n, ci, ci2);
 }
 
 }  // namespace dev
@@ -1016,7 +1059,15 @@ void AmgHierarchy::buildDevice(const FinestDevice& in, const SolverOptions& opt,
   w.flag = (int*)arena_.alloc(size_class(sizeof(int) * n0));
   w.pos = (int*)arena_.alloc(size_class(sizeof(int) * (n0 + 1)));
   w.scan = (int*)arena_.alloc(size_class(sizeof(int) * (dev::scan_scratch_ints(n0 + 1) + 1)));
-  int* flags = (int*)arena_.alloc(4096);  // [0] overflow, [1] max width, [2] not dominant
+  int* cnt = (int*)arena_.alloc(size_class(sizeof(int) * n0));  // zero between uses
+  CUDA_OK(cudaMemsetAsync(cnt, 0, sizeof(int) * (size_t)n0, st));
+  // [2] not dominant; from [4] on an overflow flag and a largest width for
+  // each Galerkin product
+  constexpr int kFlags = 1024;
+  int* flags = (int*)arena_.alloc(kFlags * sizeof(int));
+  CUDA_OK(cudaMemsetAsync(flags, 0, kFlags * sizeof(int), st));
+  int product = 4;
+  // what the host waits for is written straight to pinned memory
   int* hflags = reinterpret_cast<int*>(pinnedScalars());
   lap("level 0 values");
 
@@ -1028,18 +1079,22 @@ void AmgHierarchy::buildDevice(const FinestDevice& in, const SolverOptions& opt,
     fine.nCoarse = nc;
     fine.c2fRow = (int*)arena_.alloc(size_class(sizeof(int) * (nc + 1)));
     fine.c2fCol = (int*)arena_.alloc(size_class(sizeof(int) * fine.n));
-    dev::coarse_to_fine(fine.n, nc, ci, w.flag, fine.c2fRow, fine.c2fCol, w.scan, st);
+    dev::coarse_to_fine(fine.n, nc, ci, cnt, fine.c2fRow, fine.c2fCol, w.scan, st);
     const dev::LevelRows af{fine.n, fine.cols, fine.vals, fine.diag, fine.meta, fine.rowSlice, fine.ellWidth};
     const int nSlices = (nc + 31) / 32;
     int* sliceOff = (int*)arena_.alloc(size_class(sizeof(int) * (nSlices + 1)));
-    CUDA_OK(cudaMemsetAsync(flags, 0, 3 * sizeof(int), st));
-    dev::galerkin_count(af, nc, ci, fine.c2fRow, fine.c2fCol, w.best, flags, st);
-    dev::slice_widths(nc, w.best, w.join, st);
-    dev::scan_exclusive(w.join, sliceOff, nSlices, w.scan, st);
-    CUDA_OK(cudaMemcpyAsync(hflags, sliceOff + nSlices, sizeof(int), cudaMemcpyDeviceToHost, st));
-    CUDA_OK(cudaMemcpyAsync(hflags + 1, flags, sizeof(int), cudaMemcpyDeviceToHost, st));
+    if (product + 2 > kFlags) {
+      CUDA_OK(cudaMemsetAsync(flags + 4, 0, (kFlags - 4) * sizeof(int), st));
+      product = 4;
+    }
+    int* state = flags + product;
+    product += 2;
+    dev::galerkin_count(af, nc, ci, fine.c2fRow, fine.c2fCol, w.best, state, st);
+    dev::slice_widths(nc, w.best, w.join, state + 1, st);
+    dev::scan_exclusive(w.join, sliceOff, nSlices, w.scan, st, hflags, state);
     CUDA_OK(cudaStreamSynchronize(st));
     const long long E = hflags[0];
+    c.maxWidth = hflags[2];
     FVM_REQUIRE(hflags[1] == 0, kUnsupported,
                 "device-built hierarchy: an aggregate's entries exceed the Galerkin kernel's capacity");
     const size_t e1 = (size_t)std::max<long long>(E, 1);
@@ -1059,22 +1114,14 @@ void AmgHierarchy::buildDevice(const FinestDevice& in, const SolverOptions& opt,
     c.sliceRow = (int*)arena_.alloc(size_class(sizeof(int) * nSlices));
     c.sliceRows = (int*)arena_.alloc(size_class(sizeof(int) * nSlices));
     c.rowSlice = (int*)arena_.alloc(size_class(sizeof(int) * nc));
-    // the fill writes every row's entries and padding; the lanes of the last
-    // slice past the last row keep these (column 0) so that no index in the
-    // level is undefined
-    CUDA_OK(cudaMemsetAsync(c.cols, 0, sizeof(int) * e1, st));
     dev::galerkin_fill(af, nc, ci, fine.c2fRow, fine.c2fCol, sliceOff, c.cols, c.vals, c.valsF, c.diag, c.diagF,
-                       st);
-    dev::slice_meta_fill(nc, sliceOff, c.meta, c.sliceRow, c.sliceRows, c.rowSlice, flags + 1, st);
-    CUDA_OK(cudaMemcpyAsync(hflags, flags + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
-    CUDA_OK(cudaStreamSynchronize(st));
-    c.maxWidth = hflags[0];
+                       state, st);
+    dev::slice_meta_fill(nc, sliceOff, c.meta, c.sliceRow, c.sliceRows, c.rowSlice, st);
     return E;
   };
   // one matching: coarse size of `a`'s pairs (ci written)
   auto match = [&](const dev::LevelRows& a, const int* order, int* ci) {
-    dev::aggregate_pairs(a, opt.matchBeta, opt.matchRounds, order, w, ci, st);
-    CUDA_OK(cudaMemcpyAsync(hflags, w.pos + a.n, sizeof(int), cudaMemcpyDeviceToHost, st));
+    dev::aggregate_pairs(a, opt.matchBeta, opt.matchRounds, order, w, ci, hflags, st);
     CUDA_OK(cudaStreamSynchronize(st));
     return hflags[0];
   };

@@ -15,6 +15,7 @@
 #include <cstdint>
 
 #include "kernels.cuh"
+#include "pdl.cuh"
 
 namespace fvm {
 namespace dev {
@@ -136,13 +137,6 @@ __device__ __forceinline__ T row_sum(const SellView<T>& a, const int4 m, int lan
 // registers when the wait ends and only gathers then. (The vectors such a
 // kernel reads after the wait are not declared __restrict__: as read-only
 // parameters the compiler would be free to load them ahead of it.)
-#define FVM_PDL_TRIGGER() asm volatile("griddepcontrol.launch_dependents;" ::: "memory")
-#define FVM_PDL_WAIT() asm volatile("griddepcontrol.wait;" ::: "memory")
-#define FVM_PDL()      \
-  do {                 \
-    FVM_PDL_TRIGGER(); \
-    FVM_PDL_WAIT();    \
-  } while (0)
 
 // A slice's {first row, rows, offset, width}: loaded (SELL-32) or computed
 // (ELL-32: aligned 32-row groups of one width)
@@ -1597,22 +1591,6 @@ __global__ void k_update_ghosts(BoundaryData bd, const int* __restrict__ perm,
 // ---------------------------------------------------------------------------
 // wrappers
 
-namespace {
-template <typename... KArgs, typename... Args>
-void pdl_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStream_t st, Args... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = 0;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
-}
-}  // namespace
 template <class T>
 void gs_color(const SellView<T>& a, int s0, int s1, T* x, const T* b, cudaStream_t st, RowPlan plan, const T* xc,
               const int* ci) {

@@ -15,6 +15,7 @@
 
 #include "common.hpp"
 #include "learned.hpp"
+#include "pdl.cuh"
 #include "umma.cuh"
 
 namespace fvm {
@@ -35,33 +36,6 @@ int node_blocks(int n) {
   return b < 148 * 16 ? (b < 1 ? 1 : b) : 148 * 16;
 }
 
-// Every kernel of a pass lets the next one start (its launch, TMEM and
-// shared-memory set-up) and waits for all before it ahead of its first read
-// of anything a pass writes. Pointers to what a pass writes carry no
-// __restrict__ here: such loads may be moved above the wait.
-#define NN_PDL_TRIGGER() asm volatile("griddepcontrol.launch_dependents;" ::: "memory")
-#define NN_PDL_WAIT() asm volatile("griddepcontrol.wait;" ::: "memory")
-#define NN_PDL()      \
-  do {                \
-    NN_PDL_TRIGGER(); \
-    NN_PDL_WAIT();    \
-  } while (0)
-
-template <typename... KArgs, typename... Args>
-void launch(void (*kernel)(KArgs...), int grid, int block, size_t smem, cudaStream_t st, Args... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(block);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
-}
-
 __device__ __forceinline__ float relu(float x) { return x > 0.f ? x : 0.f; }
 
 __device__ __forceinline__ double block_sum(double v) {
@@ -79,7 +53,7 @@ __device__ __forceinline__ double block_sum(double v) {
 
 // sum_i e_i^2 per block
 __global__ void k_sq_partials(int n, const double* __restrict__ e, double* partials) {
-  NN_PDL();
+  FVM_PDL();
   double s = 0.0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) s += e[i] * e[i];
   s = block_sum(s);
@@ -91,7 +65,7 @@ __global__ void k_sq_partials(int n, const double* __restrict__ e, double* parti
 __global__ void __launch_bounds__(kBlock) k_encode(int n, const double* r, const double* __restrict__ diag,
                                                    const double* sum, const float* P, float* u, double* scale,
                                                    float* H0) {
-  NN_PDL();
+  FVM_PDL();
   const int lane = threadIdx.x & 31;
   const int i0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 8;
   const double s = sum[0] / (double)n;
@@ -129,7 +103,7 @@ __global__ void __launch_bounds__(kBlock) k_pass_start(int n, const double* r, i
                                                        int nSlices, const int4* __restrict__ meta,
                                                        const int* __restrict__ cols, const double* vals,
                                                        const double* diag, float* wf, float* wb) {
-  NN_PDL();
+  FVM_PDL();
   if (blockIdx.x < scaleBlocks) {
     double s = 0.0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += scaleBlocks * blockDim.x)
@@ -254,7 +228,7 @@ __device__ __forceinline__ void rotate8(float (&v)[8], int g) {
 __global__ void __launch_bounds__(kBlock) k_layer(int n, GraphArgs g, const float* P, const float* Hin, float* Hout,
                                                   float* Mout) {
   __shared__ float sWsT[32 * 32], sWmT[32 * 32], sb[32];
-  NN_PDL();
+  FVM_PDL();
   for (int t = threadIdx.x; t < 1024; t += blockDim.x) {
     const int c = t >> 5, k = t & 31;
     sWsT[k * 32 + c] = P[t];
@@ -335,11 +309,11 @@ __global__ void __launch_bounds__(kTcThreads, kTcBlocks) k_layer_tc(int n, Graph
   __shared__ uint32_t sTmem;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   float* stage = sB + 32 * 64 + warp * kStage;
-  NN_PDL_TRIGGER();
+  FVM_PDL_TRIGGER();
   if (warp == 0) umma::tmem_alloc(&sTmem, 32);
   if (threadIdx.x == 32) umma::mbar_init(&bar, 1);
   Rows8 rows = rows8(g, blockIdx.x * kTcRows + 8 * warp, 1, n, lane);
-  NN_PDL_WAIT();
+  FVM_PDL_WAIT();
   gather8_issue(Hin, rows, stage, lane);
   // B = [Ws Wm]: row = output channel, K = the 64 inputs (h then m); a thread
   // takes 4 inputs of a channel (every CTA reads these 8 KB at once: whole
@@ -454,7 +428,7 @@ __device__ __forceinline__ float warp_sum(float v) {
 
 __global__ void __launch_bounds__(kBlock) k_decode(int n, const float* P, const float* H3, const double* scale,
                                                    double* out) {
-  NN_PDL();
+  FVM_PDL();
   const int lane = threadIdx.x & 31;
   const int nw = (gridDim.x * blockDim.x) >> 5;
   const float wd = P[kDecW + lane], bd = P[kDecB];
@@ -488,7 +462,7 @@ __global__ void __launch_bounds__(kBlock) k_decode_bwd(int n, const float* P, co
                                                        const double* __restrict__ e, const double* e2, float* dH3,
                                                        float* gp, double* lossPartials) {
   __shared__ float sv[kWarps * 33];
-  NN_PDL();
+  FVM_PDL();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int nw = (gridDim.x * blockDim.x) >> 5;
   const float wd = P[kDecW + lane], bd = P[kDecB];
@@ -519,7 +493,7 @@ __global__ void __launch_bounds__(kBlock) k_decode_bwd_grad(int n, const float* 
                                                             const double* scale, const double* gd,
                                                             const double* gdScale, float* dH3, float* gp) {
   __shared__ float sv[kWarps * 33];
-  NN_PDL();
+  FVM_PDL();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int nw = (gridDim.x * blockDim.x) >> 5;
   const float wd = P[kDecW + lane];
@@ -552,7 +526,7 @@ __global__ void __launch_bounds__(kBlock) k_decode_bwd_grad(int n, const float* 
 
 // t = r + q in place of q, with block partials of t.t and r.r
 __global__ void k_residual_loss(int n, const double* r, double* q, double* partials) {
-  NN_PDL();
+  FVM_PDL();
   double a = 0.0, b = 0.0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const double ri = r[i];
@@ -571,7 +545,7 @@ __global__ void k_residual_loss(int n, const double* r, double* q, double* parti
 
 // loss = sum t.t / sum r.r; gscale = 2 / sum r.r
 __global__ void k_residual_loss_finish(int np, const double* partials, double* loss, double* gscale) {
-  NN_PDL();
+  FVM_PDL();
   double a = 0.0, b = 0.0;
   for (int k = threadIdx.x; k < np; k += blockDim.x) {
     a += partials[2 * k];
@@ -592,7 +566,7 @@ __global__ void __launch_bounds__(kBlock) k_layer_bwd_a(int n, const float* P, c
                                                         float* gp, int off) {
   extern __shared__ float sv[];  // kWarps * kLayerSize (per-warp gradient sums)
   __shared__ float sWs[1024], sWm[1024];
-  NN_PDL();
+  FVM_PDL();
   for (int t = threadIdx.x; t < 1024; t += blockDim.x) {
     sWs[t] = P[t];
     sWm[t] = P[1024 + t];
@@ -637,7 +611,7 @@ __global__ void __launch_bounds__(kBlock) k_layer_bwd_a(int n, const float* P, c
 // (the FP32 layers; the tensor-core ones form it where they read it)
 __global__ void __launch_bounds__(kBlock) k_layer_bwd_b(int n, GraphArgs g, const float* dS, const float* dM,
                                                         float* dHin) {
-  NN_PDL();
+  FVM_PDL();
   const int lane = threadIdx.x & 31;
   const int nw = (gridDim.x * blockDim.x) >> 5;
   for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += nw) {
@@ -679,7 +653,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_layer_bwd_tc(int n, GraphArgs
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   float* stage = smem + warp * kStage;
   static_assert(kTcThreads / 32 * kStage == 2 * kTcRows * 32 + 64 * kTcRows, "staging overlays Z, ZT and 64 features");
-  NN_PDL_TRIGGER();
+  FVM_PDL_TRIGGER();
   if (warp == 0) umma::tmem_alloc(&sTmem, 128);
   if (threadIdx.x == 32) umma::mbar_init(&bar, 1);
   // features 64 .. 127 of XT: the constant 1, then zeros
@@ -689,7 +663,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_layer_bwd_tc(int n, GraphArgs
   }
   Rows8 rows = {0, 0, -1};
   if (dMout) rows = rows8(g, blockIdx.x * kTcRows + 8 * warp, 1, n, lane);
-  NN_PDL_WAIT();
+  FVM_PDL_WAIT();
   if (dMout) gather8_issue(dMout, rows, stage, lane);
   {
     const int f = threadIdx.x & 63, c = (threadIdx.x >> 6) << 2;  // W^T[f][c] = Ws[c][f] or Wm[c][f - 32]
@@ -817,7 +791,7 @@ __global__ void __launch_bounds__(kBlock) k_encode_bwd(int n, GraphArgs g, const
                                                        const float* dH0, const float* dM, float* gp) {
   __shared__ float sv[kWarps * 64];
   __shared__ __align__(16) float sStage[kWarps * kStage];
-  NN_PDL();
+  FVM_PDL();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int nw = (gridDim.x * blockDim.x) >> 5;
   float gw = 0.f, gb = 0.f;
@@ -857,7 +831,7 @@ __global__ void __launch_bounds__(kBlock) k_encode_bwd(int n, GraphArgs g, const
 // took 9.4 us, now 6.7.)
 __global__ void __launch_bounds__(kBlock) k_grad_reduce(int layerBlocks, const float* gp, float* grad) {
   __shared__ float part[kGradBlocks][32];
-  NN_PDL();
+  FVM_PDL();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int p = blockIdx.x * 32 + lane;
   const bool layer = blockIdx.x * 32 >= kLayer0 && blockIdx.x * 32 + 32 <= kDecW;
@@ -880,7 +854,7 @@ static_assert(kGradBlocks % kWarps == 0 && kLayer0 % 32 == 0 && kDecW % 32 == 0,
               "the reduction's blocks hold parameters of one kind");
 
 __global__ void k_adam(float* P, const float* g, float* m, float* v, float lr, float c1, float c2) {
-  NN_PDL();
+  FVM_PDL();
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= kParams) return;
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
@@ -913,10 +887,10 @@ void run_forward(const Graph& g, const float* P, const double* r, Workspace& w, 
   const int n = w.n;
   FVM_REQUIRE(g.entries > 0 && g.entries <= w.wcap, kBadArgument,
               "learned correction: workspace not prepared for this graph's entries");
-  launch(k_pass_start, kReduceBlocks + ceil_div(4LL * g.nSlices, kWarps), kBlock, 0, st, n, r, kReduceBlocks,
+  pdl_launch_smem(k_pass_start, kReduceBlocks + ceil_div(4LL * g.nSlices, kWarps), kBlock, 0, st, n, r, kReduceBlocks,
          w.partials, g.nSlices, g.a.meta, g.a.cols, g.a.vals, g.a.diag, w.wf, w.wb);
   dev::sum_partials(kReduceBlocks, w.partials, scal + 1, st);
-  launch(k_encode, ceil_div(n, 8 * kWarps), kBlock, 0, st, n, r, g.a.diag, scal + 1, P, w.u, scal, w.H[0]);
+  pdl_launch_smem(k_encode, ceil_div(n, 8 * kWarps), kBlock, 0, st, n, r, g.a.diag, scal + 1, P, w.u, scal, w.H[0]);
   FVM_REQUIRE(((uintptr_t)P & 15) == 0, kBadArgument, "learned correction: parameters not 16-byte aligned");
   const GraphArgs ga = args(g, w);
   if (w.tensorCores)
@@ -926,9 +900,9 @@ void run_forward(const Graph& g, const float* P, const double* r, Workspace& w, 
     const float* Pl = P + kLayer0 + l * kLayerSize;
     float* Ml = keepMessages ? w.M[l] : nullptr;
     if (w.tensorCores)
-      launch(k_layer_tc, tc_blocks(n), kTcThreads, kFwdSmem, st, n, ga, Pl, w.H[l], w.H[l + 1], Ml, w.status);
+      pdl_launch_smem(k_layer_tc, tc_blocks(n), kTcThreads, kFwdSmem, st, n, ga, Pl, w.H[l], w.H[l + 1], Ml, w.status);
     else
-      launch(k_layer, node_blocks(n), kBlock, 0, st, n, ga, Pl, w.H[l], w.H[l + 1], Ml);
+      pdl_launch_smem(k_layer, node_blocks(n), kBlock, 0, st, n, ga, Pl, w.H[l], w.H[l + 1], Ml);
   }
 }
 
@@ -951,7 +925,7 @@ void run_backward(const Graph& g, const float* P, float* grad, Workspace& w, cud
       const bool odd = (kLayers - 1 - l) & 1;
       float* outS = odd ? w.dA : w.dS;
       float* outM = odd ? w.M[kLayers - 1] : w.dB;
-      launch(k_layer_bwd_tc, layerBlocks, kTcThreads, kBwdSmem, st, n, ga, P + off, w.H[l], w.H[l + 1], w.M[l], dH, dM,
+      pdl_launch_smem(k_layer_bwd_tc, layerBlocks, kTcThreads, kBwdSmem, st, n, ga, P + off, w.H[l], w.H[l + 1], w.M[l], dH, dM,
              outS, outM, w.gradPartials, off, w.status);
       check(cudaGetLastError(), "layer backward launch");
       dH = outS;
@@ -963,14 +937,14 @@ void run_backward(const Graph& g, const float* P, float* grad, Workspace& w, cud
           "k_layer_bwd_a shared memory");
     for (int l = kLayers - 1; l >= 0; l--) {
       const int off = kLayer0 + l * kLayerSize;
-      launch(k_layer_bwd_a, kGradBlocks, kBlock, smem, st, n, P + off, w.H[l], w.H[l + 1], w.M[l], w.dA, w.dS, w.dB,
+      pdl_launch_smem(k_layer_bwd_a, kGradBlocks, kBlock, smem, st, n, P + off, w.H[l], w.H[l + 1], w.M[l], w.dA, w.dS, w.dB,
              w.gradPartials, off);
       check(cudaGetLastError(), "layer backward launch");
-      launch(k_layer_bwd_b, node_blocks(n), kBlock, 0, st, n, ga, w.dS, w.dB, w.dA);
+      pdl_launch_smem(k_layer_bwd_b, node_blocks(n), kBlock, 0, st, n, ga, w.dS, w.dB, w.dA);
     }
   }
-  launch(k_encode_bwd, kGradBlocks, kBlock, 0, st, n, ga, w.u, w.H[0], dH, dM, w.gradPartials);
-  launch(k_grad_reduce, ceil_div(kParams, 32), kBlock, 0, st, layerBlocks, w.gradPartials, grad);
+  pdl_launch_smem(k_encode_bwd, kGradBlocks, kBlock, 0, st, n, ga, w.u, w.H[0], dH, dM, w.gradPartials);
+  pdl_launch_smem(k_grad_reduce, ceil_div(kParams, 32), kBlock, 0, st, layerBlocks, w.gradPartials, grad);
 }
 
 }  // namespace
@@ -1044,16 +1018,16 @@ void Workspace::checkStatus() {
 void forward(const Graph& g, const float* params, const double* r, double* out, Workspace& w, double* scal,
              cudaStream_t st) {
   run_forward(g, params, r, w, scal, false, st);
-  launch(k_decode, node_blocks(ceil_div(w.n, 4)), kBlock, 0, st, w.n, params, w.H[kLayers], scal, out);
+  pdl_launch_smem(k_decode, node_blocks(ceil_div(w.n, 4)), kBlock, 0, st, w.n, params, w.H[kLayers], scal, out);
 }
 
 void forward_backward(const Graph& g, const float* P, const double* r, const double* e, float* grad, double* loss,
                       Workspace& w, double* scal, cudaStream_t st) {
   const int n = w.n;
   run_forward(g, P, r, w, scal, true, st);
-  launch(k_sq_partials, kReduceBlocks, kBlock, 0, st, n, e, w.partials);
+  pdl_launch_smem(k_sq_partials, kReduceBlocks, kBlock, 0, st, n, e, w.partials);
   dev::sum_partials(kReduceBlocks, w.partials, scal + 2, st);
-  launch(k_decode_bwd, kGradBlocks, kBlock, 0, st, n, P, w.H[kLayers], scal, e, scal + 2, w.dA, w.gradPartials,
+  pdl_launch_smem(k_decode_bwd, kGradBlocks, kBlock, 0, st, n, P, w.H[kLayers], scal, e, scal + 2, w.dA, w.gradPartials,
          w.partials);
   dev::sum_partials(kGradBlocks, w.partials, loss, st);
   run_backward(g, P, grad, w, st);
@@ -1065,12 +1039,12 @@ void forward_backward_residual(const Graph& g, const float* P, const double* r, 
   double* d = w.dv;
   double* t = w.dv + n;
   run_forward(g, P, r, w, scal, true, st);
-  launch(k_decode, node_blocks(ceil_div(n, 4)), kBlock, 0, st, n, P, w.H[kLayers], scal, d);
+  pdl_launch_smem(k_decode, node_blocks(ceil_div(n, 4)), kBlock, 0, st, n, P, w.H[kLayers], scal, d);
   dev::spmv(g.a, g.nSlices, d, t, st);  // t = A d
-  launch(k_residual_loss, kReduceBlocks, kBlock, 0, st, n, r, t, w.partials);  // t = r + A d
-  launch(k_residual_loss_finish, 1, kBlock, 0, st, kReduceBlocks, w.partials, loss, scal + 3);
+  pdl_launch_smem(k_residual_loss, kReduceBlocks, kBlock, 0, st, n, r, t, w.partials);  // t = r + A d
+  pdl_launch_smem(k_residual_loss_finish, 1, kBlock, 0, st, kReduceBlocks, w.partials, loss, scal + 3);
   dev::spmv(g.a, g.nSlices, t, d, st);  // d = A (r + A d): dL/dd / (2 / |r|^2)
-  launch(k_decode_bwd_grad, kGradBlocks, kBlock, 0, st, n, P, w.H[kLayers], scal, d, scal + 3, w.dA,
+  pdl_launch_smem(k_decode_bwd_grad, kGradBlocks, kBlock, 0, st, n, P, w.H[kLayers], scal, d, scal + 3, w.dA,
          w.gradPartials);
   run_backward(g, P, grad, w, st);
 }
@@ -1093,7 +1067,7 @@ int tc_wait_probe(unsigned limit) {
 void adam_step(float* params, const float* grad, float* m, float* v, float lr, int t, cudaStream_t st) {
   const float c1 = 1.f - std::pow(0.9f, (float)t);
   const float c2 = 1.f - std::pow(0.999f, (float)t);
-  launch(k_adam, ceil_div(kParams, kBlock), kBlock, 0, st, params, grad, m, v, lr, c1, c2);
+  pdl_launch_smem(k_adam, ceil_div(kParams, kBlock), kBlock, 0, st, params, grad, m, v, lr, c1, c2);
 }
 
 std::vector<float> initial_parameters(uint64_t seed) {
