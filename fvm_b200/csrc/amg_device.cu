@@ -351,71 +351,56 @@ __global__ void k_c2f_sort(int nc, const int* c2fRow, int* cnt, int* c2fCol) {
 // ---- Galerkin ----------------------------------------------------------------------
 
 constexpr int kGalWarps = 4;
+constexpr int kGalSmall = 64;  // entries of a coarse row that half a warp takes
 
-// One warp per coarse row. The entries of its fine rows (rows ascending,
-// entries in stored order) are taken 32 at a time, one a lane: lanes of one
-// coarse column find each other with a match, the lowest looks the column up
-// among those found before (U, in first-visit order; S their sums) and adds
-// the lanes' values in lane order, so every sum is in stored order. Scanning
-// all earlier entries of the row for each entry, and lane 0 summing the
-// diagonal over all of them, took 190 us a launch (70 for the counts) on the
-// levels of 1.5M tets; this takes GAL_US.
-template <bool kFill>
-__global__ void __launch_bounds__(32 * kGalWarps) k_galerkin(LevelRows a, int nc, const int* ci, const int* c2fRow,
-                                                             const int* c2fCol, int* count, int* overflow,
-                                                             const int* sliceOff, int* ccols, double* cvals,
-                                                             float* cvalsF, double* cdiag, float* cdiagF) {
-  __shared__ int sU[kGalWarps][kGalerkinCap];
-  __shared__ double sS[kFill ? kGalWarps : 1][kFill ? kGalerkinCap : 1];
-  __shared__ int sOff[kGalWarps][32], sBase[kGalWarps][32], sRow[kGalWarps][32];
-  __shared__ double sDiag[kGalWarps][32];
-  FVM_PDL();
-  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int I = blockIdx.x * kGalWarps + wid;
-  if (I >= nc) {  // the whole warp leaves together
-    // lanes of the last slice past the last row: column 0, so that no index
-    // in the level is undefined (the fill covers whole slices)
-    if (kFill && I < ((nc + 31) & ~31)) {
-      const int s = I >> 5, cw = (sliceOff[s + 1] - sliceOff[s]) >> 5;
-      for (int slot = lane; slot < cw; slot += 32) ccols[sliceOff[s] + (I & 31) + 32 * (size_t)slot] = 0;
-    }
-    return;
-  }
-  int* U = sU[wid];
-  double* S = sS[kFill ? wid : 0];
-  const int f0 = c2fRow[I], f1 = c2fRow[I + 1];
+// One coarse row I per group of G lanes (I < 0: none; the whole warp calls
+// together). The entries of its fine rows (rows ascending, entries in stored
+// order) are taken G at a time, one a lane: lanes of one coarse column find
+// each other with a match, the lowest looks the column up among those found
+// before (U, in first-visit order; S their sums) and adds the lanes' values
+// in lane order, so every sum is in stored order. False when the row has more
+// than cap entries (nothing is written then).
+template <bool kFill, int G>
+__device__ __forceinline__ bool galerkin_row(const LevelRows& a, int I, int cap, const int* ci, const int* c2fRow,
+                                             const int* c2fCol, int* count, const int* sliceOff, int* ccols,
+                                             double* cvals, float* cvalsF, double* cdiag, float* cdiagF, int* U,
+                                             double* S, int* sOff, int* sBase, int* sRow, double* sDiag) {
+  const int lane = threadIdx.x & 31, gl = lane & (G - 1), g0 = lane & ~(G - 1);
+  constexpr unsigned kGroup = G == 32 ? kFull : (1u << (G & 31)) - 1u;
+  const int f0 = I >= 0 ? c2fRow[I] : 0;
+  int f1 = I >= 0 ? c2fRow[I + 1] : 0;
   double dsum = 0.0;  // fine diagonals plus the entries inside the aggregate
   int L = 0, nU = 0;
-  for (int q0 = f0; q0 < f1; q0 += 32) {
-    // up to 32 fine rows: each lane looks one up, a warp scan places them
-    const int nq = min(32, f1 - q0);
+  bool fits = true;
+  for (int q0 = f0; __any_sync(kFull, q0 < f1); q0 += G) {
+    // up to G fine rows: each lane looks one up, a scan places them
+    int nq = min(G, f1 - q0);
     int base = 0, w = 0, f = -1;
-    if (lane < nq) {
-      f = c2fCol[q0 + lane];
+    if (gl < nq) {
+      f = c2fCol[q0 + gl];
       row_range(a, f, base, w);
-      if (kFill) sDiag[wid][lane] = a.diag[f];
+      if (kFill) sDiag[gl] = a.diag[f];
     }
     int incl = w;
-    for (int o = 1; o < 32; o <<= 1) {
-      const int t = __shfl_up_sync(kFull, incl, o);
-      if (lane >= o) incl += t;
+#pragma unroll
+    for (int o = 1; o < G; o <<= 1) {
+      const int t = __shfl_up_sync(kFull, incl, o, G);
+      if (gl >= o) incl += t;
     }
-    const int tot = __shfl_sync(kFull, incl, 31);
-    if (L + tot > kGalerkinCap) {
-      if (lane == 0) {
-        atomicExch(overflow, 1);
-        if (!kFill) count[I] = 0;
-      }
-      return;
-    }
+    int tot = __shfl_sync(kFull, incl, G - 1, G);
     L += tot;
-    sOff[wid][lane] = incl - w;
-    sBase[wid][lane] = base;
-    sRow[wid][lane] = f;
+    if (L > cap) {
+      fits = false;
+      f1 = q0;
+      tot = nq = 0;
+    }
+    sOff[gl] = incl - w;
+    sBase[gl] = base;
+    sRow[gl] = f;
     __syncwarp();
     int qd = 0;  // rows whose diagonal is in dsum
-    for (int e0 = 0; e0 < tot; e0 += 32) {
-      const int e = e0 + lane;
+    for (int e0 = 0; __any_sync(kFull, e0 < tot); e0 += G) {
+      const int e = e0 + gl;
       int J = -1;
       double v = 0.0;
       if (e < tot) {
@@ -423,34 +408,37 @@ __global__ void __launch_bounds__(32 * kGalWarps) k_galerkin(LevelRows a, int nc
         int lo = 0, hi = nq - 1;
         while (lo < hi) {
           const int mid = (lo + hi + 1) >> 1;
-          if (sOff[wid][mid] <= e)
+          if (sOff[mid] <= e)
             lo = mid;
           else
             hi = mid - 1;
         }
-        const int idx = sBase[wid][lo] + 32 * (e - sOff[wid][lo]);
+        const int idx = sBase[lo] + 32 * (e - sOff[lo]);
         const int j = a.cols[idx];
         v = a.vals[idx];
-        if (j != sRow[wid][lo] && v != 0.0) J = ci[j];  // else padding
+        if (j != sRow[lo] && v != 0.0) J = ci[j];  // else padding
       }
       if (kFill) {
-        unsigned in = __ballot_sync(kFull, J == I);
-        while (in) {
-          const int b = __ffs(in) - 1;
-          in &= in - 1;
-          while (qd < nq && sOff[wid][qd] <= e0 + b) dsum += sDiag[wid][qd++];
-          dsum += __shfl_sync(kFull, v, b);
+        unsigned in = (__ballot_sync(kFull, J >= 0 && J == I) >> g0) & kGroup;
+        while (__any_sync(kFull, in != 0u)) {
+          const int b = in ? __ffs(in) - 1 : 0;
+          const double vb = __shfl_sync(kFull, v, b, G);
+          if (in) {
+            while (qd < nq && sOff[qd] <= e0 + b) dsum += sDiag[qd++];
+            dsum += vb;
+          }
+          in &= in - 1u;
         }
       }
       const bool live = J >= 0 && J != I;
       int slot = -1;
       for (int k = 0; k < nU; k++)
         if (U[k] == J) slot = k;
-      const unsigned same = __match_any_sync(kFull, live ? J : -2 - lane);
+      const unsigned same = __match_any_sync(kFull, live ? J * (32 / G) + g0 / G : -2 - lane);
       const bool leader = live && __ffs(same) - 1 == lane;
-      const unsigned found = __ballot_sync(kFull, leader && slot < 0);
       const bool isNew = leader && slot < 0;
-      if (isNew) slot = nU + __popc(found & ((1u << lane) - 1u));
+      const unsigned found = (__ballot_sync(kFull, isNew) >> g0) & kGroup;
+      if (isNew) slot = nU + __popc(found & ((1u << gl) - 1u));
       if (kFill) {
         double s = leader && !isNew ? S[slot] : 0.0;
         unsigned rest = leader ? same : 0u;
@@ -467,15 +455,16 @@ __global__ void __launch_bounds__(32 * kGalWarps) k_galerkin(LevelRows a, int nc
       __syncwarp();
     }
     if (kFill)
-      while (qd < nq) dsum += sDiag[wid][qd++];
+      while (qd < nq) dsum += sDiag[qd++];
     __syncwarp();
   }
+  if (I < 0 || !fits) return fits;
   if constexpr (!kFill) {
-    if (lane == 0) count[I] = nU;
+    if (gl == 0) count[I] = nU;
   } else {
     const int s = I >> 5;
     const int cbase = sliceOff[s] + (I & 31), cw = (sliceOff[s + 1] - sliceOff[s]) >> 5;
-    for (int slot = lane; slot < cw; slot += 32) {
+    for (int slot = gl; slot < cw; slot += G) {
       const size_t o = (size_t)cbase + 32 * (size_t)slot;
       const bool used = slot < nU;  // else padding: own row, zero
       const double v = used ? S[slot] : 0.0;
@@ -483,10 +472,67 @@ __global__ void __launch_bounds__(32 * kGalWarps) k_galerkin(LevelRows a, int nc
       cvals[o] = v;
       if (cvalsF) cvalsF[o] = (float)v;
     }
-    if (lane == 0) {
+    if (gl == 0) {
       cdiag[I] = dsum;
       if (cdiagF) cdiagF[I] = (float)dsum;
     }
+  }
+  return true;
+}
+
+// Groups of G lanes a coarse row. With G = 16 rows of more than kGalSmall
+// entries are left to the block's first warp. What bounds it is the chain of
+// five dependent loads of a row, so rows in flight count: half a warp needs
+// 0.8 KB of shared memory a row where a whole one needs 6. (Levels of 1.5M
+// tets, 8 launches: a scan of all earlier entries for each entry, a warp a row
+// 190 us a launch and 70 for the counts; match, a warp a row 151 and 65; half
+// a warp a row 83 and 45.)
+template <bool kFill, int G>
+__global__ void __launch_bounds__(32 * kGalWarps) k_galerkin(LevelRows a, int nc, const int* ci, const int* c2fRow,
+                                                             const int* c2fCol, int* count, int* overflow,
+                                                             const int* sliceOff, int* ccols, double* cvals,
+                                                             float* cvalsF, double* cdiag, float* cdiagF) {
+  constexpr int kGroups = kGalWarps * 32 / G;
+  constexpr int kCap = G == 32 ? kGalerkinCap : kGalSmall;
+  __shared__ int sU[kGroups][kCap];
+  __shared__ double sS[kFill ? kGroups : 1][kFill ? kCap : 1];
+  __shared__ int sOff[kGroups][G], sBase[kGroups][G], sRow[kGroups][G];
+  __shared__ double sDiag[kGroups][G];
+  FVM_PDL();
+  const int lane = threadIdx.x & 31, g = threadIdx.x / G;
+  int I = blockIdx.x * kGroups + g;
+  // lanes of the last slice past the last row: column 0, so that no index in
+  // the level is undefined (the fill covers whole slices)
+  if (kFill && I >= nc && I < ((nc + 31) & ~31)) {
+    const int s = I >> 5, cw = (sliceOff[s + 1] - sliceOff[s]) >> 5;
+    for (int slot = lane & (G - 1); slot < cw; slot += G) ccols[sliceOff[s] + (I & 31) + 32 * (size_t)slot] = 0;
+  }
+  if (I >= nc) I = -1;
+  const bool fits =
+      galerkin_row<kFill, G>(a, I, kCap, ci, c2fRow, c2fCol, count, sliceOff, ccols, cvals, cvalsF, cdiag, cdiagF,
+                             sU[g], sS[kFill ? g : 0], sOff[g], sBase[g], sRow[g], sDiag[g]);
+  if constexpr (G == 32) {
+    if (!fits && lane == 0) {
+      atomicExch(overflow, 1);
+      if (!kFill) count[I] = 0;
+    }
+  } else {
+    __shared__ int nLong, longRow[kGroups];
+    if (!__syncthreads_or(!fits)) return;
+    if (threadIdx.x == 0) nLong = 0;
+    __syncthreads();
+    if (!fits && (lane & (G - 1)) == 0) longRow[atomicAdd(&nLong, 1)] = I;
+    __syncthreads();
+    if (threadIdx.x >= 32) return;
+    __shared__ int bU[kGalerkinCap], bOff[32], bBase[32], bRow[32];
+    __shared__ double bS[kFill ? kGalerkinCap : 1], bDiag[32];
+    for (int k = 0; k < nLong; k++)
+      if (!galerkin_row<kFill, 32>(a, longRow[k], kGalerkinCap, ci, c2fRow, c2fCol, count, sliceOff, ccols, cvals,
+                                   cvalsF, cdiag, cdiagF, bU, bS, bOff, bBase, bRow, bDiag) &&
+          lane == 0) {
+        atomicExch(overflow, 1);
+        if (!kFill) count[longRow[k]] = 0;
+      }
   }
 }
 
@@ -721,17 +767,26 @@ void coarse_to_fine(int n, int nc, const int* ci, int* cnt, int* c2fRow, int* c2
   pdl_launch(k_c2f_sort, cdiv(nc, kT), kT, st, nc, c2fRow, cnt, c2fCol);
 }
 
-void galerkin_count(const LevelRows& a, int nc, const int* ci, const int* c2fRow, const int* c2fCol, int* count,
-                    int* overflow, cudaStream_t st) {
-  pdl_launch(k_galerkin<false>, cdiv(nc, kGalWarps), 32 * kGalWarps, st, a, nc, ci, c2fRow, c2fCol, count, overflow,
-             nullptr, nullptr, nullptr, nullptr, nullptr, nullptr);
+// half a warp a row while a coarse row has at most 32 entries on average: two
+// rounds of 16 lanes (pairs of tets 8 to 12, of hexes 12 to 18, the levels'
+// aggregates of 5 rows of a tet 20); from there on a warp's 32 lanes are used
+static bool short_rows(long long entries, int nc) { return entries <= 32ll * nc; }
+
+void galerkin_count(const LevelRows& a, long long entries, int nc, const int* ci, const int* c2fRow,
+                    const int* c2fCol, int* count, int* overflow, cudaStream_t st) {
+  const auto f = short_rows(entries, nc) ? k_galerkin<false, 16> : k_galerkin<false, 32>;
+  const int rows = short_rows(entries, nc) ? 2 * kGalWarps : kGalWarps;
+  pdl_launch(f, cdiv(nc, rows), 32 * kGalWarps, st, a, nc, ci, c2fRow, c2fCol, count, overflow, nullptr, nullptr,
+             nullptr, nullptr, nullptr, nullptr);
 }
 
-void galerkin_fill(const LevelRows& a, int nc, const int* ci, const int* c2fRow, const int* c2fCol,
-                   const int* sliceOff, int* cols, double* vals, float* valsF, double* diag, float* diagF,
-                   int* overflow, cudaStream_t st) {
-  pdl_launch(k_galerkin<true>, cdiv(cdiv(nc, 32) * 32, kGalWarps), 32 * kGalWarps, st, a, nc, ci, c2fRow, c2fCol,
-             nullptr, overflow, sliceOff, cols, vals, valsF, diag, diagF);
+void galerkin_fill(const LevelRows& a, long long entries, int nc, const int* ci, const int* c2fRow,
+                   const int* c2fCol, const int* sliceOff, int* cols, double* vals, float* valsF, double* diag,
+                   float* diagF, int* overflow, cudaStream_t st) {
+  const auto f = short_rows(entries, nc) ? k_galerkin<true, 16> : k_galerkin<true, 32>;
+  const int rows = short_rows(entries, nc) ? 2 * kGalWarps : kGalWarps;
+  pdl_launch(f, cdiv(cdiv(nc, 32) * 32, rows), 32 * kGalWarps, st, a, nc, ci, c2fRow, c2fCol, nullptr, overflow,
+             sliceOff, cols, vals, valsF, diag, diagF);
 }
 
 void slice_widths(int n, const int* count, int* width32, int* maxWidth, cudaStream_t st) {
@@ -1089,7 +1144,7 @@ void AmgHierarchy::buildDevice(const FinestDevice& in, const SolverOptions& opt,
     }
     int* state = flags + product;
     product += 2;
-    dev::galerkin_count(af, nc, ci, fine.c2fRow, fine.c2fCol, w.best, state, st);
+    dev::galerkin_count(af, (long long)fine.entries, nc, ci, fine.c2fRow, fine.c2fCol, w.best, state, st);
     dev::slice_widths(nc, w.best, w.join, state + 1, st);
     dev::scan_exclusive(w.join, sliceOff, nSlices, w.scan, st, hflags, state);
     CUDA_OK(cudaStreamSynchronize(st));
@@ -1114,7 +1169,7 @@ void AmgHierarchy::buildDevice(const FinestDevice& in, const SolverOptions& opt,
     c.sliceRow = (int*)arena_.alloc(size_class(sizeof(int) * nSlices));
     c.sliceRows = (int*)arena_.alloc(size_class(sizeof(int) * nSlices));
     c.rowSlice = (int*)arena_.alloc(size_class(sizeof(int) * nc));
-    dev::galerkin_fill(af, nc, ci, fine.c2fRow, fine.c2fCol, sliceOff, c.cols, c.vals, c.valsF, c.diag, c.diagF,
+    dev::galerkin_fill(af, (long long)fine.entries, nc, ci, fine.c2fRow, fine.c2fCol, sliceOff, c.cols, c.vals, c.valsF, c.diag, c.diagF,
                        state, st);
     dev::slice_meta_fill(nc, sliceOff, c.meta, c.sliceRow, c.sliceRows, c.rowSlice, st);
     return E;

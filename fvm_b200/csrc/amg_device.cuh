@@ -58,8 +58,8 @@ void aggregate_pairs(const LevelRows& a, double beta, int rounds, const int* ord
 void coarse_to_fine(int n, int nc, const int* ci, int* cnt, int* c2fRow, int* c2fCol, int* scanScratch,
                     cudaStream_t st);
 
-// Galerkin product Ac = P^T A P for piecewise-constant P, one warp per
-// coarse row. Pass 1 (count != null): unique off-diagonal coarse columns
+// Galerkin product Ac = P^T A P for piecewise-constant P, a warp or half of
+// one per coarse row (entries: those of the fine level). Pass 1 (count != null): unique off-diagonal coarse columns
 // per row into count[I]. Pass 2: the row's columns (first-visit order over
 // its fine rows ascending, entries in stored order) and sums into the
 // coarse SELL-32 level (natural row order, 32-row slices described by
@@ -69,9 +69,9 @@ void coarse_to_fine(int n, int nc, const int* ci, int* cnt, int* c2fRow, int* c2
 // 0. *overflow is set when an aggregate's entries exceed the per-warp
 // capacity.
 constexpr int kGalerkinCap = 512;
-void galerkin_count(const LevelRows& a, int nc, const int* ci, const int* c2fRow, const int* c2fCol, int* count,
+void galerkin_count(const LevelRows& a, long long entries, int nc, const int* ci, const int* c2fRow, const int* c2fCol, int* count,
                     int* overflow, cudaStream_t st);
-void galerkin_fill(const LevelRows& a, int nc, const int* ci, const int* c2fRow, const int* c2fCol,
+void galerkin_fill(const LevelRows& a, long long entries, int nc, const int* ci, const int* c2fRow, const int* c2fCol,
                    const int* sliceOff, int* cols, double* vals, float* valsF, double* diag, float* diagF,
                    int* overflow, cudaStream_t st);
 
