@@ -33,6 +33,7 @@
 #include <vector>
 
 #include "common.hpp"
+#include "pdl.cuh"
 
 namespace fvm {
 namespace dev {
@@ -522,27 +523,31 @@ __device__ __forceinline__ size_t block_at(int NB, int I, int J) {
 
 // which blocks hold entries (one byte per block pair)
 __global__ void __launch_bounds__(128) k_inv_flag(SellView<double> a, const int* __restrict__ rowSlice,
-                                                  const int* __restrict__ pos, int NB, unsigned char* nz) {
+                                                  const int* pos, int NB, unsigned char* nz, int* rowAt) {
+  FVM_PDL();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < NB) nz[(size_t)i * NB + i] = 1;
   if (i >= a.n) return;
   int lane;
   const int4 m = slice_of_row(a, rowSlice, i, lane);
   const int bi = pos[i] / kBlk;
+  rowAt[pos[i]] = i;
   for (int k = 0; k < m.w; k++) {
     const int bj = pos[a.cols[m.z + 32 * k + lane]] / kBlk;
     if (bi <= bj) nz[(size_t)bi * NB + bj] = 1;
   }
 }
 // flagged blocks to zero, the diagonal to one (the padding rows keep it)
-__global__ void __launch_bounds__(256) k_inv_clear(int NB, const unsigned char* __restrict__ nz, double* A) {
+__global__ void __launch_bounds__(256) k_inv_clear(int NB, const unsigned char* nz, double* A) {
+  FVM_PDL();
   const int I = blockIdx.y, J = blockIdx.x;
   if (J < I || !nz[(size_t)I * NB + J]) return;
   double* b = A + block_at(NB, I, J);
   for (int e = threadIdx.x; e < kBlk * kBlk; e += 256) b[e] = I == J && e / kBlk == e % kBlk ? 1.0 : 0.0;
 }
 __global__ void __launch_bounds__(128) k_inv_scatter(SellView<double> a, const int* __restrict__ rowSlice,
-                                                     const int* __restrict__ pos, int NB, double* A) {
+                                                     const int* pos, int NB, double* A) {
+  FVM_PDL();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.n) return;
   int lane;
@@ -565,7 +570,7 @@ __global__ void __launch_bounds__(128) k_inv_scatter(SellView<double> a, const i
 struct BlockInverse {
   double row[2][kBlk];
 };
-__device__ void invert_block(double (&d)[4], BlockInverse& s, double* __restrict__ out, int* status) {
+__device__ void invert_block(double (&d)[4], BlockInverse& s, double* out, int* status) {
   const int w = threadIdx.x >> 5, c = threadIdx.x & 31;
   if (w == 0) s.row[0][c] = d[0];
 #pragma unroll
@@ -589,9 +594,10 @@ __device__ void invert_block(double (&d)[4], BlockInverse& s, double* __restrict
 }
 
 // the first step's pivot blocks inverted
-__global__ void __launch_bounds__(256) k_inv_first(int NB, const int* __restrict__ pivots,
-                                                   const double* __restrict__ A, double* Dinv, int* status) {
+__global__ void __launch_bounds__(256) k_inv_first(int NB, const int* pivots, const double* A, double* Dinv,
+                                                   int* status) {
   __shared__ BlockInverse ws;
+  FVM_PDL();
   const int K = pivots[blockIdx.x];
   const double* b = A + block_at(NB, K, K);
   double d[4];
@@ -603,12 +609,14 @@ __global__ void __launch_bounds__(256) k_inv_first(int NB, const int* __restrict
 // For block row i and the step's q-th pivot block K: C = A[i][K] (old) and
 // R = D^-1 A[K][i], both 32 x 32 at slot (q, i); act[q][i] says whether
 // they couple at all.
-__global__ void __launch_bounds__(256) k_inv_panel(int NB, const int* __restrict__ pivots,
-                                                   const double* __restrict__ A, const double* __restrict__ Dinv,
-                                                   const unsigned char* __restrict__ nz, double* __restrict__ C,
-                                                   double* __restrict__ R, unsigned char* __restrict__ act) {
+// (pivots: complete before the first step, read ahead of the wait)
+__global__ void __launch_bounds__(256) k_inv_panel(int NB, const int* __restrict__ pivots, const double* A,
+                                                   const double* Dinv, const unsigned char* nz, double* C, double* R,
+                                                   unsigned char* act) {
   __shared__ double S[kBlk][kBlk + 1], D[kBlk][kBlk + 1];
+  FVM_PDL_TRIGGER();
   const int i = blockIdx.x, q = blockIdx.y, K = pivots[q];
+  FVM_PDL_WAIT();
   const bool on = i != K && nz[(size_t)min(i, K) * NB + max(i, K)];
   if (threadIdx.x == 0) act[(size_t)q * NB + i] = on;
   if (!on) return;
@@ -648,21 +656,33 @@ __device__ __forceinline__ void copy16(void* smem, const void* gmem) {
 }
 
 struct UpdateStage {
-  double C[64][kBlk + 2], R[kBlk][64 + 2];
+  double C[64][kBlk + 4], R[kBlk][64 + 4];  // (rows 4 banks of 8 bytes on: fragment loads without conflicts)
 };
 
+// D (8 x 8) += A (8 x 4) B (4 x 8): lane l holds A[l / 4][l % 4], B[l % 4][l / 4]
+// and D[l / 4][2 (l % 4) .. + 1]
+__device__ __forceinline__ void mma_f64(double (&d)[2], double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+      : "+d"(d[0]), "+d"(d[1])
+      : "d"(a), "d"(b));
+}
+
 // One step over the 64 x 64 tiles on and above the diagonal (four blocks
-// each, one CTA per tile). A tile that no pivot of the step reaches returns
-// at once. A step over a full matrix of 3840 padded rows takes 41 us: 11 us
-// of FP64 at the chip's rate, 96 KB of L2 traffic per tile, and three CTAs
-// of 80 registers per SM to hide either behind the other. Splitting off the
-// pivot tiles' writes and fixed copy addresses took it from 49 to 41 us.
+// each, one CTA per tile, two warps per block). A tile that no pivot of the
+// step reaches returns at once. With a 4 x 4 register tile of FP64 FMAs a
+// thread a step over a full matrix of 3840 padded rows took 41 us: 11 us of
+// FP64 at the chip's rate, as long again in shared-memory reads, and three
+// CTAs of 80 registers per SM to hide those and the tile's loads behind each
+// other. The FP64 matrix instruction reads 6 operands for 8 products of 8 x 8
+// x 4 where that read 8 for 16 FMAs, and one stage suffices where the step has
+// one pivot: 28 us.
 __global__ void __launch_bounds__(256, 3) k_inv_update(int NB, int np, const int* __restrict__ pivots, int nNext,
-                                                       const int* __restrict__ next, double* __restrict__ A,
-                                                       const double* __restrict__ C, const double* __restrict__ R,
-                                                       const unsigned char* __restrict__ act, double* Dinv,
+                                                       const int* __restrict__ next, double* A, const double* C,
+                                                       const double* R, const unsigned char* act, double* Dinv,
                                                        unsigned char* nz, int* status) {
-  // two stages: the next pivot's operands arrive while one is multiplied
+  // two stages (one when np = 1): the next pivot's operands arrive while one
+  // is multiplied
+  FVM_PDL_TRIGGER();
   extern __shared__ __align__(16) unsigned char raw[];
   UpdateStage* stage = reinterpret_cast<UpdateStage*>(raw);
   // the diagonal tiles first (they may go on to invert a pivot block), then
@@ -683,16 +703,22 @@ __global__ void __launch_bounds__(256, 3) k_inv_update(int NB, int np, const int
   int K = -1;
   // the blocks of the tile: (I, J), (I, J+), (I+, J), (I+, J+); on the
   // diagonal (I+, J) lies below it and is not stored
-  bool stored[2][2], filled[2][2];
-#pragma unroll
-  for (int x = 0; x < 2; x++)
-#pragma unroll
-    for (int y = 0; y < 2; y++) {
-      stored[x][y] = 2 * I + x <= 2 * J + y;
-      filled[x][y] = stored[x][y] && nz[(size_t)(2 * I + x) * NB + 2 * J + y];
+  // (warp w: block (x, y), its rows 16 (w / 2 % 2) .. + 15)
+  const int warp = tid >> 5, x = warp >> 2, y = warp & 1, h = (warp >> 1) & 1;
+  if (lane < np) K = pivots[lane];
+  int nextHere = 0;  // pivots of the next step on this tile's diagonal
+  if (I == J) {
+    int v = 0;
+    for (int k = lane; k < nNext; k += 32) {
+      const int b = next[k];
+      v |= b == 2 * I ? 1 : b == 2 * I + 1 ? 2 : 0;
     }
+    nextHere = __reduce_or_sync(0xffffffffu, v);
+  }
+  FVM_PDL_WAIT();
+  const int bi = 2 * I + x, bj = 2 * J + y;
+  const bool stored = bi <= bj, filled = stored && nz[(size_t)bi * NB + bj];
   if (lane < np) {
-    K = pivots[lane];
     const unsigned char* f = act + (size_t)lane * NB;
     r0 = f[2 * I];
     r1 = f[2 * I + 1];
@@ -708,29 +734,23 @@ __global__ void __launch_bounds__(256, 3) k_inv_update(int NB, int np, const int
     return m ? __ffs(m) - 1 : -1;
   };
   const int pr0 = pivotAt(2 * I), pr1 = pivotAt(2 * I + 1), pc0 = pivotAt(2 * J), pc1 = pivotAt(2 * J + 1);
-  // pivots of the next step on this tile's diagonal
-  int nextHere = 0;
-  if (I == J) {
-    int v = 0;
-    for (int k = lane; k < nNext; k += 32) {
-      const int b = next[k];
-      v |= b == 2 * I ? 1 : b == 2 * I + 1 ? 2 : 0;
-    }
-    nextHere = __reduce_or_sync(kAll, v);
-  }
   const unsigned work = (mr0 | mr1) & (mc0 | mc1);
   const bool meets = pr0 >= 0 || pr1 >= 0 || pc0 >= 0 || pc1 >= 0;
   if (!work && !meets && !nextHere) return;
-  const int ty = tid >> 4, tx = tid & 15;
-  double acc[4][4];
+  // the warp's 16 x 32 as two rows of four 8 x 8 fragments
+  const int fr = 16 * h + (lane >> 2), fc = 2 * (lane & 3);  // the lane's first element in the block
+  double acc[2][4][2];
+  {
+    const double* b = A + block_at(NB, min(bi, bj), max(bi, bj)) + fr * kBlk + fc;
 #pragma unroll
-  for (int u = 0; u < 4; u++)
+    for (int u = 0; u < 2; u++)
 #pragma unroll
-    for (int v = 0; v < 4; v++) {
-      const int x = u >> 1, y = v >> 1;
-      acc[u][v] = filled[x][y] ? A[block_at(NB, 2 * I + x, 2 * J + y) + (ty + 16 * (u & 1)) * kBlk + tx + 16 * (v & 1)]
-                               : 0.0;
-    }
+      for (int v = 0; v < 4; v++) {
+        const double2 d = filled ? *reinterpret_cast<const double2*>(b + 8 * u * kBlk + 8 * v) : make_double2(0.0, 0.0);
+        acc[u][v][0] = d.x;
+        acc[u][v][1] = d.y;
+      }
+  }
   // thread t copies C row t / 16 (+ 16 u), columns 2 (t mod 16), and R row
   // t / 32 (+ 8 u), columns 2 (t mod 32)
   const unsigned mcT = (lane >> 4) ? mc1 : mc0;
@@ -766,75 +786,77 @@ __global__ void __launch_bounds__(256, 3) k_inv_update(int NB, int np, const int
     }
     __syncthreads();
     const UpdateStage& g = stage[cur];
-#pragma unroll 4
-    for (int t = 0; t < kBlk; t++) {
-      double c[4], r[4];
+    const double* ca = &g.C[32 * x + fr][lane & 3];
+    const double* rb = &g.R[lane & 3][32 * y + (lane >> 2)];
 #pragma unroll
-      for (int u = 0; u < 4; u++) c[u] = g.C[ty + 16 * u][t];
+    for (int k = 0; k < kBlk; k += 4) {
+      double c[2], r[4];
 #pragma unroll
-      for (int v = 0; v < 4; v++) r[v] = g.R[t][tx + 16 * v];
+      for (int u = 0; u < 2; u++) c[u] = -ca[8 * u * (kBlk + 4) + k];
 #pragma unroll
-      for (int u = 0; u < 4; u++)
+      for (int v = 0; v < 4; v++) r[v] = rb[k * (64 + 4) + 8 * v];
 #pragma unroll
-        for (int v = 0; v < 4; v++) acc[u][v] -= c[u] * r[v];
+      for (int u = 0; u < 2; u++)
+#pragma unroll
+        for (int v = 0; v < 4; v++) mma_f64(acc[u][v], c[u], r[v]);
     }
     __syncthreads();  // the stage is free for the pivot after the next
   }
-  // write each block: pivot rows and columns take R, the pivot block -D^-1
-#pragma unroll
-  for (int x = 0; x < 2; x++)
-#pragma unroll
-    for (int y = 0; y < 2; y++) {
-      if (!stored[x][y]) continue;
-      const int bi = 2 * I + x, bj = 2 * J + y;
-      double* b = A + block_at(NB, bi, bj) + ty * kBlk + tx;
-      const unsigned mrx = x ? mr1 : mr0, mcy = y ? mc1 : mc0;
-      const int kr = x ? pr1 : pr0, kc = y ? pc1 : pc0;
-      if (kr < 0 && kc < 0) {
-        if (!(mrx & mcy)) continue;
+  // write the block: pivot rows and columns take R, the pivot block -D^-1
+  const unsigned mrx = x ? mr1 : mr0, mcy = y ? mc1 : mc0;
+  const int kr = x ? pr1 : pr0, kc = y ? pc1 : pc0;
+  if (stored) {
+    double* b = A + block_at(NB, bi, bj) + fr * kBlk + fc;
+    if (kr < 0 && kc < 0) {
+      if (mrx & mcy) {
 #pragma unroll
         for (int u = 0; u < 2; u++)
 #pragma unroll
-          for (int v = 0; v < 2; v++) b[16 * u * kBlk + 16 * v] = acc[2 * x + u][2 * y + v];
-        if (!filled[x][y] && tid == 0) nz[(size_t)bi * NB + bj] = 1;
-        continue;
+          for (int v = 0; v < 4; v++)
+            *reinterpret_cast<double2*>(b + 8 * u * kBlk + 8 * v) = make_double2(acc[u][v][0], acc[u][v][1]);
+        if (!filled && h == 0 && lane == 0) nz[(size_t)bi * NB + bj] = 1;
       }
+    } else {
       // R of column bj, R^T of row bi, or -D^-1; a block that the pivot does
       // not couple to stays as it is
-      const double* from;
+      const double* from = nullptr;
       int rs = kBlk, cs = 1;
       double sign = 1.0;
       if (bi == bj) {
         from = Dinv + (size_t)bi * kBlk * kBlk;
         sign = -1.0;
       } else if (kr >= 0) {
-        if (!(mcy >> kr & 1)) continue;
-        from = R + ((size_t)kr * NB + bj) * kBlk * kBlk;
-      } else {
-        if (!(mrx >> kc & 1)) continue;
+        if (mcy >> kr & 1) from = R + ((size_t)kr * NB + bj) * kBlk * kBlk;
+      } else if (mrx >> kc & 1) {
         from = R + ((size_t)kc * NB + bi) * kBlk * kBlk;
         rs = 1;
         cs = kBlk;
       }
-      for (int u = 0; u < 2; u++)
-        for (int v = 0; v < 2; v++)
-          b[16 * u * kBlk + 16 * v] = sign * from[(ty + 16 * u) * rs + (tx + 16 * v) * cs];
+      if (from)
+        for (int u = 0; u < 2; u++)
+          for (int v = 0; v < 4; v++)
+            for (int e = 0; e < 2; e++)
+              b[8 * u * kBlk + 8 * v + e] = sign * from[(fr + 8 * u) * rs + (fc + 8 * v + e) * cs];
     }
-  for (int x = 0; x < 2; x++) {
-    if (!(nextHere >> x & 1)) continue;
+  }
+  for (int z = 0; z < 2; z++) {
+    if (!(nextHere >> z & 1)) continue;
     // the block's values from the registers (a pivot of the next step is no
     // pivot of this one)
     __syncthreads();
+    if (x == z && y == z)
 #pragma unroll
-    for (int u = 0; u < 4; u++)
+      for (int u = 0; u < 2; u++)
 #pragma unroll
-      for (int v = 0; v < 4; v++)
-        if (u >> 1 == x && v >> 1 == x) stage[0].C[ty + 16 * (u & 1)][tx + 16 * (v & 1)] = acc[u][v];
+        for (int v = 0; v < 4; v++) {
+          stage[0].C[fr + 8 * u][fc + 8 * v] = acc[u][v][0];
+          stage[0].C[fr + 8 * u][fc + 8 * v + 1] = acc[u][v][1];
+        }
     __syncthreads();
     double d[4];
 #pragma unroll
     for (int k = 0; k < 4; k++) d[k] = stage[0].C[4 * (tid >> 5) + k][lane];
-    invert_block(d, *reinterpret_cast<BlockInverse*>(&stage[0].R[0][0]), Dinv + (size_t)(2 * I + x) * kBlk * kBlk, status);
+    invert_block(d, *reinterpret_cast<BlockInverse*>(&stage[0].R[0][0]), Dinv + (size_t)(2 * I + z) * kBlk * kBlk, status);
   }
 }
 
@@ -843,35 +865,33 @@ __global__ void __launch_bounds__(256, 3) k_inv_update(int NB, int np, const int
 // memory and writes each to its own row (ld apart, zero past column n),
 // columns gathered there
 template <class T, int W>
-__global__ void __launch_bounds__(512) k_inv_finish(int n, int NB, const int* __restrict__ pos,
-                                                    const int* __restrict__ rowAt, const double* __restrict__ A,
-                                                    const unsigned char* __restrict__ nz, T* __restrict__ out, int ld) {
+__global__ void __launch_bounds__(512) k_inv_finish(int n, int NB, const int* pos, const int* rowAt, const double* A,
+                                                    const unsigned char* nz, T* out, int ld) {
   extern __shared__ __align__(16) unsigned char raw[];
+  FVM_PDL();
   T* strip = reinterpret_cast<T*>(raw);  // [W][NB * 32]
   const int N = NB * kBlk, p0 = blockIdx.x * W, I = p0 / kBlk, r0 = p0 % kBlk;
+  const int lane = threadIdx.x & 31;
   for (int J = threadIdx.x >> 5; J < NB; J += 16) {
-    const int lane = threadIdx.x & 31;
     const bool on = nz[(size_t)min(I, J) * NB + max(I, J)];
     const double* b = A + block_at(NB, min(I, J), max(I, J));
-    if (I <= J) {
-      for (int r = 0; r < W; r++)
-        strip[(size_t)r * N + J * kBlk + lane] = on ? (T)-b[(r0 + r) * kBlk + lane] : T(0);
-    } else {
-      for (int r = 0; r < W; r++)
-        strip[(size_t)r * N + J * kBlk + lane] = on ? (T)-b[lane * kBlk + r0 + r] : T(0);
-    }
+    const int rs = I <= J ? kBlk : 1, cs = I <= J ? 1 : kBlk;
+    double v[W];
+#pragma unroll
+    for (int r = 0; r < W; r++) v[r] = on ? -b[(r0 + r) * rs + lane * cs] : 0.0;
+#pragma unroll
+    for (int r = 0; r < W; r++) strip[(size_t)r * N + J * kBlk + lane] = (T)v[r];
   }
+  int row[W];
+#pragma unroll
+  for (int r = 0; r < W; r++) row[r] = rowAt[p0 + r];
   __syncthreads();
-  for (int r = 0; r < W; r++) {
-    const int i = rowAt[p0 + r];
-    if (i < 0) continue;
-    for (int j = threadIdx.x; j < ld; j += 512)
-      out[(size_t)i * ld + j] = j < n ? strip[(size_t)r * N + pos[j]] : T(0);
+  for (int j = threadIdx.x; j < ld; j += 512) {
+    const int at = j < n ? pos[j] : -1;
+#pragma unroll
+    for (int r = 0; r < W; r++)
+      if (row[r] >= 0) out[(size_t)row[r] * ld + j] = at >= 0 ? strip[(size_t)r * N + at] : T(0);
   }
-}
-__global__ void k_inv_rows(int n, const int* __restrict__ pos, int* rowAt) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) rowAt[pos[i]] = i;
 }
 
 // a coarse row's point: the mean of its fine rows'
@@ -934,34 +954,33 @@ void inverse_symmetric(const SellView<double>& a, const int* rowSlice, const flo
   ok(cudaMemsetAsync(nz, 0, (size_t)NB * NB, st), "cudaMemsetAsync");
   ok(cudaMemsetAsync(rowAt, 0xff, sizeof(int) * (size_t)NB * kBlk, st), "cudaMemsetAsync");
   const int rows = (std::max(n, NB) + 127) / 128;
-  k_inv_flag<<<rows, 128, 0, st>>>(a, rowSlice, pos, NB, nz);
-  k_inv_rows<<<rows, 128, 0, st>>>(n, pos, rowAt);
-  k_inv_clear<<<dim3(NB, NB), 256, 0, st>>>(NB, nz, A);
-  k_inv_scatter<<<rows, 128, 0, st>>>(a, rowSlice, pos, NB, A);
+  pdl_launch(k_inv_flag, rows, 128, st, a, rowSlice, pos, NB, nz, rowAt);
+  pdl_launch(k_inv_clear, dim3(NB, NB), 256, st, NB, nz, A);
+  pdl_launch(k_inv_scatter, rows, 128, st, a, rowSlice, pos, NB, A);
   const int* pivots = dPlan->pivot;  // (device address arithmetic only)
-  k_inv_first<<<plan.start[1], 256, 0, st>>>(NB, pivots, A, Dinv, status);
+  pdl_launch(k_inv_first, plan.start[1], 256, st, NB, pivots, A, Dinv, status);
   const int tiles = (NB / 2) * (NB / 2 + 1) / 2;
-  constexpr int smem = 2 * (int)sizeof(UpdateStage);
-  ok(cudaFuncSetAttribute(k_inv_update, cudaFuncAttributeMaxDynamicSharedMemorySize, smem), "cudaFuncSetAttribute");
+  ok(cudaFuncSetAttribute(k_inv_update, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * (int)sizeof(UpdateStage)),
+     "cudaFuncSetAttribute");
   for (int s = 0; s < plan.steps; s++) {
     const int np = plan.start[s + 1] - plan.start[s];
     const int nNext = s + 1 < plan.steps ? plan.start[s + 2] - plan.start[s + 1] : 0;
     const int* at = pivots + plan.start[s];
-    k_inv_panel<<<dim3(NB, np), 256, 0, st>>>(NB, at, A, Dinv, nz, C, R, act);
-    k_inv_update<<<tiles, 256, smem, st>>>(NB, np, at, nNext, pivots + plan.start[s + 1], A, C, R, act, Dinv, nz, status);
+    pdl_launch(k_inv_panel, dim3(NB, np), 256, st, NB, at, A, Dinv, nz, C, R, act);
+    pdl_launch_smem(k_inv_update, tiles, 256, (np > 1 ? 2 : 1) * sizeof(UpdateStage), st, NB, np, at, nNext,
+                    pivots + plan.start[s + 1], A, C, R, act, Dinv, nz, status);
   }
   const int N = NB * kBlk;
   if (out64) {
     const size_t smem = sizeof(double) * 4 * (size_t)N;
     ok(cudaFuncSetAttribute(k_inv_finish<double, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
        "cudaFuncSetAttribute");
-    k_inv_finish<double, 4><<<N / 4, 512, smem, st>>>(n, NB, pos, rowAt, A, nz, out64, n);
+    pdl_launch_smem(k_inv_finish<double, 4>, N / 4, 512, smem, st, n, NB, pos, rowAt, A, nz, out64, n);
   } else {
     const size_t smem = sizeof(float) * 8 * (size_t)N;
     ok(cudaFuncSetAttribute(k_inv_finish<float, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
        "cudaFuncSetAttribute");
-    k_inv_finish<float, 8><<<N / 8, 512, smem, st>>>(n, NB, pos, rowAt, A, nz, outF,
-                                                             inverse_f32_stride(n));
+    pdl_launch_smem(k_inv_finish<float, 8>, N / 8, 512, smem, st, n, NB, pos, rowAt, A, nz, outF, inverse_f32_stride(n));
   }
   ok(cudaGetLastError(), "coarsest inverse");
 }
