@@ -1438,6 +1438,12 @@ void LinearSolve::run(cudaGraphExec_t& exec, cudaStream_t st, const std::functio
     body();
     return;
   }
+  if (singleUse_ && eagerRuns_ < kEagerRuns) {
+    eagerRuns_++;
+    body();
+    launches += h_.kernelsPerCycle() + 7;  // the cycle and a CG iteration's own
+    return;
+  }
   if (!exec) {
     cudaGraph_t g = nullptr;
     CUDA_OK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
@@ -2107,7 +2113,7 @@ bool LinearSolve::cgFlexible() const {
 bool LinearSolve::deviceSolvable() const {
   const SolverOptions& o = h_.options();
   return o.solver != kSolverJacobi && (o.preconditioner == kPrecAMG || o.solver == kSolverBCGStab) && o.useGraphs &&
-         o.verbosity <= 0 && !(learned_ && learnedActive_) && !graphsFailed_ && !loopFailed_;
+         o.verbosity <= 0 && !(learned_ && learnedActive_) && !graphsFailed_ && !loopFailed_ && !singleUse_;
 }
 
 LinearSolve::LoopKey LinearSolve::loopKey() const {

@@ -410,6 +410,13 @@ class LinearSolve {
   // builds the graph of the solve's device loop now (when it will be used)
   // rather than in the first solve
   void prebuild(cudaStream_t st);
+  // The hierarchy is rebuilt before the next solve (a matrix that follows the
+  // solution): no graph of the whole solve, and the first iterations launch
+  // their kernels one by one. Capturing and instantiating the solve's graph
+  // took 0.7 ms where the solve itself, two or three iterations on 41k cells,
+  // takes 0.2; from iteration kEagerRuns on an iteration's own graph (built
+  // then) is the cheaper way again.
+  void setSingleUse(bool on) { singleUse_ = on; }
   const int* deviceLoopState() const { return loopInt_; }
   const double* deviceInitialNorm() const { return history_; }
   long long loopBodyNodes() const { return loopBodyNodes_; }
@@ -480,6 +487,9 @@ class LinearSolve {
   void learnedStep(cudaStream_t st, double* x, double* r, double acceptFactor);
   std::map<const void*, long long> nodeCounts_;
   bool graphsFailed_ = false;
+  static constexpr int kEagerRuns = 4;
+  bool singleUse_ = false;
+  int eagerRuns_ = 0;
 
  public:
   long long launches = 0;  // kernels + copies enqueued (graph nodes counted per replay)

@@ -979,6 +979,7 @@ void ThermalModel::ensureMatrix() {
     lap("hierarchy on the device");
     dPerm_ = const_cast<int*>(hier_.finestPermDevice());
     solver_.reset(new LinearSolve(hier_));
+    solver_->setSingleUse(matrixDependsOnT_);
     solverGen_++;
     solver_->setLearned(learned_);
     // the solve's graphs are built while the GPU computes the coarsest
@@ -1044,6 +1045,7 @@ void ThermalModel::ensureMatrix() {
   CUDA_OK(cudaMemcpyAsync(dPerm_, hier_.packed(0).perm.data(), sizeof(int) * (size_t)n, cudaMemcpyHostToDevice,
                           stream_));
   solver_.reset(new LinearSolve(hier_));
+  solver_->setSingleUse(matrixDependsOnT_);
   solverGen_++;
   solver_->setLearned(learned_);
   lap("solver workspace");
