@@ -110,6 +110,7 @@ struct OrderShared {
   int nodeDepth[kNodes], nodeCount[kNodes], nodeBlock[kNodes];
   int warpCount[kOrderThreads / 32][kNodes];
   int parts, nodes;
+  unsigned short place[kMaxN];
 };
 
 // floats as integers of the same order, and back
@@ -146,15 +147,22 @@ __global__ void __launch_bounds__(kOrderThreads) k_inv_order(SellView<double> a,
     s.node[i] = kNone;
     for (int d = 0; d < 3; d++) s.at[d][i] = points ? points[(size_t)d * n + i] : 0.0f;
   }
-  // fn(j) for every column j of the thread's q-th row, four loads in flight
+  // fn(j) for every column j of the thread's q-th row, eight loads in flight
   auto columns = [&](int q, auto&& fn) {
-    for (int k = 0; k < width[q]; k += 4) {
-      int j[4];
+    for (int k = 0; k < width[q]; k += 8) {
+      int j[8];
 #pragma unroll
-      for (int u = 0; u < 4; u++) j[u] = __ldg(a.cols + base[q] + 32 * min(k + u, width[q] - 1));
+      for (int u = 0; u < 8; u++) j[u] = __ldg(a.cols + base[q] + 32 * min(k + u, width[q] - 1));
 #pragma unroll
-      for (int u = 0; u < 4; u++) fn(j[u]);
+      for (int u = 0; u < 8; u++) fn(j[u]);
     }
+  };
+  // count[key] += 1 for every lane with a key >= 0: one atomic per warp and
+  // key (most rows share a component and a node; 3313 atomics on one address
+  // took 43k cycles)
+  auto tally = [&](int* count, int key) {
+    const unsigned same = __match_any_sync(0xffffffffu, key);
+    if (key >= 0 && lane == __ffs(same) - 1) atomicAdd(&count[key], __popc(same));
   };
   if (t == 0) {
     s.parts = 1;
@@ -185,9 +193,15 @@ __global__ void __launch_bounds__(kOrderThreads) k_inv_order(SellView<double> a,
   __syncthreads();
   for (int k = 1; k < kMaxN; k *= 2) {
     int up[kPer];
+    bool moved = false;
 #pragma unroll
-    for (int q = 0; q < kPer; q++) up[q] = t + q * kOrderThreads < n ? s.label[s.label[t + q * kOrderThreads]] : 0;
-    __syncthreads();
+    for (int q = 0; q < kPer; q++) {
+      const int i = t + q * kOrderThreads;
+      const int l = i < n ? s.label[i] : 0;
+      up[q] = i < n ? s.label[l] : 0;
+      moved = moved || up[q] != l;
+    }
+    if (!__syncthreads_or(moved)) break;
 #pragma unroll
     for (int q = 0; q < kPer; q++)
       if (t + q * kOrderThreads < n) s.label[t + q * kOrderThreads] = up[q];
@@ -198,7 +212,7 @@ __global__ void __launch_bounds__(kOrderThreads) k_inv_order(SellView<double> a,
     const int i = t + q * kOrderThreads;
     if (i >= n) continue;
     columns(q, [&](int j) {
-      if (j >= i) return;
+      if (j >= i || parent[j] == parent[i]) return;  // mostly one tree already
       int x = i, y = j;
       while (true) {
         x = find(x);
@@ -216,11 +230,11 @@ __global__ void __launch_bounds__(kOrderThreads) k_inv_order(SellView<double> a,
   for (int e = t; e < n; e += kOrderThreads) s.dist[e] = 0;
   __syncthreads();
 #pragma unroll
-  for (int q = 0; q < kPer; q++)
-    if (t + q * kOrderThreads < n) {
-      s.label[t + q * kOrderThreads] = root[q];
-      atomicAdd(&s.dist[root[q]], 1);
-    }
+  for (int q = 0; q < kPer; q++) {
+    const int i = t + q * kOrderThreads;
+    if (i < n) s.label[i] = root[q];
+    tally(s.dist, i < n ? root[q] : -1);
+  }
   __syncthreads();
   // rows of each row's component; the largest component's first row
 #pragma unroll
@@ -372,8 +386,16 @@ __global__ void __launch_bounds__(kOrderThreads) k_inv_order(SellView<double> a,
       }
     }
     __syncthreads();
-    for (int i = t; i < n; i += kOrderThreads)
-      if (s.node[i] == kNone && s.mode[s.part[i]]) s.side[i] = bin(i, s.part[i]) > s.cut[s.part[i]];
+    // (place: a row's part and side in one word, none for rows not being split)
+    for (int i = t; i < n; i += kOrderThreads) {
+      int place = 0xffff;
+      if (s.node[i] == kNone && s.mode[s.part[i]]) {
+        const int side = bin(i, s.part[i]) > s.cut[s.part[i]] ? 1 : 0;
+        s.side[i] = (unsigned char)side;
+        place = 2 * s.part[i] + side;
+      }
+      s.place[i] = (unsigned short)place;
+    }
     __syncthreads();
     // the rows of either side that touch the other
 #pragma unroll
@@ -381,9 +403,9 @@ __global__ void __launch_bounds__(kOrderThreads) k_inv_order(SellView<double> a,
       const int i = t + q * kOrderThreads;
       int key = -1;
       if (i < n && s.node[i] == kNone && s.mode[s.part[i]] == 2) {
-        const int p = s.part[i], mine = s.side[i] & 1;
+        const int p = s.part[i], mine = s.side[i] & 1, across = 2 * p + 1 - mine;
         bool hit = false;
-        columns(q, [&](int j) { hit = hit || (s.part[j] == p && s.node[j] == kNone && (s.side[j] & 1) != mine); });
+        columns(q, [&](int j) { hit = hit || s.place[j] == across; });
         if (hit) {
           s.side[i] = (unsigned char)(mine | 2);
           key = 2 * p + mine;
@@ -435,9 +457,8 @@ __global__ void __launch_bounds__(kOrderThreads) k_inv_order(SellView<double> a,
 #pragma unroll
   for (int q = 0; q < kPer; q++) {
     const int i = t + q * kOrderThreads;
-    if (i >= n) continue;
-    if (s.node[i] == kNone) s.node[i] = (unsigned short)(separators + s.part[i]);
-    atomicAdd(&s.nodeCount[s.node[i]], 1);
+    if (i < n && s.node[i] == kNone) s.node[i] = (unsigned short)(separators + s.part[i]);
+    tally(s.nodeCount, i < n ? (int)s.node[i] : -1);
   }
   __syncthreads();
   // leaves first, then the separators from the deepest up; in each group
