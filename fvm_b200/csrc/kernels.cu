@@ -390,6 +390,79 @@ __global__ void k_csr_residual(int n, const int* __restrict__ row, const int* __
   if (threadIdx.x == 0) partials[blockIdx.x] = t;
 }
 
+// The same for large systems: one CTA of 32 warps per SM over a contiguous
+// share of the rows, a warp 32 rows at a time. Its lanes take the rows'
+// entries side by side (whole lines of columns and values, 192 entries in
+// flight), leave the products in shared memory and then add them up row by
+// row, in stored order: the same bits. What bounds both is the gather of x,
+// an L1 line per entry (15M of them are 52 of the 96 us of 3M rows); here
+// neighbouring rows meet in one SM's L1, and what is read once does not push
+// x out of it (evict-first). Against a thread per row, 3 to 7 entries: 200k
+// rows 14.4 us both, 300k 16.4 / 18.5, 600k 22.6 / 28.7, 1M 30.8 / 41.1, 3M
+// 84 / 96; below 2^18 rows a share is too short to pay. (A window of x in
+// shared memory was slower the larger it was: 92 to 141 us.)
+constexpr int kCsrTileRows = 1 << 18, kCsrCtas = 148, kCsrChunk = 6;
+__global__ void __launch_bounds__(1024, 1) k_csr_residual_tiles(int n, const int* __restrict__ row,
+                                                                const int* __restrict__ col,
+                                                                const double* __restrict__ diag,
+                                                                const double* __restrict__ off,
+                                                                const double* __restrict__ x,
+                                                                const double* __restrict__ b, double* r,
+                                                                double* partials) {
+  __shared__ double product[32][32 * kCsrChunk];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  double* p = product[w];
+  const int tiles = (n + 31) >> 5;
+  const int t1 = (int)((long long)tiles * (blockIdx.x + 1) / gridDim.x);
+  int t = (int)((long long)tiles * blockIdx.x / gridDim.x) + w;
+  // a lane's row: its entries are k0 .. k1 - 1; the next tile's bounds are
+  // fetched a tile ahead
+  int n0 = 0, n1 = 0;
+  if (t < t1) {
+    n0 = row[min(32 * t + lane, n)];
+    n1 = row[min(32 * t + lane + 1, n)];
+  }
+  double l1 = 0.0;
+  for (; t < t1; t += 32) {
+    const int i = 32 * t + lane, k0 = n0, k1 = n1;
+    if (t + 32 < t1) {
+      n0 = row[min(i + 1024, n)];
+      n1 = row[min(i + 1025, n)];
+    }
+    double s = i < n ? __ldcs(b + i) + __ldcs(diag + i) * x[i] : 0.0;
+    const int e0 = __shfl_sync(0xffffffffu, k0, 0), len = __shfl_sync(0xffffffffu, k1, 31) - e0;
+    const int a0 = k0 - e0, a1 = k1 - e0;
+    for (int c = 0; c < len; c += 32 * kCsrChunk) {
+      int j[kCsrChunk];
+      double v[kCsrChunk];
+#pragma unroll
+      for (int u = 0; u < kCsrChunk; u++) {
+        const int k = c + 32 * u + lane;
+        j[u] = k < len ? __ldcs(col + e0 + k) : -1;
+        v[u] = k < len ? __ldcs(off + e0 + k) : 0.0;
+      }
+#pragma unroll
+      for (int u = 0; u < kCsrChunk; u++)
+        if (j[u] >= 0) p[32 * u + lane] = v[u] * x[j[u]];
+      __syncwarp();
+      const int first = max(a0, c), last = min(a1, c + 32 * kCsrChunk);
+      for (int k = first; k < last; k++) s = s + p[k - c];
+      __syncwarp();
+    }
+    if (i < n) {
+      if (r) __stcs(r + i, s);
+      l1 += fabs(s);
+    }
+  }
+  for (int o = 16; o > 0; o >>= 1) l1 += __shfl_down_sync(0xffffffffu, l1, o);
+  __syncthreads();
+  if (lane == 0) product[0][w] = l1;
+  __syncthreads();
+  if (threadIdx.x) return;
+  for (int k = 1; k < 32; k++) l1 += product[0][k];
+  partials[blockIdx.x] = l1;
+}
+
 __global__ void __launch_bounds__(kBlock, 4) k_spmv(SellView<double> a, int nSlices, const double* __restrict__ x, double* y) {
   FVM_PDL();
   const int lane = threadIdx.x & 31;
@@ -1693,10 +1766,13 @@ int residual_partials(int nSlices, int n, int ellWidth) {
   if (ellWidth >= 1 && ellWidth <= 8) return ceil_div(n, kBlock) < 1 ? 1 : ceil_div(n, kBlock);
   return reduce_blocks(nSlices);
 }
-int csr_residual_blocks(int n) { return ceil_div(n, kBlock); }
+int csr_residual_blocks(int n) { return n >= kCsrTileRows ? kCsrCtas : ceil_div(n, kBlock); }
 void csr_residual(int n, const int* row, const int* col, const double* diag, const double* off,
                   const double* x, const double* b, double* r, double* partials, cudaStream_t st) {
-  k_csr_residual<<<csr_residual_blocks(n), kBlock, 0, st>>>(n, row, col, diag, off, x, b, r, partials);
+  if (n >= kCsrTileRows)
+    k_csr_residual_tiles<<<kCsrCtas, 1024, 0, st>>>(n, row, col, diag, off, x, b, r, partials);
+  else
+    k_csr_residual<<<csr_residual_blocks(n), kBlock, 0, st>>>(n, row, col, diag, off, x, b, r, partials);
 }
 void csr_residual_finish(int nPartials, const double* partials, double* l1, cudaStream_t st) {
   pdl_launch(k_sum_partials, 1, 1024, st, nPartials, partials, l1);

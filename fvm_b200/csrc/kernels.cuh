@@ -117,8 +117,8 @@ void cg_update(int n, const double* alpha, const double* p, const double* q, dou
 int residual_partials(int nSlices, int n, int ellWidth);
 
 // r = b + D x + O x on a plain CSR matrix (implicit diagonal, reference
-// column order), one thread per row; block k writes the L1 sum of its 256
-// rows to partials[k] (csr_residual_blocks(n) of them), then
+// column order); block k writes the L1 sum of its rows to partials[k]
+// (csr_residual_blocks(n) of them, at most one per 256 rows), then
 // csr_residual_finish sums them in a fixed order into *l1.
 int csr_residual_blocks(int n);
 void csr_residual(int n, const int* row, const int* col, const double* diag, const double* off,

@@ -29,8 +29,10 @@
 
 namespace {
 
-// one partial per 256-row block: up to 65536 blocks = 16,777,216 rows
+// room for one partial per 256 rows, the most any kernel leaves: 65536 for
+// 16,777,216 rows
 constexpr int kMaxPartials = 65536;
+constexpr int kMaxRows = 256 * kMaxPartials;
 
 __device__ __align__(256) double g_residual_scratch[kMaxPartials + 1];
 
@@ -106,7 +108,7 @@ extern "C" int fvm_csr_residual_device_noalloc(int n, const int* row, const int*
     FVM_REQUIRE(row && col && diag && off && x && b && l1norm, fvm::kBadArgument,
                 "null device pointer");
     const int np = fvm::dev::csr_residual_blocks(n);
-    FVM_REQUIRE(np <= kMaxPartials, fvm::kTooLarge,
+    FVM_REQUIRE(n <= kMaxRows && np <= kMaxPartials, fvm::kTooLarge,
                 "fvm_csr_residual_device_noalloc handles at most 16777216 rows (its fixed "
                 "scratch holds 65536 block sums); use fvm_csr_residual for larger systems");
     double* scratch = scratch_for_current_context();

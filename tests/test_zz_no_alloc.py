@@ -143,3 +143,47 @@ def test_no_alloc_after_device_reset():
     out = subprocess.run([sys.executable, "-c", _RESET_CHILD, root, here], capture_output=True, text=True,
                          timeout=300)
     assert out.returncode == 0 and "reset ok" in out.stdout, out.stdout + out.stderr
+
+
+@pytest.mark.parametrize("n", [(1 << 18) - 1, 1 << 18, (1 << 18) + 1, 300_017])
+def test_large_systems_in_reference_order(n):
+    """From 2^18 rows on a warp takes 32 rows' entries side by side: rows with
+    none, rows longer than a warp's 192 products, and the last, partial tile.
+    r equals the scalar sums in stored order bit for bit; the norm is the sum
+    of n positive terms in another order: n 2^-53 <= 4e-11 at the very most,
+    1e-13 asked as elsewhere (a tree of 148 x 1024 chains of 10 rows)."""
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    rng = np.random.default_rng(n)
+    cnt = rng.integers(0, 8, n)
+    cnt[[0, 5, n // 2, n - 1]] = [0, 700, 193, 192]
+    cnt[1000:1064] = 0
+    row = np.zeros(n + 1, np.int32)
+    row[1:] = np.cumsum(cnt)
+    of = np.repeat(np.arange(n), cnt)
+    col = np.clip(of + rng.integers(-5000, 5001, len(of)), 0, n - 1).astype(np.int32)
+    off = rng.uniform(0.1, 1.0, len(of))
+    diag = -rng.uniform(4.0, 5.0, n)
+    x = rng.standard_normal(n)
+    b = rng.standard_normal(n)
+    ref = b + diag * x
+    k = row[:-1].copy()
+    for _ in range(int(cnt.max())):  # one stored entry of every row at a time
+        live = np.flatnonzero(k < row[1:])
+        ref[live] = ref[live] + off[k[live]] * x[col[k[live]]]
+        k[live] += 1
+    lib = _lib.load()
+    dev = torch.device("cuda:0")
+    d = [torch.as_tensor(a, device=dev) for a in (row, col, diag, off, x, b)]
+    for keep in (True, False):
+        d_r = torch.full((n,), float("nan"), dtype=torch.float64, device=dev)
+        d_norm = torch.full((1,), float("nan"), dtype=torch.float64, device=dev)
+        rc = lib.fvm_csr_residual_device_noalloc(
+            n, *[ctypes.c_void_p(t.data_ptr()) for t in d], ctypes.c_void_p(d_r.data_ptr()) if keep else None,
+            ctypes.c_void_p(d_norm.data_ptr()), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+        assert rc == 0, lib.fvm_last_error().decode()
+        torch.cuda.synchronize()
+        if keep:
+            np.testing.assert_array_equal(d_r.cpu().numpy(), ref)
+        assert abs(float(d_norm[0]) - np.abs(ref).sum()) <= 1e-13 * np.abs(ref).sum()
