@@ -208,3 +208,67 @@ def test_fused_prolongation_is_bitwise_neutral(kind):
     (T0, o0, c0), (T1, o1, c1) = out
     assert (o0, c0) == (o1, c1)
     np.testing.assert_array_equal(T0, T1)
+
+
+def _disk(sides, rings, seed):
+    """A polygon of `sides` sides inside rings of quads: one row with `sides`
+    entries among rows of four."""
+    a = 2.0 * np.pi * np.arange(sides) / sides
+    nodes = np.zeros((sides * (rings + 1), 3))
+    for k in range(rings + 1):
+        nodes[k * sides: (k + 1) * sides, :2] = (1.0 + 0.5 * k) * np.stack([np.cos(a), np.sin(a)], 1)
+    s = np.arange(sides)
+    nid = lambda k, s: k * sides + s % sides  # noqa: E731
+    cid = lambda k, s: 1 + k * sides + s % sides  # noqa: E731
+    fc, fn = [np.stack([0 * s, cid(0, s)], 1)], [np.stack([nid(0, s), nid(0, s + 1)], 1)]
+    for k in range(rings):
+        fc.append(np.stack([cid(k, s), cid(k, s + 1)], 1))
+        fn.append(np.stack([nid(k, s + 1), nid(k + 1, s + 1)], 1))
+        if k:
+            fc.append(np.stack([cid(k - 1, s), cid(k, s)], 1))
+            fn.append(np.stack([nid(k, s), nid(k, s + 1)], 1))
+    fc, fn = np.concatenate(fc), np.concatenate(fn)
+    cen = np.zeros((1 + sides * rings, 2))
+    for k in range(rings):
+        r = 1.25 + 0.5 * k
+        cen[1 + k * sides: 1 + (k + 1) * sides] = r * np.stack([np.cos(a + np.pi / sides), np.sin(a + np.pi / sides)], 1)
+    fn = meshgen._orient_2node(nodes, fn, cen[fc[:, 0]], cen[fc[:, 1]])
+    gfc, gfn = [], []
+    for part in (s[: sides // 2], s[sides // 2:]):
+        cells = cid(rings - 1, part)
+        f = np.stack([nid(rings, part), nid(rings, part + 1)], 1)
+        gfn.append(meshgen._orient_2node(nodes, f, cen[cells], 2.0 * cen[cells]))
+        gfc.append(np.stack([cells, 0 * cells], 1))
+    mesh = meshgen._pack(2, 1 + sides * rings, nodes, fc, fn, gfc, gfn)
+    rng = np.random.default_rng(seed)
+    return mesh, np.exp(rng.normal(size=mesh["nCells"])), rng.uniform(size=mesh["nCells"])
+
+
+@pytest.mark.parametrize("sides", [30, 61, 66, 240])
+def test_galerkin_of_one_long_row_among_short_ones(sides):
+    """Levels of short rows give a coarse row half a warp and 64 entries; an
+    aggregate with more is left to the block's first warp."""
+    mesh, k, s = _disk(sides, 5, seed=sides)
+    tm, _, _ = gpu_model(mesh, {1: ("T", 300.0), 2: ("T", 400.0)}, solver=_cg(_amg(coarsest=20)),
+                         fields={"conductivity": k, "source": s}, opts={"relativeTolerance": 1e-8})
+    sizes, cis = tm.getHierarchy()
+    A = tm.getLevelMatrix(0)
+    assert np.diff(A["row"]).max() == sides
+    for lvl, ci in enumerate(cis):
+        Ac = tm.getLevelMatrix(lvl + 1)
+        cd, off = _galerkin(A, ci, sizes[lvl])
+        scale = np.abs(cd).max()
+        np.testing.assert_allclose(Ac["diag"], cd, rtol=1e-12, atol=1e-12 * scale)
+        got, want = _as_dict(Ac), {key: v for key, v in off.items() if v != 0.0}
+        assert set(got) == set(want)
+        np.testing.assert_allclose([got[key] for key in want], list(want.values()), rtol=1e-12, atol=1e-12 * scale)
+        A = Ac
+    assert tm.advance(100).converged
+
+
+def test_galerkin_refuses_an_aggregate_beyond_its_capacity():
+    mesh, k, s = _disk(600, 3, seed=1)
+    tm, _, _ = gpu_model(mesh, {1: ("T", 300.0), 2: ("T", 400.0)}, solver=_cg(_amg(coarsest=20)),
+                         fields={"conductivity": k, "source": s})
+    with pytest.raises(Exception, match="capacity"):
+        tm.advance(1)

@@ -158,3 +158,46 @@ def test_outer_acceleration_option_range():
     a.outerAcceleration = 6
     with pytest.raises(Exception):
         _ = gpu_model(*_mesh("tet")[:1], {}, solver=a)
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+def test_single_use_hierarchies_launch_without_a_graph(precision):
+    """Radiative and mixed conditions rebuild the hierarchy before every solve:
+    no loop graph, the first iterations as single launches, the following ones
+    as one graph each. Bitwise the same as with graphs off; the inner
+    tolerance makes the solves go past that change."""
+    from fvm_b200 import models
+
+    out = []
+    for graphs in (True, False):
+        mesh, f = _mesh("hex")
+        solver = _solver(precision, True)
+        solver.preconditioner.useGraphs = graphs
+        solver.useGraphs = graphs
+        m = fvmbaseExt.Mesh.from_dict(mesh)
+        tf = models.ThermalFields("therm")
+        tm = models.ThermalModelA(models.GeomFields("geom"), tf, [m])
+        for gid, (kind, vals) in {
+            1: ("SpecifiedTemperature", {"specifiedTemperature": 300.0}),
+            2: ("SpecifiedTemperature", {"specifiedTemperature": 400.0}),
+            3: ("Radiative", {"farFieldTemperature": 310.0, "surfaceEmissivity": 0.7}),
+            4: ("Mixed", {"convectiveCoefficient": 8.0, "farFieldTemperature": 320.0, "surfaceEmissivity": 0.5}),
+        }.items():
+            bc = tm.getBCMap()[gid]
+            bc.bcType = kind
+            for name, v in vals.items():
+                bc.setVar(name, v)
+        o = tm.getOptions()
+        o.linearSolver = solver
+        o.relativeTolerance = 1e-10
+        tm.init()
+        tf.conductivity[m.getCells()] = f["k"]
+        tf.source[m.getCells()] = f["s"]
+        rep = tm.advance(30)
+        assert rep.linearIterations > 6 * rep.iterations
+        out.append((rep.iterations, rep.linearIterations, tf.temperature[m.getCells()].copy(),
+                    np.array(tm.getNormHistory())))
+    (i1, l1, t1, h1), (i0, l0, t0, h0) = out
+    assert (i1, l1) == (i0, l0)
+    np.testing.assert_array_equal(h1, h0)
+    np.testing.assert_array_equal(t1, t0)
