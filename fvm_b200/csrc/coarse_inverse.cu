@@ -19,8 +19,9 @@
 // A step is two kernels: k_inv_panel forms the new pivot rows R = D^-1 A[K][:]
 // of every pivot block of the step, k_inv_update applies them to the 64 x 64
 // tiles on and above the diagonal and inverts the next step's pivot blocks.
-// Measured, order and unpermuting included: 3313 rows (41k tets) 5.4 -> 1.1
-// ms in 23 steps instead of 104, 3385 rows (100^3 hexes, two phases) 5.6 ->
+// Measured, order and unpermuting included: 3313 rows (41k tets) 5.4 -> 0.9
+// ms in 23 steps instead of 104 (1.1 before the FP64 matrix instructions and
+// the chained launches), 3385 rows (100^3 hexes, two phases) 5.6 ->
 // 1.6 ms in 29 instead of 106, 2151 rows (1.5M tets) 2.4 -> 0.9 ms in 22
 // instead of 68, 24 independent meshes of 3930 rows 7.7 -> 0.5 ms in 11
 // instead of 123.
@@ -695,8 +696,9 @@ __device__ __forceinline__ void mma_f64(double (&d)[2], double a, double b) {
 // FP64 at the chip's rate, as long again in shared-memory reads, and three
 // CTAs of 80 registers per SM to hide those and the tile's loads behind each
 // other. The FP64 matrix instruction reads 6 operands for 8 products of 8 x 8
-// x 4 where that read 8 for 16 FMAs, and one stage suffices where the step has
-// one pivot: 28 us.
+// x 4 where that read 8 for 16 FMAs; one stage suffices where the step has
+// one pivot; the pivots are read ahead of the wait. Over the 23 steps of 3313
+// rows 31 -> 21.5 us a step (64 registers and four CTAs, with spills: 22.8).
 __global__ void __launch_bounds__(256, 3) k_inv_update(int NB, int np, const int* __restrict__ pivots, int nNext,
                                                        const int* __restrict__ next, double* A, const double* C,
                                                        const double* R, const unsigned char* act, double* Dinv,
