@@ -956,7 +956,8 @@ void Workspace::allocate(int n_, bool training, long long entries) {
     const size_t hb = sizeof(float) * (size_t)n * 32;
     check(cudaMalloc(&u, sizeof(float) * (size_t)n), "cudaMalloc");
     for (int l = 0; l <= kLayers; l++) check(cudaMalloc(&H[l], hb), "cudaMalloc");
-    check(cudaMalloc(&partials, sizeof(double) * (kReduceBlocks + 8)), "cudaMalloc");
+    // two sums a block (k_residual_loss)
+    check(cudaMalloc(&partials, sizeof(double) * (2 * kReduceBlocks + 8)), "cudaMalloc");
     check(cudaMalloc(&status, sizeof(int)), "cudaMalloc");
     check(cudaMemset(status, 0, sizeof(int)), "cudaMemset");
     if (training) {

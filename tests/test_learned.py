@@ -190,6 +190,26 @@ def test_tensor_core_layers_on_many_tiles():
     assert rel_l2(res[True][1], res[False][1]) <= 2e-2
 
 
+@pytest.mark.gpu
+def test_residual_losses_are_those_of_their_pairs():
+    """The loss of the residual objective, |r + A d|^2 / |r|^2, summed by two
+    partial sums a block: with a decoder that outputs zero it is exactly 1 for
+    every pair, whatever else the process has allocated around the sums."""
+    from fvm_b200.learned import LearnedCorrection
+
+    for keep in range(3):
+        lc = LearnedCorrection(seed=keep)
+        lc.setObjective(LearnedCorrection.RESIDUAL)
+        mesh, f, bcs, fields = _case(31 + keep)
+        tm, _, _ = gpu_model(mesh, bcs, solver=_plain(), fields=fields, opts={"relativeTolerance": 1e-10})
+        assert lc.harvest(tm, nOuter=3, perSolve=4, relativeTolerance=1e-10) == 12
+        p = lc.getParams()
+        p[mo.DEC_W:] = 0.0
+        lc.setParams(p)
+        assert lc.evaluate() == 1.0
+        assert np.all(lc.train(steps=6, lr=1e-12, seed=1)[:1] == 1.0)
+
+
 def _irregular(n, most, seed):
     """Symmetric M-matrix whose rows hold between 0 and about 2 `most` entries."""
     rng = np.random.default_rng(seed)
