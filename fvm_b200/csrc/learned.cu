@@ -791,18 +791,18 @@ __global__ void __launch_bounds__(kBlock) k_encode_bwd(int n, GraphArgs g, const
                                                        const float* dH0, const float* dM, float* gp) {
   __shared__ float sv[kWarps * 64];
   __shared__ __align__(16) float sStage[kWarps * kStage];
-  FVM_PDL();
+  FVM_PDL_TRIGGER();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int nw = (gridDim.x * blockDim.x) >> 5;
-  float gw = 0.f, gb = 0.f;
   float* stage = sStage + w * kStage;
-  for (int i0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i0 < n; i0 += 8 * nw) {
+  int i0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  Rows8 rows = {0, 0, -1};
+  if (dM) rows = rows8(g, i0, nw, n, lane);
+  FVM_PDL_WAIT();
+  float gw = 0.f, gb = 0.f;
+  for (; i0 < n; i0 += 8 * nw) {
     float dh[8], h0[8], uq[8];
-    Rows8 rows = {0, 0, -1};
-    if (dM) {
-      rows = rows8(g, i0, nw, n, lane);
-      gather8_issue(dM, rows, stage, lane);
-    }
+    if (dM) gather8_issue(dM, rows, stage, lane);
 #pragma unroll
     for (int q = 0; q < 8; q++) {
       const int i = i0 + q * nw;
@@ -810,7 +810,11 @@ __global__ void __launch_bounds__(kBlock) k_encode_bwd(int n, GraphArgs g, const
       h0[q] = i < n ? H0[(size_t)i * 32 + lane] : 0.f;
       uq[q] = i < n ? u[i] : 0.f;
     }
-    if (dM) gather8_sum(g, g.wb, dM, rows, stage, lane, dh);
+    if (dM) {
+      const Rows8 next = rows8(g, i0 + 8 * nw, nw, n, lane);
+      gather8_sum(g, g.wb, dM, rows, stage, lane, dh);
+      rows = next;
+    }
 #pragma unroll
     for (int q = 0; q < 8; q++) {
       if (i0 + q * nw >= n) break;
@@ -837,11 +841,12 @@ __global__ void __launch_bounds__(kBlock) k_grad_reduce(int layerBlocks, const f
   const bool layer = blockIdx.x * 32 >= kLayer0 && blockIdx.x * 32 + 32 <= kDecW;
   const int nb = layer ? layerBlocks : kGradBlocks;
   if (p < kParams) {
+    float v[kGradBlocks / kWarps];  // (all in flight before the first is stored)
 #pragma unroll
-    for (int k = 0; k < kGradBlocks / kWarps; k++) {
-      const int b = w + k * kWarps;
-      if (b < nb) part[b][lane] = gp[(size_t)b * kParams + p];
-    }
+    for (int k = 0; k < kGradBlocks / kWarps; k++)
+      v[k] = w + k * kWarps < nb ? gp[(size_t)(w + k * kWarps) * kParams + p] : 0.f;
+#pragma unroll
+    for (int k = 0; k < kGradBlocks / kWarps; k++) part[w + k * kWarps][lane] = v[k];
   }
   __syncthreads();
   if (w || p >= kParams) return;
