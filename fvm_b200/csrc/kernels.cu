@@ -1445,54 +1445,98 @@ __global__ void k_face_coefficients(FaceGeom g, const double* __restrict__ k, do
       make_double4(kf * (A[0] - ds[0] * dm), kf * (A[1] - ds[1] * dm), kf * (A[2] - ds[2] * dm), 0.0);
 }
 
+// The linearization's kernels read the mesh (and, for the faces, the matrix's
+// coefficients) ahead of the wait: a cell's first four neighbours and weights,
+// a face's cells and coefficients. x, grad and flux are written by the chain.
+// Volumes travel in the gradient's record, and a cell knows its side of a face
+// without reading the face's cells. (1.5M tets: gradient 50.2 -> 49.1 us, face
+// flux 49.3 -> 41.7, right-hand side 39.0 -> 33.9.)
 __global__ void k_gradient(int nCells, const int* __restrict__ row, const int* __restrict__ col,
-                           const double* __restrict__ w, const double* __restrict__ x, double* grad) {
-  FVM_PDL();
+                           const double* __restrict__ w, const double* __restrict__ vol, const double* x,
+                           double* grad) {
+  FVM_PDL_TRIGGER();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nCells) return;
+  const bool live = i < nCells;
+  const int k0 = live ? row[i] : 0, k1 = live ? row[i + 1] : 0;
+  const double v = live ? vol[i] : 0.0;
+  int c[4];
+  double wk[12];
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    c[q] = k0 + q < k1 ? col[k0 + q] : -1;
+#pragma unroll
+    for (int d = 0; d < 3; d++) wk[3 * q + d] = c[q] >= 0 ? w[3 * (k0 + q) + d] : 0.0;
+  }
+  FVM_PDL_WAIT();
+  if (!live) return;
   double g0 = 0.0, g1 = 0.0, g2 = 0.0;
   const double xi = x[i];
-  for (int k = row[i]; k < row[i + 1]; k++) {
+  double xc[4];
+#pragma unroll
+  for (int q = 0; q < 4; q++) xc[q] = c[q] >= 0 ? x[c[q]] : 0.0;
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    if (c[q] < 0) continue;
+    const double dx = xc[q] - xi;
+    g0 += wk[3 * q] * dx;
+    g1 += wk[3 * q + 1] * dx;
+    g2 += wk[3 * q + 2] * dx;
+  }
+  for (int k = k0 + 4; k < k1; k++) {
     const double dx = x[col[k]] - xi;
     g0 += w[3 * k] * dx;
     g1 += w[3 * k + 1] * dx;
     g2 += w[3 * k + 2] * dx;
   }
-  // one 32-byte record per cell (the fourth entry pads)
-  reinterpret_cast<double4*>(grad)[i] = make_double4(g0, g1, g2, 0.0);
+  // one 32-byte record per cell, its volume the fourth entry
+  reinterpret_cast<double4*>(grad)[i] = make_double4(g0, g1, g2, v);
 }
 
 __global__ void k_ghost_gradient(int nB, const int* __restrict__ bFaces, const int* __restrict__ fc,
-                                 double* grad) {
-  FVM_PDL();
+                                 const double* __restrict__ vol, double* grad) {
+  FVM_PDL_TRIGGER();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nB) return;
-  const int f = bFaces[t];
+  const int f = t < nB ? bFaces[t] : 0;
   const int c0 = fc[2 * f], c1 = fc[2 * f + 1];
+  const double v = vol[c1];
+  FVM_PDL_WAIT();
+  if (t >= nB) return;
   double4* g4 = reinterpret_cast<double4*>(grad);
-  g4[c1] = g4[c0];
+  const double4 g = g4[c0];
+  g4[c1] = make_double4(g.x, g.y, g.z, v);
 }
 
-__global__ void k_face_flux(FaceGeom g, const double* __restrict__ coeff,
-                            const double* __restrict__ sec, const double* __restrict__ grad,
-                            const double* __restrict__ x, double* flux) {
-  FVM_PDL();
+__global__ void k_face_flux(FaceGeom g, const double* __restrict__ coeff, const double* __restrict__ sec,
+                            const double* grad, const double* x, double* flux) {
+  FVM_PDL_TRIGGER();
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= g.nFaces) return;
-  // faceCells as one 8-byte load, the two gradients and the secondary
-  // coefficient as 32-byte records (vector loads); same arithmetic order
-  const int2 cc = reinterpret_cast<const int2*>(g.faceCells)[f];
+  const bool live = f < g.nFaces;
+  // faceCells as one 8-byte load, the two gradients (with the volumes) and the
+  // secondary coefficient as 32-byte records; same arithmetic order
+  const int2 cc = live ? reinterpret_cast<const int2*>(g.faceCells)[f] : make_int2(0, 0);
+  const double4 sc = live ? reinterpret_cast<const double4*>(sec)[f] : make_double4(0.0, 0.0, 0.0, 0.0);
+  const double cf = live ? coeff[f] : 0.0;
+  FVM_PDL_WAIT();
+  if (!live) return;
   const int c0 = cc.x, c1 = cc.y;
-  const double vol0 = g.cellVolume[c0], vol1 = g.cellVolume[c1];
   const double4 ga = reinterpret_cast<const double4*>(grad)[c0];
   const double4 gb = reinterpret_cast<const double4*>(grad)[c1];
-  const double4 sc = reinterpret_cast<const double4*>(sec)[f];
-  const double vs = vol0 + vol1;
+  const double x0 = x[c0], x1 = x[c1];
+  const double vs = ga.w + gb.w;
   double s = 0.0;
-  s += ((ga.x * vol0 + gb.x * vol1) / vs) * sc.x;
-  s += ((ga.y * vol0 + gb.y * vol1) / vs) * sc.y;
-  s += ((ga.z * vol0 + gb.z * vol1) / vs) * sc.z;
-  flux[f] = coeff[f] * (x[c1] - x[c0]) + s;
+  s += ((ga.x * ga.w + gb.x * gb.w) / vs) * sc.x;
+  s += ((ga.y * ga.w + gb.y * gb.w) / vs) * sc.y;
+  s += ((ga.z * ga.w + gb.z * gb.w) / vs) * sc.z;
+  flux[f] = cf * (x1 - x0) + s;
+}
+
+// side[k] = 2 f + (cell i is the second of face f), for the k-th entry of the
+// cells' face lists
+__global__ void k_face_sides(int nCells, const int* __restrict__ row, const int* __restrict__ col,
+                             const int* __restrict__ fc, int* side) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= nCells) return;
+  for (int k = row[i]; k < row[i + 1]; k++) side[k] = 2 * col[k] + (fc[2 * col[k]] == i ? 0 : 1);
 }
 
 // Ghost row of a flux-type boundary face as GenericBCS leaves it
@@ -1532,24 +1576,39 @@ __device__ __forceinline__ void flux_bc(int kind, double q, const double* p, dou
   }
 }
 
-__global__ void k_assemble_rhs(int nCells, CellFaceView cf, const int* __restrict__ fc,
-                               const double* __restrict__ flux, const double* __restrict__ coeff,
-                               const double* __restrict__ am, const double* __restrict__ vol,
-                               const double* __restrict__ source, const double* __restrict__ rhoVdt,
-                               const double* __restrict__ xN1, BoundaryData bd,
-                               const int* __restrict__ bIndexOfFace, double* x,
-                               const int* __restrict__ perm, double* b) {
-  FVM_PDL();
+__global__ void k_assemble_rhs(int nCells, CellFaceView cf, const int* __restrict__ fc, const double* flux,
+                               const double* __restrict__ coeff, const double* __restrict__ am,
+                               const double* __restrict__ vol, const double* __restrict__ source,
+                               const double* __restrict__ rhoVdt, const double* xN1, BoundaryData bd,
+                               const int* __restrict__ bIndexOfFace, double* x, const int* __restrict__ perm,
+                               double* b) {
+  FVM_PDL_TRIGGER();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nCells) return;
+  const bool live = i < nCells;
+  const int k0 = live ? cf.row[i] : 0, k1 = live ? cf.row[i + 1] : 0;
+  int side[6];
+#pragma unroll
+  for (int q = 0; q < 6; q++) side[q] = k0 + q < k1 ? cf.side[k0 + q] : -1;
+  FVM_PDL_WAIT();
+  if (!live) return;
   // DiffusionDiscretization: r0 += flux, r1 -= flux, faces ascending
   double r = 0.0;
-  for (int k = cf.row[i]; k < cf.row[i + 1]; k++) {
-    const int f = cf.col[k];
-    if (fc[2 * f] == i)
-      r += flux[f];
+  double fl[6];
+#pragma unroll
+  for (int q = 0; q < 6; q++) fl[q] = side[q] >= 0 ? flux[side[q] >> 1] : 0.0;
+#pragma unroll
+  for (int q = 0; q < 6; q++) {
+    if (side[q] < 0) continue;
+    if (side[q] & 1)
+      r -= fl[q];
     else
-      r -= flux[f];
+      r += fl[q];
+  }
+  for (int k = k0 + 6; k < k1; k++) {
+    if (cf.side[k] & 1)
+      r -= flux[cf.side[k] >> 1];
+    else
+      r += flux[cf.side[k] >> 1];
   }
   // SourceDiscretization
   r += vol[i] * source[i];
@@ -2322,12 +2381,16 @@ void face_coefficients(const FaceGeom& g, const double* k, double* coeff, double
                        cudaStream_t st) {
   k_face_coefficients<<<ceil_div(g.nFaces, kBlock), kBlock, 0, st>>>(g, k, coeff, secCoeff);
 }
-void gradient(int nCells, const int* ccRow, const int* ccCol, const double* w, const double* x,
+void gradient(int nCells, const int* ccRow, const int* ccCol, const double* w, const double* vol, const double* x,
               double* grad, cudaStream_t st) {
-  pdl_launch(k_gradient, ceil_div(nCells, kBlock), kBlock, st, nCells, ccRow, ccCol, w, x, grad);
+  pdl_launch(k_gradient, ceil_div(nCells, kBlock), kBlock, st, nCells, ccRow, ccCol, w, vol, x, grad);
 }
-void ghost_gradient(int nB, const int* bFaces, const int* faceCells, double* grad, cudaStream_t st) {
-  if (nB > 0) pdl_launch(k_ghost_gradient, ceil_div(nB, kBlock), kBlock, st, nB, bFaces, faceCells, grad);
+void ghost_gradient(int nB, const int* bFaces, const int* faceCells, const double* vol, double* grad,
+                    cudaStream_t st) {
+  if (nB > 0) pdl_launch(k_ghost_gradient, ceil_div(nB, kBlock), kBlock, st, nB, bFaces, faceCells, vol, grad);
+}
+void face_sides(int nCells, const int* cfRow, const int* cfCol, const int* faceCells, int* side, cudaStream_t st) {
+  k_face_sides<<<ceil_div(nCells, kBlock), kBlock, 0, st>>>(nCells, cfRow, cfCol, faceCells, side);
 }
 void face_flux(const FaceGeom& g, const double* coeff, const double* secCoeff, const double* grad,
                const double* x, double* flux, cudaStream_t st) {

@@ -222,10 +222,11 @@ struct FaceGeom {
 void face_coefficients(const FaceGeom& g, const double* k, double* coeff, double* secCoeff,
                        cudaStream_t st);
 // least-squares gradient of x on self rows, then boundary ghosts copy c0;
-// grad holds one 32-byte record per cell (x, y, z, pad), 32-byte aligned
-void gradient(int nCells, const int* ccRow, const int* ccCol, const double* w, const double* x,
+// grad holds one 32-byte record per cell (x, y, z, the cell's volume), 32-byte
+// aligned
+void gradient(int nCells, const int* ccRow, const int* ccCol, const double* w, const double* vol, const double* x,
               double* grad, cudaStream_t st);
-void ghost_gradient(int nBFaces, const int* bFaces, const int* faceCells, double* grad,
+void ghost_gradient(int nBFaces, const int* bFaces, const int* faceCells, const double* vol, double* grad,
                     cudaStream_t st);
 // flux_f = c_f (x1 - x0) + gradF . sec_f
 void face_flux(const FaceGeom& g, const double* coeff, const double* secCoeff,
@@ -252,7 +253,9 @@ struct CellFaceView {
   const int* bRow;   // per self cell: range into the boundary-face lists
   const int* bCol;   // boundary faces, ascending face index (BC application order)
   const int* bColG;  // the same faces by ascending ghost index (elimination order)
+  const int* side;   // per entry of col: 2 face + (the cell is the face's second), by face_sides
 };
+void face_sides(int nCells, const int* cfRow, const int* cfCol, const int* faceCells, int* side, cudaStream_t st);
 // Assembles the delta-form right-hand side of every self cell exactly as
 // DiffusionDiscretization + Source + TimeDerivative + GenericBCS +
 // eliminateBoundaryEquations produce it, writing b[perm[i]]; also records

@@ -810,6 +810,9 @@ void ThermalModel::ensureDevice() {
   dVol_ = arena_.upload(m.cellVolume);
   dCfRow_ = arena_.upload(cfRow);
   dCfCol_ = arena_.upload(cfCol);
+  dCfSide_ = (int*)arena_.alloc(sizeof(int) * std::max<size_t>(cfCol.size(), 1));
+  CUDA_OK(cudaStreamSynchronize(nullptr));  // (a copy from pageable memory may still be on its way)
+  dev::face_sides(n, dCfRow_, dCfCol_, dFaceCells_, dCfSide_, stream_);
   dBRow_ = arena_.upload(bRow);
   dBCol_ = arena_.upload(bCol);
   dBColG_ = arena_.upload(bColG);
@@ -951,7 +954,7 @@ void ThermalModel::ensureMatrix() {
     dev::transient_coeff(n, dRc_, dVol_, opt_.timeStep, dRhoVdt_, stream_);
     rhoVdt = dRhoVdt_;
   }
-  dev::CellFaceView cf{dCfRow_, dCfCol_, dBRow_, dBCol_, dBColG_};
+  dev::CellFaceView cf{dCfRow_, dCfCol_, dBRow_, dBCol_, dBColG_, dCfSide_};
   const dev::BoundaryData bd = boundaryData();
   dev::assemble_matrix(n, cf, dFaceCells_, dCoeff_, dAreaMag_, rhoVdt, bd, dBIndexOfFace_, dT_, dDiagOrig_, stream_);
   if (opt_.linear.setupOnDevice && !opt_.linear.finestOnly()) {
@@ -1055,11 +1058,11 @@ void ThermalModel::ensureMatrix() {
 void ThermalModel::linearize() {
   HostMesh& m = *mesh_;
   const int n = m.nCells, F = m.nFaces;
-  dev::gradient(n, dCcRow_, dCcCol_, dGradW_, dT_, dGrad_, stream_);
-  dev::ghost_gradient((int)boundaryFaces_.size(), dBFace_, dFaceCells_, dGrad_, stream_);
+  dev::gradient(n, dCcRow_, dCcCol_, dGradW_, dVol_, dT_, dGrad_, stream_);
+  dev::ghost_gradient((int)boundaryFaces_.size(), dBFace_, dFaceCells_, dVol_, dGrad_, stream_);
   dev::FaceGeom g{F, n, dFaceCells_, dArea_, dAreaMag_, dCentroid_, dVol_};
   dev::face_flux(g, dCoeff_, dSec_, dGrad_, dT_, dFlux_, stream_);
-  dev::CellFaceView cf{dCfRow_, dCfCol_, dBRow_, dBCol_, dBColG_};
+  dev::CellFaceView cf{dCfRow_, dCfCol_, dBRow_, dBCol_, dBColG_, dCfSide_};
   const dev::BoundaryData bd = boundaryData();
   dev::assemble_rhs(n, cf, dFaceCells_, dFlux_, dCoeff_, dAreaMag_, dVol_, dSrc_,
                     opt_.transient ? dRhoVdt_ : nullptr, dTN1_, bd, dBIndexOfFace_, dT_,

@@ -229,7 +229,7 @@ class ThermalModel {
   bool deviceReady_ = false;
   DeviceArena arena_;
   int *dFaceCells_ = nullptr, *dCcRow_ = nullptr, *dCcCol_ = nullptr;
-  int *dCfRow_ = nullptr, *dCfCol_ = nullptr, *dBRow_ = nullptr, *dBCol_ = nullptr, *dBColG_ = nullptr;
+  int *dCfRow_ = nullptr, *dCfCol_ = nullptr, *dCfSide_ = nullptr, *dBRow_ = nullptr, *dBCol_ = nullptr, *dBColG_ = nullptr;
   int *dBFace_ = nullptr, *dBKind_ = nullptr, *dBIndexOfFace_ = nullptr, *dPerm_ = nullptr;
   double* hPinned_ = nullptr;  // pinned host staging of the face coefficients and diagonal
   size_t hPinnedBytes_ = 0;

@@ -272,3 +272,36 @@ def test_galerkin_refuses_an_aggregate_beyond_its_capacity():
                          fields={"conductivity": k, "source": s})
     with pytest.raises(Exception, match="capacity"):
         tm.advance(1)
+
+
+@pytest.mark.parametrize("sides", [5, 7, 40])
+def test_linearization_of_cells_with_many_faces(sides):
+    """The linearization's kernels fetch a cell's first four neighbours and six
+    faces ahead of the rest. Three outer iterations on a skewed disk (the
+    non-orthogonal correction acts) against the C restatement, each linear
+    solve to 1e-12: the fields agree to the solves' tolerance times the
+    system's condition, below 1e-9."""
+    from oracle import oracle_c
+
+    mesh, k, s = _disk(sides, 4, seed=sides)
+    rng = np.random.default_rng(2)
+    nodes = np.array(mesh["nodes"]).reshape(-1, 3)
+    nodes[sides: 4 * sides, :2] += 0.1 * min(1.0, 6.0 / sides) * rng.uniform(-1, 1, (3 * sides, 2))
+    mesh["nodes"] = nodes.reshape(np.shape(mesh["nodes"]))
+    amg = fvmbaseExt.AMG()
+    amg.relativeTolerance = 1e-12
+    amg.nMaxIterations = 500
+    tm, tf, m = gpu_model(mesh, {1: ("T", 300.0), 2: ("T", 400.0)}, solver=amg,
+                          fields={"conductivity": k, "source": s}, opts={"relativeTolerance": 1e-30})
+    tm.advance(3)
+    r = oracle_c.OracleThermal(mesh)
+    r.set_options(n_pre=1, n_post=1, lin_rel=1e-12, max_iter=500, rel=1e-30)
+    for gid, t in ((1, 300.0), (2, 400.0)):
+        r.set_bc(gid, 0, [t])
+    r.init()
+    r.set_field(1, meshgen.extend_to_ghosts(mesh, k))
+    r.set_field(2, meshgen.extend_to_ghosts(mesh, s))
+    norms, _ = r.advance(3)
+    n = mesh["nCells"]
+    assert norms[1] > 1e-6 * norms[0]  # the correction is not nothing
+    assert rel_l2(tf.temperature[m.getCells()][:n], r.get_field(0)[:n]) <= 1e-9
