@@ -97,7 +97,7 @@ __device__ __forceinline__ T row_chunk_g(const SellView<T>& a, int e0, int cnt, 
   return sum;
 }
 template <class T, int K>
-__device__ __forceinline__ T row_chunk(const SellView<T>& a, int e0, int cnt, const T* __restrict__ x, T sum) {
+__device__ __forceinline__ T row_chunk(const SellView<T>& a, int e0, int cnt, const T* x, T sum) {
   return row_chunk_g<T, K>(a, e0, cnt, XDirect<T>{x}, sum);
 }
 
@@ -134,9 +134,10 @@ __device__ __forceinline__ T row_sum(const SellView<T>& a, const int4 m, int lan
 // slice metadata and transfer maps, complete before the solve's first launch
 // (the setup ends with a synchronisation) -- is loaded between the two
 // instructions, so a pass whose predecessor is still running has its row in
-// registers when the wait ends and only gathers then. (The vectors such a
-// kernel reads after the wait are not declared __restrict__: as read-only
-// parameters the compiler would be free to load them ahead of it.)
+// registers when the wait ends and only gathers then. No vector that an
+// earlier kernel of a chain writes is declared __restrict__, in whatever
+// kernel of the chain it is read: as a read-only parameter the compiler would
+// be free to load it ahead of the wait.
 
 // A slice's {first row, rows, offset, width}: loaded (SELL-32) or computed
 // (ELL-32: aligned 32-row groups of one width)
@@ -162,7 +163,7 @@ __global__ void k_zero(int n, T* x) {
 
 // ---------------------------------------------------------------------------
 template <class T>
-__global__ void k_gs_sequential(SellView<T> a, T* x, const T* __restrict__ b, int reverse) {
+__global__ void k_gs_sequential(SellView<T> a, T* x, const T* b, int reverse) {
   FVM_PDL();
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   for (int t = 0; t < a.n; t++) {
@@ -174,8 +175,8 @@ __global__ void k_gs_sequential(SellView<T> a, T* x, const T* __restrict__ b, in
 }
 
 template <class T>
-__global__ void __launch_bounds__(kBlock, 4) k_jacobi(SellView<T> a, int nSlices, const T* __restrict__ xold, T* xnew,
-                         const T* __restrict__ b) {
+__global__ void __launch_bounds__(kBlock, 4) k_jacobi(SellView<T> a, int nSlices, const T* xold, T* xnew,
+                                                      const T* b) {
   FVM_PDL();
   const int lane = threadIdx.x & 31;
   for (int s = blockIdx.x * kSlicesPerBlock + (threadIdx.x >> 5); s < nSlices; s += gridDim.x * kSlicesPerBlock) {
@@ -318,8 +319,8 @@ __global__ void __launch_bounds__(kBlock) k_jacobi_damped(SellView<T> a, int nSl
 // written, not read) and xnew = x + dv. dv is indexed by row only, so it
 // is updated in place; x and xnew are distinct.
 template <class T, bool First>
-__global__ void __launch_bounds__(kBlock, 4) k_cheb(SellView<T> a, int nSlices, const T* __restrict__ x, T* xnew,
-                                                    T* dv, const T* __restrict__ b, T c1, T c2) {
+__global__ void __launch_bounds__(kBlock, 4) k_cheb(SellView<T> a, int nSlices, const T* x, T* xnew,
+                                                    T* dv, const T* b, T c1, T c2) {
   FVM_PDL();
   const int lane = threadIdx.x & 31;
   for (int s = blockIdx.x * kSlicesPerBlock + (threadIdx.x >> 5); s < nSlices; s += gridDim.x * kSlicesPerBlock) {
@@ -353,8 +354,8 @@ __global__ void __launch_bounds__(kBlock) k_gershgorin(SellView<double> a, int n
 }
 
 template <class T>
-__global__ void __launch_bounds__(kBlock, 4) k_residual(SellView<T> a, int nSlices, const T* __restrict__ x,
-                           const T* __restrict__ b, T* r, double* partials) {
+__global__ void __launch_bounds__(kBlock, 4) k_residual(SellView<T> a, int nSlices, const T* x, const T* b, T* r,
+                                                        double* partials) {
   FVM_PDL();
   const int lane = threadIdx.x & 31;
   double l1 = 0.0;
@@ -463,7 +464,7 @@ __global__ void __launch_bounds__(1024, 1) k_csr_residual_tiles(int n, const int
   partials[blockIdx.x] = l1;
 }
 
-__global__ void __launch_bounds__(kBlock, 4) k_spmv(SellView<double> a, int nSlices, const double* __restrict__ x, double* y) {
+__global__ void __launch_bounds__(kBlock, 4) k_spmv(SellView<double> a, int nSlices, const double* x, double* y) {
   FVM_PDL();
   const int lane = threadIdx.x & 31;
   for (int s = blockIdx.x * kSlicesPerBlock + (threadIdx.x >> 5); s < nSlices; s += gridDim.x * kSlicesPerBlock) {
@@ -494,7 +495,7 @@ __device__ __forceinline__ T ell_row_g(const SellView<T>& a, int i, const X& xg,
   }
 }
 template <class T, int W>
-__device__ __forceinline__ T ell_row(const SellView<T>& a, int i, const T* __restrict__ x, T sum) {
+__device__ __forceinline__ T ell_row(const SellView<T>& a, int i, const T* x, T sum) {
   return ell_row_g<T, W>(a, i, XDirect<T>{x}, sum);
 }
 
@@ -598,8 +599,7 @@ __global__ void __launch_bounds__(kBlock) k_gs_color_ell2(SellView<T> a, int r0,
 }
 
 template <class T, int W>
-__global__ void __launch_bounds__(kBlock, 8) k_jacobi_ell(SellView<T> a, const T* __restrict__ xold, T* xnew,
-                                                          const T* __restrict__ b) {
+__global__ void __launch_bounds__(kBlock, 8) k_jacobi_ell(SellView<T> a, const T* xold, T* xnew, const T* b) {
   FVM_PDL();
   const int i = blockIdx.x * kBlock + threadIdx.x;
   if (i >= a.n) return;
@@ -608,8 +608,8 @@ __global__ void __launch_bounds__(kBlock, 8) k_jacobi_ell(SellView<T> a, const T
 }
 
 template <class T, int W>
-__global__ void __launch_bounds__(kBlock, 8) k_jacobi_damped_ell(SellView<T> a, const T* __restrict__ xold, T* xnew,
-                                                                 const T* __restrict__ b, T w) {
+__global__ void __launch_bounds__(kBlock, 8) k_jacobi_damped_ell(SellView<T> a, const T* xold, T* xnew, const T* b,
+                                                                 T w) {
   FVM_PDL();
   const int i = blockIdx.x * kBlock + threadIdx.x;
   if (i >= a.n) return;
@@ -619,8 +619,8 @@ __global__ void __launch_bounds__(kBlock, 8) k_jacobi_damped_ell(SellView<T> a, 
 }
 
 template <class T, int W, bool First>
-__global__ void __launch_bounds__(kBlock, 8) k_cheb_ell(SellView<T> a, const T* __restrict__ x, T* xnew, T* dv,
-                                                        const T* __restrict__ b, T c1, T c2) {
+__global__ void __launch_bounds__(kBlock, 8) k_cheb_ell(SellView<T> a, const T* x, T* xnew, T* dv,
+                                                        const T* b, T c1, T c2) {
   FVM_PDL();
   const int i = blockIdx.x * kBlock + threadIdx.x;
   if (i >= a.n) return;
@@ -659,7 +659,7 @@ __global__ void __launch_bounds__(kBlock, ell_blocks<T, W>()) k_residual_ell(Sel
 }
 
 template <int W>
-__global__ void __launch_bounds__(kBlock, 8) k_spmv_ell(SellView<double> a, const double* __restrict__ x, double* y) {
+__global__ void __launch_bounds__(kBlock, 8) k_spmv_ell(SellView<double> a, const double* x, double* y) {
   FVM_PDL();
   const int i = blockIdx.x * kBlock + threadIdx.x;
   if (i >= a.n) return;
@@ -690,7 +690,7 @@ __device__ __forceinline__ void block_sum2(double& a, double& b) {
 
 // y = A x over an ELL-32 level, with one partial of x.y per block
 template <int W>
-__global__ void __launch_bounds__(kBlock, 8) k_spmv_dot_ell(SellView<double> a, const double* __restrict__ x, double* y,
+__global__ void __launch_bounds__(kBlock, 8) k_spmv_dot_ell(SellView<double> a, const double* x, double* y,
                                                             double* partials) {
   FVM_PDL();
   const int i = blockIdx.x * kBlock + threadIdx.x;
@@ -708,8 +708,10 @@ __global__ void __launch_bounds__(kBlock, 8) k_spmv_dot_ell(SellView<double> a, 
 // q = A p with p = p_old * beta + z formed on the fly (p itself is written
 // by k_cg_update_pby, after every row has read its neighbours' p_old), one
 // partial of p.q per block. z is the cycle's own result (FP32 for the FP32
-// cycle: the conversion is exact). p_old and the matrix, which the kernels
-// just before do not write, are loaded ahead of the wait.
+// cycle: the conversion is exact). p_old and the matrix are loaded ahead of
+// the wait: the update that wrote p_old is complete, because the loop's test
+// (k_loop_init, k_loop_check) or a host wait lies between and neither is a
+// dependent launch.
 template <class S, int W>
 __global__ void __launch_bounds__(kBlock, W <= 6 ? 6 : 5) k_spmv_dot_pby_ell(SellView<double> a, const S* z,
                                                                 const double* p, const double* beta,
@@ -737,8 +739,8 @@ __global__ void __launch_bounds__(kBlock, W <= 6 ? 6 : 5) k_spmv_dot_pby_ell(Sel
 }
 
 template <class S>
-__global__ void __launch_bounds__(kBlock, 4) k_spmv_dot_pby(SellView<double> a, int nSlices, const S* __restrict__ z,
-                                                            const double* __restrict__ p, const double* beta,
+__global__ void __launch_bounds__(kBlock, 4) k_spmv_dot_pby(SellView<double> a, int nSlices, const S* z,
+                                                            const double* p, const double* beta,
                                                             double* y, double* partials) {
   FVM_PDL();
   const int lane = threadIdx.x & 31;
@@ -758,7 +760,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_spmv_dot_pby(SellView<double> a, 
 }
 
 // the same over a SELL-32 level (grid-stride over slices)
-__global__ void __launch_bounds__(kBlock, 4) k_spmv_dot(SellView<double> a, int nSlices, const double* __restrict__ x,
+__global__ void __launch_bounds__(kBlock, 4) k_spmv_dot(SellView<double> a, int nSlices, const double* x,
                                                         double* y, double* partials) {
   FVM_PDL();
   const int lane = threadIdx.x & 31;
@@ -779,7 +781,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_spmv_dot(SellView<double> a, int 
 // block partials of (r, z), z the cycle's result, beside those of (r, z_old)
 // that the update left (pairs: z_old, z)
 template <class S>
-__global__ void k_cg_dot_z(int n, const S* __restrict__ z, const double* __restrict__ r, double* partials) {
+__global__ void k_cg_dot_z(int n, const S* z, const double* r, double* partials) {
   FVM_PDL();
   double b = 0.0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) b += r[i] * (double)z[i];
@@ -788,8 +790,7 @@ __global__ void k_cg_dot_z(int n, const S* __restrict__ z, const double* __restr
 }
 
 // rho_prev <- rho, rho <- (r, z_new), beta (flexible: (rho - (r, z_old)) / rho_prev)
-__global__ void k_cg_beta(int np, const double* __restrict__ p, double* rho, double* rhoPrev, double* beta,
-                          int flexible) {
+__global__ void k_cg_beta(int np, const double* p, double* rho, double* rhoPrev, double* beta, int flexible) {
   FVM_PDL();
   double a = 0.0, b = 0.0;
   for (int i = threadIdx.x; i < np; i += blockDim.x) {
@@ -806,7 +807,7 @@ __global__ void k_cg_beta(int np, const double* __restrict__ p, double* rho, dou
 }
 
 // alpha = rho / sum of the partials (p.Ap)
-__global__ void k_cg_alpha(int np, const double* __restrict__ p, const double* rho, double* alpha) {
+__global__ void k_cg_alpha(int np, const double* p, const double* rho, double* alpha) {
   FVM_PDL();
   // four loads in flight per thread, added in order
   double s = 0.0;
@@ -828,9 +829,8 @@ __global__ void k_cg_alpha(int np, const double* __restrict__ p, const double* r
 // flexible beta, of (r, z) with the new r and this iteration's z (pairs,
 // first entry)
 template <class S>
-__global__ void k_cg_update(int n, const double* alpha, const double* __restrict__ p, const double* __restrict__ q,
-                            double* x, double* r, const S* __restrict__ z, double* partials, double* zPartials,
-                            float* rF) {
+__global__ void k_cg_update(int n, const double* alpha, const double* p, const double* q, double* x, double* r, const S* z,
+                            double* partials, double* zPartials, float* rF) {
   FVM_PDL();
   const double am = -1.0 * alpha[0];
   double l1 = 0.0, rz = 0.0;
@@ -851,9 +851,8 @@ __global__ void k_cg_update(int n, const double* alpha, const double* __restrict
 
 // the same with p = p_old * beta + z, written here
 template <class S>
-__global__ void k_cg_update_pby(int n, const double* alpha, const S* __restrict__ z, const double* beta, double* p,
-                                const double* __restrict__ q, double* x, double* r, double* partials,
-                                double* zPartials, float* rF) {
+__global__ void k_cg_update_pby(int n, const double* alpha, const S* z, const double* beta, double* p, const double* q,
+                                double* x, double* r, double* partials, double* zPartials, float* rF) {
   FVM_PDL();
   const double am = -1.0 * alpha[0];
   const double b = beta[0];
@@ -1064,7 +1063,7 @@ __global__ void __launch_bounds__(kBlock) k_restrict(int nc, const int* __restri
 template <class T>
 __global__ void __launch_bounds__(kBlock, 4) k_residual_restrict(SellView<T> a, const int* __restrict__ rowSlice, int nc,
                                     const int* __restrict__ c2fRow, const int* __restrict__ c2fCol,
-                                    const T* __restrict__ x, const T* __restrict__ b, T* bc, T* xc) {
+                                    const T* x, const T* b, T* bc, T* xc) {
   FVM_PDL();
   const int I = blockIdx.x * blockDim.x + threadIdx.x;
   if (I >= nc) return;
@@ -1094,7 +1093,7 @@ __global__ void k_prolong(int n, const int* __restrict__ ci, const T* xc, T* x, 
 }
 
 template <class T>
-__global__ void k_dense_solve(int n, const double* __restrict__ ainv, const T* __restrict__ b, T* x) {
+__global__ void k_dense_solve(int n, const double* __restrict__ ainv, const T* b, T* x) {
   FVM_PDL();
   // one warp per row
   const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -1313,17 +1312,17 @@ __global__ void k_cast_d2f_big(size_t n, const double* __restrict__ a, float* b)
   if (i < n) b[i] = (float)a[i];
 }
 
-__global__ void k_convert_d2f(int n, const double* __restrict__ a, float* b) {
+__global__ void k_convert_d2f(int n, const double* a, float* b) {
   FVM_PDL();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) b[i] = (float)a[i];
 }
-__global__ void k_add_f2d(int n, const float* __restrict__ a, double* b) {
+__global__ void k_add_f2d(int n, const float* a, double* b) {
   FVM_PDL();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) b[i] = b[i] + (double)a[i];
 }
-__global__ void k_l1_partials(int n, const double* __restrict__ a, double* partials) {
+__global__ void k_l1_partials(int n, const double* a, double* partials) {
   FVM_PDL();
   double s = 0.0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) s += fabs(a[i]);
@@ -1333,8 +1332,8 @@ __global__ void k_l1_partials(int n, const double* __restrict__ a, double* parti
 // The start of a CG solve from x = 0: r = b + A x is b itself. r, its FP32
 // copy (the FP32 cycle's right-hand side; null: none), x = p = 0 and the
 // |r|_1 partials in k_l1_partials' layout, in one pass over b.
-__global__ void k_cg_start(int n, const double* __restrict__ b, double* __restrict__ r, float* __restrict__ rF,
-                           double* __restrict__ x, double* __restrict__ p, double* partials, double* zPartials) {
+__global__ void k_cg_start(int n, const double* b, double* r, float* rF, double* x, double* p, double* partials,
+                           double* zPartials) {
   FVM_PDL();
   double s = 0.0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -1351,15 +1350,14 @@ __global__ void k_cg_start(int n, const double* __restrict__ b, double* __restri
     zPartials[2 * blockIdx.x] = 0.0;  // (r, z_old) of the first beta
   }
 }
-__global__ void k_dot_partials(int n, const double* __restrict__ a, const double* __restrict__ b,
-                               double* partials) {
+__global__ void k_dot_partials(int n, const double* a, const double* b, double* partials) {
   FVM_PDL();
   double s = 0.0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) s += a[i] * b[i];
   s = block_sum(s);
   if (threadIdx.x == 0) partials[blockIdx.x] = s;
 }
-__global__ void k_sum_partials(int np, const double* __restrict__ p, double* out) {
+__global__ void k_sum_partials(int np, const double* p, double* out) {
   FVM_PDL();
   // four independent loads in flight per thread (ELL residuals leave one
   // partial per 256 rows: 31k partials for 8M rows); fixed order
@@ -1391,23 +1389,23 @@ __global__ void k_scalar_ratio_product(const double* a, const double* b, const d
   FVM_PDL();
   out[0] = (a[0] / b[0]) * (c[0] / d[0]);
 }
-__global__ void k_axpy_dev(int n, const double* s, double sign, const double* __restrict__ x, double* y) {
+__global__ void k_axpy_dev(int n, const double* s, double sign, const double* x, double* y) {
   FVM_PDL();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) y[i] = y[i] + (sign * s[0]) * x[i];
 }
-__global__ void k_xpby_dev(int n, const double* __restrict__ z, const double* beta, double* p) {
+__global__ void k_xpby_dev(int n, const double* z, const double* beta, double* p) {
   FVM_PDL();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) p[i] = p[i] * beta[0] + z[i];
 }
-__global__ void k_bicg_p(int n, const double* __restrict__ r, const double* __restrict__ v,
-                         const double* omega, const double* beta, double* p) {
+__global__ void k_bicg_p(int n, const double* r, const double* v, const double* omega, const double* beta,
+                         double* p) {
   FVM_PDL();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) p[i] = (p[i] - omega[0] * v[i]) * beta[0] + r[i];
 }
-__global__ void k_copy_d(int n, const double* __restrict__ a, double* b) {
+__global__ void k_copy_d(int n, const double* a, double* b) {
   FVM_PDL();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) b[i] = a[i];
@@ -1687,7 +1685,7 @@ __global__ void k_cast_d2f(int n, const double* __restrict__ a, float* b) {
   if (i < n) b[i] = (float)a[i];
 }
 
-__global__ void k_update_self(int nCells, const int* __restrict__ perm, const double* __restrict__ delta,
+__global__ void k_update_self(int nCells, const int* __restrict__ perm, const double* delta,
                               double* x) {
   FVM_PDL();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1699,7 +1697,7 @@ __global__ void k_update_self(int nCells, const int* __restrict__ perm, const do
 // Then the boundary heat flux: q += -(r_q + (L dx0 + R dx1)) / (-1)
 // (FluxJacobianMatrix::multiplyAndAdd, DiagonalMatrix::solveBoundary).
 __global__ void k_update_ghosts(BoundaryData bd, const int* __restrict__ perm,
-                                const double* __restrict__ delta, const int* __restrict__ fc,
+                                const double* delta, const int* __restrict__ fc,
                                 const double* __restrict__ coeff, double* x) {
   FVM_PDL();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;

@@ -52,7 +52,7 @@ __device__ __forceinline__ double block_sum(double v) {
 }
 
 // sum_i e_i^2 per block
-__global__ void k_sq_partials(int n, const double* __restrict__ e, double* partials) {
+__global__ void k_sq_partials(int n, const double* e, double* partials) {
   FVM_PDL();
   double s = 0.0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) s += e[i] * e[i];
@@ -459,7 +459,7 @@ __device__ void block_grad_store(const float* sv, int nv, float* gp, int off) {
 }
 
 __global__ void __launch_bounds__(kBlock) k_decode_bwd(int n, const float* P, const float* H3, const double* scale,
-                                                       const double* __restrict__ e, const double* e2, float* dH3,
+                                                       const double* e, const double* e2, float* dH3,
                                                        float* gp, double* lossPartials) {
   __shared__ float sv[kWarps * 33];
   FVM_PDL();

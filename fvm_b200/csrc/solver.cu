@@ -1345,6 +1345,9 @@ __global__ void k_loop_init(double* scal, int* loopInt, double* history, double 
 // sum_partials sums them) and the test on it. Half: the test BiCGStab makes
 // half way, on the absolute tolerance alone; the second half runs unless the
 // solve ended (condition hHalf).
+// Neither this nor k_loop_init may become a dependent launch: the CG update
+// before it has to be complete when the next iteration's k_spmv_dot_pby_ell
+// loads p ahead of its wait.
 template <bool Half>
 __global__ void __launch_bounds__(1024) k_loop_check(int np, const double* __restrict__ p, double* scal, int* loopInt,
                                                      double* history, double relTol, double absTol, int maxIt,
