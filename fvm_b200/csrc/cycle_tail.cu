@@ -26,9 +26,10 @@
 // The passes are a list of steps made on the host (AmgHierarchy::buildTail),
 // so V, W and F cycles and all smoothers go through the same kernel. The
 // file is built without contraction: bitwise the values of the separate
-// kernels.
+// kernels, over the whole range of the formats (divide).
 #include "cycle_tail.cuh"
 
+#include <cmath>
 #include <cstdint>
 
 namespace fvm {
@@ -86,16 +87,50 @@ __device__ __forceinline__ void pass_barrier() {
 // multiply-add gives exactly. a * rd is within two units in the last place,
 // the first step brings it within one, and from there the step with the
 // correctly rounded reciprocal rounds correctly (Markstein, IBM J. Res.
-// Dev. 34, 1990).
-__device__ __forceinline__ double divide(double a, double d, double rd) {
-  double q = a * rd;
-  q = __fma_rn(__fma_rn(-q, d, a), rd, q);
-  return __fma_rn(__fma_rn(-q, d, a), rd, q);
+// Dev. 34, 1990). That holds while rd and the quotient are normal numbers and
+// the remainder, a multiple of the product of both last places, is
+// representable: for d and a * rd within the bounds below (|a| is then within
+// 2^-811 and 2^813, the remainder a multiple of 2^-915; FP32 2^-93, 2^125
+// and 2^-139). Outside them, and for infinities and NaN, the division itself;
+// reciprocal() marks a d out of bounds with NaN, so that one test of a * rd
+// sees all of it. (Values of a heat problem's rows lie inside; zeros, which
+// a * rd has right with their sign, do not take the division either.)
+//
+// word: the part of a number that has its sign and exponent; the exponent's
+// upper two bits differ (01, 10) in the middle half of its range, which is
+// where a * rd has to lie: 2^-511 to 2^513, FP32 2^-63 to 2^65.
+__device__ __forceinline__ unsigned word(double v) { return (unsigned)__double2hiint(v); }
+__device__ __forceinline__ unsigned word(float v) { return __float_as_uint(v); }
+template <class T>
+__device__ __forceinline__ bool middle(T v) {
+  const unsigned w = word(v);
+  return ((w ^ (w << 1)) & 0x40000000u) != 0u;
 }
-__device__ __forceinline__ float divide(float a, float d, float rd) {
-  float q = a * rd;
-  q = __fmaf_rn(__fmaf_rn(-q, d, a), rd, q);
-  return __fmaf_rn(__fmaf_rn(-q, d, a), rd, q);
+__device__ __forceinline__ double reciprocal(double d) {
+  return fabs(d) >= 0x1p-300 && fabs(d) <= 0x1p300 ? 1.0 / d : double(NAN);
+}
+__device__ __forceinline__ float reciprocal(float d) {
+  return fabsf(d) >= 0x1p-30f && fabsf(d) <= 0x1p60f ? 1.0f / d : float(NAN);
+}
+__device__ __forceinline__ double fused(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float fused(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+// (The test runs beside the Newton steps: a cycle of 576 rows, all on one CTA,
+// 28.3 us without a test, 29.0 so, 29.6 with the steps behind the test; of
+// 65536 rows 117.0, 118.0 and 119.8.)
+__device__ __forceinline__ void hold(double& v) { asm volatile("" : "+d"(v)); }
+__device__ __forceinline__ void hold(float& v) { asm volatile("" : "+f"(v)); }
+template <class T>
+__device__ __noinline__ T divide_any(T a, T d) {
+  return a / d;
+}
+template <class T>
+__device__ __forceinline__ T divide(T a, T d, T rd) {
+  const T q0 = a * rd;
+  T q = fused(fused(-q0, d, a), rd, q0);
+  q = fused(fused(-q, d, a), rd, q);
+  hold(q);
+  if (!middle(q0)) q = a == T(0) && rd == rd ? q0 : divide_any(a, d);
+  return q;
 }
 
 // the barrier a step begins with (arrived at when the last one ended)
@@ -407,7 +442,7 @@ __global__ void __launch_bounds__(128) k_tail_pack(const __grid_constant__ TailA
     P.slot[q] = live ? i | colour << 20 : -1;
     const T d = live ? P.a.diag[i] : T(1);
     P.diag[q] = d;
-    P.rdiag[q] = T(1) / d;
+    P.rdiag[q] = reciprocal(d);
     const int self = (((h % L.per) * 32 + lane) << 4) | (h / L.per);
     for (int k = 0; k < L.width; k++) {
       const int e = (h * L.width + k) * 32 + lane;

@@ -57,7 +57,7 @@ struct TailLevel {
   const int* slot;       // row | colour << 20, -1: none
   const int* idx;        // (slice * width + k) * 32 + lane: column's place
   const T* val;
-  const T *diag, *rdiag;       // by slot: diagonal and its reciprocal
+  const T *diag, *rdiag;       // by slot: diagonal and its reciprocal (NaN: see divide)
   const int* ci;               // by slot: coarse row's place (-1: none)
   const int *c2fRow, *c2fIdx;  // by coarse row: places of its rows
   unsigned x, b, r;            // byte offsets in shared memory

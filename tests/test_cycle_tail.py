@@ -104,3 +104,53 @@ def test_smoothers(knobs, precision):
 @pytest.mark.parametrize("pre", [0, 1])
 def test_as_preconditioner(kind, pre):
     _both(_grid(100, 67), kind, nPreSweeps=pre)
+
+
+def _scaled(scales, precision, kind):
+    """Histories and solutions of both paths, matrix and right-hand side
+    scaled: neither the place nor the size of a rounding may differ. Row by
+    row the scale of the matrix varies by 2^20 in the last of them."""
+    row, col, diag, off, b = _grid(60, 41)
+    matrix, rhs, vary = scales
+    s = np.full(len(diag), matrix)
+    if vary:
+        # symmetric: couplings take the smaller scale of their two rows
+        s = matrix * 2.0 ** np.random.default_rng(5).integers(-10, 11, len(diag))
+    rows = np.repeat(np.arange(len(diag)), np.diff(row))
+    out = []
+    for launches in (False, True):
+        amg = fvmbaseExt.AMG()
+        amg.precision = precision
+        amg.nPreSweeps = 1
+        amg.smootherType = kind
+        amg.nMaxIterations = 3
+        amg.relativeTolerance = 1e-30
+        amg.absoluteTolerance = 0.0
+        if launches:
+            amg.planThreadsPerRow = 1
+        x, info = amg.solve_csr(row, col, diag * s, off * np.minimum(s[rows], s[col]), b * rhs)
+        out.append((x, info["history"], info["launches"]))
+    (x0, h0, l0), (x1, h1, l1) = out
+    assert np.all(np.isfinite(x1)) and len(h1) > 1 and l0 < l1
+    np.testing.assert_array_equal(h0, h1)
+    np.testing.assert_array_equal(x0, x1)
+    np.testing.assert_array_equal(np.signbit(x0), np.signbit(x1))
+
+
+# FP64: subnormal and nearly so (reciprocals that overflow), at both ends,
+# quotients near the ends of the format
+@pytest.mark.parametrize("kind", [0, 1])
+@pytest.mark.parametrize("scales", [(1.0, 1e-305, False), (1.0, 1e290, False), (1e-310, 1e-310, False),
+                                    (1e-305, 1e-290, False), (1e290, 1e290, False), (1e-150, 1e150, False),
+                                    (1e200, 1e-100, False), (2.0 ** -300, 1.0, True), (2.0 ** 300, 1.0, True)], ids=str)
+def test_scales_fp64(scales, kind):
+    _scaled(scales, fvmbaseExt.AMG.FP64, kind)
+
+
+@pytest.mark.parametrize("kind", [0, 1])
+@pytest.mark.parametrize("scales", [(1.0, 1e-33, False), (1.0, 1e-42, False), (1.0, 1e33, False),
+                                    (1e-42, 1e-42, False), (1e-38, 1e-33, False), (1e33, 1e33, False),
+                                    (1e-15, 1e15, False), (1e20, 1e-20, False), (2.0 ** -30, 1.0, True),
+                                    (2.0 ** 60, 1.0, True)], ids=str)
+def test_scales_mixed(scales, kind):
+    _scaled(scales, fvmbaseExt.AMG.MIXED, kind)
