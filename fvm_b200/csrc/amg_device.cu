@@ -959,6 +959,7 @@ bool AmgHierarchy::prepareFinestPatternDevice(const FinestDevice& in) {
   fp.sliceRows = fp.arena.upload(pk.sliceRows);
   fp.sliceOff = fp.arena.upload(pk.sliceOff);
   fp.meta = fp.arena.upload(meta);
+  settle_device();
   // the permutation on the host too (exports of level 0 use it)
   pk.perm.resize(n);
   pk.iperm.resize(n);
@@ -1011,6 +1012,7 @@ void AmgHierarchy::prepareFinestPattern(const FinestDevice& in, int ordering) {
   fp.posSrc = fp.arena.upload(posSrc.get(), E);
   fp.iperm = fp.arena.upload(p.iperm);
   fp.perm = fp.arena.upload(p.perm);
+  settle_device();
 }
 
 void AmgHierarchy::allocVectors(DevLevel& d, bool mixed) {
@@ -1261,6 +1263,7 @@ void AmgHierarchy::buildDevice(const FinestDevice& in, const SolverOptions& opt,
       std::vector<double> inv;
       dense_inverse(h, inv);
       coarseInv_ = arena_.upload(inv);
+      settle_device();
     } else {
       FVM_REQUIRE(c.ellWidth == 0, kUnsupported, "coarsest level in ELL-32 layout");
       auto alloc = [&](size_t bytes) { return arena_.alloc(size_class(bytes)); };

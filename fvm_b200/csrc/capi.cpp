@@ -703,14 +703,13 @@ int fvm_amg_solve_csr(int n, const int* row, const int* col, const double* diag,
       std::vector<double> bp(n);
       for (int i = 0; i < n; i++) bp[p0.perm[i]] = b[i];
       DevLevel& d = hier.level(0);
-      if (cudaMemcpy(d.b, bp.data(), sizeof(double) * n, cudaMemcpyHostToDevice) != cudaSuccess)
-        throw Error(kDeviceError, "copy of b failed");
+      copy_to_device(d.b, bp.data(), sizeof(double) * n);
       cudaEvent_t e0, e1;
       cudaEventCreate(&e0);
       cudaEventCreate(&e1);
       cudaEventRecord(e0, st);
       {
-        LinearSolve ls(hier);
+        LinearSolve ls(hier, st);
         sr = ls.solve(st);
         if (rep) {
           fill_report(rep, sr);

@@ -51,6 +51,15 @@ const char* last_error();
     if (!(cond)) throw ::fvm::Error((status), (msg)); \
   } while (0)
 
+// cudaMemcpy from pageable memory returns once the data is in its staging
+// buffer, and cudaMemset does not wait at all; both are ordered before later
+// work of the default stream only, and most work here runs on streams that do
+// not wait for it. settle_device() waits until everything given to the default
+// stream so far is done; the other two are a copy and a fill that are.
+void settle_device();
+void copy_to_device(void* d, const void* h, size_t bytes);
+void clear_device(void* d, size_t bytes);
+
 // Compressed rows: row[i]..row[i+1] index col[] (and any value arrays kept
 // alongside). Matches the reference's CRConnectivity layout.
 struct CSR {

@@ -964,7 +964,7 @@ void Workspace::allocate(int n_, bool training, long long entries) {
     // two sums a block (k_residual_loss)
     check(cudaMalloc(&partials, sizeof(double) * (2 * kReduceBlocks + 8)), "cudaMalloc");
     check(cudaMalloc(&status, sizeof(int)), "cudaMalloc");
-    check(cudaMemset(status, 0, sizeof(int)), "cudaMemset");
+    clear_device(status, sizeof(int));
     if (training) {
       for (int l = 0; l < kLayers; l++) check(cudaMalloc(&M[l], hb), "cudaMalloc");
       check(cudaMalloc(&dA, hb), "cudaMalloc");
@@ -1016,7 +1016,7 @@ void Workspace::checkStatus() {
   int h = 0;
   check(cudaMemcpy(&h, status, sizeof(int), cudaMemcpyDeviceToHost), "status copy");
   if (h) {
-    check(cudaMemset(status, 0, sizeof(int)), "cudaMemset");
+    clear_device(status, sizeof(int));
     throw Error(kDeviceError, "learned correction: a tensor-core completion wait ran out");
   }
 }
@@ -1059,7 +1059,7 @@ int tc_wait_probe(unsigned limit) {
   int* status = nullptr;
   check(cudaMalloc(&status, sizeof(int)), "cudaMalloc");
   int h = 0;
-  cudaError_t e = cudaMemset(status, 0, sizeof(int));
+  cudaError_t e = cudaMemsetAsync(status, 0, sizeof(int), nullptr);
   if (e == cudaSuccess) {
     k_tc_wait_probe<<<1, 64>>>(limit, status);
     e = cudaGetLastError();
@@ -1175,8 +1175,8 @@ LearnedCorrection::LearnedCorrection(uint64_t seed) {
   nn::check(cudaMalloc(&dM_, sizeof(float) * nn::kParams), "cudaMalloc");
   nn::check(cudaMalloc(&dV_, sizeof(float) * nn::kParams), "cudaMalloc");
   nn::check(cudaMalloc(&dScal_, sizeof(double) * 16), "cudaMalloc");
-  nn::check(cudaMemset(dM_, 0, sizeof(float) * nn::kParams), "cudaMemset");
-  nn::check(cudaMemset(dV_, 0, sizeof(float) * nn::kParams), "cudaMemset");
+  clear_device(dM_, sizeof(float) * nn::kParams);
+  clear_device(dV_, sizeof(float) * nn::kParams);
   setParams(nn::initial_parameters(seed));
 }
 
@@ -1203,9 +1203,9 @@ std::vector<float> LearnedCorrection::params() const {
 
 void LearnedCorrection::setParams(const std::vector<float>& p) {
   FVM_REQUIRE((int)p.size() == nn::kParams, kBadArgument, "learned correction: wrong parameter count");
-  nn::check(cudaMemcpy(dParams_, p.data(), sizeof(float) * nn::kParams, cudaMemcpyHostToDevice), "cudaMemcpy");
-  nn::check(cudaMemset(dM_, 0, sizeof(float) * nn::kParams), "cudaMemset");
-  nn::check(cudaMemset(dV_, 0, sizeof(float) * nn::kParams), "cudaMemset");
+  copy_to_device(dParams_, p.data(), sizeof(float) * nn::kParams);
+  clear_device(dM_, sizeof(float) * nn::kParams);
+  clear_device(dV_, sizeof(float) * nn::kParams);
   adamT_ = 0;
 }
 

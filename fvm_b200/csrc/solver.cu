@@ -83,6 +83,16 @@ void DeviceArena::copy_h2d(void* d, const void* h, size_t n) {
   CUDA_OK(cudaMemcpy(d, h, n, cudaMemcpyHostToDevice));
 }
 
+void settle_device() { CUDA_OK(cudaStreamSynchronize(nullptr)); }
+void copy_to_device(void* d, const void* h, size_t bytes) {
+  CUDA_OK(cudaMemcpy(d, h, bytes, cudaMemcpyHostToDevice));
+  settle_device();
+}
+void clear_device(void* d, size_t bytes) {
+  CUDA_OK(cudaMemset(d, 0, bytes));
+  settle_device();
+}
+
 void DeviceArena::release() {
   std::lock_guard<std::mutex> lock(mu_);
   for (auto& pb : ptrs_) free_.insert({pb.second, pb.first});
@@ -337,6 +347,7 @@ void AmgHierarchy::build(std::vector<RefLevel>& levels, int finestLocalSize, con
   }
   prepareChebyshev();
   buildTail();
+  settle_device();
   tunePlans();
   lap("launch plans");
   if (trace) {
@@ -548,6 +559,7 @@ void AmgHierarchy::tunePlans() {
       if (d.xF) CUDA_OK(cudaMemset(d.xF, 0, sizeof(float) * d.n));
       if (d.tmpF) CUDA_OK(cudaMemset(d.tmpF, 0, sizeof(float) * d.n));
     }
+    settle_device();
   }
 }
 
@@ -633,6 +645,7 @@ void AmgHierarchy::uploadMatrix(const PackedLevel& p, DevLevel& d, bool mixed) {
     d.tmpF = (float*)arena_.alloc(fb);
     CUDA_OK(cudaMemset(d.xF, 0, fb));
   }
+  settle_device();
 }
 
 void AmgHierarchy::uploadTransfer(const PackedLevel& p, DevLevel& d, int nCoarse) {
@@ -640,6 +653,7 @@ void AmgHierarchy::uploadTransfer(const PackedLevel& p, DevLevel& d, int nCoarse
   d.ci = arena_.upload(p.coarseIndex);
   d.c2fRow = arena_.upload(p.c2fRow);
   d.c2fCol = arena_.upload(p.c2fCol);
+  settle_device();
 }
 
 template <>
@@ -974,7 +988,7 @@ void AmgHierarchy::buildTail() {
   if (opt_.cycleType == kFCycle) ok = ok && program(kVCycle, true) && program(kVCycle, false);
   if (!ok) return;  // a W cycle of very many levels: launches of their own
   const dev::TailStep* d = arena_.upload(all);
-  CUDA_OK(cudaStreamSynchronize(nullptr));
+  settle_device();
   for (size_t k = 0; k < programs.size(); k++) programs[k].steps = d + start[k];
   tailPrograms_ = std::move(programs);
   tailSmem_ = used;
@@ -1394,10 +1408,10 @@ __global__ void __launch_bounds__(1024) k_loop_check(int np, const double* __res
 // Device workspace comes from the hierarchy's arena (recycled by the next
 // build of the same sizes, so a rebuild allocates nothing); the pinned
 // scalars are the hierarchy's too.
-LinearSolve::LinearSolve(AmgHierarchy& h) : h_(h), n_(h.level(0).n) {
+LinearSolve::LinearSolve(AmgHierarchy& h, cudaStream_t st) : h_(h), n_(h.level(0).n) {
   work_ = (double*)h.scratch(sizeof(double) * (size_t)n_ * kWorkVectors);
   scal_ = (double*)h.scratch(sizeof(double) * 32);
-  CUDA_OK(cudaMemset(scal_, 0, sizeof(double) * 32));
+  CUDA_OK(cudaMemsetAsync(scal_, 0, sizeof(double) * 32, st));
   partials_ = (double*)h.scratch(sizeof(double) * (dev::vec_blocks(n_) + 1));
   {
     const DevLevel& d = h.level(0);

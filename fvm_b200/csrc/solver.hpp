@@ -147,6 +147,7 @@ class DeviceArena {
  public:
   ~DeviceArena();
   void* alloc(size_t bytes);
+  // on the default stream: settle_device() before another stream reads it
   template <class T>
   T* upload(const std::vector<T>& v) {
     return upload(v.data(), v.size());
@@ -381,7 +382,8 @@ bool graph_conditional(cudaGraph_t g, cudaGraphConditionalHandle h, cudaGraphCon
 // the right-hand side, level 0's x the delta (zeroed on entry).
 class LinearSolve {
  public:
-  explicit LinearSolve(AmgHierarchy& h);
+  // st: the stream solve() will be given
+  LinearSolve(AmgHierarchy& h, cudaStream_t st);
   ~LinearSolve();
   SolveReport solve(cudaStream_t st);
   // Learned correction applied after every refinement iteration of the AMG

@@ -113,13 +113,13 @@ void ThermalModel::setSegments(const std::vector<int>& offsets) {
       FVM_REQUIRE(offsets[s + 1] > offsets[s], kBadArgument, "segments: offsets must increase");
     segOff_ = offsets;
     CUDA_OK(cudaMalloc(&dSegOff_, sizeof(int) * segOff_.size()));
-    CUDA_OK(cudaMemcpy(dSegOff_, segOff_.data(), sizeof(int) * segOff_.size(), cudaMemcpyHostToDevice));
+    copy_to_device(dSegOff_, segOff_.data(), sizeof(int) * segOff_.size());
     std::vector<int> chunk(1, 0);
     for (size_t s = 0; s + 1 < segOff_.size(); s++)
       chunk.push_back(chunk.back() + (segOff_[s + 1] - segOff_[s] + kSegChunk - 1) / kSegChunk);
     segChunks_ = chunk.back();
     CUDA_OK(cudaMalloc(&dSegChunk_, sizeof(int) * chunk.size()));
-    CUDA_OK(cudaMemcpy(dSegChunk_, chunk.data(), sizeof(int) * chunk.size(), cudaMemcpyHostToDevice));
+    copy_to_device(dSegChunk_, chunk.data(), sizeof(int) * chunk.size());
     CUDA_OK(cudaMalloc(&dSegPart_, sizeof(double) * (size_t)segChunks_));
     CUDA_OK(cudaMalloc(&dSegNorm_, sizeof(double) * (segOff_.size() - 1)));
   }
@@ -810,14 +810,14 @@ void ThermalModel::ensureDevice() {
   dVol_ = arena_.upload(m.cellVolume);
   dCfRow_ = arena_.upload(cfRow);
   dCfCol_ = arena_.upload(cfCol);
-  dCfSide_ = (int*)arena_.alloc(sizeof(int) * std::max<size_t>(cfCol.size(), 1));
-  CUDA_OK(cudaStreamSynchronize(nullptr));  // (a copy from pageable memory may still be on its way)
-  dev::face_sides(n, dCfRow_, dCfCol_, dFaceCells_, dCfSide_, stream_);
   dBRow_ = arena_.upload(bRow);
   dBCol_ = arena_.upload(bCol);
   dBColG_ = arena_.upload(bColG);
   dBFace_ = arena_.upload(boundaryFaces_);
   dBIndexOfFace_ = arena_.upload(bIndexOfFace);
+  dCfSide_ = (int*)arena_.alloc(sizeof(int) * std::max<size_t>(cfCol.size(), 1));
+  settle_device();
+  dev::face_sides(n, dCfRow_, dCfCol_, dFaceCells_, dCfSide_, stream_);
   const int nB = (int)boundaryFaces_.size();
   dBKind_ = (int*)arena_.alloc(sizeof(int) * (nB + 1));
   dBValue_ = (double*)arena_.alloc(sizeof(double) * (nB + 1));
@@ -826,7 +826,7 @@ void ThermalModel::ensureDevice() {
   dBGhostDiag_ = (double*)arena_.alloc(sizeof(double) * (nB + 1));
   dHf_ = (double*)arena_.alloc(sizeof(double) * 4 * (nB + 1));
   dHeatFlux_ = (double*)arena_.alloc(sizeof(double) * (nB + 1));
-  CUDA_OK(cudaMemset(dHeatFlux_, 0, sizeof(double) * (nB + 1)));
+  clear_device(dHeatFlux_, sizeof(double) * (nB + 1));
   const size_t cb = sizeof(double) * (size_t)nAll;
   dT_ = (double*)arena_.alloc(cb);
   dK_ = (double*)arena_.alloc(cb);
@@ -839,7 +839,7 @@ void ThermalModel::ensureDevice() {
   dFlux_ = (double*)arena_.alloc(sizeof(double) * (size_t)F);
   dCoeff_ = (double*)arena_.alloc(sizeof(double) * (size_t)F);
   dSec_ = (double*)arena_.alloc(4 * sizeof(double) * (size_t)F);  // 32-byte record per face
-  CUDA_OK(cudaMemset(dGrad_, 0, 4 * cb));
+  clear_device(dGrad_, 4 * cb);
   {
     // identifies this model's level-0 pattern (interiorConn_, entryFace_)
     static std::atomic<unsigned long long> nextKey{1};
@@ -918,9 +918,9 @@ void ThermalModel::uploadFields() {
       par[3 * t + 2] = b.values[4];  // surfaceEmissivity
     }
   }
-  CUDA_OK(cudaMemcpy(dBKind_, kind.data(), sizeof(int) * (nB + 1), cudaMemcpyHostToDevice));
-  CUDA_OK(cudaMemcpy(dBValue_, val.data(), sizeof(double) * (nB + 1), cudaMemcpyHostToDevice));
-  CUDA_OK(cudaMemcpy(dBParam_, par.data(), sizeof(double) * 3 * (nB + 1), cudaMemcpyHostToDevice));
+  CUDA_OK(cudaMemcpyAsync(dBKind_, kind.data(), sizeof(int) * (nB + 1), cudaMemcpyHostToDevice, stream_));
+  CUDA_OK(cudaMemcpyAsync(dBValue_, val.data(), sizeof(double) * (nB + 1), cudaMemcpyHostToDevice, stream_));
+  CUDA_OK(cudaMemcpyAsync(dBParam_, par.data(), sizeof(double) * 3 * (nB + 1), cudaMemcpyHostToDevice, stream_));
   if (par != bParamHost_) {
     bParamHost_ = par;
     matrixDirty_ = true;
@@ -981,7 +981,7 @@ void ThermalModel::ensureMatrix() {
     hier_.buildDevice(in, opt_.linear, true);
     lap("hierarchy on the device");
     dPerm_ = const_cast<int*>(hier_.finestPermDevice());
-    solver_.reset(new LinearSolve(hier_));
+    solver_.reset(new LinearSolve(hier_, stream_));
     solver_->setSingleUse(matrixDependsOnT_);
     solverGen_++;
     solver_->setLearned(learned_);
@@ -1047,7 +1047,7 @@ void ThermalModel::ensureMatrix() {
   dPerm_ = (int*)hier_.scratch(sizeof(int) * (size_t)n);
   CUDA_OK(cudaMemcpyAsync(dPerm_, hier_.packed(0).perm.data(), sizeof(int) * (size_t)n, cudaMemcpyHostToDevice,
                           stream_));
-  solver_.reset(new LinearSolve(hier_));
+  solver_.reset(new LinearSolve(hier_, stream_));
   solver_->setSingleUse(matrixDependsOnT_);
   solverGen_++;
   solver_->setLearned(learned_);

@@ -101,3 +101,49 @@ def test_loop_control_ends_a_chain():
         assert re.search(r"\b%s(?:<\w+>)?<<<" % k, solver)
         assert not re.search(r"pdl_launch(?:_smem)?\(\s*%s\b" % k, solver)
         assert not any(waits(body) for n, _, body in kernels("solver.cu") if n == k)
+
+
+def functions(name):
+    """(name, body) of every function definition of a file, roughly: an
+    identifier, a parameter list and a body."""
+    s = text(name)
+    for m in re.finditer(r"^[A-Za-z][^\n;#(){}=]*?([\w:~]+)\(", s, flags=re.M):
+        depth, j = 1, m.end()
+        while depth and j < len(s):
+            depth += {"(": 1, ")": -1}.get(s[j], 0)
+            j += 1
+        if re.match(r"\s*(const\s*)?(:[^{;]*)?\{", s[j:]):
+            yield m.group(1), block(s, j)
+
+
+HOST = sorted(f for f in os.listdir(CSRC) if f.endswith((".cu", ".cpp", ".hpp")))
+COPIES = r"cudaMemset\(|cudaMemcpy\([^;]*cudaMemcpyHostToDevice|\bupload\("
+# the arena's own members, and callers whose kernels run on the default stream
+DEFAULT_STREAM = {"copy_h2d", "DeviceArena::copy_h2d", "upload", "CsrGraph", "fvm_csr_residual",
+                  "fvm_learned_forward_csr", "fvm_learned_gradient_csr"}
+
+
+@pytest.mark.parametrize("name", HOST)
+def test_host_copies_end_before_another_stream_reads_them(name):
+    """cudaMemcpy from pageable memory and cudaMemset are ordered before later
+    work of the default stream only; level arrays, mesh arrays and network
+    parameters are read on streams that do not wait for it. Whoever makes such
+    a copy waits for the default stream (settle_device) after the last one."""
+    s = text(name)
+    checked = 0
+    for fn, body in functions(name):
+        at = [m.start() for m in re.finditer(COPIES, body)]
+        checked += len(at)
+        if at and fn not in DEFAULT_STREAM:
+            assert "settle_device();" in body[at[-1]:], f"{name}: {fn}"
+    if name.endswith(".cu"):
+        assert checked == len(re.findall(COPIES, s))
+
+
+def test_settle_waits_for_the_default_stream():
+    assert "cudaStreamSynchronize(nullptr)" in dict(functions("solver.cu"))["settle_device"]
+
+
+def test_host_build_ends_with_the_default_stream_empty():
+    body = dict(functions("solver.cu"))["AmgHierarchy::build"]
+    assert body.index("buildTail();") < body.index("settle_device();") < body.index("tunePlans();")
