@@ -32,6 +32,8 @@
 #include <cmath>
 #include <cstdint>
 
+#include "pdl.cuh"
+
 namespace fvm {
 namespace dev {
 namespace {
@@ -519,6 +521,7 @@ template <class T>
 void cycle_tail(const TailArgs<T>& a, size_t smemBytes, cudaStream_t st) {
   cudaLaunchAttribute attr[2];
   cudaLaunchConfig_t cfg = config<T>(a.lc, smemBytes, st, attr);
+  launchesIssued++;
   cudaLaunchKernelEx(&cfg, k_cycle_tail<T>, a);
 }
 template void cycle_tail<float>(const TailArgs<float>&, size_t, cudaStream_t);

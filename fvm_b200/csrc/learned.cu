@@ -1151,18 +1151,22 @@ __global__ void k_step_finish(double* norm, const double* trial, double* accepte
 }  // namespace
 
 void step_alpha(const double* rq, const double* qq, double* alpha, cudaStream_t st) {
+  launchesIssued++;
   k_step_alpha<<<1, 1, 0, st>>>(rq, qq, alpha);
 }
 void step_trial(int n, const double* r, const double* q, const double* alpha, double* rt, double* partials,
                 cudaStream_t st) {
+  launchesIssued++;
   k_step_trial<<<dev::vec_blocks(n), kBlock, 0, st>>>(n, r, q, alpha, rt, partials);
 }
 void step_accept(int n, double* x, const double* d, double* r, const double* rt, const double* alpha,
                  const double* norm, const double* trialNorm, double acceptFactor, cudaStream_t st) {
+  launchesIssued++;
   k_step_accept<<<dev::vec_blocks(n), kBlock, 0, st>>>(n, x, d, r, rt, alpha, norm, trialNorm, acceptFactor);
 }
 void step_finish(double* norm, const double* trialNorm, double* accepted, double* steps, double* useful,
                  double usefulFactor, double acceptFactor, cudaStream_t st) {
+  launchesIssued++;
   k_step_finish<<<1, 1, 0, st>>>(norm, trialNorm, accepted, steps, useful, usefulFactor, acceptFactor);
 }
 

@@ -17,6 +17,9 @@
 
 namespace fvm {
 
+// kernels and copies that this thread has issued on the paths of a solve
+inline thread_local long long launchesIssued = 0;
+
 template <typename... KArgs, typename... Args>
 inline void pdl_launch_smem(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
                             Args... args) {
@@ -30,6 +33,7 @@ inline void pdl_launch_smem(void (*kernel)(KArgs...), dim3 grid, dim3 block, siz
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
+  launchesIssued++;
   cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 

@@ -2,6 +2,7 @@
 #include "solver.hpp"
 
 #include "coarse_inverse.cuh"
+#include "pdl.cuh"
 
 #include <math_constants.h>
 
@@ -716,7 +717,10 @@ void AmgHierarchy::sweeps(int nSweeps, int l, cudaStream_t st, const T* xc, cons
                                st);
         cur ^= 1;
       }
-    if (cur) CUDA_OK(cudaMemcpyAsync(x, bufs[1], sizeof(T) * (size_t)d.n, cudaMemcpyDeviceToDevice, st));
+    if (cur) {
+      CUDA_OK(cudaMemcpyAsync(x, bufs[1], sizeof(T) * (size_t)d.n, cudaMemcpyDeviceToDevice, st));
+      launchesIssued++;
+    }
     return;
   }
   for (int s = 0; s < nSweeps; s++) {
@@ -1440,8 +1444,13 @@ void LinearSolve::dot_into(const double* a, const double* b, double* scalar, cud
   dev::sum_partials(dev::vec_blocks(n_), partials_, scalar, st);
 }
 
+void LinearSolve::toHost(int slot, const double* scalar, cudaStream_t st) {
+  CUDA_OK(cudaMemcpyAsync(hostScal_ + slot, scalar, sizeof(double), cudaMemcpyDeviceToHost, st));
+  launchesIssued++;
+}
+
 double LinearSolve::fetch(const double* scalar, cudaStream_t st) {
-  CUDA_OK(cudaMemcpyAsync(hostScal_, scalar, sizeof(double), cudaMemcpyDeviceToHost, st));
+  toHost(0, scalar, st);
   CUDA_OK(cudaStreamSynchronize(st));
   return hostScal_[0];
 }
@@ -1457,8 +1466,9 @@ void LinearSolve::run(cudaGraphExec_t& exec, cudaStream_t st, const std::functio
   }
   if (singleUse_ && eagerRuns_ < kEagerRuns) {
     eagerRuns_++;
+    const long long total = launches, issued = launchesIssued;
     body();
-    launches += h_.kernelsPerCycle() + 7;  // the cycle and a CG iteration's own
+    launches = total + (launchesIssued - issued);  // as many as the graph will have nodes
     return;
   }
   if (!exec) {
@@ -1548,10 +1558,10 @@ SolveReport LinearSolve::solveAMG(cudaStream_t st) {
       dev::sum_partials(d.nPartials, d.partials, scal_ + kNorm, st);
       if (useLs) {
         learnedStep(st, d.x, d.r, 1.0);
-        CUDA_OK(cudaMemcpyAsync(hostScal_ + 1, scal_ + kLsAccepted, sizeof(double), cudaMemcpyDeviceToHost, st));
-        CUDA_OK(cudaMemcpyAsync(hostScal_ + 2, scal_ + kLsUseful, sizeof(double), cudaMemcpyDeviceToHost, st));
+        toHost(1, scal_ + kLsAccepted, st);
+        toHost(2, scal_ + kLsUseful, st);
       }
-      CUDA_OK(cudaMemcpyAsync(hostScal_, scal_ + kNorm, sizeof(double), cudaMemcpyDeviceToHost, st));
+      toHost(0, scal_ + kNorm, st);
     });
     CUDA_OK(cudaStreamSynchronize(st));
     const double rn = hostScal_[0];
@@ -1605,7 +1615,7 @@ SolveReport LinearSolve::solveJacobi(cudaStream_t st) {
       dev::copy_d(n_, d.tmp, d.x, st);
       dev::residual<double>(d.view64(), d.nSlices, d.x, d.b, d.r, d.partials, st);
       dev::sum_partials(d.nPartials, d.partials, scal_ + kNorm, st);
-      CUDA_OK(cudaMemcpyAsync(hostScal_, scal_ + kNorm, sizeof(double), cudaMemcpyDeviceToHost, st));
+      toHost(0, scal_ + kNorm, st);
     });
     CUDA_OK(cudaStreamSynchronize(st));
     const double rn = hostScal_[0];
@@ -1767,12 +1777,15 @@ SolveReport LinearSolve::solveCG(cudaStream_t st) {
       run(g4_, st, [&] {
         h_.applyCycle(R, st);
         const int gb = (n_ + 255) / 256;
-        if (mixedCycle)
+        if (mixedCycle) {
           k_f2d<<<gb, 256, 0, st>>>(n_, d.xF, D1);
-        else
+          launchesIssued++;
+        } else {
           dev::copy_d(n_, d.x, D1, st);
+        }
         dev::spmv(d.view64(), d.nSlices, D1, R1, st);
         k_add_vec<<<gb, 256, 0, st>>>(n_, R, R1, R1);
+        launchesIssued++;
         const nn::Graph g{d.view64(), d.rowSlice, d.nSlices, (long long)d.entries};
         learned_->apply(g, R1, DN, scal_ + kLsScale, st);
         dev::spmv(d.view64(), d.nSlices, DN, Q2, st);
@@ -1783,6 +1796,7 @@ SolveReport LinearSolve::solveCG(cudaStream_t st) {
         nn::step_trial(n_, R1, Q2, scal_ + kLsAlpha, RT, partials_, st);
         dev::sum_partials(dev::vec_blocks(n_), partials_, scal_ + kLsTrial, st);
         k_combine<<<gb, 256, 0, st>>>(n_, D1, scal_ + kLsAlpha, DN, D1);
+        launchesIssued++;
         dev::cg_dot_z<double>(n_, D1, R, partials2_, st);
         dev::cg_beta(dev::vec_blocks(n_), partials2_, scal_ + kRho, scal_ + kRhoPrev, scal_ + kBeta, flexible, st);
         dev::xpby_dev(n_, D1, scal_ + kBeta, P, st);
@@ -1790,9 +1804,9 @@ SolveReport LinearSolve::solveCG(cudaStream_t st) {
         dev::cg_alpha(dev::spmv_dot_blocks(d.view64(), d.nSlices), partials2_, scal_ + kRho, scal_ + kAlpha, st);
         dev::cg_update<double>(n_, scal_ + kAlpha, P, Q, X, R, D1, partials_, partials2_, st, rF);
         dev::sum_partials(dev::vec_blocks(n_), partials_, scal_ + kNorm, st);
-        CUDA_OK(cudaMemcpyAsync(hostScal_, scal_ + kNorm, sizeof(double), cudaMemcpyDeviceToHost, st));
-        CUDA_OK(cudaMemcpyAsync(hostScal_ + 1, scal_ + kLsBefore, sizeof(double), cudaMemcpyDeviceToHost, st));
-        CUDA_OK(cudaMemcpyAsync(hostScal_ + 2, scal_ + kLsTrial, sizeof(double), cudaMemcpyDeviceToHost, st));
+        toHost(0, scal_ + kNorm, st);
+        toHost(1, scal_ + kLsBefore, st);
+        toHost(2, scal_ + kLsTrial, st);
       });
       launches += 6;
     } else if (fused) {
@@ -1806,7 +1820,7 @@ SolveReport LinearSolve::solveCG(cudaStream_t st) {
         else
           cgStep<double>(d.x, R, P, Q, X, flexible, rF, st);
         dev::sum_partials(dev::vec_blocks(n_), partials_, scal_ + kNorm, st);
-        CUDA_OK(cudaMemcpyAsync(hostScal_, scal_ + kNorm, sizeof(double), cudaMemcpyDeviceToHost, st));
+        toHost(0, scal_ + kNorm, st);
       });
     } else {
       run(g1_, st, [&] {
@@ -1825,7 +1839,7 @@ SolveReport LinearSolve::solveCG(cudaStream_t st) {
         dev::axpy_dev(n_, scal_ + kAlpha, -1.0, P, X, st);
         dev::axpy_dev(n_, scal_ + kAlpha, -1.0, Q, R, st);
         norm_into(R, scal_ + kNorm, st);
-        CUDA_OK(cudaMemcpyAsync(hostScal_, scal_ + kNorm, sizeof(double), cudaMemcpyDeviceToHost, st));
+        toHost(0, scal_ + kNorm, st);
       });
     }
     CUDA_OK(cudaStreamSynchronize(st));
@@ -1970,8 +1984,8 @@ bool LinearSolve::addDeviceLoop(cudaGraph_t g, cudaStream_t st, bool hostCopies)
   // the results to the pinned host scalars
   auto copies = [&] {
     if (!hostCopies) return;
-    CUDA_OK(cudaMemcpyAsync(hostScal_, scal_ + kNorm, sizeof(double), cudaMemcpyDeviceToHost, st));
-    CUDA_OK(cudaMemcpyAsync(hostScal_ + 1, history_, sizeof(double), cudaMemcpyDeviceToHost, st));
+    toHost(0, scal_ + kNorm, st);
+    toHost(1, history_, st);
     CUDA_OK(cudaMemcpyAsync(hostScal_ + 2, loopInt_, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
   };
   const size_t nb = sizeof(double) * (size_t)n_;
@@ -2237,7 +2251,7 @@ SolveReport LinearSolve::solveBCGStab(cudaStream_t st) {
     run(g1_, st, [&] {
       bcgFirst(R, RT, V, P, PH, X, st);
       dev::sum_partials(dev::vec_blocks(n_), partials_, scal_ + kNorm, st);
-      CUDA_OK(cudaMemcpyAsync(hostScal_, scal_ + kNorm, sizeof(double), cudaMemcpyDeviceToHost, st));
+      toHost(0, scal_ + kNorm, st);
     });
     CUDA_OK(cudaStreamSynchronize(st));
     double rn = hostScal_[0];
@@ -2252,7 +2266,7 @@ SolveReport LinearSolve::solveBCGStab(cudaStream_t st) {
     run(g2_, st, [&] {
       bcgSecond(R, Tt, PH, X, st);
       dev::sum_partials(dev::vec_blocks(n_), partials_, scal_ + kNorm, st);
-      CUDA_OK(cudaMemcpyAsync(hostScal_, scal_ + kNorm, sizeof(double), cudaMemcpyDeviceToHost, st));
+      toHost(0, scal_ + kNorm, st);
     });
     CUDA_OK(cudaStreamSynchronize(st));
     rn = hostScal_[0];

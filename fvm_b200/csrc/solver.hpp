@@ -465,6 +465,8 @@ class LinearSolve {
   SolveReport solveJacobi(cudaStream_t st);
   void norm_into(const double* v, double* scalar, cudaStream_t st);
   void dot_into(const double* a, const double* b, double* scalar, cudaStream_t st);
+  // scalar to the pinned host scalars, asynchronously
+  void toHost(int slot, const double* scalar, cudaStream_t st);
   double fetch(const double* scalar, cudaStream_t st);
   // Runs body on st; with graphs enabled the first call captures it and
   // later calls replay the instantiated graph.

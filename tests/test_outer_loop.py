@@ -201,3 +201,60 @@ def test_single_use_hierarchies_launch_without_a_graph(precision):
     assert (i1, l1) == (i0, l0)
     np.testing.assert_array_equal(h1, h0)
     np.testing.assert_array_equal(t1, t0)
+
+
+def _radiative_launches(linear, iterations):
+    """Kernels and copies of one outer iteration whose solve makes the given
+    number of iterations; radiative faces make its hierarchy a single-use one."""
+    from fvm_b200 import models
+
+    kind, knobs = linear
+    amg = fvmbaseExt.AMG()
+    for name, value in knobs.items():
+        setattr(amg, name, value)
+    solver = amg
+    if kind is not fvmbaseExt.AMG:
+        solver = kind()
+        if kind is not fvmbaseExt.JacobiSolver:
+            solver.preconditioner = amg
+    solver.nMaxIterations = iterations
+    solver.relativeTolerance = 1e-300
+    solver.absoluteTolerance = 0.0
+    mesh, f = _mesh("hex")
+    m = fvmbaseExt.Mesh.from_dict(mesh)
+    tf = models.ThermalFields("therm")
+    tm = models.ThermalModelA(models.GeomFields("geom"), tf, [m])
+    for gid, (bc_kind, vals) in {
+        1: ("SpecifiedTemperature", {"specifiedTemperature": 300.0}),
+        2: ("SpecifiedTemperature", {"specifiedTemperature": 400.0}),
+        3: ("Radiative", {"farFieldTemperature": 310.0, "surfaceEmissivity": 0.7}),
+    }.items():
+        bc = tm.getBCMap()[gid]
+        bc.bcType = bc_kind
+        for name, v in vals.items():
+            bc.setVar(name, v)
+    tm.getOptions().linearSolver = solver
+    tm.init()
+    tf.conductivity[m.getCells()] = f["k"]
+    tf.source[m.getCells()] = f["s"]
+    return tm.advance(1).launches
+
+
+MIXED = dict(precision=fvmbaseExt.AMG.MIXED, coarseSolver=fvmbaseExt.AMG.COARSE_DIRECT, coarsestSize=100,
+             coarseJacobiRows=1 << 30, nPreSweeps=0, nPostSweeps=2, setupOnDevice=True)
+
+
+@pytest.mark.parametrize("linear", [
+    (fvmbaseExt.CG, {}), (fvmbaseExt.CG, MIXED), (fvmbaseExt.CG, dict(cycleType=1, planThreadsPerRow=1)),
+    (fvmbaseExt.CG, dict(chebyshevDegree=3)), (fvmbaseExt.AMG, {}), (fvmbaseExt.AMG, MIXED),
+    (fvmbaseExt.BCGStab, {}), (fvmbaseExt.BCGStab, MIXED), (fvmbaseExt.JacobiSolver, {}),
+], ids=["cg", "cg-mixed", "cg-w", "cg-cheb", "amg", "amg-mixed", "bcgstab", "bcgstab-mixed", "jacobi"])
+def test_single_use_hierarchies_count_what_they_launch(linear):
+    """The report's launches (kernels and copies issued): an iteration whose
+    kernels are launched one by one counts as many as the same iteration as a
+    graph, whose nodes are counted. The first four pieces of a solve are
+    launched (BiCGStab has two an iteration), the later ones are graphs."""
+    first = 1 if linear[0] is fvmbaseExt.BCGStab else 2
+    launched = _radiative_launches(linear, first + 1) - _radiative_launches(linear, first)
+    graph = _radiative_launches(linear, 8) - _radiative_launches(linear, 7)
+    assert launched == graph > 0
