@@ -452,3 +452,38 @@ def test_trained_network_prediction_on_held_out_draws():
                                                             cycles[True][0], cycles[True][1], cycles[True][2]))
     assert loss_trained < 0.8 * loss_init
     assert cycles[True][0] <= cycles[False][0] + 2
+
+
+@pytest.mark.gpu
+def test_tensor_core_gradient_misses_no_entry_of_a_small_graph():
+    """Nine nodes with 0 to 4 neighbours, all parameters and inputs positive: no
+    unit is near its ReLU's edge and no sum cancels, so TF32 alone separates the
+    two sides. A gradient entry has at most 20 operands cut to 10 bits behind it
+    (two a layer forward, in the loss and in the layer's input, two a layer
+    backward, two in the product of the gradient): 20 * 2^-10 = 2e-2. Leaving
+    one entry of the matrix out moves a block by more than 9e-2."""
+    from fvm_b200.learned import LearnedCorrection
+
+    n, tol = 9, 20 * 2.0 ** -10
+    row, col, _, off = _irregular(n, 2, seed=29)
+    off = np.ones_like(off)
+    diag = -np.maximum(np.diff(row), 1).astype(float)
+    rng = np.random.default_rng(22)
+    P = rng.uniform(0.01, 0.05, mo.N_PARAMS).astype(np.float32)
+    P64 = P.astype(np.float64)
+    r = rng.uniform(0.5, 1.5, n) * np.abs(diag)
+    e = -np.ones(n)
+    lref, gref = mo.loss_and_gradient(P64, row, col, diag, off, r, e)
+
+    def worst(g):
+        return max(rel_l2(g[a:b], gref[a:b]) for a, b in _BLOCKS)
+
+    for k in range(len(off)):
+        missed = off.copy()
+        missed[k] = 0.0
+        assert worst(mo.loss_and_gradient(P64, row, col, diag, missed, r, e)[1]) > 9e-2
+    lc = LearnedCorrection(seed=0)
+    lc.setParams(P)
+    g, loss = lc.gradient_csr(row, col, diag, off, r, e)
+    assert abs(loss - lref) <= tol * lref
+    assert worst(g) <= tol
