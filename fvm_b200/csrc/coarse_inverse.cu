@@ -19,12 +19,12 @@
 // A step is two kernels: k_inv_panel forms the new pivot rows R = D^-1 A[K][:]
 // of every pivot block of the step, k_inv_update applies them to the 64 x 64
 // tiles on and above the diagonal and inverts the next step's pivot blocks.
-// Measured, order and unpermuting included: 3313 rows (41k tets) 5.4 -> 0.9
+// Measured, order and unpermuting included: 3313 rows (41k tets) 5.4 -> 0.93
 // ms in 23 steps instead of 104 (1.1 before the FP64 matrix instructions and
-// the chained launches), 3385 rows (100^3 hexes, two phases) 5.6 ->
-// 1.6 ms in 29 instead of 106, 2151 rows (1.5M tets) 2.4 -> 0.9 ms in 22
-// instead of 68, 24 independent meshes of 3930 rows 7.7 -> 0.5 ms in 11
-// instead of 123.
+// the chained launches), 3385 rows (100^3 hexes, two phases) 5.6 -> 1.22 ms
+// in 29 instead of 106, 2151 rows (1.5M tets) 2.4 -> 0.73 ms in 22 instead of
+// 68, 24 independent meshes of 3930 rows 7.7 -> 0.44 ms in 11 instead of 123.
+// The order alone is 0.13, 0.26, 0.16 and 0.12 ms of them.
 //
 // The result depends on nothing but the matrix (ties by row index, sums in
 // a fixed order). Built with contraction: no reference arithmetic here.

@@ -396,11 +396,11 @@ __global__ void k_csr_residual(int n, const int* __restrict__ row, const int* __
 // entries side by side (whole lines of columns and values, 192 entries in
 // flight), leave the products in shared memory and then add them up row by
 // row, in stored order: the same bits. What bounds both is the gather of x,
-// an L1 line per entry (15M of them are 52 of the 96 us of 3M rows); here
+// an L1 line per entry (15M of them are 52 of the 80 us of 3M rows); here
 // neighbouring rows meet in one SM's L1, and what is read once does not push
 // x out of it (evict-first). Against a thread per row, 3 to 7 entries: 200k
 // rows 14.4 us both, 300k 16.4 / 18.5, 600k 22.6 / 28.7, 1M 30.8 / 41.1, 3M
-// 84 / 96; below 2^18 rows a share is too short to pay. (A window of x in
+// 80.4 / 92.7; below 2^18 rows a share is too short to pay. (A window of x in
 // shared memory was slower the larger it was: 92 to 141 us.)
 constexpr int kCsrTileRows = 1 << 18, kCsrCtas = 148, kCsrChunk = 6;
 __global__ void __launch_bounds__(1024, 1) k_csr_residual_tiles(int n, const int* __restrict__ row,

@@ -174,7 +174,7 @@ __device__ __forceinline__ Rows8 rows8(const GraphArgs& g, int i0, int stride, i
 // other SMs have just written the line). Here gather8_issue starts the copies
 // of the first four neighbours of all 8 rows into the warp's 4 KB of shared
 // memory (16 bytes a lane, no registers held), the caller loads what else it
-// needs, and gather8_sum waits once. (24.6k nodes: the forward layer 24.6 ->
+// needs, and gather8_sum waits once. (29.5k nodes: the forward layer 24.6 ->
 // 8.4 us.)
 constexpr int kStage = 8 * 4 * 32;  // floats of a warp's staging
 __device__ __forceinline__ void gather8_issue(const float* X, Rows8 p, float* stage, int lane) {
@@ -635,7 +635,7 @@ constexpr int kBwdSmem = (128 * kTcRows + kTcRows * 32 + 32 * kTcRows + 64 * 32)
 // The incoming gradient is dHout as given (dMout null), or the previous
 // layer's input gradient, formed here row by row (dHout = its dS plus the
 // gather of its dM = dMout) instead of by a pass of its own between the two:
-// the layer with that pass took 22.9 + 6.5 us at 24.6k nodes, now 10.3.
+// the layer with that pass took 22.9 + 6.5 us at 29.5k nodes, now 10.3.
 __global__ void __launch_bounds__(kTcThreads, 2) k_layer_bwd_tc(int n, GraphArgs g, const float* P, const float* Hin,
                                                                 const float* Hout, const float* Min,
                                                                 const float* dHout, const float* dMout, float* dS,
@@ -832,7 +832,7 @@ __global__ void __launch_bounds__(kBlock) k_encode_bwd(int n, GraphArgs g, const
 // have layerBlocks of them, the others kGradBlocks). A block takes 32
 // parameters: its warps bring all their partials to shared memory at once and
 // one warp adds them up. (One thread a parameter with four loads in flight
-// took 9.4 us, now 6.7.)
+// took 9.4 us, now 5.6.)
 __global__ void __launch_bounds__(kBlock) k_grad_reduce(int layerBlocks, const float* gp, float* grad) {
   __shared__ float part[kGradBlocks][32];
   FVM_PDL();
